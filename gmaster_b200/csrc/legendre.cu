@@ -9,8 +9,10 @@
 // turns the two hemispheres into the Sum / Diff right-hand sides of `rhs`.
 //
 // The contraction is carried in T (double for GM_FP64, float for GM_MIXED); the
-// recurrence is always double.  These kernels are the plain-FP64 path and the
-// narrow-batch mixed path; the tensor-core path (legendre_tc.cu) takes wide batches.
+// recurrence is always double.  These kernels are the plain-FP64 path, and the mixed path of
+// a few maps where no checkpoint tables exist (spins other than 0 and 2, Nside above 2048;
+// with tables: legendre_rows.cu); the tensor-core path (legendre_ck.cu, legendre_tc.cu) takes
+// wide batches.
 //
 // Replaces gmaster/_native/cuda/march_v2.cu:155-407 (march_analysis /
 // march_synthesis: float32 difference-form recurrence, SIMT FMA contraction).
@@ -88,64 +90,6 @@ __device__ __forceinline__ Coef make_coef(int l, int m, int s, int l0)
     return c;
 }
 
-// Checkpoint tables of the single-precision rows (legendre_ck.cu): segment k of order m
-// starts at row l0 + 128 k; per (segment, lane) the scaled pre-state (v_{l-1}, D_l) and its
-// shift n (actual = stored * 2^(-64 n)).  Variant q = 0: s' = 0 (spin 0) or -2; q = 1: +2.
-struct CkTab {
-    const int64_t *segoff;
-    const float2 *ck[2];
-    const uint8_t *cn[2];
-    // optional (NULL: every segment generated): per segment, bit g set when a lane of the
-    // 64-lane group g has a non-zero stored state (legendre_ck.cu:gm_ck_masks)
-    const unsigned long long *mask[2];
-};
-constexpr int kCkSeg = 128;
-
-// Whether some lane of this CTA (lanes [j0, j0 + nl)) has a non-zero state at segment seg
-// of either row variant: a CTA whose lanes all start the segment from zero gives exactly
-// zero rows for its 128 rows and skips them (the decision is uniform over the CTA).
-__device__ __forceinline__ bool ck_segment_active(const CkTab &tab, int nvar, int64_t seg, int64_t j0, int64_t nl,
-                                                  int64_t nlanes)
-{
-    if (!tab.mask[0] || nlanes > 4096) return true;
-    const int64_t j1 = (j0 + nl < nlanes ? j0 + nl : nlanes) - 1;
-    const int g0 = (int)(j0 >> 6), g1 = (int)(j1 >> 6);
-    const unsigned long long hi = g1 >= 63 ? ~0ull : ((1ull << (g1 + 1)) - 1ull);
-    const unsigned long long bits = hi & ~((1ull << g0) - 1ull);
-    unsigned long long mk = __ldg(tab.mask[0] + seg);
-    if (nvar > 1 && tab.mask[1]) mk |= __ldg(tab.mask[1] + seg);
-    return (mk & bits) != 0ull;
-}
-
-// Single-precision difference-form coefficients of row l (legendre_ck.cu): (c1, E for
-// s' = -s, E for s' = +s, b); a segment's first row is the restart step (0, 0, 0, 1).
-__device__ __forceinline__ float4 ck_coef(int l, int m, int s, int l0)
-{
-    if ((l - l0) % kCkSeg == 0) return make_float4(0.f, 0.f, 0.f, 1.f);
-    const Coef c = make_coef(l, m, s, l0);
-    const double e = c.alpha - c.beta - 1.0;
-    return make_float4((float)c.alpha, (float)(e + c.c0), (float)(e - c.c0), (float)c.beta);
-}
-
-// One FP32 difference-form step, then the emitted value (scaled lanes: n > 0).
-__device__ __forceinline__ float ck_step(float c1, float E, float b, float y, float &v, float &D, int &n,
-                                         bool scaled)
-{
-    const float C = fmaf(c1, y, E);
-    const float bD = b * D;
-    D = fmaf(C, v, bD);
-    v = v + D;
-    if (!scaled) return v;
-    const float out = v * (n == 0 ? 1.0f : (n == 1 ? 0x1p-64f : 0.0f));
-    // a row grows a value by at most 2^8 (alpha <= sqrt(2m) + 1 at Nside <= 8192)
-    if (n != 0 && fabsf(v) > 0x1p48f) {
-        v *= 0x1p-64f;
-        D *= 0x1p-64f;
-        --n;
-    }
-    return out;
-}
-
 template <typename T, int V>
 __device__ __forceinline__ T warp_reduce_scatter(T (&v)[V], int lane)
 {
@@ -174,14 +118,11 @@ __device__ __forceinline__ int64_t alm_index(int64_t lmax, int64_t l, int64_t m)
 
 // NC components per CTA (spin 0: NC maps; spin 2: NC = 2, one (Q, U) pair).
 // NV values per degree: spin 0: 2 NC; spin 2: 8.  LB degrees per reduce-scatter block.
-//
-// CK: the rows come from the single-precision difference form restarted from the checkpoint
-// tables every 128 rows (mixed precision, spin 0 and 2) instead of the FP64 recurrence.
-template <typename T, int SPIN, int NC, int R, bool CK>
+template <typename T, int SPIN, int NC, int R>
 __global__ void __launch_bounds__(kThreads) k_legendre_ana(
     int64_t nside, int64_t lmax, int64_t ncomp, const double *__restrict__ geom,
     const double *__restrict__ seeds, const T *__restrict__ rhs, double *__restrict__ alm,
-    double scale, int spin, CkTab tab)
+    double scale, int spin)
 {
     constexpr int NV = SPIN == 0 ? 2 * NC : 8;
     constexpr int LB = 32 / NV;
@@ -189,7 +130,6 @@ __global__ void __launch_bounds__(kThreads) k_legendre_ana(
     static_assert(LB * NV == 32, "reduce-scatter width");
     static_assert(LB % 2 == 0 && kWindow % 2 == 0, "row parity is fixed by the row index");
     __shared__ Coef coef[kWindow];
-    __shared__ float4 fcoef[kWindow];
     __shared__ double red[kWarps][kWindow * NV];
 
     const int64_t L = lmax + 1, nlanes = 2 * nside, nelem = L * (L + 1) / 2;
@@ -202,29 +142,24 @@ __global__ void __launch_bounds__(kThreads) k_legendre_ana(
 
     double x[R], v[NVAR][R], vp[NVAR][R];
     int kx[NVAR][R];
-    float fy[R], fv[NVAR][R], fD[NVAR][R];
-    int fn[NVAR][R];
     T rh[R][NC][4];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int64_t j = (int64_t)blockIdx.x * kThreads * R + r * kThreads + threadIdx.x;
         const bool ok = j < nlanes;
         x[r] = ok ? geom[j] : 0.0;
-        fy[r] = ok ? (float)(geom[j] - 1.0) : 0.0f;
         const double ls = ok ? geom[nlanes + j] : 0.0, lc = ok ? geom[2 * nlanes + j] : 0.0;
 #pragma unroll
         for (int q = 0; q < NVAR; ++q) {
             // seed variants: s' = -s (lambda+), then s' = +s (lambda-, times (-1)^s)
             const int var = SPIN == 0 ? 0 : seed_variant(sv) + q;
-            if (!CK && ok) {
+            if (ok) {
                 seed_lane(seeds + ((int64_t)var * L + m) * 4, ls, lc, v[q][r], kx[q][r]);
             } else {
                 v[q][r] = 0.0;
                 kx[q][r] = 0;
             }
             vp[q][r] = 0.0;
-            fv[q][r] = fD[q][r] = 0.0f;
-            fn[q][r] = 0;
         }
 #pragma unroll
         for (int c = 0; c < NC; ++c)
@@ -254,45 +189,9 @@ __global__ void __launch_bounds__(kThreads) k_legendre_ana(
             }
     }
     for (int lb = l0; lb < L; lb += kWindow) {
-        if (CK && (lb - l0) % kCkSeg == 0 &&
-            !ck_segment_active(tab, NVAR, tab.segoff[m] + (lb - l0) / kCkSeg,
-                               (int64_t)blockIdx.x * kThreads * R, (int64_t)kThreads * R, nlanes)) {
-            lb += kCkSeg - kWindow;   // the segment's rows are zero on all lanes of this CTA
-            continue;
-        }
         if (threadIdx.x < kWindow) {
             const int l = lb + threadIdx.x;
-            if (CK) fcoef[threadIdx.x] = ck_coef(l, m, sv, l0);
-            else coef[threadIdx.x] = make_coef(l, m, sv, l0);
-        }
-        bool scaled = false;
-        if (CK) {
-            if ((lb - l0) % kCkSeg == 0) {
-                // a new segment: the lane states restart from the checkpoint table
-                const int64_t seg = tab.segoff[m] + (lb - l0) / kCkSeg;
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const int64_t j = (int64_t)blockIdx.x * kThreads * R + r * kThreads + threadIdx.x;
-#pragma unroll
-                    for (int q = 0; q < NVAR; ++q) {
-                        float2 st = make_float2(0.f, 0.f);
-                        int n = 0;
-                        if (j < nlanes) {
-                            st = __ldg(tab.ck[q] + seg * nlanes + j);
-                            n = __ldg(tab.cn[q] + seg * nlanes + j);
-                        }
-                        fv[q][r] = st.x;
-                        fD[q][r] = st.y;
-                        fn[q][r] = n;
-                    }
-                }
-            }
-            int any = 0;
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-#pragma unroll
-                for (int q = 0; q < NVAR; ++q) any |= fn[q][r];
-            scaled = __any_sync(0xffffffffu, any != 0);
+            coef[threadIdx.x] = make_coef(l, m, sv, l0);
         }
         __syncthreads();
 #pragma unroll 1
@@ -304,16 +203,7 @@ __global__ void __launch_bounds__(kThreads) k_legendre_ana(
             for (int s = 0; s < LB; ++s) {
                 const int l = lb + i + s;
                 if (l < L) {
-                    float fval[NVAR][R];
-                    if (CK) {
-                        const float4 cq = fcoef[i + s];
-#pragma unroll
-                        for (int r = 0; r < R; ++r)
-#pragma unroll
-                            for (int q = 0; q < NVAR; ++q)
-                                fval[q][r] = ck_step(cq.x, q == 0 ? cq.y : cq.z, cq.w, fy[r], fv[q][r],
-                                                     fD[q][r], fn[q][r], scaled);
-                    } else if (l > l0) {
+                    if (l > l0) {
                         const Coef cf = coef[i + s];
 #pragma unroll
                         for (int r = 0; r < R; ++r) {
@@ -340,7 +230,7 @@ __global__ void __launch_bounds__(kThreads) k_legendre_ana(
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
                         if (SPIN == 0) {
-                            const T val = CK ? (T)fval[0][r] : (kx[0][r] == 0 ? (T)v[0][r] : (T)0);
+                            const T val = kx[0][r] == 0 ? (T)v[0][r] : (T)0;
 #pragma unroll
                             for (int c = 0; c < NC; ++c) {
                                 const T hr = par ? rh[r][c][2] : rh[r][c][0];
@@ -349,16 +239,9 @@ __global__ void __launch_bounds__(kThreads) k_legendre_ana(
                                 acc[s * NV + 2 * c + 1] += val * hi;
                             }
                         } else {
-                            T f1, f2;
-                            if (CK) {
-                                f1 = (T)(0.5f * (fval[0][r] + fval[NVAR - 1][r]));
-                                f2 = (T)(0.5f * (fval[0][r] - fval[NVAR - 1][r]));
-                            } else {
-                                const double lp = kx[0][r] == 0 ? v[0][r] : 0.0;
-                                const double lm = kx[NVAR - 1][r] == 0 ? v[NVAR - 1][r] : 0.0;
-                                f1 = (T)(0.5 * (lp + lm));
-                                f2 = (T)(0.5 * (lp - lm));
-                            }
+                            const double lp = kx[0][r] == 0 ? v[0][r] : 0.0;
+                            const double lm = kx[NVAR - 1][r] == 0 ? v[NVAR - 1][r] : 0.0;
+                            const T f1 = (T)(0.5 * (lp + lm)), f2 = (T)(0.5 * (lp - lm));
                             // same-parity side P = Sum (even) / Diff (odd); other side D
                             const T qpr = par ? rh[r][0][2] : rh[r][0][0];
                             const T qpi = par ? rh[r][0][3] : rh[r][0][1];
@@ -422,17 +305,16 @@ __global__ void __launch_bounds__(kThreads) k_legendre_ana(
 
 // ---------------------------------------------------------------- synthesis
 
-template <typename T, int SPIN, int NC, int R, bool CK>
+template <typename T, int SPIN, int NC, int R>
 __global__ void __launch_bounds__(kThreads) k_legendre_syn(
     int64_t nside, int64_t lmax, int64_t ncomp, const double *__restrict__ geom,
     const double *__restrict__ seeds, const double *__restrict__ alm, T *__restrict__ syn,
-    int spin, CkTab tab)
+    int spin)
 {
     constexpr int NVAR = SPIN == 0 ? 1 : 2;
     constexpr int NA = SPIN == 0 ? NC : 2;  // complex alm rows per degree (maps, or E and B)
     constexpr int NACC = SPIN == 0 ? 4 * NC : 16;
     __shared__ Coef coef[2][kWindow];
-    __shared__ float4 fcoef[2][kWindow];
     __shared__ T aw[2][kWindow][NA][2];
 
     const int64_t L = lmax + 1, nlanes = 2 * nside, nelem = L * (L + 1) / 2;
@@ -443,28 +325,23 @@ __global__ void __launch_bounds__(kThreads) k_legendre_syn(
 
     double x[R], v[NVAR][R], vp[NVAR][R];
     int kx[NVAR][R];
-    float fy[R], fv[NVAR][R], fD[NVAR][R];
-    int fn[NVAR][R];
     T acc[R][NACC];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int64_t j = (int64_t)blockIdx.x * kThreads * R + r * kThreads + threadIdx.x;
         const bool ok = j < nlanes && l0 <= lmax;
         x[r] = ok ? geom[j] : 0.0;
-        fy[r] = ok ? (float)(geom[j] - 1.0) : 0.0f;
         const double ls = ok ? geom[nlanes + j] : 0.0, lc = ok ? geom[2 * nlanes + j] : 0.0;
 #pragma unroll
         for (int q = 0; q < NVAR; ++q) {
             const int var = SPIN == 0 ? 0 : seed_variant(sv) + q;
-            if (!CK && ok) {
+            if (ok) {
                 seed_lane(seeds + ((int64_t)var * L + m) * 4, ls, lc, v[q][r], kx[q][r]);
             } else {
                 v[q][r] = 0.0;
                 kx[q][r] = 0;
             }
             vp[q][r] = 0.0;
-            fv[q][r] = fD[q][r] = 0.0f;
-            fn[q][r] = 0;
         }
 #pragma unroll
         for (int q = 0; q < NACC; ++q) acc[r][q] = (T)0;
@@ -472,48 +349,9 @@ __global__ void __launch_bounds__(kThreads) k_legendre_syn(
 
     int buf = 0;
     for (int lb = l0; lb < L; lb += kWindow, buf ^= 1) {
-        if (CK && (lb - l0) % kCkSeg == 0 &&
-            !ck_segment_active(tab, NVAR, tab.segoff[m] + (lb - l0) / kCkSeg,
-                               (int64_t)blockIdx.x * kThreads * R, (int64_t)kThreads * R, nlanes)) {
-            // the segment's rows are zero on all lanes of this CTA; the next window that runs
-            // takes the other buffer, as it would have after this one
-            lb += kCkSeg - kWindow;
-            buf ^= 1;
-            continue;
-        }
-        bool scaled = false;
-        if (CK) {
-            if ((lb - l0) % kCkSeg == 0) {
-                // a new segment: the lane states restart from the checkpoint table
-                const int64_t seg = tab.segoff[m] + (lb - l0) / kCkSeg;
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const int64_t j = (int64_t)blockIdx.x * kThreads * R + r * kThreads + threadIdx.x;
-#pragma unroll
-                    for (int q = 0; q < NVAR; ++q) {
-                        float2 st = make_float2(0.f, 0.f);
-                        int n = 0;
-                        if (j < nlanes) {
-                            st = __ldg(tab.ck[q] + seg * nlanes + j);
-                            n = __ldg(tab.cn[q] + seg * nlanes + j);
-                        }
-                        fv[q][r] = st.x;
-                        fD[q][r] = st.y;
-                        fn[q][r] = n;
-                    }
-                }
-            }
-            int any = 0;
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-#pragma unroll
-                for (int q = 0; q < NVAR; ++q) any |= fn[q][r];
-            scaled = __any_sync(0xffffffffu, any != 0);
-        }
         if (threadIdx.x < kWindow) {
             const int l = lb + threadIdx.x;
-            if (CK) fcoef[buf][threadIdx.x] = ck_coef(l, m, sv, l0);
-            else coef[buf][threadIdx.x] = make_coef(l, m, sv, l0);
+            coef[buf][threadIdx.x] = make_coef(l, m, sv, l0);
 #pragma unroll
             for (int a = 0; a < NA; ++a) {
                 T re = 0, im = 0;
@@ -542,16 +380,7 @@ __global__ void __launch_bounds__(kThreads) k_legendre_syn(
                 const int s = s0 + hh;
                 if (s >= lend) break;
                 const int l = lb + s;
-                float fval[NVAR][R];
-                if (CK) {
-                    const float4 cq = fcoef[buf][s];
-#pragma unroll
-                    for (int r = 0; r < R; ++r)
-#pragma unroll
-                        for (int q = 0; q < NVAR; ++q)
-                            fval[q][r] = ck_step(cq.x, q == 0 ? cq.y : cq.z, cq.w, fy[r], fv[q][r], fD[q][r],
-                                                 fn[q][r], scaled);
-                } else if (l > l0) {
+                if (l > l0) {
                     const Coef cf = coef[buf][s];
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
@@ -575,23 +404,16 @@ __global__ void __launch_bounds__(kThreads) k_legendre_syn(
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     if (SPIN == 0) {
-                        const T val = CK ? (T)fval[0][r] : (kx[0][r] == 0 ? (T)v[0][r] : (T)0);
+                        const T val = kx[0][r] == 0 ? (T)v[0][r] : (T)0;
 #pragma unroll
                         for (int c = 0; c < NC; ++c) {
                             acc[r][4 * c + 2 * hh] += val * aw[buf][s][c][0];
                             acc[r][4 * c + 2 * hh + 1] += val * aw[buf][s][c][1];
                         }
                     } else {
-                        T f1, f2;
-                        if (CK) {
-                            f1 = (T)(0.5f * (fval[0][r] + fval[NVAR - 1][r]));
-                            f2 = (T)(0.5f * (fval[0][r] - fval[NVAR - 1][r]));
-                        } else {
-                            const double lp = kx[0][r] == 0 ? v[0][r] : 0.0;
-                            const double lm = kx[NVAR - 1][r] == 0 ? v[NVAR - 1][r] : 0.0;
-                            f1 = (T)(0.5 * (lp + lm));
-                            f2 = (T)(0.5 * (lp - lm));
-                        }
+                        const double lp = kx[0][r] == 0 ? v[0][r] : 0.0;
+                        const double lm = kx[NVAR - 1][r] == 0 ? v[NVAR - 1][r] : 0.0;
+                        const T f1 = (T)(0.5 * (lp + lm)), f2 = (T)(0.5 * (lp - lm));
                         const T er = aw[buf][s][0][0], ei = aw[buf][s][0][1];
                         const T br = aw[buf][s][1][0], bi = aw[buf][s][1][1];
                         // per parity: [S1E re, im, S1B re, im, S2E re, im, S2B re, im]
@@ -682,63 +504,53 @@ extern "C" int64_t gm_seed_table_len(int64_t L) { return (2 * kMaxSpin + 1) * 4 
 template <typename T, int SPIN, int NC, int R>
 static int launch_ana(int spin, int64_t nside, int64_t lmax, int64_t ncomp, const double *geom,
                       const double *seeds, const void *rhs, double *alm, double scale,
-                      cudaStream_t s, const CkTab *tab = nullptr)
+                      cudaStream_t s)
 {
     const int64_t nlanes = 2 * nside;
     dim3 grid((unsigned)((nlanes + kThreads * R - 1) / (kThreads * R)), (unsigned)(lmax + 1),
               (unsigned)((ncomp + NC - 1) / NC));
-    if (tab)
-        k_legendre_ana<float, SPIN, NC, R, true><<<grid, kThreads, 0, s>>>(
-            nside, lmax, ncomp, geom, seeds, (const float *)rhs, alm, scale, spin, *tab);
-    else
-        k_legendre_ana<T, SPIN, NC, R, false><<<grid, kThreads, 0, s>>>(
-            nside, lmax, ncomp, geom, seeds, (const T *)rhs, alm, scale, spin, CkTab{});
+    k_legendre_ana<T, SPIN, NC, R><<<grid, kThreads, 0, s>>>(nside, lmax, ncomp, geom, seeds, (const T *)rhs,
+                                                             alm, scale, spin);
     return check_launch("gm_legendre_analysis");
 }
 
 template <typename T, int SPIN, int NC, int R>
 static int launch_syn(int spin, int64_t nside, int64_t lmax, int64_t ncomp, const double *geom,
-                      const double *seeds, const double *alm, void *syn, cudaStream_t s,
-                      const CkTab *tab = nullptr)
+                      const double *seeds, const double *alm, void *syn, cudaStream_t s)
 {
     const int64_t nlanes = 2 * nside;
     dim3 grid((unsigned)((nlanes + kThreads * R - 1) / (kThreads * R)), (unsigned)(lmax + 1),
               (unsigned)((ncomp + NC - 1) / NC));
-    if (tab)
-        k_legendre_syn<float, SPIN, NC, R, true><<<grid, kThreads, 0, s>>>(
-            nside, lmax, ncomp, geom, seeds, alm, (float *)syn, spin, *tab);
-    else
-        k_legendre_syn<T, SPIN, NC, R, false><<<grid, kThreads, 0, s>>>(
-            nside, lmax, ncomp, geom, seeds, alm, (T *)syn, spin, CkTab{});
+    k_legendre_syn<T, SPIN, NC, R><<<grid, kThreads, 0, s>>>(nside, lmax, ncomp, geom, seeds, alm, (T *)syn,
+                                                             spin);
     return check_launch("gm_legendre_synthesis");
 }
 
 template <typename T>
 static int dispatch_ana(int spin, int64_t nside, int64_t lmax, int64_t ncomp, const double *geom,
                         const double *seeds, const void *rhs, double *alm, double scale,
-                        cudaStream_t s, const CkTab *tab = nullptr)
+                        cudaStream_t s)
 {
     if (spin == 0) {
         if (ncomp == 1)
-            return launch_ana<T, 0, 1, 4>(spin, nside, lmax, ncomp, geom, seeds, rhs, alm, scale, s, tab);
+            return launch_ana<T, 0, 1, 4>(spin, nside, lmax, ncomp, geom, seeds, rhs, alm, scale, s);
         if (ncomp == 2)
-            return launch_ana<T, 0, 2, 4>(spin, nside, lmax, ncomp, geom, seeds, rhs, alm, scale, s, tab);
-        return launch_ana<T, 0, 4, 2>(spin, nside, lmax, ncomp, geom, seeds, rhs, alm, scale, s, tab);
+            return launch_ana<T, 0, 2, 4>(spin, nside, lmax, ncomp, geom, seeds, rhs, alm, scale, s);
+        return launch_ana<T, 0, 4, 2>(spin, nside, lmax, ncomp, geom, seeds, rhs, alm, scale, s);
     }
-    return launch_ana<T, 2, 2, 2>(spin, nside, lmax, ncomp, geom, seeds, rhs, alm, scale, s, tab);
+    return launch_ana<T, 2, 2, 2>(spin, nside, lmax, ncomp, geom, seeds, rhs, alm, scale, s);
 }
 
 template <typename T>
 static int dispatch_syn(int spin, int64_t nside, int64_t lmax, int64_t ncomp, const double *geom,
-                        const double *seeds, const double *alm, void *syn, cudaStream_t s,
-                        const CkTab *tab = nullptr)
+                        const double *seeds, const double *alm, void *syn, cudaStream_t s)
 {
     if (spin == 0) {
-        if (ncomp == 1) return launch_syn<T, 0, 1, 2>(spin, nside, lmax, ncomp, geom, seeds, alm, syn, s, tab);
-        if (ncomp == 2) return launch_syn<T, 0, 2, 2>(spin, nside, lmax, ncomp, geom, seeds, alm, syn, s, tab);
-        return launch_syn<T, 0, 4, 1>(spin, nside, lmax, ncomp, geom, seeds, alm, syn, s, tab);
+        if (ncomp == 1) return launch_syn<T, 0, 1, 2>(spin, nside, lmax, ncomp, geom, seeds, alm, syn, s);
+        if (ncomp == 2) return launch_syn<T, 0, 2, 2>(spin, nside, lmax, ncomp, geom, seeds, alm, syn, s);
+        return launch_syn<T, 0, 4, 1>(spin, nside, lmax, ncomp, geom, seeds, alm, syn, s);
     }
-    return launch_syn<T, 2, 2, 2>(spin, nside, lmax, ncomp, geom, seeds, alm, syn, s, tab);
+    return launch_syn<T, 2, 2, 2>(spin, nside, lmax, ncomp, geom, seeds, alm, syn, s);
 }
 
 // Tile shapes the autotuner chooses from: (NC, R) = (components per CTA, lanes per thread).
@@ -746,7 +558,8 @@ static int dispatch_syn(int spin, int64_t nside, int64_t lmax, int64_t ncomp, co
 // handles one (Q, U) pair per CTA (NC = 2).  Index -1 selects the built-in heuristic.
 // The last tile of each list (8 lanes per thread: a reduce-scatter tree per 8 rows shared by
 // 64 elements of a thread instead of 32) is compiled for single precision only; the FP64
-// kernels run it as the tile with 4 lanes per thread.
+// kernels run it as the tile with 4 lanes per thread.  The checkpointed single-precision
+// passes (legendre_rows.cu) read R as the pairs of lanes (spin 0) or lanes (spin 2) of a thread.
 static const int kTiles0[][2] = {{1, 1}, {1, 2}, {1, 4}, {2, 1}, {2, 2}, {2, 4}, {4, 1}, {4, 2}, {8, 1}, {2, 8}};
 static const int kTiles2[][2] = {{2, 1}, {2, 2}, {2, 4}, {2, 8}};
 constexpr int kNTiles0 = sizeof(kTiles0) / sizeof(kTiles0[0]);
@@ -755,9 +568,9 @@ constexpr int kNTiles2 = sizeof(kTiles2) / sizeof(kTiles2[0]);
 template <typename T>
 static int tile_ana(int spin, int tile, int64_t nside, int64_t lmax, int64_t ncomp,
                     const double *geom, const double *seeds, const void *rhs, double *alm,
-                    double scale, cudaStream_t s, const CkTab *tab = nullptr)
+                    double scale, cudaStream_t s)
 {
-#define GM_ANA(SP, NC, R) return launch_ana<T, SP, NC, R>(spin, nside, lmax, ncomp, geom, seeds, rhs, alm, scale, s, tab)
+#define GM_ANA(SP, NC, R) return launch_ana<T, SP, NC, R>(spin, nside, lmax, ncomp, geom, seeds, rhs, alm, scale, s)
     if (spin == 0) {
         switch (tile) {
         case 0: GM_ANA(0, 1, 1);
@@ -788,9 +601,9 @@ static int tile_ana(int spin, int tile, int64_t nside, int64_t lmax, int64_t nco
 template <typename T>
 static int tile_syn(int spin, int tile, int64_t nside, int64_t lmax, int64_t ncomp,
                     const double *geom, const double *seeds, const double *alm, void *syn,
-                    cudaStream_t s, const CkTab *tab = nullptr)
+                    cudaStream_t s)
 {
-#define GM_SYN(SP, NC, R) return launch_syn<T, SP, NC, R>(spin, nside, lmax, ncomp, geom, seeds, alm, syn, s, tab)
+#define GM_SYN(SP, NC, R) return launch_syn<T, SP, NC, R>(spin, nside, lmax, ncomp, geom, seeds, alm, syn, s)
     if (spin == 0) {
         switch (tile) {
         case 0: GM_SYN(0, 1, 1);
@@ -902,62 +715,4 @@ extern "C" int gm_legendre_synthesis(int precision, int spin, int64_t nside, int
     if (precision == GM_MIXED)
         return dispatch_syn<float>(spin, nside, lmax, ncomp, lane_geom, seeds, alm, syn, s);
     return GM_ERR_UNSUPPORTED;
-}
-
-// Mixed-precision spin-0 / spin-2 transforms with the checkpointed single-precision rows.
-static int ck_args_ok(int spin, int64_t nside, int64_t lmax, int64_t ncomp, int tile)
-{
-    if (nside < 1 || lmax < 2 || lmax + 1 > 65535 || ncomp < 1 || ncomp > 65535) return GM_ERR_BAD_SHAPE;
-    if (spin != 0 && spin != 2) return GM_ERR_UNSUPPORTED;
-    if (spin == 2 && (ncomp % 2)) return GM_ERR_BAD_SHAPE;
-    if (tile < -1 || tile >= (spin == 0 ? kNTiles0 : kNTiles2)) return GM_ERR_BAD_SHAPE;
-    return GM_OK;
-}
-
-static CkTab ck_tab(const int64_t *segoff, const void *ck_a, const uint8_t *cn_a, const void *ck_b,
-                    const uint8_t *cn_b, const uint64_t *mask_a, const uint64_t *mask_b)
-{
-    CkTab t;
-    t.segoff = segoff;
-    t.ck[0] = (const float2 *)ck_a;
-    t.cn[0] = cn_a;
-    t.ck[1] = (const float2 *)ck_b;
-    t.cn[1] = cn_b;
-    // both variants' masks or neither
-    const bool masked = mask_a && (mask_b || ck_b == nullptr);
-    t.mask[0] = masked ? (const unsigned long long *)mask_a : nullptr;
-    t.mask[1] = masked ? (const unsigned long long *)mask_b : nullptr;
-    return t;
-}
-
-extern "C" int gm_legendre_analysis_ck(int spin, int64_t nside, int64_t lmax, int64_t ncomp,
-                                       const double *lane_geom, const void *rhs, double *alm,
-                                       double scale, const int64_t *segoff, const void *ck_a,
-                                       const uint8_t *cn_a, const void *ck_b, const uint8_t *cn_b,
-                                       const uint64_t *mask_a, const uint64_t *mask_b, int tile, void *stream)
-{
-    const int st = ck_args_ok(spin, nside, lmax, ncomp, tile);
-    if (st != GM_OK) return st;
-    if (!lane_geom || !rhs || !alm || !segoff || !ck_a || !cn_a || (spin == 2 && (!ck_b || !cn_b)))
-        return GM_ERR_BAD_PTR;
-    const CkTab tab = ck_tab(segoff, ck_a, cn_a, spin == 2 ? ck_b : nullptr, cn_b, mask_a, spin == 2 ? mask_b : nullptr);
-    cudaStream_t s = as_stream(stream);
-    return tile < 0 ? dispatch_ana<float>(spin, nside, lmax, ncomp, lane_geom, nullptr, rhs, alm, scale, s, &tab)
-                    : tile_ana<float>(spin, tile, nside, lmax, ncomp, lane_geom, nullptr, rhs, alm, scale, s, &tab);
-}
-
-extern "C" int gm_legendre_synthesis_ck(int spin, int64_t nside, int64_t lmax, int64_t ncomp,
-                                        const double *lane_geom, const double *alm, void *syn,
-                                        const int64_t *segoff, const void *ck_a, const uint8_t *cn_a,
-                                        const void *ck_b, const uint8_t *cn_b, const uint64_t *mask_a,
-                                        const uint64_t *mask_b, int tile, void *stream)
-{
-    const int st = ck_args_ok(spin, nside, lmax, ncomp, tile);
-    if (st != GM_OK) return st;
-    if (!lane_geom || !alm || !syn || !segoff || !ck_a || !cn_a || (spin == 2 && (!ck_b || !cn_b)))
-        return GM_ERR_BAD_PTR;
-    const CkTab tab = ck_tab(segoff, ck_a, cn_a, spin == 2 ? ck_b : nullptr, cn_b, mask_a, spin == 2 ? mask_b : nullptr);
-    cudaStream_t s = as_stream(stream);
-    return tile < 0 ? dispatch_syn<float>(spin, nside, lmax, ncomp, lane_geom, nullptr, alm, syn, s, &tab)
-                    : tile_syn<float>(spin, tile, nside, lmax, ncomp, lane_geom, nullptr, alm, syn, s, &tab);
 }
