@@ -333,8 +333,12 @@ __device__ __forceinline__ void ana8(Rows<SPIN, R> &w, const u64 (&rh)[R][4 * NC
     if (SCALED) w.renormalise();
 }
 
+// Resident CTAs asked for: four of one spin-0 map at R = 4 (128 registers; 139 and three CTAs
+// measured 18.0 instead of 16.9 ms at Nside 2048).
+__host__ __device__ constexpr int ana_ctas(int spin, int nc, int r) { return spin == 0 && nc == 1 && r == 4 ? 4 : 1; }
+
 template <int SPIN, int NC, int R>
-__global__ void __launch_bounds__(32 * max_warps(SPIN, R)) k_rows_ana(int64_t nside, int64_t lmax, int64_t ncomp,
+__global__ void __launch_bounds__(32 * max_warps(SPIN, R), ana_ctas(SPIN, NC, R)) k_rows_ana(int64_t nside, int64_t lmax, int64_t ncomp,
                                                           const double *__restrict__ geom,
                                                           const float *__restrict__ rhs,
                                                           double *__restrict__ alm, double scale, Tab tab)
