@@ -99,14 +99,28 @@ __device__ __forceinline__ T2 phase_pi(const T2 *__restrict__ tw, int h, int q2,
 
 // ---------------------------------------------------------------- FFT core
 
+// Radices of h into rad (4s, a 2, then odd primes ascending), written by one warp of 32
+// threads that test 32 odd divisors at a time; returns their number.
 __device__ int factorize(int h, int *rad)
 {
+    const int lane = threadIdx.x & 31;
     int n = 0;
-    while (h % 4 == 0) { rad[n++] = 4; h /= 4; }
-    if (h % 2 == 0) { rad[n++] = 2; h /= 2; }
-    for (int p = 3; p * p <= h; p += 2)
-        while (h % p == 0) { rad[n++] = p; h /= p; }
-    if (h > 1) rad[n++] = h;
+    auto put = [&](int p) {
+        if (lane == 0) rad[n] = p;
+        ++n;
+    };
+    while (h % 4 == 0) { put(4); h /= 4; }
+    if (h % 2 == 0) { put(2); h /= 2; }
+    for (int base = 3; base * base <= h; base += 64) {
+        const int d = base + 2 * lane;
+        unsigned hit = __ballot_sync(0xffffffffu, d <= h && h % d == 0);
+        while (hit) {   // ascending: a composite divisor no longer divides
+            const int p = base + 2 * (__ffs(hit) - 1);
+            hit &= hit - 1;
+            while (p * p <= h && h % p == 0) { put(p); h /= p; }
+        }
+    }
+    if (h > 1) put(h);
     return n;
 }
 
@@ -191,7 +205,10 @@ __device__ T2 *fft_shared(T2 *a, T2 *b, int h, const T2 *__restrict__ tw, int si
 {
     __shared__ int rad[40];
     __shared__ int nst;
-    if (threadIdx.x == 0) nst = factorize(h, rad);
+    if (threadIdx.x < 32) {
+        const int k = factorize(h, rad);
+        if (threadIdx.x == 0) nst = k;
+    }
     __syncthreads();
     int Ls = 1;
     for (int s = 0; s < nst; ++s) {
@@ -257,6 +274,61 @@ __host__ __device__ __forceinline__ bool bluestein_big(int h, int nside, int bsm
 __host__ __device__ __forceinline__ bool ring_big(int h, int hcap, int nside, int bsmin)
 {
     return h > hcap || bluestein_big(h, nside, bsmin);
+}
+
+// ---- Bluestein's method: the DFT of length h as a circular convolution of length M
+
+template <typename T2>
+__device__ __forceinline__ T2 bs_chirp(const T2 *__restrict__ tw, int h, int n, int j, int sign)
+{
+    const unsigned q = ((unsigned)j * (unsigned)j) % (unsigned)n;
+    return twiddle_n(tw, h, (int)q, sign);   // e^{sign i pi j^2 / h}
+}
+
+// Bluestein filter: the transform of the wrapped conjugate chirp of length M; returns the
+// buffer holding it (b0 or b1).
+template <typename T2>
+__device__ T2 *bs_filter(int h, int n, int M, const T2 *__restrict__ tw, const T2 *__restrict__ twM, int sign,
+                         T2 *b0, T2 *b1)
+{
+    for (int m = threadIdx.x; m < M; m += blockDim.x) {
+        T2 v{};
+        int j = -1;
+        if (m < h) j = m;
+        else if (m > M - h) j = M - m;
+        if (j >= 0) {
+            v = bs_chirp(tw, h, n, j, sign);
+            v.y = -v.y;
+        }
+        b0[m] = v;
+    }
+    __syncthreads();
+    return fft_shared<1>(b0, b1, M, twM, -1);
+}
+
+// X[0, h) holds z_j c_j; zero-pads to M, convolves with the filter FB and returns the buffer
+// holding the DFT sum_j z_j e^{sign 2 pi i jk / h}, k < h.
+template <typename T2>
+__device__ T2 *bs_apply(T2 *X, T2 *Y, const T2 *FB, int h, int n, int M, const T2 *__restrict__ tw,
+                        const T2 *__restrict__ twM, int sign)
+{
+    for (int j = h + threadIdx.x; j < M; j += blockDim.x) X[j] = T2{};
+    __syncthreads();
+    T2 *FA = fft_shared<1>(X, Y, M, twM, -1);
+    T2 *G = (FA == X) ? Y : X;
+    const auto invM = (decltype(X->x))1 / (decltype(X->x))M;
+    for (int m = threadIdx.x; m < M; m += blockDim.x) {
+        T2 v = cmul(FA[m], FB[m]);
+        v.x *= invM;
+        v.y *= invM;
+        FA[m] = v;
+    }
+    __syncthreads();
+    T2 *R = fft_shared<1>(FA, G, M, twM, +1);
+    T2 *Z = (R == FA) ? G : FA;
+    for (int k = threadIdx.x; k < h; k += blockDim.x) Z[k] = cmul(R[k], bs_chirp(tw, h, n, k, sign));
+    __syncthreads();
+    return Z;
 }
 
 // Load one ring of one map (times the mask) as h complex z_t = x_2t + i x_2t+1, each
@@ -506,33 +578,128 @@ __device__ __forceinline__ void residue_sums(const T *__restrict__ syn, int64_t 
     ps[1] = si;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) k_fold_residual(int64_t nside, int64_t L, int64_t ncomp,
-                                                       const T *__restrict__ syn,
-                                                       const T *__restrict__ rhs_map,
-                                                       const uint8_t *__restrict__ shifted,
-                                                       T *__restrict__ rhs_out)
+// Both hemispheres' coefficients of one order: (north re, im, south re, im).
+template <typename T> struct alignas(16) Quad {
+    T x, y, z, w;
+};
+
+// Ring fold of J consecutive (lane, component) columns of syn (L, nlanes, ncomp, 4): for every
+// residue k of the ring length n,
+//   P_k = sum_t sigma^t c(k + t n) + sum_{t >= 1} sigma^t conj c(t n - k),  sigma = -1 if shifted,
+// from A_k = sum_{t >= 0} sigma^t c(k + t n) as P_k = A_k + sigma conj A_{n-k}: residues k and
+// n - k are summed together, so every coefficient is read once.  A CTA's threads run along
+// the J columns first (J x 16 or 32 contiguous bytes a row), then over the residue pairs; on
+// short rings (pairs fewer than half the slots) several slots share a pair, each summing every
+// s-th alias, and their sums are added in a fixed order.
+//   RESIDUAL: out(m) = sigma^t w n P_k - rhs_map(m) for m = k + t n, as Sum / Diff halves;
+//   otherwise spec[comp][ring][k] = P_k, k <= n / 2, of the north and the south ring.
+// Bound by memory: reads syn (and rhs_map) once, writes once.  One thread block per lane with
+// the threads along m read 16 bytes per 32-byte sector 128 lanes apart and summed the aliases
+// of the polar rings (n = 4, 8, ...) in a few threads: 2.2 -> 0.45 ms a pass at Nside 2048 with
+// one map (1.2 GB: 2.7 TB/s), 370 -> 78 us at Nside 512 with a (Q, U) pair.
+__host__ __device__ constexpr int fold_threads(int J) { return J == 8 ? 512 : 256; }
+
+template <typename T, int J, bool RESIDUAL>
+__global__ void __launch_bounds__(fold_threads(J)) k_fold_lanes(int64_t nside, int64_t L, int64_t ncomp, int64_t cbeg, int64_t cw,
+                                                    const Quad<T> *__restrict__ syn,
+                                                    const Quad<T> *__restrict__ rhs_map,
+                                                    const uint8_t *__restrict__ shifted, Quad<T> *__restrict__ out,
+                                                    typename vec2<T>::type *__restrict__ spec, int64_t sstride)
 {
-    const int64_t j = blockIdx.x, c = blockIdx.y;
-    const int64_t nlanes = 2 * nside, npix = 12 * nside * nside;
-    const int n = (int)ring_nphi(nside, north_ring(j));
-    const bool sh = shifted[north_ring(j)] != 0;
-    const bool two = j != nlanes - 1;
-    const T wn = (T)(4.0 * M_PI / (double)npix * (double)n);
-    for (int k = threadIdx.x; k < n && k < L; k += blockDim.x) {
-        T pn[2], ps[2];
-        residue_sums(syn, L, nlanes, ncomp, j, c, k, n, sh, two, pn, ps);
-        int t = 0;
-        for (int64_t m = k; m < L; m += n, ++t) {
-            T sg = (sh && (t & 1)) ? -wn : wn;
-            T gnr = sg * pn[0], gni = sg * pn[1], gsr = sg * ps[0], gsi = sg * ps[1];
-            const int64_t idx = ((m * nlanes + j) * ncomp + c) * 4;
-            T *o = rhs_out + idx;
-            const T *b = rhs_map + idx;
-            o[0] = gnr + gsr - b[0];
-            o[1] = gni + gsi - b[1];
-            o[2] = gnr - gsr - b[2];
-            o[3] = gni - gsi - b[3];
+    using T2 = typename vec2<T>::type;
+    constexpr int NT = fold_threads(J), Q = NT / J;
+    __shared__ Quad<T> pa[NT], pb[NT];
+    const int64_t nlanes = 2 * nside, stride = nlanes * ncomp;
+    const int q = threadIdx.x / J;
+    const int64_t item = (int64_t)blockIdx.x * J + threadIdx.x % J;
+    const bool ok = item < nlanes * cw;
+    const int64_t j = ok ? item / cw : 0, c = cbeg + (ok ? item % cw : 0);
+    const int64_t col = j * ncomp + c;
+    const int n = (int)ring_nphi(nside, north_ring(j)), np = n / 2 + 1;
+    const bool sh = shifted[north_ring(j)] != 0, two = j != nlanes - 1;
+    const T sigma = sh ? (T)-1 : (T)1;
+    const T wn = (T)(4.0 * M_PI / (double)(12 * nside * nside) * (double)n);
+    const Quad<T> *src = syn + col;
+    int s = 1;
+    while (2 * s * np <= Q) s *= 2;
+    const int part = q & (s - 1);
+
+    // aliases k + t n, t = t0, t0 + s, ...
+    auto sum = [&](int k, int t0) {
+        Quad<T> a{0, 0, 0, 0};
+        const int64_t dm = (int64_t)s * n;
+        int t = t0;
+#pragma unroll 4
+        for (int64_t m = k + (int64_t)t0 * n; m < L; m += dm, t += s) {
+            const Quad<T> v = src[m * stride];
+            const T sg = (sh && (t & 1)) ? (T)-1 : (T)1;
+            a.x += sg * v.x;
+            a.y += sg * v.y;
+            a.z += sg * v.z;
+            a.w += sg * v.w;
+        }
+        return a;
+    };
+    auto pair_sums = [&](int p, Quad<T> &A, Quad<T> &B) {
+        // residue 0 leaves order 0 to the caller
+        A = sum(p, p == 0 && part == 0 ? s : part);
+        B = (p > 0 && 2 * p < n) ? sum(n - p, part) : Quad<T>{0, 0, 0, 0};
+    };
+    auto emit = [&](int k, const Quad<T> &P) {
+        if (RESIDUAL) {
+            const int64_t dm = (int64_t)s * n;
+            int t = part;
+#pragma unroll 4
+            for (int64_t m = k + (int64_t)part * n; m < L; m += dm, t += s) {
+                const T f = (sh && (t & 1)) ? -wn : wn;
+                const T nr = f * P.x, ni = f * P.y, sr = two ? f * P.z : (T)0, si = two ? f * P.w : (T)0;
+                const int64_t idx = m * stride + col;
+                const Quad<T> b = rhs_map[idx];
+                out[idx] = Quad<T>{nr + sr - b.x, ni + si - b.y, nr - sr - b.z, ni - si - b.w};
+            }
+        } else if (part == 0 && 2 * k <= n) {
+            const int64_t base = (c - cbeg) * (4 * nside - 1);
+            spec[(base + north_ring(j)) * sstride + k] = make2<T2, T>(P.x, P.y);
+            if (two) spec[(base + south_ring(nside, j)) * sstride + k] = make2<T2, T>(P.z, P.w);
+        }
+    };
+    auto finish = [&](int p, const Quad<T> &A, const Quad<T> &B) {
+        if (p == 0) {
+            const Quad<T> z = src[0];
+            emit(0, Quad<T>{z.x + 2 * A.x, z.y, z.z + 2 * A.z, z.w});
+        } else if (2 * p == n) {
+            emit(p, Quad<T>{A.x + sigma * A.x, A.y - sigma * A.y, A.z + sigma * A.z, A.w - sigma * A.w});
+        } else {
+            emit(p, Quad<T>{A.x + sigma * B.x, A.y - sigma * B.y, A.z + sigma * B.z, A.w - sigma * B.w});
+            if (RESIDUAL)
+                emit(n - p, Quad<T>{B.x + sigma * A.x, B.y - sigma * A.y, B.z + sigma * A.z, B.w - sigma * A.w});
+        }
+    };
+
+    const int p0 = q / s;
+    if (s > 1 && ok && p0 < np) {
+        Quad<T> A, B;
+        pair_sums(p0, A, B);
+        pa[threadIdx.x] = A;
+        pb[threadIdx.x] = B;
+    }
+    __syncthreads();
+    if (!ok) return;
+    if (s > 1) {
+        if (p0 >= np) return;
+        Quad<T> A{0, 0, 0, 0}, B{0, 0, 0, 0};
+        for (int u = 0; u < s; ++u) {
+            const int e = (p0 * s + u) * J + (int)(threadIdx.x % J);
+            const Quad<T> a = pa[e], b = pb[e];
+            A.x += a.x; A.y += a.y; A.z += a.z; A.w += a.w;
+            B.x += b.x; B.y += b.y; B.z += b.z; B.w += b.w;
+        }
+        finish(p0, A, B);
+    } else {
+        for (int p = p0; p < np; p += Q) {
+            Quad<T> A, B;
+            pair_sums(p, A, B);
+            finish(p, A, B);
         }
     }
 }
@@ -600,62 +767,83 @@ __global__ void __launch_bounds__(512) k_ring_synthesis(int64_t nside, int64_t L
 }
 
 
+// Inverse ring transform from the folded spectra of k_fold_lanes: one CTA per (ring, block of
+// cpc components).  i0 > 0: the cap rings of length 4 i, i0 <= i < i0 + cnt, of both
+// hemispheres; i0 = 0: the belt.  Rings whose half-length has a prime factor above 64 go through
+// Bluestein's method (M <= mcap: three buffers of M), the others through the mixed-radix FFT.
+// A launch covers rings of one shared-memory size, so that short rings run many CTAs per SM.
+// With the fold before it: 2235 -> 790 us for a (Q, U) pair at Nside 1024 (a ring per CTA reading
+// its coefficients 128 lanes apart and taking prime factors up to 1021 as one radix), 163 -> 61
+// us for one FP64 map at Nside 256.
+template <typename T>
+__global__ void __launch_bounds__(512) k_ring_inverse(int64_t nside, int64_t ncomp, int cpc, int64_t sstride,
+                                                      const typename vec2<T>::type *__restrict__ spec,
+                                                      const void *__restrict__ twall, int64_t twcnt,
+                                                      const uint8_t *__restrict__ shifted, double *__restrict__ maps,
+                                                      int64_t cbeg, int64_t i0, int64_t cnt, int mcap, int hcap,
+                                                      int bsmin, int buf)
+{
+    using T2 = typename vec2<T>::type;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int64_t b = blockIdx.y, nring = 4 * nside - 1, npix = 12 * nside * nside;
+    const int64_t r = i0 == 0 ? nside - 1 + b : (b < cnt ? i0 - 1 + b : 4 * nside - 1 - (i0 + b - cnt));
+    const int n = (int)ring_nphi(nside, r), h = n / 2;
+    const bool bs = mcap > 0 && use_bluestein(h, mcap);
+    if (hcap > 0 && ring_big(h, hcap, (int)nside, bsmin)) return;   // left to k_ring_synthesis_big
+    const int64_t off = ring_offset(nside, r);
+    const bool sh = shifted[r] != 0;
+    T2 *b0 = reinterpret_cast<T2 *>(smem_raw), *b1 = b0 + buf, *b2 = b1 + buf;
+    const T2 *twT = TwTable<T2>::get(twall, twcnt);
+    const T2 *tw = twT + twiddle_offset(n);
+    const int M = bs ? next_pow2(2 * h - 1) : 0;
+    const T2 *twM = bs ? twT + twiddle_offset(M) : nullptr;
+    T2 *FB = nullptr, *X = b0, *Y = b1;
+    if (bs) {
+        FB = bs_filter(h, n, M, tw, twM, +1, b0, b1);
+        X = FB == b0 ? b1 : b0;
+        Y = b2;
+    }
+    T2 cpi;   // e^{-i pi / n}
+    {
+        double s1, c1d;
+        sincospi(-1.0 / (double)n, &s1, &c1d);
+        cpi = make2<T2, T>((T)c1d, (T)s1);
+    }
+    const int64_t cend = (int64_t)(blockIdx.x + 1) * cpc < ncomp ? (int64_t)(blockIdx.x + 1) * cpc : ncomp;
+    for (int64_t c = (int64_t)blockIdx.x * cpc; c < cend; ++c) {
+        const T2 *P = spec + (c * nring + r) * sstride;
+        // Z'[k] = (C_k + C_{k+h}) + i (C_k - C_{k+h}) omega_n^{-k}, C_k = e^{i pi s k / n} P_k and
+        // C_{k+h} = conj C_{h-k} for k > 0
+        for (int k = threadIdx.x; k < h; k += blockDim.x) {
+            T2 ck = P[k], ch = P[h - k];
+            if (sh) {
+                ck = cmul(ck, phase_pi(tw, h, k, cpi, +1));
+                ch = cmul(ch, phase_pi(tw, h, h - k, cpi, +1));
+            }
+            if (k > 0) ch = cconj(ch);
+            const T2 sum = cadd(ck, ch);
+            const T2 dif = cmul(csub(ck, ch), twiddle_n(tw, h, k, +1));
+            T2 z = make2<T2, T>(sum.x - dif.y, sum.y + dif.x);
+            if (bs) z = cmul(z, bs_chirp(tw, h, n, k, +1));
+            X[k] = z;
+        }
+        __syncthreads();
+        const T2 *Z = bs ? bs_apply(X, Y, FB, h, n, M, tw, twM, +1) : fft_shared(X, Y, h, tw, +1);
+        double2 *dst = reinterpret_cast<double2 *>(maps + (cbeg + c) * npix + off);
+        for (int t = threadIdx.x; t < h; t += blockDim.x) {
+            const T2 z = Z[t];
+            dst[t] = make_double2((double)z.x, (double)z.y);
+        }
+        __syncthreads();
+    }
+}
+
 // ---------------------------------------------------------------- rings beyond shared memory
 //
 // One persistent CTA per slot of the global scratch (three buffers of Mmax complex floats
 // each) walks the rings; only the rings of ring_big are transformed, with the arithmetic of
 // the shared-memory kernels: a Stockham FFT of length h, or Bluestein's method with a
 // power-of-two length M.  __syncthreads orders the CTA's global-memory accesses.
-
-__device__ __forceinline__ float2 bs_chirp(const float2 *__restrict__ tw, int h, int n, int j, int sign)
-{
-    const unsigned q = ((unsigned)j * (unsigned)j) % (unsigned)n;
-    return twiddle_n(tw, h, (int)q, sign);   // e^{sign i pi j^2 / h}
-}
-
-// Bluestein filter: the transform of the wrapped conjugate chirp of length M; returns the
-// buffer holding it (b0 or b1).
-__device__ float2 *bs_filter(int h, int n, int M, const float2 *__restrict__ tw,
-                             const float2 *__restrict__ twM, int sign, float2 *b0, float2 *b1)
-{
-    for (int m = threadIdx.x; m < M; m += blockDim.x) {
-        float2 v = make_float2(0.f, 0.f);
-        int j = -1;
-        if (m < h) j = m;
-        else if (m > M - h) j = M - m;
-        if (j >= 0) {
-            v = bs_chirp(tw, h, n, j, sign);
-            v.y = -v.y;
-        }
-        b0[m] = v;
-    }
-    __syncthreads();
-    return fft_shared<1>(b0, b1, M, twM, -1);
-}
-
-// X[0, h) holds z_j c_j; zero-pads to M, convolves with the filter FB and returns the buffer
-// holding the DFT sum_j z_j e^{sign 2 pi i jk / h}, k < h.
-__device__ float2 *bs_apply(float2 *X, float2 *Y, const float2 *FB, int h, int n, int M,
-                            const float2 *__restrict__ tw, const float2 *__restrict__ twM, int sign)
-{
-    for (int j = h + threadIdx.x; j < M; j += blockDim.x) X[j] = make_float2(0.f, 0.f);
-    __syncthreads();
-    float2 *FA = fft_shared<1>(X, Y, M, twM, -1);
-    float2 *G = (FA == X) ? Y : X;
-    const float invM = 1.0f / (float)M;
-    for (int m = threadIdx.x; m < M; m += blockDim.x) {
-        float2 v = cmul(FA[m], FB[m]);
-        v.x *= invM;
-        v.y *= invM;
-        FA[m] = v;
-    }
-    __syncthreads();
-    float2 *R = fft_shared<1>(FA, G, M, twM, +1);
-    float2 *Z = (R == FA) ? G : FA;
-    for (int k = threadIdx.x; k < h; k += blockDim.x) Z[k] = cmul(R[k], bs_chirp(tw, h, n, k, sign));
-    __syncthreads();
-    return Z;
-}
 
 // T = float: three buffers of Mmax complex floats per slot (Bluestein rings included).
 // T = double: no Bluestein path (the mixed-radix FFT takes every ring, as in the FP64
@@ -973,22 +1161,35 @@ extern "C" int gm_pack_rhs(int precision, int64_t nside, int64_t L, int64_t ncom
     return check_launch("gm_pack_rhs");
 }
 
+// Columns per CTA: eight (a full 128-byte line a row in single precision) where that leaves two
+// CTAs per SM, else two.
+template <typename T, bool RESIDUAL>
+static void fold_lanes(int64_t nside, int64_t L, int64_t ncomp, int64_t cbeg, int64_t cw, const void *syn,
+                       const void *rhs_map, const uint8_t *shifted, void *out, void *spec, int64_t sstride,
+                       cudaStream_t s)
+{
+    using T2 = typename vec2<T>::type;
+    const int64_t items = 2 * nside * cw;
+    auto run = [&](auto kernel, int J) {
+        kernel<<<(unsigned)((items + J - 1) / J), fold_threads(J), 0, s>>>(nside, L, ncomp, cbeg, cw, (const Quad<T> *)syn,
+                                                               (const Quad<T> *)rhs_map, shifted, (Quad<T> *)out,
+                                                               (T2 *)spec, sstride);
+    };
+    if (items >= 8 * 296) run(k_fold_lanes<T, 8, RESIDUAL>, 8);
+    else run(k_fold_lanes<T, 2, RESIDUAL>, 2);
+}
+
 extern "C" int gm_fold_residual(int precision, int64_t nside, int64_t L, int64_t ncomp,
                                 const void *syn, const void *rhs_map, const uint8_t *shifted,
                                 void *rhs_out, void *stream)
 {
     if (nside < 1 || L < 1 || ncomp < 1 || ncomp > 65535) return GM_ERR_BAD_SHAPE;
     if (!syn || !rhs_map || !shifted || !rhs_out) return GM_ERR_BAD_PTR;
-    dim3 grid((unsigned)(2 * nside), (unsigned)ncomp);
     cudaStream_t s = as_stream(stream);
     if (precision == GM_FP64)
-        k_fold_residual<double><<<grid, 256, 0, s>>>(nside, L, ncomp, (const double *)syn,
-                                                     (const double *)rhs_map, shifted,
-                                                     (double *)rhs_out);
+        fold_lanes<double, true>(nside, L, ncomp, 0, ncomp, syn, rhs_map, shifted, rhs_out, nullptr, 0, s);
     else if (precision == GM_MIXED)
-        k_fold_residual<float><<<grid, 256, 0, s>>>(nside, L, ncomp, (const float *)syn,
-                                                    (const float *)rhs_map, shifted,
-                                                    (float *)rhs_out);
+        fold_lanes<float, true>(nside, L, ncomp, 0, ncomp, syn, rhs_map, shifted, rhs_out, nullptr, 0, s);
     else
         return GM_ERR_UNSUPPORTED;
     return check_launch("gm_fold_residual");
@@ -1042,4 +1243,90 @@ extern "C" int gm_ring_synthesis(int precision, int64_t nside, int64_t L, int64_
 {
     return gm_ring_synthesis_ws(precision, nside, L, ncomp, syn, tw, shifted, maps, nullptr, 0, 0, 0,
                                 stream);
+}
+
+// Whether some ring goes to the *_big kernels (ring_big of the longest ring).
+static bool any_ring_big(int64_t nside, int hcap, int bsmin)
+{
+    return 2 * nside > hcap || (bsmin > 0 && next_pow2((int)(4 * nside - 1)) > bsmin);
+}
+
+extern "C" int64_t gm_ring_fold_bytes(int precision, int64_t nside)
+{
+    if (nside < 1) return 0;
+    return (4 * nside - 1) * (2 * nside + 1) * (int64_t)(precision == GM_FP64 ? sizeof(double2) : sizeof(float2));
+}
+
+template <typename T>
+static int ring_synthesis_fold(int64_t nside, int64_t L, int64_t ncomp, const void *syn, const void *tw,
+                               const uint8_t *shifted, double *maps, void *work, int64_t chunk, int hcap, int bsmin,
+                               bool big, cudaStream_t s)
+{
+    using T2 = typename vec2<T>::type;
+    const int64_t cnt = gm_ring_twiddle_count(nside), sstride = 2 * nside + 1;
+    const int hc = big ? hcap : 0;
+    int mcap = bluestein_mcap(nside);
+    if (sizeof(T) == 8 && mcap > 4096) mcap = 4096;   // three buffers of M in 227 KB
+    for (int64_t c0 = 0; c0 < ncomp; c0 += chunk) {
+        const int64_t cw = ncomp - c0 < chunk ? ncomp - c0 : chunk;
+        fold_lanes<T, false>(nside, L, ncomp, c0, cw, syn, nullptr, shifted, nullptr, work, sstride, s);
+        int st = check_launch("gm_ring_synthesis_fold");
+        if (st) return st;
+        // rings up to half-length hmax, with buffers for Bluestein rings of length M (0: none)
+        auto run = [&](int64_t i0, int64_t n, int hmax, int M) {
+            const int cpc = 8, buf = M > hmax ? M : hmax;
+            const size_t bytes = (size_t)(M ? 3 : 2) * buf * sizeof(T2);
+            int e = set_smem(k_ring_inverse<T>, bytes);
+            if (e) return e;
+            const int threads = hmax <= 256 ? 128 : (hmax <= 512 ? 256 : 512);
+            dim3 grid((unsigned)((cw + cpc - 1) / cpc), (unsigned)(i0 ? 2 * n : 2 * nside + 1));
+            k_ring_inverse<T><<<grid, threads, bytes, s>>>(nside, cw, cpc, sstride, (const T2 *)work, tw, cnt, shifted,
+                                                           maps, c0, i0, n, M ? mcap : 0, hc, bsmin, buf);
+            return check_launch("gm_ring_synthesis_fold");
+        };
+        // the belt (length 4 nside), then the caps by powers of two of their length
+        const int hb = (int)(2 * nside);
+        const int hfit = big && hb > hcap ? hcap : hb;
+        if ((st = run(0, 0, hfit, use_bluestein(hb, mcap) ? next_pow2(2 * hb - 1) : 0))) return st;
+        for (int64_t lo = 1, hi = 128; lo < nside; lo = hi + 1, hi *= 2) {
+            const int64_t top = hi < nside - 1 ? hi : nside - 1;
+            const int hm = (int)(2 * top), M = next_pow2(2 * hm - 1);
+            // above the first class every ring has the same M: beyond mcap none takes Bluestein
+            const int Mc = M <= mcap ? M : (lo == 1 ? mcap : 0);
+            if ((st = run(lo, top - lo + 1, big && hm > hcap ? hcap : hm, Mc))) return st;
+        }
+    }
+    return GM_OK;
+}
+
+extern "C" int gm_ring_synthesis_fold(int precision, int64_t nside, int64_t L, int64_t ncomp, const void *syn,
+                                      const void *tw, const uint8_t *shifted, double *maps, void *work,
+                                      int64_t work_bytes, void *scratch, int64_t scratch_bytes, int64_t hcap_max,
+                                      int64_t bs_min, void *stream)
+{
+    if (nside < 1 || nside > 8192 || L < 1 || ncomp < 1 || ncomp > 65535) return GM_ERR_BAD_SHAPE;
+    if (precision != GM_FP64 && precision != GM_MIXED) return GM_ERR_UNSUPPORTED;
+    if (!syn || !tw || !shifted || !maps || !work || !scratch) return GM_ERR_BAD_PTR;
+    if ((reinterpret_cast<uintptr_t>(maps) | reinterpret_cast<uintptr_t>(syn)) & 15) return GM_ERR_BAD_PTR;
+    const int64_t per = gm_ring_fold_bytes(precision, nside), chunk = work_bytes / per;
+    const int64_t slot = gm_ring_big_scratch_bytes(nside, 1), nslots = scratch_bytes / slot;
+    if (chunk < 1 || nslots < 1) return GM_ERR_BAD_SHAPE;
+    int hcap = ring_hcap(precision, nside, true);
+    if (hcap_max > 0 && hcap_max < hcap) hcap = (int)hcap_max;
+    const int bsmin = precision == GM_MIXED ? (bs_min > 0 ? (int)bs_min : 8192) : 0;
+    const bool big = any_ring_big(nside, hcap, bsmin);
+    cudaStream_t s = as_stream(stream);
+    const int st = precision == GM_FP64
+                       ? ring_synthesis_fold<double>(nside, L, ncomp, syn, tw, shifted, maps, work, chunk, hcap, bsmin, big, s)
+                       : ring_synthesis_fold<float>(nside, L, ncomp, syn, tw, shifted, maps, work, chunk, hcap, bsmin, big, s);
+    if (st || !big) return st;
+    const int64_t nring = 4 * nside - 1, cnt = gm_ring_twiddle_count(nside);
+    const unsigned gbig = (unsigned)(nslots < nring ? nslots : nring);
+    if (precision == GM_FP64)
+        k_ring_synthesis_big<double><<<gbig, 512, 0, s>>>(nside, L, ncomp, (const double *)syn, tw, cnt, shifted, maps,
+                                                          hcap, 0, scratch, slot);
+    else
+        k_ring_synthesis_big<float><<<gbig, 512, 0, s>>>(nside, L, ncomp, (const float *)syn, tw, cnt, shifted, maps,
+                                                         hcap, bsmin, scratch, slot);
+    return check_launch("gm_ring_synthesis_fold");
 }

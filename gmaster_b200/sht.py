@@ -338,12 +338,18 @@ def fold_residual(plan, syn, rhs_map, prec, out=None):
     return res
 
 
+# Folded ring spectra of the synthesis: components at a time, up to this many bytes.
+RING_FOLD_BYTES = 1 << 30
+
+
 def ring_synthesis(plan, syn, prec):
     ncomp = syn.shape[2]
     maps = torch.empty((ncomp, plan.npix), dtype=torch.float64, device=plan.device)
+    per = int(_lib.load().gm_ring_fold_bytes(prec, plan.nside))
+    work = torch.empty(per * max(1, min(ncomp, RING_FOLD_BYTES // per)), dtype=torch.uint8, device=plan.device)
     scratch, sbytes = _ring_scratch(plan, prec)
-    _lib.call("gm_ring_synthesis_ws", prec, plan.nside, plan.L, ncomp, _lib.ptr(syn), _lib.ptr(plan.tw),
-              _lib.ptr(plan.shifted), _lib.ptr(maps), _lib.ptr(scratch), sbytes,
+    _lib.call("gm_ring_synthesis_fold", prec, plan.nside, plan.L, ncomp, _lib.ptr(syn), _lib.ptr(plan.tw),
+              _lib.ptr(plan.shifted), _lib.ptr(maps), _lib.ptr(work), work.numel(), _lib.ptr(scratch), sbytes,
               RING_TUNING["hcap_max"], RING_TUNING["bs_min"], _lib.stream_handle(plan.device))
     return maps
 

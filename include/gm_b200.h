@@ -115,6 +115,18 @@ int gm_ring_synthesis_ws(int precision, int64_t nside, int64_t L, int64_t ncomp,
                          const void *tw, const uint8_t *shifted, double *maps, void *scratch,
                          int64_t scratch_bytes, int64_t hcap_max, int64_t bs_min, void *stream);
 
+/* gm_ring_synthesis_ws in two steps: the coefficients folded into the half spectra of the
+ * rings (read once, in rows of neighbouring lanes), then the inverse transforms, rings with a
+ * prime factor above 64 by Bluestein's method in both precisions (the entries above take the
+ * mixed-radix FFT).  work holds the folded spectra of as many components at a time as
+ * work_bytes allow, gm_ring_fold_bytes each; scratch as in gm_ring_synthesis_ws (required).
+ * syn and maps must be 16-byte aligned. */
+int64_t gm_ring_fold_bytes(int precision, int64_t nside);
+int gm_ring_synthesis_fold(int precision, int64_t nside, int64_t L, int64_t ncomp, const void *syn,
+                           const void *tw, const uint8_t *shifted, double *maps, void *work,
+                           int64_t work_bytes, void *scratch, int64_t scratch_bytes,
+                           int64_t hcap_max, int64_t bs_min, void *stream);
+
 /* ----------------------------------------------------------- Legendre stage */
 
 /* Seed table length (doubles): 17 variants x L orders x 4.  Variant 0 is spin 0; spin
