@@ -400,77 +400,166 @@ __global__ void k_bin_cells(int64_t lmax, int64_t nb, int64_t ncls, const double
 
 // ---------------------------------------------------------------- LU
 
-// Single-CTA right-looking LU with partial pivoting, row-major a (n x n).
-__global__ void __launch_bounds__(1024) k_lu_factor(int64_t n, double *__restrict__ a,
-                                                    int32_t *__restrict__ piv,
-                                                    int32_t *__restrict__ status)
+// Blocked LU, panel step in shared memory: columns [k0, k0 + kb) of rows k0..n-1 of the
+// row-major (n, n) matrix, one CTA, partial pivoting (largest magnitude, lowest row on ties; a
+// NaN is never chosen over a number).  Row interchanges are confined to the panel here; k_lu_rest
+// applies them to the other columns.  piv[k] is the row exchanged with row k; *status receives
+// k + 1 for the first column without a non-zero pivot.
+//
+// Bound by latency: two barriers, a warp reduction of the pivot candidates and kb - k
+// multiply-adds a row per column.  The panel is read and written once; held in global memory it
+// took 7 us a column, here 1.9 (a 612 x 612 matrix: panels 4.3 -> 1.16 ms, with the other
+// columns' kernels 5.4 -> 1.5 ms).
+__global__ void __launch_bounds__(1024) k_lu_panel_smem(int n, int k0, int kb, double *__restrict__ a,
+                                                        int32_t *__restrict__ piv, int32_t *__restrict__ status)
 {
-    __shared__ double sval[32];
-    __shared__ int sidx[32];
-    __shared__ int pivot_row;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    if (tid == 0) *status = 0;
-    for (int64_t k = 0; k < n; ++k) {
-        // pivot search in column k
-        double best = -1.0;
-        int bi = (int)k;
-        for (int64_t i = k + tid; i < n; i += blockDim.x) {
-            const double v = fabs(a[i * n + k]);
-            if (v > best) {
-                best = v;
-                bi = (int)i;
+    extern __shared__ double pan[];   // [kb][ld], column c at pan + c * ld
+    __shared__ unsigned long long skey[2][32];
+    __shared__ int srow[2][32];
+    const int rows = n - k0, ld = rows | 1;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    if (k0 == 0 && tid == 0) *status = 0;
+    for (int64_t e = tid; e < (int64_t)rows * kb; e += blockDim.x) {
+        const int i = (int)(e / kb), c = (int)(e % kb);
+        pan[(int64_t)c * ld + i] = a[(int64_t)(k0 + i) * n + k0 + c];
+    }
+    __syncthreads();
+    // order of candidates: NaN, then by magnitude
+    auto key_of = [](double v) -> unsigned long long {
+        const double f = fabs(v);
+        return f >= 0.0 ? (unsigned long long)__double_as_longlong(f) + 1ull : 0ull;
+    };
+    for (int k = 0; k < kb; ++k) {
+        double *col = pan + (int64_t)k * ld;
+        unsigned long long key = 0;
+        int row = k;
+        for (int i = k + tid; i < rows; i += blockDim.x) {
+            const unsigned long long q = key_of(col[i]);
+            if (q > key) {
+                key = q;
+                row = i;
             }
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            const double ov = __shfl_down_sync(0xffffffffu, best, o);
-            const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-            if (ov > best || (ov == best && oi < bi)) {
-                best = ov;
-                bi = oi;
+        auto better = [](unsigned long long q, int r, unsigned long long &bq, int &br) {
+            if (q > bq || (q == bq && r < br)) {
+                bq = q;
+                br = r;
             }
+        };
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long q = __shfl_xor_sync(0xffffffffu, key, o);
+            const int r = __shfl_xor_sync(0xffffffffu, row, o);
+            better(q, r, key, row);
         }
         if (lane == 0) {
-            sval[warp] = best;
-            sidx[warp] = bi;
+            skey[k & 1][warp] = key;
+            srow[k & 1][warp] = row;
         }
         __syncthreads();
+        key = lane < nw ? skey[k & 1][lane] : 0ull;
+        row = lane < nw ? srow[k & 1][lane] : rows;
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long q = __shfl_xor_sync(0xffffffffu, key, o);
+            const int r = __shfl_xor_sync(0xffffffffu, row, o);
+            better(q, r, key, row);
+        }
+        if (key == 0ull) row = k;   // no number in the column
         if (tid == 0) {
-            double bv = sval[0];
-            int bix = sidx[0];
-            for (int w = 1; w < nwarps; ++w)
-                if (sval[w] > bv || (sval[w] == bv && sidx[w] < bix)) {
-                    bv = sval[w];
-                    bix = sidx[w];
-                }
-            pivot_row = bix;
-            piv[k] = bix;
-            if (bv == 0.0 && *status == 0) *status = (int32_t)(k + 1);
+            piv[k0 + k] = k0 + row;
+            if (key == 1ull && *status == 0) *status = k0 + k + 1;
         }
-        __syncthreads();
-        const int64_t p = pivot_row;
-        if (p != k)
-            for (int64_t jj = tid; jj < n; jj += blockDim.x) {
-                const double t = a[k * n + jj];
-                a[k * n + jj] = a[p * n + jj];
-                a[p * n + jj] = t;
+        if (row != k)
+            for (int c = tid; c < kb; c += blockDim.x) {
+                const double t = pan[(int64_t)c * ld + k];
+                pan[(int64_t)c * ld + k] = pan[(int64_t)c * ld + row];
+                pan[(int64_t)c * ld + row] = t;
             }
         __syncthreads();
-        const double d = a[k * n + k];
-        const double inv = d != 0.0 ? 1.0 / d : 0.0;
-        for (int64_t i = k + 1 + tid; i < n; i += blockDim.x) a[i * n + k] *= inv;
-        __syncthreads();
-        // trailing update, one warp per row, lanes along columns
-        for (int64_t i = k + 1 + warp; i < n; i += nwarps) {
-            const double lik = a[i * n + k];
-            if (lik != 0.0)
-                for (int64_t jj = k + 1 + lane; jj < n; jj += 32) a[i * n + jj] -= lik * a[k * n + jj];
+        const double d = col[k], inv = d != 0.0 ? 1.0 / d : 0.0;
+        for (int i = k + 1 + tid; i < rows; i += blockDim.x) {
+            const double l = col[i] * inv;
+            col[i] = l;
+#pragma unroll 4
+            for (int c = k + 1; c < kb; ++c) {
+                double *pc = pan + (int64_t)c * ld;
+                pc[i] = fma(-l, pc[k], pc[i]);
+            }
         }
         __syncthreads();
     }
+    for (int64_t e = tid; e < (int64_t)rows * kb; e += blockDim.x) {
+        const int i = (int)(e / kb), c = (int)(e % kb);
+        a[(int64_t)(k0 + i) * n + k0 + c] = pan[(int64_t)c * ld + i];
+    }
 }
 
-// Blocked LU, panel step: columns [k0, k1) of the row-major (n, n) matrix, rows k0..n-1,
-// one CTA.  Partial pivoting as in k_lu_factor (the pivot swap moves whole rows, all n
+// Blocked LU, the columns outside the panel [k0, k0 + kb), kb <= 32: the panel's row
+// interchanges as one permutation (every row read before any is written), and right of the panel
+// the U rows, L11^-1 times themselves with L11 unit lower triangular; one thread per column.
+constexpr int kLuPan = 32;
+__global__ void __launch_bounds__(128) k_lu_rest(int n, int k0, int kb, double *__restrict__ a,
+                                                 const int32_t *__restrict__ piv)
+{
+    __shared__ double l11[kLuPan][kLuPan];
+    __shared__ int top[kLuPan], ext[kLuPan], dst[kLuPan];   // sources of the panel's rows and of the rows below
+    __shared__ bool below[kLuPan];                          // dst is below the panel and named for the first time
+    const int tid = threadIdx.x, k1 = k0 + kb;
+    for (int e = tid; e < kb * kb; e += blockDim.x) l11[e / kb][e % kb] = a[(int64_t)(k0 + e / kb) * n + k0 + e % kb];
+    if (tid < kb) {
+        top[tid] = k0 + tid;
+        const int p = piv[k0 + tid];
+        dst[tid] = p;
+        ext[tid] = p;
+    }
+    __syncthreads();
+    if (tid < kb) {
+        bool first = dst[tid] >= k1;
+        for (int e = 0; e < tid && first; ++e) first = dst[e] != dst[tid];
+        below[tid] = first;
+    }
+    if (tid == 0) {
+        for (int i = 0; i < kb; ++i) {
+            const int p = dst[i], t = top[i];
+            if (p < k1) {
+                top[i] = top[p - k0];
+                top[p - k0] = t;
+            } else {
+                int e = 0;   // the first step that exchanged with row p holds its content
+                while (dst[e] != p) ++e;
+                top[i] = ext[e];
+                ext[e] = t;
+            }
+        }
+    }
+    __syncthreads();
+    int col = blockIdx.x * blockDim.x + tid;
+    if (col >= n - kb) return;
+    if (col >= k0) col += kb;
+    double u[kLuPan], w[kLuPan];
+#pragma unroll
+    for (int i = 0; i < kLuPan; ++i) {
+        if (i >= kb) break;
+        u[i] = a[(int64_t)top[i] * n + col];
+        w[i] = below[i] ? a[(int64_t)ext[i] * n + col] : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < kLuPan; ++i) {
+        if (i >= kb) break;
+        if (below[i]) a[(int64_t)dst[i] * n + col] = w[i];
+        if (col >= k1) {
+#pragma unroll
+            for (int j = 0; j < kLuPan; ++j) {
+                if (j >= i) break;
+                u[i] = fma(-l11[i][j], u[j], u[i]);
+            }
+        }
+        a[(int64_t)(k0 + i) * n + col] = u[i];
+    }
+}
+
+// Blocked LU, panel step in global memory for matrices whose panels do not fit shared memory:
+// columns [k0, k1) of the row-major (n, n) matrix, rows k0..n-1,
+// one CTA.  Partial pivoting as in k_lu_panel_smem (the pivot swap moves whole rows, all n
 // columns, so the left factor and the trailing part stay consistent); the rank-1 updates
 // are confined to the panel's columns.  The caller then solves for the U rows right of
 // the panel (k_lu_trsm) and updates the trailing matrix with one GEMM.
@@ -750,6 +839,133 @@ __global__ void __launch_bounds__(256) k_lu_solve_blk(int64_t n, const double *_
     }
 }
 
+// Prepared solves.  The row interchanges of the factorisation as one permutation, and the
+// inverses of the 32 x 32 diagonal blocks of L and U (the last block padded with the identity):
+// a solve then has no sequential chain inside a block, only a product of 32 x 32.
+constexpr int kLuSB = 32;
+
+// Block 0: perm (n rows: row perm[i] of b becomes row i); block 1 + i: the inverses of diagonal
+// block i.  inv holds (block, L or U, row, column).
+__global__ void __launch_bounds__(64) k_lu_prepare(int n, const double *__restrict__ lu,
+                                                   const int32_t *__restrict__ piv, int32_t *__restrict__ perm,
+                                                   double *__restrict__ inv)
+{
+    __shared__ double d[kLuSB][kLuSB + 1];
+    extern __shared__ int32_t sidx[];   // n entries, then the interchanges
+    const int tid = threadIdx.x;
+    if (blockIdx.x == 0) {
+        int32_t *sp = sidx + n;
+        for (int i = tid; i < n; i += blockDim.x) {
+            sidx[i] = i;
+            sp[i] = piv[i];
+        }
+        __syncthreads();
+        if (tid == 0)
+            for (int k = 0; k < n; ++k) {
+                const int32_t p = sp[k], t = sidx[k];
+                sidx[k] = sidx[p];
+                sidx[p] = t;
+            }
+        __syncthreads();
+        for (int i = tid; i < n; i += blockDim.x) perm[i] = sidx[i];
+        return;
+    }
+    const int blk = blockIdx.x - 1, r0 = blk * kLuSB, lane = tid & 31, upper = tid >> 5;
+    for (int e = tid; e < kLuSB * kLuSB; e += blockDim.x) {
+        const int i = e / kLuSB, k = e % kLuSB;
+        d[i][k] = r0 + i < n && r0 + k < n ? lu[(int64_t)(r0 + i) * n + r0 + k] : (i == k ? 1.0 : 0.0);
+    }
+    __syncthreads();
+    // one warp per triangle, one column of the inverse per lane
+    double y[kLuSB];
+    if (!upper) {
+#pragma unroll
+        for (int i = 0; i < kLuSB; ++i) {
+            double v = i == lane ? 1.0 : 0.0;
+#pragma unroll
+            for (int k = 0; k < kLuSB; ++k)
+                if (k < i) v = fma(-d[i][k], y[k], v);
+            y[i] = v;
+        }
+    } else {
+#pragma unroll
+        for (int i = kLuSB - 1; i >= 0; --i) {
+            double v = i == lane ? 1.0 : 0.0;
+#pragma unroll
+            for (int k = 0; k < kLuSB; ++k)
+                if (k > i) v = fma(-d[i][k], y[k], v);
+            y[i] = v / d[i][i];
+        }
+    }
+    double *o = inv + ((int64_t)blk * 2 + upper) * kLuSB * kLuSB;
+#pragma unroll
+    for (int i = 0; i < kLuSB; ++i) o[i * kLuSB + lane] = y[i];
+}
+
+// x = A^-1 b with the prepared factors; b and x (n, nrhs) row-major.  One CTA per CB columns of
+// b, held in shared memory; one warp per row of a 32-row block: the products with the rows solved
+// so far and with the inverse of the diagonal block are each a sum over the lanes, so a column's
+// arithmetic does not depend on CB or on its neighbours.  Bound by the latency of 2 n / 32 block
+// steps (two barriers, a row read and two reductions each); with the interchanges applied one by
+// one and 32-step substitutions inside a block a solve of n = 92 took 42 us, of 612 438
+// us; here 6.8 and 77 us.
+template <int CB>
+__global__ void __launch_bounds__(1024) k_lu_solve_prepared(int n, const double *__restrict__ lu,
+                                                            const int32_t *__restrict__ perm,
+                                                            const double *__restrict__ inv, int64_t nrhs,
+                                                            const double *__restrict__ b, double *__restrict__ x)
+{
+    extern __shared__ double xs[];   // [n rounded up to 32][CB]
+    __shared__ double part[kLuSB][CB];
+    const int tid = threadIdx.x, lane = tid & 31, r = tid >> 5;
+    const int64_t c0 = (int64_t)blockIdx.x * CB;
+    const int ncol = (int)(nrhs - c0 < CB ? nrhs - c0 : CB);
+    const int nblk = (n + kLuSB - 1) / kLuSB;
+    for (int i = tid; i < nblk * kLuSB * CB; i += blockDim.x) {
+        const int row = i / CB, c = i % CB;
+        xs[i] = row < n && c < ncol ? b[(int64_t)perm[row] * nrhs + c0 + c] : 0.0;
+    }
+    __syncthreads();
+    auto step = [&](int blk, int jbeg, int jend, int upper) {
+        const int row = blk * kLuSB + r;
+        const double di = inv[((int64_t)blk * 2 + upper) * kLuSB * kLuSB + r * kLuSB + lane];
+        double acc[CB];
+#pragma unroll
+        for (int c = 0; c < CB; ++c) acc[c] = 0.0;
+        if (row < n) {
+            const double *src = lu + (int64_t)row * n;
+#pragma unroll 4
+            for (int j = jbeg + lane; j < jend; j += 32) {
+                const double l = __ldg(src + j);
+#pragma unroll
+                for (int c = 0; c < CB; ++c) acc[c] = fma(l, xs[j * CB + c], acc[c]);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < CB; ++c)
+            for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+        if (lane == 0)
+#pragma unroll
+            for (int c = 0; c < CB; ++c) part[r][c] = xs[row * CB + c] - acc[c];
+        __syncthreads();
+#pragma unroll
+        for (int c = 0; c < CB; ++c) {
+            acc[c] = di * part[lane][c];
+            for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+        }
+        if (lane == 0)
+#pragma unroll
+            for (int c = 0; c < CB; ++c) xs[row * CB + c] = acc[c];
+        __syncthreads();
+    };
+    for (int blk = 0; blk < nblk; ++blk) step(blk, 0, blk * kLuSB, 0);
+    for (int blk = nblk - 1; blk >= 0; --blk) step(blk, (blk + 1) * kLuSB, n, 1);
+    for (int i = tid; i < n * CB; i += blockDim.x) {
+        const int row = i / CB, c = i % CB;
+        if (c < ncol) x[(int64_t)row * nrhs + c0 + c] = xs[i];
+    }
+}
+
 }  // namespace gm
 
 using namespace gm;
@@ -878,11 +1094,55 @@ extern "C" int gm_bin_cells_csr(int64_t lmax, int64_t nbands, int64_t ncls, cons
     return check_launch("gm_bin_cells");
 }
 
+// Panel width of the shared-memory panels: the widest of 32, 16, 8, 4 columns that fit (the
+// whole matrix up to n = 160), 0 when none does.
+static int lu_panel_width(int64_t n)
+{
+    const int64_t fit = 200 * 1024 / (8 * (n | 1));
+    if (fit >= n) return (int)n;
+    for (int kb = kLuPan; kb >= 4; kb /= 2)
+        if (fit >= kb) return kb;
+    return 0;
+}
+
 extern "C" int gm_lu_factor(int64_t n, double *a, int32_t *piv, int32_t *status, void *stream)
 {
     if (n < 1 || n > 65535) return GM_ERR_BAD_SHAPE;
     if (!a || !piv || !status) return GM_ERR_BAD_PTR;
-    k_lu_factor<<<1, 1024, 0, as_stream(stream)>>>(n, a, piv, status);
+    cudaStream_t s = as_stream(stream);
+    const int w = lu_panel_width(n);
+    if (w == 0) {   // panels in global memory
+        cudaError_t e = cudaMemsetAsync(status, 0, sizeof(int32_t), s);
+        if (e != cudaSuccess) {
+            set_error("gm_lu_factor memset", e);
+            return GM_ERR_LAUNCH;
+        }
+        for (int64_t k0 = 0; k0 < n; k0 += kLuTile) {
+            const int64_t k1 = k0 + kLuTile < n ? k0 + kLuTile : n;
+            int st = gm_lu_panel(n, a, k0, k1, piv, status, stream);
+            if (st == GM_OK && k1 < n) st = gm_lu_trsm(n, a, k0, k1, stream);
+            if (st == GM_OK && k1 < n) st = gm_lu_update(n, a, k0, k1, stream);
+            if (st != GM_OK) return st;
+        }
+        return GM_OK;
+    }
+    const size_t smem = (size_t)w * (n | 1) * sizeof(double);
+    cudaError_t e = cudaFuncSetAttribute(k_lu_panel_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) {
+        set_error("gm_lu_factor attr", e);
+        return GM_ERR_LAUNCH;
+    }
+    for (int64_t k0 = 0; k0 < n; k0 += w) {
+        const int kb = (int)(n - k0 < w ? n - k0 : w);
+        const int64_t rows = n - k0, k1 = k0 + kb;
+        const int threads = rows >= 1024 ? 1024 : (int)((rows + 31) / 32 * 32);
+        k_lu_panel_smem<<<1, threads, smem, s>>>((int)n, (int)k0, kb, a, piv, status);
+        if (n > kb) k_lu_rest<<<(unsigned)((n - kb + 127) / 128), 128, 0, s>>>((int)n, (int)k0, kb, a, piv);
+        if (k1 < n) {
+            const int st = gm_lu_update(n, a, k0, k1, stream);
+            if (st != GM_OK) return st;
+        }
+    }
     return check_launch("gm_lu_factor");
 }
 
@@ -936,4 +1196,53 @@ extern "C" int gm_lu_solve(int64_t n, const double *lu, const int32_t *piv, int6
     k_lu_solve<<<(unsigned)((nrhs + warps_per - 1) / warps_per), (unsigned)threads, 0,
                  as_stream(stream)>>>(n, lu, piv, nrhs, b);
     return check_launch("gm_lu_solve");
+}
+
+extern "C" int64_t gm_lu_prepared_bytes(int64_t n)
+{
+    if (n < 1) return 0;
+    const int64_t nblk = (n + kLuSB - 1) / kLuSB;
+    return nblk * (2 * kLuSB * kLuSB * (int64_t)sizeof(double) + kLuSB * (int64_t)sizeof(int32_t));
+}
+
+// The columns of b in shared memory: 4 per CTA up to this many rows.
+constexpr int64_t kLuPreparedMax = 200 * 1024 / (4 * 8);
+
+extern "C" int gm_lu_prepare(int64_t n, const double *lu, const int32_t *piv, void *work, void *stream)
+{
+    if (n < 1 || n > kLuPreparedMax) return GM_ERR_BAD_SHAPE;
+    if (!lu || !piv || !work) return GM_ERR_BAD_PTR;
+    const int64_t nblk = (n + kLuSB - 1) / kLuSB;
+    double *inv = (double *)work;
+    int32_t *perm = (int32_t *)(inv + nblk * 2 * kLuSB * kLuSB);
+    const size_t smem = 2 * (size_t)n * sizeof(int32_t);
+    cudaError_t e = cudaFuncSetAttribute(k_lu_prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) {
+        set_error("gm_lu_prepare attr", e);
+        return GM_ERR_LAUNCH;
+    }
+    k_lu_prepare<<<(unsigned)(1 + nblk), 64, smem, as_stream(stream)>>>((int)n, lu, piv, perm, inv);
+    return check_launch("gm_lu_prepare");
+}
+
+extern "C" int gm_lu_solve_prepared(int64_t n, const double *lu, const void *work, int64_t nrhs, const double *b,
+                                    double *x, void *stream)
+{
+    if (n < 1 || n > kLuPreparedMax || nrhs < 1) return GM_ERR_BAD_SHAPE;
+    if (!lu || !work || !b || !x || b == x) return GM_ERR_BAD_PTR;
+    const int64_t nblk = (n + kLuSB - 1) / kLuSB;
+    const double *inv = (const double *)work;
+    const int32_t *perm = (const int32_t *)(inv + nblk * 2 * kLuSB * kLuSB);
+    // four columns a CTA share every row of the factors; few columns spread over more CTAs
+    const bool wide = nrhs > 2 * 148;
+    auto kern = wide ? k_lu_solve_prepared<4> : k_lu_solve_prepared<1>;
+    const int cb = wide ? 4 : 1;
+    const size_t smem = (size_t)nblk * kLuSB * cb * sizeof(double);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) {
+        set_error("gm_lu_solve_prepared attr", e);
+        return GM_ERR_LAUNCH;
+    }
+    kern<<<(unsigned)((nrhs + cb - 1) / cb), 1024, smem, as_stream(stream)>>>((int)n, lu, perm, inv, nrhs, b, x);
+    return check_launch("gm_lu_solve_prepared");
 }

@@ -229,28 +229,22 @@ def _slots(ncls):
 class LUFactor:
     """FP64 LU factorisation with partial pivoting of a square device matrix."""
 
-    # matrices above this order are factored in panels of _PANEL columns (the trailing
-    # updates by the FP64 tile kernel gm_lu_update); smaller ones in one single-CTA kernel
-    _BLOCKED_FROM = 256
-    _PANEL = 64
+    # matrices up to this order are solved with prepared factors (one permutation, inverted
+    # diagonal blocks; the right-hand sides held in shared memory), larger ones from the factors
+    _PREPARED_MAX = 6400
 
     def __init__(self, a):
         self.n = a.shape[0]
         self.lu = a.contiguous().clone()
         self.piv = torch.empty(self.n, dtype=torch.int32, device=a.device)
         self.status = torch.zeros(1, dtype=torch.int32, device=a.device)
+        self._prepared = None
         st = _lib.stream_handle(a.device)
-        if self.n <= self._BLOCKED_FROM:
-            _lib.call("gm_lu_factor", self.n, _lib.ptr(self.lu), _lib.ptr(self.piv),
-                      _lib.ptr(self.status), st)
-            return
-        n, A = self.n, self.lu
-        for k0 in range(0, n, self._PANEL):
-            k1 = min(n, k0 + self._PANEL)
-            _lib.call("gm_lu_panel", n, _lib.ptr(A), k0, k1, _lib.ptr(self.piv), _lib.ptr(self.status), st)
-            if k1 < n:
-                _lib.call("gm_lu_trsm", n, _lib.ptr(A), k0, k1, st)
-                _lib.call("gm_lu_update", n, _lib.ptr(A), k0, k1, st)
+        _lib.call("gm_lu_factor", self.n, _lib.ptr(self.lu), _lib.ptr(self.piv), _lib.ptr(self.status), st)
+        if self.n <= self._PREPARED_MAX:
+            self._prepared = torch.empty(int(_lib.load().gm_lu_prepared_bytes(self.n)), dtype=torch.uint8,
+                                         device=a.device)
+            _lib.call("gm_lu_prepare", self.n, _lib.ptr(self.lu), _lib.ptr(self.piv), _lib.ptr(self._prepared), st)
 
     def check(self):
         st = int(self.status.item())
@@ -259,6 +253,13 @@ class LUFactor:
 
     def solve(self, b):
         """Solve A x = b for b of shape (n,) or (n, nrhs)."""
+        if self._prepared is not None:
+            b = b.contiguous()
+            x = torch.empty_like(b)
+            nrhs = 1 if b.ndim == 1 else b.shape[1]
+            _lib.call("gm_lu_solve_prepared", self.n, _lib.ptr(self.lu), _lib.ptr(self._prepared), nrhs, _lib.ptr(b),
+                      _lib.ptr(x), _lib.stream_handle(b.device))
+            return x
         x = b.contiguous().clone()
         nrhs = 1 if x.ndim == 1 else x.shape[1]
         _lib.call("gm_lu_solve", self.n, _lib.ptr(self.lu), _lib.ptr(self.piv), nrhs, _lib.ptr(x),

@@ -242,8 +242,9 @@ int gm_bin_cells_csr(int64_t lmax, int64_t nbands, int64_t ncls, const double *c
  * jnp.linalg.solve, workspaces.py:2146).  piv: n int32.  status: one int32 set to
  * 0 on success or k+1 when the k-th pivot is exactly zero. */
 int gm_lu_factor(int64_t n, double *a, int32_t *piv, int32_t *status, void *stream);
-/* Blocked form of gm_lu_factor (same factors, pivots and status; the caller zeroes
- * `status`): for each panel [k0, k1): gm_lu_panel (pivoting and factoring the panel's
+/* The steps of a blocked factorisation with panels in global memory, which gm_lu_factor takes
+ * where no panel of four columns fits shared memory (same factors, pivots and status; the
+ * caller zeroes `status`): for each panel [k0, k1): gm_lu_panel (pivoting and factoring the panel's
  * columns, whole-row swaps), gm_lu_trsm (the U rows right of the panel), then
  * gm_lu_update (A[k1:, k1:] -= A[k1:, k0:k1] A[k0:k1, k1:]).  Replaces the reference's
  * jnp.linalg.solve factorisation (workspaces.py:2146) for large binned matrices. */
@@ -255,6 +256,13 @@ int gm_lu_trsm(int64_t n, double *a, int64_t k0, int64_t k1, void *stream);
 int gm_lu_update(int64_t n, double *a, int64_t k0, int64_t k1, void *stream);
 int gm_lu_solve(int64_t n, const double *lu, const int32_t *piv, int64_t nrhs,
                 double *b, void *stream);
+/* Solves with prepared factors, n <= 6400.  work (gm_lu_prepared_bytes) receives the row
+ * interchanges as one permutation and the inverses of the 32 x 32 diagonal blocks of L and U;
+ * gm_lu_solve_prepared then writes x = A^-1 b, both (n, nrhs) row-major, x not b. */
+int64_t gm_lu_prepared_bytes(int64_t n);
+int gm_lu_prepare(int64_t n, const double *lu, const int32_t *piv, void *work, void *stream);
+int gm_lu_solve_prepared(int64_t n, const double *lu, const void *work, int64_t nrhs,
+                         const double *b, double *x, void *stream);
 
 /* ----------------------------------------------- batched tensor-core Legendre stage */
 
