@@ -100,6 +100,8 @@ SIGNATURES = {
     "gm_mask_ring_runs": ([_c_i64, _c_vp, _c_vp, _c_vp, _c_vp], _c_int),
     "gm_cov_binned": ([_c_i64, _c_i64, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_i64, _c_vp, _c_vp, _c_vp,
                        _c_i64, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp], _c_int),
+    "gm_cov_bands": ([_c_i64, _c_i64, _c_i64, _c_vp, _c_i64, _c_vp, _c_vp, _c_vp, _c_vp, _c_i64, _c_vp, _c_vp,
+                      _c_vp, _c_i64, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp], _c_int),
     "gm_cov_coupled": ([_c_i64, _c_i64, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp], _c_int),
     "gm_gl_nodes": ([_c_i64, _c_vp, _c_vp, _c_vp], _c_int),
     "gm_wigner_table": ([_c_i64, _c_vp, _c_i64, _c_int, _c_int, _c_vp, _c_vp, _c_vp], _c_int),
@@ -195,6 +197,13 @@ def ptr(t):
     if not t.is_cuda:
         raise ValueError("gmaster_b200 kernels take CUDA tensors")
     return ctypes.c_void_p(t.data_ptr())
+
+
+def ptr_array(tensors):
+    """Host array of the raw device pointers of CUDA tensors."""
+    if not all(t.is_cuda for t in tensors):
+        raise ValueError("gmaster_b200 kernels take CUDA tensors")
+    return (ctypes.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
 
 
 def stream_handle(device=None):

@@ -4,7 +4,7 @@
 (NaMaster's; gmaster/covariance.py:197-406): the coupling blocks of the power spectra of
 the mask products, from the same FP64 3j kernel as the mode-coupling matrices, divided
 by 2 l' + 1.  `gaussian_covariance` evaluates the signed sums of (C C + C C) / 2 * Xi
-terms of every output block and bins both sides in one CUDA kernel (`gm_cov_binned`),
+terms of every output block and bins both sides in one CUDA kernel (`gm_cov_bands`),
 then decouples with the LU factors of the two workspaces (covariance.py:479-575).
 `get_iNKA_cell` gives the improved-NKA input spectra (covariance.py:970-1024).
 
@@ -12,6 +12,7 @@ Map-based spin-0 and spin-2 fields only: the catalog shot-noise terms and the fl
 variant of the reference are outside this build.
 """
 
+import ctypes
 import itertools
 
 import numpy as np
@@ -243,14 +244,14 @@ class NmtCovarianceWorkspace:
         kernels, rows, signs, bptr = self._terms()
         nblocks = len(bptr) - 1
         st = _lib.stream_handle(dev)
-        if kernels:
-            xi = torch.stack(kernels).contiguous()
-        else:
-            xi = torch.zeros((1, L, L), dtype=torch.float64, device=dev)
-        terms = torch.tensor(rows if rows else [(0, 0, 0)], dtype=torch.int32).to(dev)
-        sg = torch.tensor(signs if signs else [0.0], dtype=torch.float64).to(dev)
-        bp = torch.tensor(bptr, dtype=torch.int32).to(dev)
         if coupled:
+            if kernels:
+                xi = torch.stack(kernels).contiguous()
+            else:
+                xi = torch.zeros((1, L, L), dtype=torch.float64, device=dev)
+            terms = torch.tensor(rows if rows else [(0, 0, 0)], dtype=torch.int32).to(dev)
+            sg = torch.tensor(signs if signs else [0.0], dtype=torch.float64).to(dev)
+            bp = torch.tensor(bptr, dtype=torch.int32).to(dev)
             out = torch.empty((nblocks, L, L), dtype=torch.float64, device=dev)
             _lib.call("gm_cov_coupled", self.lmax, nblocks, _lib.ptr(xi), _lib.ptr(spec),
                       _lib.ptr(terms), _lib.ptr(sg), _lib.ptr(bp), _lib.ptr(out), st)
@@ -259,11 +260,20 @@ class NmtCovarianceWorkspace:
             opa = wa.bins.device_operators(dev)
             opb = wb.bins.device_operators(dev)
             nx, ny = wa.nbands, wb.nbands
+            # contractions that share a kernel tensor (one mask) read it once
+            xi, where = [], {}
+            for k in kernels:
+                where.setdefault(k.data_ptr(), len(where))
+                if len(where) > len(xi):
+                    xi.append(k.contiguous())
+            index = [where[k.data_ptr()] for k in kernels]
+            table = np.array([(index[k], ra, rb) for k, ra, rb in rows], dtype=np.int32).reshape(-1, 3)
+            sg, bp = np.array(signs, dtype=np.float64), np.array(bptr, dtype=np.int32)
+            host = [np.ascontiguousarray(x).ctypes.data_as(ctypes.c_void_p) for x in (table, sg, bp)]
             out = torch.empty((nblocks, nx, ny), dtype=torch.float64, device=dev)
-            _lib.call("gm_cov_binned", self.lmax, nblocks, _lib.ptr(xi), _lib.ptr(spec),
-                      _lib.ptr(terms), _lib.ptr(sg), _lib.ptr(bp), nx, _lib.ptr(opa["ptr"]),
-                      _lib.ptr(opa["ells"]), _lib.ptr(opa["wfl"]), ny, _lib.ptr(opb["ptr"]),
-                      _lib.ptr(opb["ells"]), _lib.ptr(opb["wfl"]), _lib.ptr(out), st)
+            _lib.call("gm_cov_bands", self.lmax, nblocks, len(xi), _lib.ptr_array(xi), spec.shape[0], _lib.ptr(spec),
+                      *host, nx, _lib.ptr(opa["ptr"]), _lib.ptr(opa["ells"]), _lib.ptr(opa["wfl"]), ny,
+                      _lib.ptr(opb["ptr"]), _lib.ptr(opb["ells"]), _lib.ptr(opb["wfl"]), _lib.ptr(out), st)
         cov = out.view(self.nclsa, self.nclsb, nx, ny).permute(2, 0, 3, 1)
         cov = cov.reshape(nx * self.nclsa, ny * self.nclsb)
         if coupled:

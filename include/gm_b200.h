@@ -493,6 +493,16 @@ int gm_cov_binned(int64_t lmax, int64_t nblocks, const double *xi, const double 
                   int64_t nbands_a, const int32_t *ptr_a, const int32_t *ells_a,
                   const double *w_a, int64_t nbands_b, const int32_t *ptr_b,
                   const int32_t *ells_b, const double *w_b, double *out, void *stream);
+
+/* gm_cov_binned with the term table on the host: terms, signs (+1 or -1), block_ptr (at most 512
+ * terms) and xi (nk <= 8 device pointers to (L, L) kernels) are host arrays, spec has nrows <= 16
+ * rows.  The indices are checked. */
+int gm_cov_bands(int64_t lmax, int64_t nblocks, int64_t nk, const double *const *xi, int64_t nrows,
+                 const double *spec, const int32_t *terms, const double *signs,
+                 const int32_t *block_ptr, int64_t nbands_a, const int32_t *ptr_a,
+                 const int32_t *ells_a, const double *w_a, int64_t nbands_b,
+                 const int32_t *ptr_b, const int32_t *ells_b, const double *w_b, double *out,
+                 void *stream);
 int gm_cov_coupled(int64_t lmax, int64_t nblocks, const double *xi, const double *spec,
                    const int32_t *terms, const double *signs, const int32_t *block_ptr,
                    double *out, void *stream);
