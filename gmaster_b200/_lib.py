@@ -38,6 +38,9 @@ SIGNATURES = {
     "gm_legendre_synthesis": ([_c_int, _c_int, _c_i64, _c_i64, _c_i64, _c_vp, _c_vp, _c_vp, _c_vp,
                                _c_vp], _c_int),
     "gm_pseudo_cl": ([_c_i64, _c_i64, _c_vp, _c_i64, _c_vp, _c_vp, _c_vp], _c_int),
+    "gm_pseudo_cl_pairs": ([_c_i64, _c_i64, _c_i64, _c_vp, _c_i64, _c_vp, _c_vp, _c_vp], _c_int),
+    "gm_decouple_cells": ([_c_i64, _c_i64, _c_i64, _c_vp, _c_i64, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp,
+                           _c_vp], _c_int),
     "gm_coupling_blocks": ([_c_i64, _c_vp, _c_i64, _c_int, _c_vp, _c_vp, _c_vp], _c_int),
     "gm_coupling_units": ([_c_i64], _c_i64),
     "gm_coupling_blocks_multi": ([_c_i64, _c_vp, _c_i64, _c_vp, _c_vp, _c_vp, _c_vp], _c_int),

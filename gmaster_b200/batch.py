@@ -32,7 +32,7 @@ from ._config import get_precision, nmt_params
 from .field import NmtField
 from .utils import as_device
 from .workspaces import (NmtWorkspace, _which, compute_coupled_cell, coupling_blocks_multi,
-                         pseudo_cl)
+                         pseudo_cl, pseudo_cl_pairs)
 
 
 def fields_from_maps(mask, maps, *, spin=None, n_iter=None, beam=None, lmax=None,
@@ -104,7 +104,22 @@ def compute_coupled_cells(fields1, fields2):
     """Coupled pseudo-C_ell of each pair (fields1[i], fields2[i])."""
     if len(fields1) != len(fields2):
         raise ValueError("the two field lists must have the same length")
-    return [compute_coupled_cell(a, b) for a, b in zip(fields1, fields2)]
+    out = [None] * len(fields1)
+    groups = {}   # pairs of equal lmax and shapes share a launch
+    for i, (a, b) in enumerate(zip(fields1, fields2)):
+        if not a.is_compatible(b, strict=False):
+            raise ValueError("You're trying to correlate incompatible fields")
+        x, y = a.get_alms(), b.get_alms()
+        lmax = min(a.ainfo.lmax, b.ainfo.lmax)
+        if x.ndim != 2 or y.ndim != 2 or x.device != y.device:
+            out[i] = compute_coupled_cell(a, b)
+            continue
+        groups.setdefault((lmax, x.shape, y.shape, x.device), []).append((i, x, y))
+    for (lmax, *_), items in groups.items():
+        cls = pseudo_cl_pairs([x for _, x, _ in items], [y for _, _, y in items], lmax)
+        for (i, _, _), c in zip(items, cls):
+            out[i] = c
+    return out
 
 
 def decouple_cells(workspace, cls, cl_bias=None, cl_noise=None):
@@ -122,7 +137,8 @@ def decouple_cells(workspace, cls, cl_bias=None, cl_noise=None):
         if c.ndim != 2 or c.shape[0] != w.ncls or c.shape[1] < w.lmax + 1:
             raise ValueError(f"Input power spectrum has wrong shape. Expected "
                              f"({w.ncls}, {w.lmax + 1}), but got {tuple(c.shape)}")
-        c = c[:, : w.lmax + 1]
+        if cl_bias is not None or cl_noise is not None:
+            c = c[:, : w.lmax + 1]
         for name, bias in (("bias", cl_bias), ("noise", cl_noise)):
             if bias is not None:
                 bias = as_device(bias, torch.float64)
@@ -130,14 +146,16 @@ def decouple_cells(workspace, cls, cl_bias=None, cl_noise=None):
                     raise ValueError(f"Input {name} power spectrum has wrong shape")
                 c = c - bias[:, : w.lmax + 1]
         stack.append(c)
-    allcl = torch.cat(stack).contiguous()                      # (nsims ncls, L)
-    binned = w.bins.bin_cell(allcl)                            # (nsims ncls, nb)
-    nb = binned.shape[1]
-    rhs = binned.reshape(len(cls), w.ncls, nb).permute(2, 1, 0).reshape(nb * w.ncls, len(cls))
     w._lu.check()
     # every simulation is one right-hand side of the LU solve (the factors of the binned
-    # coupling matrix, as decouple_cell uses them), all in one launch
-    sol = w._lu.solve(rhs)                                     # (nb ncls, nsims)
+    # coupling matrix, as decouple_cell uses them), all in one launch with the binning
+    nb = w.nbands
+    sol = None
+    if w.bins.lmax == w.lmax and len({c.shape for c in stack}) == 1 and len({c.device for c in stack}) == 1:
+        sol = w._lu.decouple([c.contiguous() for c in stack], w.bins)
+    if sol is None:
+        binned = w.bins.bin_cell(torch.cat([c[:, : w.lmax + 1] for c in stack]).contiguous())   # (nsims ncls, nb)
+        sol = w._lu.solve(binned.reshape(len(cls), w.ncls, nb).permute(2, 1, 0).reshape(nb * w.ncls, len(cls)))
     out = sol.reshape(nb, w.ncls, len(cls)).permute(2, 1, 0)
     return [out[i] for i in range(len(cls))]
 

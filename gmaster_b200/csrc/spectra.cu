@@ -20,40 +20,61 @@ __device__ __forceinline__ int64_t alm_idx(int64_t lmax, int64_t l, int64_t m)
 
 // ---------------------------------------------------------------- pseudo-C_ell
 
-constexpr int kPclLanes = 32;   // degrees per CTA (one per lane: coalesced over l)
-constexpr int kPclWarps = 8;    // orders interleaved over the warps of a CTA
+constexpr int kPclLanes = 32;    // degrees per CTA (one per lane: coalesced over l)
+constexpr int kPclWarps = 32;    // orders interleaved over the warps of a CTA
+constexpr int kPclPairs = 64;    // field pairs of one launch
 
-// grid (l-blocks of 32, pairs), 256 threads: lane = degree l, warp w sums the orders
-// m = w, w + 8, ... <= l; the eight partial sums are then added in a fixed order, so the
-// result does not depend on scheduling (equal inputs give bit-equal spectra).
-__global__ void __launch_bounds__(kPclLanes * kPclWarps) k_pseudo_cl(int64_t lmax, int64_t n1,
-                                                                     const double2 *__restrict__ a, int64_t n2,
-                                                                     const double2 *__restrict__ b,
-                                                                     double *__restrict__ cls)
+// Field pairs of a launch: pair p has the alms a (N1 rows of nelem) and b (N2 rows), spectra out
+// (N1 N2 rows of L).
+struct PclPairs {
+    const double2 *a[kPclPairs], *b[kPclPairs];
+    double *out[kPclPairs];
+};
+
+// grid (l-blocks of 32, pairs), 1024 threads: lane = degree l, warp w sums the orders m = w,
+// w + 32, ... <= l of every component product (each alm read once); the partial sums are then
+// added in a fixed order, so the result does not depend on scheduling (equal inputs give
+// bit-equal spectra).  Bound by the latency of the order loop at small lmax and by memory at
+// large: 32 warps keep it at lmax / 32 steps, and a batch of pairs is one launch.  32 pairs of
+// (E, B) at lmax 767: 74 us (4.1 TB/s); 911 us in 32 launches of eight warps and one product a CTA.
+template <int N1, int N2>
+__global__ void __launch_bounds__(kPclLanes * kPclWarps) k_pseudo_cl(int64_t lmax, const __grid_constant__ PclPairs p)
 {
-    __shared__ double part[kPclWarps][kPclLanes];
+    __shared__ double part[N1 * N2][kPclWarps][kPclLanes];
     const int64_t L = lmax + 1, nelem = L * (L + 1) / 2;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t l = (int64_t)blockIdx.x * kPclLanes + lane;
-    const int64_t pair = blockIdx.y, i = pair / n2, j = pair % n2;
-    const double2 *ai = a + i * nelem;
-    const double2 *bj = b + j * nelem;
-    double s = 0.0;
+    const double2 *a = p.a[blockIdx.y], *b = p.b[blockIdx.y];
+    const bool same = N1 == N2 && a == b;
+    double s[N1 * N2];
+#pragma unroll
+    for (int q = 0; q < N1 * N2; ++q) s[q] = 0.0;
     if (l < L) {
+#pragma unroll 4
         for (int64_t m = w; m <= l; m += kPclWarps) {
             const int64_t k = alm_idx(lmax, l, m);
-            const double2 x = ai[k], y = bj[k];
-            const double re = x.x * y.x + x.y * y.y;
-            s += m == 0 ? re : 2.0 * re;
+            double2 x[N1], y[N2];
+#pragma unroll
+            for (int i = 0; i < N1; ++i) x[i] = a[i * nelem + k];
+#pragma unroll
+            for (int j = 0; j < N2; ++j) y[j] = same ? x[j % N1] : b[j * nelem + k];
+#pragma unroll
+            for (int i = 0; i < N1; ++i)
+#pragma unroll
+                for (int j = 0; j < N2; ++j) {
+                    const double re = x[i].x * y[j].x + x[i].y * y[j].y;
+                    s[i * N2 + j] += m == 0 ? re : 2.0 * re;
+                }
         }
     }
-    part[w][lane] = s;
+#pragma unroll
+    for (int q = 0; q < N1 * N2; ++q) part[q][w][lane] = s[q];
     __syncthreads();
-    if (w == 0 && l < L) {
+    if (w < N1 * N2 && l < L) {
         double t = 0.0;
 #pragma unroll
-        for (int q = 0; q < kPclWarps; ++q) t += part[q][lane];
-        cls[pair * L + l] = t / (2.0 * (double)l + 1.0);
+        for (int q = 0; q < kPclWarps; ++q) t += part[w][q][lane];
+        p.out[blockIdx.y][w * L + l] = t / (2.0 * (double)l + 1.0);
     }
 }
 
@@ -909,11 +930,11 @@ __global__ void __launch_bounds__(64) k_lu_prepare(int n, const double *__restri
 // steps (two barriers, a row read and two reductions each); with the interchanges applied one by
 // one and 32-step substitutions inside a block a solve of n = 92 took 42 us, of 612 438
 // us; here 6.8 and 77 us.
-template <int CB>
-__global__ void __launch_bounds__(1024) k_lu_solve_prepared(int n, const double *__restrict__ lu,
-                                                            const int32_t *__restrict__ perm,
-                                                            const double *__restrict__ inv, int64_t nrhs,
-                                                            const double *__restrict__ b, double *__restrict__ x)
+// load(row, column): entry of b.
+template <int CB, class Load>
+__device__ __forceinline__ void lu_solve_columns(int n, const double *__restrict__ lu,
+                                                 const int32_t *__restrict__ perm, const double *__restrict__ inv,
+                                                 int64_t nrhs, Load load, double *__restrict__ x)
 {
     extern __shared__ double xs[];   // [n rounded up to 32][CB]
     __shared__ double part[kLuSB][CB];
@@ -923,7 +944,7 @@ __global__ void __launch_bounds__(1024) k_lu_solve_prepared(int n, const double 
     const int nblk = (n + kLuSB - 1) / kLuSB;
     for (int i = tid; i < nblk * kLuSB * CB; i += blockDim.x) {
         const int row = i / CB, c = i % CB;
-        xs[i] = row < n && c < ncol ? b[(int64_t)perm[row] * nrhs + c0 + c] : 0.0;
+        xs[i] = row < n && c < ncol ? load(perm[row], c0 + c) : 0.0;
     }
     __syncthreads();
     auto step = [&](int blk, int jbeg, int jend, int upper) {
@@ -966,21 +987,89 @@ __global__ void __launch_bounds__(1024) k_lu_solve_prepared(int n, const double 
     }
 }
 
+template <int CB>
+__global__ void __launch_bounds__(1024) k_lu_solve_prepared(int n, const double *__restrict__ lu,
+                                                            const int32_t *__restrict__ perm,
+                                                            const double *__restrict__ inv, int64_t nrhs,
+                                                            const double *__restrict__ b, double *__restrict__ x)
+{
+    lu_solve_columns<CB>(n, lu, perm, inv, nrhs,
+                         [&](int row, int64_t c) { return b[(int64_t)row * nrhs + c]; }, x);
+}
+
+// Binning and decoupling of many spectra in one launch: right-hand side c is the binned cell c,
+// rows band-major with the ncls spectra of a band adjacent (k_bin_cells' sums, entry by entry as
+// they are needed).  Cell c: ncls rows of stride ld.
+constexpr int kDecoupleCells = 256;
+struct Cells {
+    const double *c[kDecoupleCells];
+};
+template <int CB>
+__global__ void __launch_bounds__(1024) k_decouple(int n, int ncls, int64_t ld, const __grid_constant__ Cells cells,
+                                                   const int32_t *__restrict__ band_ptr,
+                                                   const int32_t *__restrict__ band_ells,
+                                                   const double *__restrict__ wfl, const double *__restrict__ lu,
+                                                   const int32_t *__restrict__ perm, const double *__restrict__ inv,
+                                                   int64_t nrhs, double *__restrict__ x)
+{
+    lu_solve_columns<CB>(n, lu, perm, inv, nrhs,
+                         [&](int row, int64_t c) {
+                             const int b = row / ncls, q = row - b * ncls;
+                             const double *src = cells.c[c] + q * ld;
+                             double s = 0.0;
+#pragma unroll 4
+                             for (int i = band_ptr[b]; i < band_ptr[b + 1]; ++i) {
+                                 const int l = band_ells[i];
+                                 s += wfl[l] * src[l];
+                             }
+                             return s;
+                         },
+                         x);
+}
+
 }  // namespace gm
 
 using namespace gm;
 
+extern "C" int gm_pseudo_cl_pairs(int64_t lmax, int64_t npairs, int64_t n1, const double *const *alm1, int64_t n2,
+                                  const double *const *alm2, double *const *cls, void *stream)
+{
+    if (lmax < 0 || npairs < 1 || n1 < 1 || n2 < 1 || n1 * n2 > 65535) return GM_ERR_BAD_SHAPE;
+    if (!alm1 || !alm2 || !cls) return GM_ERR_BAD_PTR;
+    for (int64_t i = 0; i < npairs; ++i)
+        if (!alm1[i] || !alm2[i] || !cls[i]) return GM_ERR_BAD_PTR;
+    const int64_t L = lmax + 1, nelem = L * (L + 1) / 2;
+    cudaStream_t s = as_stream(stream);
+    // fields of one or two components run all their products together; more components as
+    // pairs of single rows
+    const bool whole = n1 <= 2 && n2 <= 2;
+    const int64_t per = whole ? 1 : n1 * n2, total = npairs * per;
+    for (int64_t i0 = 0; i0 < total; i0 += kPclPairs) {
+        const int64_t cnt = total - i0 < kPclPairs ? total - i0 : kPclPairs;
+        PclPairs p;
+        for (int64_t i = 0; i < cnt; ++i) {
+            const int64_t f = (i0 + i) / per, q = (i0 + i) % per;
+            p.a[i] = (const double2 *)alm1[f] + (whole ? 0 : q / n2) * nelem;
+            p.b[i] = (const double2 *)alm2[f] + (whole ? 0 : q % n2) * nelem;
+            p.out[i] = cls[f] + q * L;
+        }
+        const dim3 grid((unsigned)((L + kPclLanes - 1) / kPclLanes), (unsigned)cnt);
+        const int threads = kPclLanes * kPclWarps;
+        if (!whole || (n1 == 1 && n2 == 1)) k_pseudo_cl<1, 1><<<grid, threads, 0, s>>>(lmax, p);
+        else if (n1 == 1) k_pseudo_cl<1, 2><<<grid, threads, 0, s>>>(lmax, p);
+        else if (n2 == 1) k_pseudo_cl<2, 1><<<grid, threads, 0, s>>>(lmax, p);
+        else k_pseudo_cl<2, 2><<<grid, threads, 0, s>>>(lmax, p);
+        const int st = check_launch("gm_pseudo_cl");
+        if (st != GM_OK) return st;
+    }
+    return GM_OK;
+}
+
 extern "C" int gm_pseudo_cl(int64_t lmax, int64_t n1, const double *alm1, int64_t n2,
                             const double *alm2, double *cls, void *stream)
 {
-    if (lmax < 0 || n1 < 1 || n2 < 1 || n1 * n2 > 65535) return GM_ERR_BAD_SHAPE;
-    if (!alm1 || !alm2 || !cls) return GM_ERR_BAD_PTR;
-    const int64_t L = lmax + 1;
-    cudaStream_t s = as_stream(stream);
-    dim3 grid((unsigned)((L + kPclLanes - 1) / kPclLanes), (unsigned)(n1 * n2));
-    k_pseudo_cl<<<grid, kPclLanes * kPclWarps, 0, s>>>(lmax, n1, (const double2 *)alm1, n2,
-                                                       (const double2 *)alm2, cls);
-    return check_launch("gm_pseudo_cl");
+    if (!alm1 || !alm2 || !cls) return lmax < 0 || n1 < 1 || n2 < 1 || n1 * n2 > 65535 ? GM_ERR_BAD_SHAPE : GM_ERR_BAD_PTR;
+    return gm_pseudo_cl_pairs(lmax, 1, n1, &alm1, n2, &alm2, &cls, stream);
 }
 
 extern "C" int gm_coupling_blocks(int64_t lmax, const double *window, int64_t nw, int which,
@@ -1245,4 +1334,34 @@ extern "C" int gm_lu_solve_prepared(int64_t n, const double *lu, const void *wor
     }
     kern<<<(unsigned)((nrhs + cb - 1) / cb), 1024, smem, as_stream(stream)>>>((int)n, lu, perm, inv, nrhs, b, x);
     return check_launch("gm_lu_solve_prepared");
+}
+
+extern "C" int gm_decouple_cells(int64_t nbands, int64_t ncls, int64_t ncells, const double *const *cells, int64_t ld,
+                                 const int32_t *band_ptr, const int32_t *band_ells, const double *wfl,
+                                 const double *lu, const void *work, double *x, void *stream)
+{
+    const int64_t n = nbands * ncls;
+    if (nbands < 1 || ncls < 1 || n > kLuPreparedMax || ncells < 1 || ncells > kDecoupleCells || ld < 1)
+        return GM_ERR_BAD_SHAPE;
+    if (!cells || !band_ptr || !band_ells || !wfl || !lu || !work || !x) return GM_ERR_BAD_PTR;
+    Cells c;
+    for (int64_t i = 0; i < ncells; ++i) {
+        if (!cells[i]) return GM_ERR_BAD_PTR;
+        c.c[i] = cells[i];
+    }
+    const int64_t nblk = (n + kLuSB - 1) / kLuSB;
+    const double *inv = (const double *)work;
+    const int32_t *perm = (const int32_t *)(inv + nblk * 2 * kLuSB * kLuSB);
+    const bool wide = ncells > 148;   // four columns share the rows of the factors
+    auto kern = wide ? k_decouple<4> : k_decouple<1>;
+    const int cb = wide ? 4 : 1;
+    const size_t smem = (size_t)nblk * kLuSB * cb * sizeof(double);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) {
+        set_error("gm_decouple_cells attr", e);
+        return GM_ERR_LAUNCH;
+    }
+    kern<<<(unsigned)((ncells + cb - 1) / cb), 1024, smem, as_stream(stream)>>>(
+        (int)n, (int)ncls, ld, c, band_ptr, band_ells, wfl, lu, perm, inv, ncells, x);
+    return check_launch("gm_decouple_cells");
 }

@@ -28,6 +28,19 @@ def pseudo_cl(alm1, alm2, lmax):
     return out
 
 
+def pseudo_cl_pairs(alms1, alms2, lmax):
+    """`pseudo_cl` of every pair (alms1[i], alms2[i]) of equal shapes in one launch: a list of
+    (n1 n2, lmax+1) views of one tensor."""
+    a = [x.contiguous() for x in alms1]
+    b = [y if y is x else y.contiguous() for x, y in zip(a, alms2)]
+    n1, n2, dev = a[0].shape[0], b[0].shape[0], a[0].device
+    out = torch.empty((len(a), n1 * n2, lmax + 1), dtype=torch.float64, device=dev)
+    cls = list(out.unbind(0))
+    _lib.call("gm_pseudo_cl_pairs", lmax, len(a), n1, _lib.ptr_array(a), n2, _lib.ptr_array(b), _lib.ptr_array(cls),
+              _lib.stream_handle(dev))
+    return cls
+
+
 def compute_coupled_cell(f1, f2):
     """Coupled pseudo-C_ell of two fields: (n1 n2, lmax+1) (workspaces.py:98-125)."""
     if not f1.is_compatible(f2, strict=False):
@@ -239,6 +252,7 @@ class LUFactor:
         self.piv = torch.empty(self.n, dtype=torch.int32, device=a.device)
         self.status = torch.zeros(1, dtype=torch.int32, device=a.device)
         self._prepared = None
+        self._regular = False   # set once `check` has read the status of this factorisation
         st = _lib.stream_handle(a.device)
         _lib.call("gm_lu_factor", self.n, _lib.ptr(self.lu), _lib.ptr(self.piv), _lib.ptr(self.status), st)
         if self.n <= self._PREPARED_MAX:
@@ -247,9 +261,34 @@ class LUFactor:
             _lib.call("gm_lu_prepare", self.n, _lib.ptr(self.lu), _lib.ptr(self.piv), _lib.ptr(self._prepared), st)
 
     def check(self):
+        if self._regular:
+            return
         st = int(self.status.item())
         if st:
             raise np.linalg.LinAlgError(f"binned coupling matrix is singular (pivot {st - 1})")
+        self._regular = True
+
+    # cells of one launch of `decouple`
+    _CELLS = 256
+
+    def decouple(self, cells, bins):
+        """A^-1 of the binned `cells` (contiguous (ncls, >= lmax+1) float64 device tensors of one
+        shape) in one launch: (n, len(cells)), rows band-major with a band's spectra adjacent;
+        None where the factors are not prepared."""
+        if self._prepared is None:
+            return None
+        ncls, ld = cells[0].shape
+        dev = cells[0].device
+        ops = bins.device_operators(dev)
+        out = []
+        for i in range(0, len(cells), self._CELLS):
+            part = cells[i:i + self._CELLS]
+            x = torch.empty((self.n, len(part)), dtype=torch.float64, device=dev)
+            _lib.call("gm_decouple_cells", bins.n_bands, ncls, len(part), _lib.ptr_array(part), ld, _lib.ptr(ops["ptr"]),
+                      _lib.ptr(ops["ells"]), _lib.ptr(ops["wfl"]), _lib.ptr(self.lu), _lib.ptr(self._prepared),
+                      _lib.ptr(x), _lib.stream_handle(dev))
+            out.append(x)
+        return out[0] if len(out) == 1 else torch.cat(out, 1)
 
     def solve(self, b):
         """Solve A x = b for b of shape (n,) or (n, nrhs)."""
@@ -645,17 +684,18 @@ class NmtWorkspace:
         if cl.ndim != 2 or cl.shape[0] != self.ncls or cl.shape[1] < self.lmax + 1:
             raise ValueError(f"Input power spectrum has wrong shape. Expected "
                              f"({self.ncls}, {self.lmax + 1}), but got {tuple(cl.shape)}")
-        total = cl[:, : self.lmax + 1]
+        total = cl if cl_bias is None and cl_noise is None else cl[:, : self.lmax + 1]
         for name, bias in (("bias", cl_bias), ("noise", cl_noise)):
             if bias is not None:
                 bias = as_device(bias, torch.float64)
                 if bias.ndim != 2 or bias.shape[0] != self.ncls or bias.shape[1] < self.lmax + 1:
                     raise ValueError(f"Input {name} power spectrum has wrong shape")
                 total = total - bias[:, : self.lmax + 1]
-        binned = self.bins.bin_cell(total.contiguous())
-        vec = binned.T.reshape(-1).contiguous()
         self._lu.check()
-        sol = self._lu.solve(vec)
+        sol = self._lu.decouple([total], self.bins) if self.bins.lmax == self.lmax else None
+        if sol is None:
+            binned = self.bins.bin_cell(total[:, : self.lmax + 1].contiguous())
+            sol = self._lu.solve(binned.T.reshape(-1).contiguous())
         return sol.reshape(self.nbands, self.ncls).T
 
     def _dense_operators(self, dev):

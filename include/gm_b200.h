@@ -173,6 +173,10 @@ int gm_legendre_synthesis_tile(int precision, int spin, int64_t nside, int64_t l
  * fixed order: equal inputs give bit-equal spectra. */
 int gm_pseudo_cl(int64_t lmax, int64_t n1, const double *alm1, int64_t n2,
                  const double *alm2, double *cls, void *stream);
+/* gm_pseudo_cl of npairs field pairs in one launch per 64: alm1, alm2 and cls are host arrays of
+ * npairs device pointers; bit-equal to separate calls. */
+int gm_pseudo_cl_pairs(int64_t lmax, int64_t npairs, int64_t n1, const double *const *alm1,
+                       int64_t n2, const double *const *alm2, double *const *cls, void *stream);
 
 /* Coupling blocks by the Wigner-3j three-term recursion in l3 (replaces
  * workspaces.py:352-517 `_coupling_matrix_tt` and 682-924 `_general_coupling_matrix`
@@ -263,6 +267,13 @@ int64_t gm_lu_prepared_bytes(int64_t n);
 int gm_lu_prepare(int64_t n, const double *lu, const int32_t *piv, void *work, void *stream);
 int gm_lu_solve_prepared(int64_t n, const double *lu, const void *work, int64_t nrhs,
                          const double *b, double *x, void *stream);
+/* Binning (gm_bin_cells_csr) and decoupling in one launch: x (nbands ncls, ncells) row-major =
+ * A^-1 of the binned cells, rows band-major with a band's ncls spectra adjacent.  cells: host
+ * array of ncells <= 256 device pointers, each ncls rows of stride ld. */
+int gm_decouple_cells(int64_t nbands, int64_t ncls, int64_t ncells, const double *const *cells,
+                      int64_t ld, const int32_t *band_ptr, const int32_t *band_ells,
+                      const double *wfl, const double *lu, const void *work, double *x,
+                      void *stream);
 
 /* ----------------------------------------------- batched tensor-core Legendre stage */
 
@@ -493,7 +504,6 @@ int gm_cov_binned(int64_t lmax, int64_t nblocks, const double *xi, const double 
                   int64_t nbands_a, const int32_t *ptr_a, const int32_t *ells_a,
                   const double *w_a, int64_t nbands_b, const int32_t *ptr_b,
                   const int32_t *ells_b, const double *w_b, double *out, void *stream);
-
 /* gm_cov_binned with the term table on the host: terms, signs (+1 or -1), block_ptr (at most 512
  * terms) and xi (nk <= 8 device pointers to (L, L) kernels) are host arrays, spec has nrows <= 16
  * rows.  The indices are checked. */
