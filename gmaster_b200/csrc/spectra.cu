@@ -429,8 +429,8 @@ __global__ void k_bin_cells(int64_t lmax, int64_t nb, int64_t ncls, const double
 //
 // Bound by latency: two barriers, a warp reduction of the pivot candidates and kb - k
 // multiply-adds a row per column.  The panel is read and written once; held in global memory it
-// took 7 us a column, here 1.9 (a 612 x 612 matrix: panels 4.3 -> 1.16 ms, with the other
-// columns' kernels 5.4 -> 1.5 ms).
+// took 7 us a column, here 1.6 (a 612 x 612 matrix: panels 4.3 -> 1.0 ms, with the other
+// columns' kernels 5.4 -> 1.4 ms).
 __global__ void __launch_bounds__(1024) k_lu_panel_smem(int n, int k0, int kb, double *__restrict__ a,
                                                         int32_t *__restrict__ piv, int32_t *__restrict__ status)
 {
@@ -461,29 +461,25 @@ __global__ void __launch_bounds__(1024) k_lu_panel_smem(int n, int k0, int kb, d
                 row = i;
             }
         }
-        auto better = [](unsigned long long q, int r, unsigned long long &bq, int &br) {
-            if (q > bq || (q == bq && r < br)) {
-                bq = q;
-                br = r;
-            }
+        // the warp's largest key and its lowest row: the key's halves and the row one after the
+        // other through the integer reductions (a shuffle tree of (key, row) takes 15 steps)
+        auto best = [](unsigned long long &q, int &r) {
+            const unsigned hi = (unsigned)(q >> 32), lo = (unsigned)q;
+            const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+            const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+            const bool mine = hi == mh && lo == ml;
+            r = __reduce_min_sync(0xffffffffu, mine ? r : 0x7fffffff);
+            q = ((unsigned long long)mh << 32) | ml;
         };
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long q = __shfl_xor_sync(0xffffffffu, key, o);
-            const int r = __shfl_xor_sync(0xffffffffu, row, o);
-            better(q, r, key, row);
-        }
+        best(key, row);
         if (lane == 0) {
             skey[k & 1][warp] = key;
             srow[k & 1][warp] = row;
         }
         __syncthreads();
         key = lane < nw ? skey[k & 1][lane] : 0ull;
-        row = lane < nw ? srow[k & 1][lane] : rows;
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long q = __shfl_xor_sync(0xffffffffu, key, o);
-            const int r = __shfl_xor_sync(0xffffffffu, row, o);
-            better(q, r, key, row);
-        }
+        row = lane < nw ? srow[k & 1][lane] : 0x7fffffff;
+        best(key, row);
         if (key == 0ull) row = k;   // no number in the column
         if (tid == 0) {
             piv[k0 + k] = k0 + row;
