@@ -1,10 +1,15 @@
 // Latitudinal (Legendre / spin-weighted Wigner-d) stage, SIMT kernels for sm_100a.
 //
 // For each order m the rows lambda^{s'}_lm(theta) = sqrt((2l+1)/4pi) d^l_{m,s'}(theta)
-// are generated on the fly by the normalised three-term recurrence in l, in double
-// precision with an explicit binary exponent per lane (values below 2^-300 are
-// carried exactly and emitted as zero), and contracted against the ring spectra.
-// Only northern lanes are marched: the hemisphere fold
+// are generated on the fly in double precision with an explicit binary exponent per lane
+// (values below 2^-300 are carried exactly and emitted as zero), and contracted against the
+// ring spectra.  With r_l = 1 / alpha_l the normalised three-term recurrence
+//     v_{l+1} = alpha_{l+1} (x - c_{l+1}) v_l - (alpha_{l+1} / alpha_l) v_{l-1}
+// is carried through the differences v_l - v_{l-1} = alpha_l d_l:
+//     d_{l+1} = d_l + ((x - 1) + e_{l+1}) v_l,   e_l = 1 - r_{l-1} - r_l - c_l,
+//     v_{l+1} = v_l + alpha_{l+1} d_{l+1},
+// three operations with two coefficients per row (legendre_rows.cu has the same form in single
+// precision).  Only northern lanes are marched: the hemisphere fold
 //   lambda^{s'}_lm(pi - theta) = (-1)^{l+m} lambda^{-s'}_lm(theta)
 // turns the two hemispheres into the Sum / Diff right-hand sides of `rhs`.
 //
@@ -13,6 +18,16 @@
 // a few maps where no checkpoint tables exist (spins other than 0 and 2, Nside above 2048;
 // with tables: legendre_rows.cu); the tensor-core path (legendre_ck.cu, legendre_tc.cu) takes
 // wide batches.
+//
+// A CTA is up to four warps of one order; the rows go in segments of up to 128 whose
+// coefficients its threads compute once, then in blocks of eight without barriers: a warp whose
+// lanes are all below 2^-300 only steps.  Spin s sums 2a and -2a directly (four values a row
+// instead of eight).  Small sizes are bound by the chain of rows (m = 0) and the reduction
+// trees, large ones by the FP64 pipe: (3 + 2 NC) operations per row and lane (spin 0), 14 (spin
+// s).  Against windows of 32 rows with coefficients by square roots and divisions in each, and
+// eight sums a row: FP64 analysis / synthesis at Nside 128 56 / 44 -> 35 / 21 us, at Nside 1024
+// 10.0 / 8.1 -> 5.1 / 3.9 ms (spin 0) and 26.8 / 21.5 -> 13.0 / 9.9 ms (spin 2); mixed spin 1 at
+// Nside 1024 20.1 / 18.4 -> 9.6 / 8.7 ms.
 //
 // Replaces gmaster/_native/cuda/march_v2.cu:155-407 (march_analysis /
 // march_synthesis: float32 difference-form recurrence, SIMT FMA contraction).
@@ -24,7 +39,6 @@ namespace gm {
 
 constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / 32;
-constexpr int kWindow = 32;
 // Spins 1..kMaxSpin share the polarised kernels (template SPIN = 2) with the spin passed at
 // run time; the seed table holds 2 kMaxSpin + 1 variants.
 constexpr int kMaxSpin = 8;
@@ -57,37 +71,26 @@ __device__ __forceinline__ void seed_lane(const double *__restrict__ sd, double 
     k = kk;
 }
 
-__device__ __forceinline__ void rescale(double &v, double &vp, int &k)
-{
-    if (k < 0 && fabs(v) > kBig) {
-        v *= kShrink;
-        vp *= kShrink;
-        ++k;
-    }
-}
-
-// Recurrence coefficients for target degree l (lambda_l from lambda_{l-1}, lambda_{l-2}):
-//   lambda_l = alpha (x - m s'/((l-1) l)) lambda_{l-1} - beta lambda_{l-2}.
+// Coefficients of the step from row l to row l + 1 (see the head of the file): e of s' = -s, e of
+// s' = +s, alpha_{l+1}.
 struct Coef {
-    double alpha, beta, c0;  // c0 = alpha s m / ((l-1) l) for spin s >= 1, 0 for spin 0
+    double ea, eb, alpha;
 };
 
-__device__ __forceinline__ Coef make_coef(int l, int m, int s, int l0)
+// r_l = 1 / alpha_l, zero at l = max(m, s).
+__device__ __forceinline__ double inv_alpha(int l, int m, int s)
 {
-    Coef c;
-    double dl = (double)l, dm = (double)m, ds = (double)s;
-    double den = sqrt((dl * dl - dm * dm) * (dl * dl - ds * ds));
-    c.alpha = sqrt((2.0 * dl + 1.0) * (2.0 * dl - 1.0)) * dl / den;
-    if (l >= l0 + 2) {
-        double dl1 = dl - 1.0;
-        double num = sqrt((dl1 * dl1 - dm * dm) * (dl1 * dl1 - ds * ds));
-        c.beta = sqrt((2.0 * dl + 1.0) / (2.0 * dl - 3.0)) * dl * num / (dl1 * den);
-    } else {
-        c.beta = 0.0;
-    }
-    // alpha (x -+ c) = fma(alpha, x, -+alpha c): one FMA per row variant in the recurrence
-    c.c0 = (s != 0 && l >= 2) ? c.alpha * (ds * dm / ((dl - 1.0) * dl)) : 0.0;
-    return c;
+    const double dl = l, dm = m, ds = s;
+    if (s == 0) return sqrt((dl * dl - dm * dm) / (4.0 * dl * dl - 1.0));
+    return sqrt((dl * dl - dm * dm) * (dl * dl - ds * ds) / (4.0 * dl * dl - 1.0)) / dl;
+}
+
+__device__ __forceinline__ Coef step_coef(int l, int m, int s)
+{
+    const double r0 = inv_alpha(l, m, s), r1 = inv_alpha(l + 1, m, s);
+    const double e = 1.0 - r0 - r1;
+    const double c = s != 0 ? (double)s * m / ((double)l * (l + 1)) : 0.0;
+    return Coef{e + c, e - c, 1.0 / r1};
 }
 
 template <typename T, int V>
@@ -114,190 +117,236 @@ __device__ __forceinline__ int64_t alm_index(int64_t lmax, int64_t l, int64_t m)
     return m * (2 * lmax + 1 - m) / 2 + l;
 }
 
+// The rows of a thread's R lanes, NVAR variants each: value v 2^(600 k), scaled difference d.
+template <int NVAR, int R> struct RowState {
+    double y[R], v[NVAR][R], d[NVAR][R];
+    int k[NVAR][R];
+
+    // Seeds at row l0.
+    __device__ __forceinline__ void start(const double *__restrict__ geom, const double *__restrict__ seeds,
+                                          int64_t nlanes, int64_t L, int64_t jw, int lane, int m, int var, bool any)
+    {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int64_t j = jw + r * 32 + lane;
+            const bool ok = any && j < nlanes;
+            y[r] = ok ? geom[j] - 1.0 : 0.0;
+            const double ls = ok ? geom[nlanes + j] : 0.0, lc = ok ? geom[2 * nlanes + j] : 0.0;
+#pragma unroll
+            for (int q = 0; q < NVAR; ++q) {
+                v[q][r] = d[q][r] = 0.0;
+                k[q][r] = 0;
+                if (ok) seed_lane(seeds + ((int64_t)(var + q) * L + m) * 4, ls, lc, v[q][r], k[q][r]);
+            }
+        }
+    }
+
+    __device__ __forceinline__ void step(const Coef &c, int r)
+    {
+#pragma unroll
+        for (int q = 0; q < NVAR; ++q) {
+            const double C = y[r] + (q == 0 ? c.ea : c.eb);
+            d[q][r] = fma(C, v[q][r], d[q][r]);
+            v[q][r] = fma(c.alpha, d[q][r], v[q][r]);
+        }
+    }
+
+    // Lanes below 2^-300 that grew past it: once per eight rows (a row grows a value by at most
+    // 2^8, alpha <= sqrt(2m) + 1).
+    __device__ __forceinline__ void rescale()
+    {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int q = 0; q < NVAR; ++q)
+                if (k[q][r] < 0 && fabs(v[q][r]) > kBig) {
+                    v[q][r] *= kShrink;
+                    d[q][r] *= kShrink;
+                    ++k[q][r];
+                }
+    }
+
+    // 0: every lane of the warp emits its rows, 1: some do, 2: none does (all below 2^-300).
+    __device__ __forceinline__ int emission() const
+    {
+        bool all = true, none = true;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int q = 0; q < NVAR; ++q) {
+                all = all && k[q][r] == 0;
+                none = none && (k[q][r] < 0 || (v[q][r] == 0.0 && d[q][r] == 0.0));
+            }
+        if (__all_sync(0xffffffffu, all)) return 0;
+        return __all_sync(0xffffffffu, none) ? 2 : 1;
+    }
+};
+
 // ---------------------------------------------------------------- analysis
 
-// NC components per CTA (spin 0: NC maps; spin 2: NC = 2, one (Q, U) pair).
-// NV values per degree: spin 0: 2 NC; spin 2: 8.  LB degrees per reduce-scatter block.
+// NC components per CTA (spin 0: NC maps; spin s: NC = 2, one (Q, U) pair), NV sums per degree.
+template <int SPIN, int NC> struct Shape {
+    static constexpr int NVAR = SPIN == 0 ? 1 : 2;
+    static constexpr int NV = SPIN == 0 ? 2 * NC : 4;
+    static constexpr int kRows = 512 / NV < 128 ? 512 / NV : 128;   // rows per staged segment
+};
+
+// Eight rows of one warp into red[8 NV].  rh: spin 0, per map Sum re, im, Diff re, im; spin s,
+// P_N, P_S, M_N, M_S (re, im).
+template <typename T, int SPIN, int NC, int R, bool PART>
+__device__ __forceinline__ void ana8(RowState<Shape<SPIN, NC>::NVAR, R> &w, const T (&rh)[R][4 * NC],
+                                     const Coef *__restrict__ cf, double *__restrict__ red, int lane)
+{
+    constexpr int NV = Shape<SPIN, NC>::NV, NVAR = Shape<SPIN, NC>::NVAR;
+    // values per reduction tree: 32 where the registers allow (half the trees, of one more level)
+    constexpr int V = (NV * 8 >= 32 && R <= 2) || NV == 16 ? 32 : 16;
+    constexpr int RB = V / NV;
+    static_assert(RB % 2 == 0 && 8 % RB == 0, "row parity is fixed by the row index");
+#pragma unroll 1
+    for (int i = 0; i < 8; i += RB) {
+        T acc[V];
+#pragma unroll
+        for (int q = 0; q < V; ++q) acc[q] = (T)0;
+#pragma unroll
+        for (int s = 0; s < RB; ++s) {
+            const Coef c = cf[i + s];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                T val[NVAR];
+#pragma unroll
+                for (int q = 0; q < NVAR; ++q) val[q] = !PART || w.k[q][r] == 0 ? (T)w.v[q][r] : (T)0;
+                if (SPIN == 0) {
+#pragma unroll
+                    for (int e = 0; e < NC; ++e) {
+                        acc[s * NV + 2 * e] += val[0] * rh[r][4 * e + 2 * (s & 1)];
+                        acc[s * NV + 2 * e + 1] += val[0] * rh[r][4 * e + 2 * (s & 1) + 1];
+                    }
+                } else {
+                    const T vp = (s & 1) ? -val[NVAR - 1] : val[NVAR - 1], vm = (s & 1) ? -val[0] : val[0];
+                    T *a = acc + s * NV;
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        a[e] += val[0] * rh[r][e];
+                        a[e] += vp * rh[r][2 + e];
+                        a[2 + e] += val[NVAR - 1] * rh[r][4 + e];
+                        a[2 + e] += vm * rh[r][6 + e];
+                    }
+                }
+                w.step(c, r);
+            }
+        }
+        const T tot = warp_reduce_scatter<T, V>(acc, lane);
+        if (lane < V) red[i * NV + lane] = (double)tot;
+    }
+    w.rescale();
+}
+
 template <typename T, int SPIN, int NC, int R>
 __global__ void __launch_bounds__(kThreads) k_legendre_ana(
     int64_t nside, int64_t lmax, int64_t ncomp, const double *__restrict__ geom,
     const double *__restrict__ seeds, const T *__restrict__ rhs, double *__restrict__ alm,
     double scale, int spin)
 {
-    constexpr int NV = SPIN == 0 ? 2 * NC : 8;
-    constexpr int LB = 32 / NV;
-    constexpr int NVAR = SPIN == 0 ? 1 : 2;
-    static_assert(LB * NV == 32, "reduce-scatter width");
-    static_assert(LB % 2 == 0 && kWindow % 2 == 0, "row parity is fixed by the row index");
-    __shared__ Coef coef[kWindow];
-    __shared__ double red[kWarps][kWindow * NV];
-
+    using S = Shape<SPIN, NC>;
+    constexpr int NV = S::NV, NVAR = S::NVAR, kRows = S::kRows;
+    __shared__ Coef cf[kRows];
+    __shared__ double red[kWarps][kRows * NV];
     const int64_t L = lmax + 1, nlanes = 2 * nside, nelem = L * (L + 1) / 2;
     const int m = blockIdx.y;
     const int64_t c0 = (int64_t)blockIdx.z * NC;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int sv = SPIN == 0 ? 0 : spin;   // the field's spin (SPIN = 2: any spin >= 1)
     const int l0 = m > sv ? m : sv;
     if (l0 > lmax) return;
+    const int64_t jw = ((int64_t)blockIdx.x * nw + warp) * 32 * R;
 
-    double x[R], v[NVAR][R], vp[NVAR][R];
-    int kx[NVAR][R];
-    T rh[R][NC][4];
+    RowState<NVAR, R> w;
+    w.start(geom, seeds, nlanes, L, jw, lane, m, SPIN == 0 ? 0 : seed_variant(sv), true);
+    T rh[R][4 * NC];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        const int64_t j = (int64_t)blockIdx.x * kThreads * R + r * kThreads + threadIdx.x;
-        const bool ok = j < nlanes;
-        x[r] = ok ? geom[j] : 0.0;
-        const double ls = ok ? geom[nlanes + j] : 0.0, lc = ok ? geom[2 * nlanes + j] : 0.0;
-#pragma unroll
-        for (int q = 0; q < NVAR; ++q) {
-            // seed variants: s' = -s (lambda+), then s' = +s (lambda-, times (-1)^s)
-            const int var = SPIN == 0 ? 0 : seed_variant(sv) + q;
-            if (ok) {
-                seed_lane(seeds + ((int64_t)var * L + m) * 4, ls, lc, v[q][r], kx[q][r]);
-            } else {
-                v[q][r] = 0.0;
-                kx[q][r] = 0;
-            }
-            vp[q][r] = 0.0;
-        }
+        const int64_t j = jw + r * 32 + lane;
+        T g[NC][4];
 #pragma unroll
         for (int c = 0; c < NC; ++c)
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-                rh[r][c][e] = (ok && c0 + c < ncomp)
-                                  ? rhs[(((int64_t)m * nlanes + j) * ncomp + c0 + c) * 4 + e]
-                                  : (T)0;
+                g[c][e] = j < nlanes && c0 + c < ncomp ? rhs[(((int64_t)m * nlanes + j) * ncomp + c0 + c) * 4 + e] : (T)0;
+        if (SPIN == 0) {
+            // l + m of a segment's even rows is even: row s takes half s & 1
+#pragma unroll
+            for (int q = 0; q < 4 * NC; ++q) rh[r][q] = g[q / 4][q % 4];
+        } else {
+            // north = (Sum + Diff) / 2, south = (Sum - Diff) / 2; P = Q + iU, M = Q - iU.  The
+            // southern rows are the northern ones of the other variant times (-1)^(l + m + s):
+            // the sign of a segment's even rows goes into the southern right-hand sides
+            const T h = (T)0.5, hs = (l0 + m + sv) & 1 ? (T)-0.5 : (T)0.5;
+            const T *q = g[0], *u = g[NC - 1];
+            const T qnr = h * (q[0] + q[2]), qni = h * (q[1] + q[3]), qsr = hs * (q[0] - q[2]), qsi = hs * (q[1] - q[3]);
+            const T unr = h * (u[0] + u[2]), uni = h * (u[1] + u[3]), usr = hs * (u[0] - u[2]), usi = hs * (u[1] - u[3]);
+            rh[r][0] = qnr - uni;
+            rh[r][1] = qni + unr;
+            rh[r][2] = qsr - usi;
+            rh[r][3] = qsi + usr;
+            rh[r][4] = qnr + uni;
+            rh[r][5] = qni - unr;
+            rh[r][6] = qsr + usi;
+            rh[r][7] = qsi - usr;
+        }
     }
 
-    // The southern ring's rows are the northern ones times (-1)^(l + m + s) (for spin s,
-    // with the (-1)^s of the +s variant in its seed).  The rows of a reduce-scatter block
-    // start at l0 + (an even offset: kWindow and LB are even), so that parity in unrolled
-    // row s is ((l0 + m + sv) + s) & 1.  With the two hemisphere halves of the right-hand
-    // side swapped once here when l0 + m + sv is odd, row s takes half s & 1, chosen at
-    // compile time instead of by selects on every element.
-    if ((l0 + m + sv) & 1) {
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                T t0 = rh[r][c][0], t1 = rh[r][c][1];
-                rh[r][c][0] = rh[r][c][2];
-                rh[r][c][1] = rh[r][c][3];
-                rh[r][c][2] = t0;
-                rh[r][c][3] = t1;
-            }
-    }
-    for (int lb = l0; lb < L; lb += kWindow) {
-        if (threadIdx.x < kWindow) {
-            const int l = lb + threadIdx.x;
-            coef[threadIdx.x] = make_coef(l, m, sv, l0);
-        }
+    for (int64_t lb = l0; lb < L; lb += kRows) {
+        const int nrow = (int)(L - lb < kRows ? L - lb : kRows);
+        __syncthreads();   // the previous segment's sums are read
+        for (int i = threadIdx.x; i < kRows; i += blockDim.x)
+            cf[i] = i < nrow ? step_coef((int)lb + i, m, sv) : Coef{0.0, 0.0, 0.0};
         __syncthreads();
 #pragma unroll 1
-        for (int i = 0; i < kWindow; i += LB) {
-            T acc[LB * NV];
+        for (int i = 0; i < nrow; i += 8) {
+            double *out = red[warp] + i * NV;
+            const int mode = w.emission();
+            if (mode == 0) {
+                ana8<T, SPIN, NC, R, false>(w, rh, cf + i, out, lane);
+            } else if (mode == 1) {
+                ana8<T, SPIN, NC, R, true>(w, rh, cf + i, out, lane);
+            } else {
+                for (int q = lane; q < 8 * NV; q += 32) out[q] = 0.0;
 #pragma unroll
-            for (int q = 0; q < LB * NV; ++q) acc[q] = (T)0;
+                for (int s = 0; s < 8; ++s) {
+                    const Coef c = cf[i + s];
 #pragma unroll
-            for (int s = 0; s < LB; ++s) {
-                const int l = lb + i + s;
-                if (l < L) {
-                    if (l > l0) {
-                        const Coef cf = coef[i + s];
-#pragma unroll
-                        for (int r = 0; r < R; ++r) {
-                            if (SPIN == 0) {
-                                double nv = fma(cf.alpha * x[r], v[0][r], -cf.beta * vp[0][r]);
-                                vp[0][r] = v[0][r];
-                                v[0][r] = nv;
-                                rescale(v[0][r], vp[0][r], kx[0][r]);
-                            } else {
-                                // s' = -2: alpha (x - m s'/((l-1)l)) = fma(alpha, x, c0);
-                                // s' = +2: fma(alpha, x, -c0)  (c0 carries alpha)
-                                double nva = fma(fma(cf.alpha, x[r], cf.c0), v[0][r], -cf.beta * vp[0][r]);
-                                double nvb = fma(fma(cf.alpha, x[r], -cf.c0), v[1][r], -cf.beta * vp[1][r]);
-                                vp[0][r] = v[0][r];
-                                v[0][r] = nva;
-                                vp[1][r] = v[1][r];
-                                v[1][r] = nvb;
-                                rescale(v[0][r], vp[0][r], kx[0][r]);
-                                rescale(v[1][r], vp[1][r], kx[1][r]);
-                            }
-                        }
-                    }
-                    const int par = s & 1;   // relative to (l0 + m + sv) & 1, see above
-#pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        if (SPIN == 0) {
-                            const T val = kx[0][r] == 0 ? (T)v[0][r] : (T)0;
-#pragma unroll
-                            for (int c = 0; c < NC; ++c) {
-                                const T hr = par ? rh[r][c][2] : rh[r][c][0];
-                                const T hi = par ? rh[r][c][3] : rh[r][c][1];
-                                acc[s * NV + 2 * c] += val * hr;
-                                acc[s * NV + 2 * c + 1] += val * hi;
-                            }
-                        } else {
-                            const double lp = kx[0][r] == 0 ? v[0][r] : 0.0;
-                            const double lm = kx[NVAR - 1][r] == 0 ? v[NVAR - 1][r] : 0.0;
-                            const T f1 = (T)(0.5 * (lp + lm)), f2 = (T)(0.5 * (lp - lm));
-                            // same-parity side P = Sum (even) / Diff (odd); other side D
-                            const T qpr = par ? rh[r][0][2] : rh[r][0][0];
-                            const T qpi = par ? rh[r][0][3] : rh[r][0][1];
-                            const T upr = par ? rh[r][1][2] : rh[r][1][0];
-                            const T upi = par ? rh[r][1][3] : rh[r][1][1];
-                            const T qdr = par ? rh[r][0][0] : rh[r][0][2];
-                            const T qdi = par ? rh[r][0][1] : rh[r][0][3];
-                            const T udr = par ? rh[r][1][0] : rh[r][1][2];
-                            const T udi = par ? rh[r][1][1] : rh[r][1][3];
-                            acc[s * NV + 0] += f1 * qpr;
-                            acc[s * NV + 1] += f1 * qpi;
-                            acc[s * NV + 2] += f1 * upr;
-                            acc[s * NV + 3] += f1 * upi;
-                            acc[s * NV + 4] += f2 * qdr;
-                            acc[s * NV + 5] += f2 * qdi;
-                            acc[s * NV + 6] += f2 * udr;
-                            acc[s * NV + 7] += f2 * udi;
-                        }
-                    }
+                    for (int r = 0; r < R; ++r) w.step(c, r);
                 }
+                w.rescale();
             }
-            const T tot = warp_reduce_scatter<T, LB * NV>(acc, lane);
-            red[warp][i * NV + lane] = (double)tot;
         }
         __syncthreads();
-        if (threadIdx.x < kWindow) {
-            const int l = lb + threadIdx.x;
-            if (l < L) {
-                double sv[NV];
+        for (int i = threadIdx.x; i < nrow; i += blockDim.x) {
+            double sum[NV];
 #pragma unroll
-                for (int q = 0; q < NV; ++q) {
-                    double t = 0.0;
+            for (int q = 0; q < NV; ++q) {
+                double t = 0.0;
+                for (int g = 0; g < nw; ++g) t += red[g][i * NV + q];
+                sum[q] = t;
+            }
+            const int64_t idx = alm_index(lmax, lb + i, m);
+            if (SPIN == 0) {
 #pragma unroll
-                    for (int w = 0; w < kWarps; ++w) t += red[w][threadIdx.x * NV + q];
-                    sv[q] = t;
-                }
-                const int64_t idx = alm_index(lmax, l, m);
-                if (SPIN == 0) {
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        if (c0 + c < ncomp) {
-                            double *a = alm + 2 * ((c0 + c) * nelem + idx);
-                            atomicAdd(a, scale * sv[2 * c]);
-                            atomicAdd(a + 1, scale * sv[2 * c + 1]);
-                        }
+                for (int c = 0; c < NC; ++c) {
+                    if (c0 + c < ncomp) {
+                        double *a = alm + 2 * ((c0 + c) * nelem + idx);
+                        atomicAdd(a, scale * sum[2 * c]);
+                        atomicAdd(a + 1, scale * sum[2 * c + 1]);
                     }
-                } else {
-                    // E = -(a1 + i-rotated a2), B likewise (see the docstring of gm_legendre_analysis)
-                    const int64_t f = c0 / 2;
-                    double *e = alm + 2 * ((2 * f) * nelem + idx);
-                    double *b = alm + 2 * ((2 * f + 1) * nelem + idx);
-                    atomicAdd(e, -scale * (sv[0] - sv[7]));
-                    atomicAdd(e + 1, -scale * (sv[1] + sv[6]));
-                    atomicAdd(b, -scale * (sv[2] + sv[5]));
-                    atomicAdd(b + 1, -scale * (sv[3] - sv[4]));
                 }
+            } else {
+                // E = -(+sa + -sa) / 2, B = i (+sa - -sa) / 2
+                double *e = alm + 2 * (c0 * nelem + idx), *b = e + 2 * nelem;
+                const double hs = 0.5 * scale;
+                atomicAdd(e, -hs * (sum[0] + sum[2]));
+                atomicAdd(e + 1, -hs * (sum[1] + sum[3]));
+                atomicAdd(b, -hs * (sum[1] - sum[3]));
+                atomicAdd(b + 1, hs * (sum[0] - sum[2]));
             }
         }
     }
@@ -305,192 +354,152 @@ __global__ void __launch_bounds__(kThreads) k_legendre_ana(
 
 // ---------------------------------------------------------------- synthesis
 
+// Eight rows of one warp added to the accumulators.  aw[row][.]: spin 0, (re, im) per map; spin s,
+// +sa and -sa (re, im).  acc: spin 0, per map the even and odd rows (re, im); spin s, U_N, V_N
+// (of +sa, -sa), U_S, V_S.
+template <typename T, int SPIN, int NC, int R, bool PART>
+__device__ __forceinline__ void syn8(RowState<Shape<SPIN, NC>::NVAR, R> &w, T (&acc)[R][4 * NC],
+                                     const Coef *__restrict__ cf, const T *__restrict__ aw)
+{
+    constexpr int NVAR = Shape<SPIN, NC>::NVAR, NA = SPIN == 0 ? NC : 2;
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+        const Coef c = cf[s];
+        T a[2 * NA];
+#pragma unroll
+        for (int q = 0; q < 2 * NA; ++q) a[q] = aw[s * 2 * NA + q];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            T val[NVAR];
+#pragma unroll
+            for (int q = 0; q < NVAR; ++q) val[q] = !PART || w.k[q][r] == 0 ? (T)w.v[q][r] : (T)0;
+            T *o = acc[r];
+            if (SPIN == 0) {
+#pragma unroll
+                for (int e = 0; e < NC; ++e) {
+                    o[4 * e + 2 * (s & 1)] += val[0] * a[2 * e];
+                    o[4 * e + 2 * (s & 1) + 1] += val[0] * a[2 * e + 1];
+                }
+            } else {
+                const T vp = (s & 1) ? -val[NVAR - 1] : val[NVAR - 1], vm = (s & 1) ? -val[0] : val[0];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    o[e] += val[0] * a[e];
+                    o[2 + e] += val[NVAR - 1] * a[2 + e];
+                    o[4 + e] += vp * a[e];
+                    o[6 + e] += vm * a[2 + e];
+                }
+            }
+            w.step(c, r);
+        }
+    }
+    w.rescale();
+}
+
 template <typename T, int SPIN, int NC, int R>
 __global__ void __launch_bounds__(kThreads) k_legendre_syn(
     int64_t nside, int64_t lmax, int64_t ncomp, const double *__restrict__ geom,
     const double *__restrict__ seeds, const double *__restrict__ alm, T *__restrict__ syn,
     int spin)
 {
-    constexpr int NVAR = SPIN == 0 ? 1 : 2;
-    constexpr int NA = SPIN == 0 ? NC : 2;  // complex alm rows per degree (maps, or E and B)
-    constexpr int NACC = SPIN == 0 ? 4 * NC : 16;
-    __shared__ Coef coef[2][kWindow];
-    __shared__ T aw[2][kWindow][NA][2];
-
+    using S = Shape<SPIN, NC>;
+    constexpr int NVAR = S::NVAR, kRows = 128;
+    constexpr int NA = SPIN == 0 ? NC : 2;  // complex alm rows per degree (maps, or +sa and -sa)
+    __shared__ Coef cf[kRows];
+    __shared__ T aw[kRows * 2 * NA];
     const int64_t L = lmax + 1, nlanes = 2 * nside, nelem = L * (L + 1) / 2;
     const int m = blockIdx.y;
     const int64_t c0 = (int64_t)blockIdx.z * NC;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int sv = SPIN == 0 ? 0 : spin;
     const int l0 = m > sv ? m : sv;
+    const int64_t jw = ((int64_t)blockIdx.x * nw + warp) * 32 * R;
 
-    double x[R], v[NVAR][R], vp[NVAR][R];
-    int kx[NVAR][R];
-    T acc[R][NACC];
+    RowState<NVAR, R> w;
+    w.start(geom, seeds, nlanes, L, jw, lane, m, SPIN == 0 ? 0 : seed_variant(sv), l0 <= lmax);
+    T acc[R][4 * NC];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int64_t j = (int64_t)blockIdx.x * kThreads * R + r * kThreads + threadIdx.x;
-        const bool ok = j < nlanes && l0 <= lmax;
-        x[r] = ok ? geom[j] : 0.0;
-        const double ls = ok ? geom[nlanes + j] : 0.0, lc = ok ? geom[2 * nlanes + j] : 0.0;
+    for (int r = 0; r < R; ++r)
 #pragma unroll
-        for (int q = 0; q < NVAR; ++q) {
-            const int var = SPIN == 0 ? 0 : seed_variant(sv) + q;
-            if (ok) {
-                seed_lane(seeds + ((int64_t)var * L + m) * 4, ls, lc, v[q][r], kx[q][r]);
-            } else {
-                v[q][r] = 0.0;
-                kx[q][r] = 0;
-            }
-            vp[q][r] = 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < NACC; ++q) acc[r][q] = (T)0;
-    }
+        for (int q = 0; q < 4 * NC; ++q) acc[r][q] = (T)0;
 
-    int buf = 0;
-    for (int lb = l0; lb < L; lb += kWindow, buf ^= 1) {
-        if (threadIdx.x < kWindow) {
-            const int l = lb + threadIdx.x;
-            coef[buf][threadIdx.x] = make_coef(l, m, sv, l0);
-#pragma unroll
-            for (int a = 0; a < NA; ++a) {
-                T re = 0, im = 0;
-                if (l < L) {
-                    const int64_t row = SPIN == 0 ? c0 + a : c0 + a;  // spin 2: rows E, B of field c0/2
-                    if (row < ncomp) {
-                        const double *p = alm + 2 * (row * nelem + alm_index(lmax, l, m));
-                        re = (T)p[0];
-                        im = (T)p[1];
-                    }
-                }
-                aw[buf][threadIdx.x][a][0] = re;
-                aw[buf][threadIdx.x][a][1] = im;
-            }
-        }
-        __syncthreads();
-        const int lend = (lb + kWindow < L) ? kWindow : (int)(L - lb);
-        // blocks start at l0 + multiples of kWindow (even), so row s has the parity of
-        // l + m relative to (l0 + m) & 1 given by s & 1: rows go in pairs and each
-        // accumulates into its half at compile time (no multiplications by zero); the
-        // halves are put in true parity order before the output
-#pragma unroll 2
-        for (int s0 = 0; s0 < lend; s0 += 2) {
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-                const int s = s0 + hh;
-                if (s >= lend) break;
-                const int l = lb + s;
-                if (l > l0) {
-                    const Coef cf = coef[buf][s];
-#pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        if (SPIN == 0) {
-                            double nv = fma(cf.alpha * x[r], v[0][r], -cf.beta * vp[0][r]);
-                            vp[0][r] = v[0][r];
-                            v[0][r] = nv;
-                            rescale(v[0][r], vp[0][r], kx[0][r]);
-                        } else {
-                            double nva = fma(fma(cf.alpha, x[r], cf.c0), v[0][r], -cf.beta * vp[0][r]);
-                            double nvb = fma(fma(cf.alpha, x[r], -cf.c0), v[1][r], -cf.beta * vp[1][r]);
-                            vp[0][r] = v[0][r];
-                            v[0][r] = nva;
-                            vp[1][r] = v[1][r];
-                            v[1][r] = nvb;
-                            rescale(v[0][r], vp[0][r], kx[0][r]);
-                            rescale(v[1][r], vp[1][r], kx[1][r]);
-                        }
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    if (SPIN == 0) {
-                        const T val = kx[0][r] == 0 ? (T)v[0][r] : (T)0;
-#pragma unroll
-                        for (int c = 0; c < NC; ++c) {
-                            acc[r][4 * c + 2 * hh] += val * aw[buf][s][c][0];
-                            acc[r][4 * c + 2 * hh + 1] += val * aw[buf][s][c][1];
-                        }
-                    } else {
-                        const double lp = kx[0][r] == 0 ? v[0][r] : 0.0;
-                        const double lm = kx[NVAR - 1][r] == 0 ? v[NVAR - 1][r] : 0.0;
-                        const T f1 = (T)(0.5 * (lp + lm)), f2 = (T)(0.5 * (lp - lm));
-                        const T er = aw[buf][s][0][0], ei = aw[buf][s][0][1];
-                        const T br = aw[buf][s][1][0], bi = aw[buf][s][1][1];
-                        // per parity: [S1E re, im, S1B re, im, S2E re, im, S2B re, im]
-                        T *a = &acc[r][8 * hh];
-                        a[0] += f1 * er;
-                        a[1] += f1 * ei;
-                        a[2] += f1 * br;
-                        a[3] += f1 * bi;
-                        a[4] += f2 * er;
-                        a[5] += f2 * ei;
-                        a[6] += f2 * br;
-                        a[7] += f2 * bi;
-                    }
-                }
-            }
-        }
-    }
-
-    if ((l0 + m + sv) & 1) {
-        // the even rows of the blocks had odd l + m + s: swap the halves into parity order
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
+    for (int64_t lb = l0; lb < L; lb += kRows) {
+        const int nrow = (int)(L - lb < kRows ? L - lb : kRows);
+        __syncthreads();   // the previous segment's rows are done with
+        for (int i = threadIdx.x; i < kRows; i += blockDim.x) {
+            const bool in = i < nrow;
+            cf[i] = in ? step_coef((int)lb + i, m, sv) : Coef{0.0, 0.0, 0.0};
+            const double2 *src = reinterpret_cast<const double2 *>(alm) + c0 * nelem + (in ? alm_index(lmax, lb + i, m) : 0);
+            T *o = aw + i * 2 * NA;
             if (SPIN == 0) {
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
-                    const T t0 = acc[r][4 * c], t1 = acc[r][4 * c + 1];
-                    acc[r][4 * c] = acc[r][4 * c + 2];
-                    acc[r][4 * c + 1] = acc[r][4 * c + 3];
-                    acc[r][4 * c + 2] = t0;
-                    acc[r][4 * c + 3] = t1;
+                    double2 a = make_double2(0.0, 0.0);
+                    if (in && c0 + c < ncomp) a = src[c * nelem];
+                    o[2 * c] = (T)a.x;
+                    o[2 * c + 1] = (T)a.y;
                 }
             } else {
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const T t = acc[r][q];
-                    acc[r][q] = acc[r][8 + q];
-                    acc[r][8 + q] = t;
+                double2 e = make_double2(0.0, 0.0), b = e;
+                if (in) {
+                    e = src[0];
+                    b = src[nelem];
                 }
+                // +sa = -(E + iB), -sa = -(E - iB)
+                o[0] = (T)(b.y - e.x);
+                o[1] = (T)(-e.y - b.x);
+                o[2] = (T)(-e.x - b.y);
+                o[3] = (T)(b.x - e.y);
+            }
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int i = 0; i < nrow; i += 8) {
+            const int mode = w.emission();
+            if (mode == 0) {
+                syn8<T, SPIN, NC, R, false>(w, acc, cf + i, aw + i * 2 * NA);
+            } else if (mode == 1) {
+                syn8<T, SPIN, NC, R, true>(w, acc, cf + i, aw + i * 2 * NA);
+            } else {
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    const Coef c = cf[i + s];
+#pragma unroll
+                    for (int r = 0; r < R; ++r) w.step(c, r);
+                }
+                w.rescale();
             }
         }
     }
 
+    const T hs = (l0 + m + sv) & 1 ? (T)-0.5 : (T)0.5;   // (-1)^(l + m + s) of the even rows
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        const int64_t j = (int64_t)blockIdx.x * kThreads * R + r * kThreads + threadIdx.x;
+        const int64_t j = jw + r * 32 + lane;
         if (j >= nlanes) continue;
+        const T *a = acc[r];
         if (SPIN == 0) {
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
                 if (c0 + c >= ncomp) continue;
                 T *o = syn + (((int64_t)m * nlanes + j) * ncomp + c0 + c) * 4;
-                const T er = acc[r][4 * c], ei = acc[r][4 * c + 1];
-                const T orr = acc[r][4 * c + 2], oi = acc[r][4 * c + 3];
-                o[0] = er + orr;
-                o[1] = ei + oi;
-                o[2] = er - orr;
-                o[3] = ei - oi;
+                o[0] = a[4 * c] + a[4 * c + 2];
+                o[1] = a[4 * c + 1] + a[4 * c + 3];
+                o[2] = a[4 * c] - a[4 * c + 2];
+                o[3] = a[4 * c + 1] - a[4 * c + 3];
             }
         } else {
-            const T *e = &acc[r][0];
-            const T *od = &acc[r][8];
-            // north: sums; south: F1 -> e - o, F2 -> o - e
-            T s1e_n[2] = {e[0] + od[0], e[1] + od[1]}, s1b_n[2] = {e[2] + od[2], e[3] + od[3]};
-            T s2e_n[2] = {e[4] + od[4], e[5] + od[5]}, s2b_n[2] = {e[6] + od[6], e[7] + od[7]};
-            T s1e_s[2] = {e[0] - od[0], e[1] - od[1]}, s1b_s[2] = {e[2] - od[2], e[3] - od[3]};
-            T s2e_s[2] = {od[4] - e[4], od[5] - e[5]}, s2b_s[2] = {od[6] - e[6], od[7] - e[7]};
-            T *oq = syn + (((int64_t)m * nlanes + j) * ncomp + c0) * 4;
-            T *ou = oq + 4;
-            // Q~ = -(S1E + i S2B), U~ = -(S1B - i S2E)
-            oq[0] = -(s1e_n[0] - s2b_n[1]);
-            oq[1] = -(s1e_n[1] + s2b_n[0]);
-            oq[2] = -(s1e_s[0] - s2b_s[1]);
-            oq[3] = -(s1e_s[1] + s2b_s[0]);
-            ou[0] = -(s1b_n[0] + s2e_n[1]);
-            ou[1] = -(s1b_n[1] - s2e_n[0]);
-            ou[2] = -(s1b_s[0] + s2e_s[1]);
-            ou[3] = -(s1b_s[1] - s2e_s[0]);
+            // Q = (U + V) / 2, U map = (U - V) / 2i, both hemispheres
+            T *oq = syn + (((int64_t)m * nlanes + j) * ncomp + c0) * 4, *ou = oq + 4;
+            const T h = (T)0.5;
+            oq[0] = h * (a[0] + a[2]);
+            oq[1] = h * (a[1] + a[3]);
+            oq[2] = hs * (a[4] + a[6]);
+            oq[3] = hs * (a[5] + a[7]);
+            ou[0] = h * (a[1] - a[3]);
+            ou[1] = -h * (a[0] - a[2]);
+            ou[2] = hs * (a[5] - a[7]);
+            ou[3] = -hs * (a[4] - a[6]);
         }
     }
 }
@@ -501,15 +510,22 @@ using namespace gm;
 
 extern "C" int64_t gm_seed_table_len(int64_t L) { return (2 * kMaxSpin + 1) * 4 * L; }
 
+// Warps of a CTA: as many as the lanes fill, up to kWarps.
+static int cta_warps(int64_t nlanes, int R)
+{
+    const int64_t need = (nlanes + 32 * R - 1) / (32 * R);
+    return (int)(need < kWarps ? need : kWarps);
+}
+
 template <typename T, int SPIN, int NC, int R>
 static int launch_ana(int spin, int64_t nside, int64_t lmax, int64_t ncomp, const double *geom,
                       const double *seeds, const void *rhs, double *alm, double scale,
                       cudaStream_t s)
 {
     const int64_t nlanes = 2 * nside;
-    dim3 grid((unsigned)((nlanes + kThreads * R - 1) / (kThreads * R)), (unsigned)(lmax + 1),
-              (unsigned)((ncomp + NC - 1) / NC));
-    k_legendre_ana<T, SPIN, NC, R><<<grid, kThreads, 0, s>>>(nside, lmax, ncomp, geom, seeds, (const T *)rhs,
+    const int nw = cta_warps(nlanes, R), per = 32 * R * nw;
+    dim3 grid((unsigned)((nlanes + per - 1) / per), (unsigned)(lmax + 1), (unsigned)((ncomp + NC - 1) / NC));
+    k_legendre_ana<T, SPIN, NC, R><<<grid, 32 * nw, 0, s>>>(nside, lmax, ncomp, geom, seeds, (const T *)rhs,
                                                              alm, scale, spin);
     return check_launch("gm_legendre_analysis");
 }
@@ -519,9 +535,9 @@ static int launch_syn(int spin, int64_t nside, int64_t lmax, int64_t ncomp, cons
                       const double *seeds, const double *alm, void *syn, cudaStream_t s)
 {
     const int64_t nlanes = 2 * nside;
-    dim3 grid((unsigned)((nlanes + kThreads * R - 1) / (kThreads * R)), (unsigned)(lmax + 1),
-              (unsigned)((ncomp + NC - 1) / NC));
-    k_legendre_syn<T, SPIN, NC, R><<<grid, kThreads, 0, s>>>(nside, lmax, ncomp, geom, seeds, alm, (T *)syn,
+    const int nw = cta_warps(nlanes, R), per = 32 * R * nw;
+    dim3 grid((unsigned)((nlanes + per - 1) / per), (unsigned)(lmax + 1), (unsigned)((ncomp + NC - 1) / NC));
+    k_legendre_syn<T, SPIN, NC, R><<<grid, 32 * nw, 0, s>>>(nside, lmax, ncomp, geom, seeds, alm, (T *)syn,
                                                              spin);
     return check_launch("gm_legendre_synthesis");
 }
