@@ -144,8 +144,10 @@ __device__ void stockham_stage(const T2 *__restrict__ in, T2 *__restrict__ out, 
     const int r = h / Lp;
     const int nb = h / p;
     if (p == 4) {
+        // the radix-4 and radix-2 stages come first: Ls is a power of two
+        const int lg = 31 - __clz(Ls);
         for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-            int kk = b / Ls, j = b - kk * Ls;
+            const int kk = b >> lg, j = b & (Ls - 1);
             T2 x0 = in[kk * Ls + j];
             T2 x1 = in[(kk + r) * Ls + j];
             T2 x2 = in[(kk + 2 * r) * Ls + j];
@@ -165,8 +167,9 @@ __device__ void stockham_stage(const T2 *__restrict__ in, T2 *__restrict__ out, 
             o[3 * Ls] = csub(bq, d);
         }
     } else if (p == 2) {
+        const int lg = 31 - __clz(Ls);
         for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-            int kk = b / Ls, j = b - kk * Ls;
+            const int kk = b >> lg, j = b & (Ls - 1);
             T2 x0 = in[kk * Ls + j];
             T2 x1 = in[(kk + r) * Ls + j];
             if (Ls > 1) x1 = cmul(x1, twiddle<TM>(tw, h, j * r, sign));   // j r < h / 2
@@ -332,20 +335,36 @@ __device__ T2 *bs_apply(T2 *X, T2 *Y, const T2 *FB, int h, int n, int M, const T
 }
 
 // Load one ring of one map (times the mask) as h complex z_t = x_2t + i x_2t+1, each
-// multiplied by f(t) (the Bluestein chirp, or 1).
+// multiplied by f(t) (the Bluestein chirp, or 1).  vec: x and mask are aligned to two elements
+// (every ring starts at an even pixel), so a pair is one load.
 template <typename T, typename Tin, typename T2, typename F>
-__device__ __forceinline__ void load_ring(const Tin *__restrict__ x, const double *__restrict__ mask,
+__device__ __forceinline__ void load_ring(const Tin *__restrict__ x, const double *__restrict__ mask, bool vec,
                                           int h, T2 *__restrict__ dst, F f)
 {
+    using Tin2 = typename vec2<Tin>::type;
     for (int t = threadIdx.x; t < h; t += blockDim.x) {
+        Tin2 p;
+        if (vec) {
+            p = reinterpret_cast<const Tin2 *>(x)[t];
+        } else {
+            p.x = x[2 * t];
+            p.y = x[2 * t + 1];
+        }
         T2 z;
         if (mask) {
             // masked field: the FP64 product map * mask, rounded once to T
-            z.x = (T)((double)x[2 * t] * mask[2 * t]);
-            z.y = (T)((double)x[2 * t + 1] * mask[2 * t + 1]);
+            double2 w;
+            if (vec) {
+                w = reinterpret_cast<const double2 *>(mask)[t];
+            } else {
+                w.x = mask[2 * t];
+                w.y = mask[2 * t + 1];
+            }
+            z.x = (T)((double)p.x * w.x);
+            z.y = (T)((double)p.y * w.y);
         } else {
-            z.x = (T)x[2 * t];
-            z.y = (T)x[2 * t + 1];
+            z.x = (T)p.x;
+            z.y = (T)p.y;
         }
         dst[t] = f(t, z);
     }
@@ -394,107 +413,64 @@ __device__ __forceinline__ void ring_outputs(const T2 *__restrict__ Z, int n, in
     }
 }
 
-// One CTA per (map component, ring), the component the fast grid index so that the CTAs of
-// one ring run together and read its mask once from DRAM: mixed-radix Stockham FFT in
-// shared memory.  In single precision the rings of the Bluestein path (use_bluestein with
-// `mcap` > 0) are left to k_ring_analysis_bluestein.
+// Rings of a launch (forward and inverse): i0 > 0, the cap rings of length 4 i, i0 <= i < i0 + cnt, of
+// both hemispheres; i0 = 0, the belt.  A launch covers rings of one shared-memory size, so
+// that short rings run many CTAs per SM.
+__device__ __forceinline__ int64_t launch_ring(int64_t nside, int64_t i0, int64_t cnt, int64_t b)
+{
+    return i0 == 0 ? nside - 1 + b : (b < cnt ? i0 - 1 + b : 4 * nside - 1 - (i0 + b - cnt));
+}
+
+// Forward ring transform: one CTA per (ring, block of cpc components), the component block the
+// fast grid index so that the CTAs of one ring run together and read its mask once from DRAM.
+// Rings whose half-length has a prime factor above 64 go through Bluestein's method (M <= mcap:
+// three buffers of M; the transform of the chirp once per CTA), the others through the
+// mixed-radix FFT.  Bound by the passes over shared memory (one per radix) and their barriers:
+// an eighth of the points as threads, two radix-4 butterflies each, fills an SM with CTAs.
 template <typename T, typename Tin>
-__global__ void __launch_bounds__(512) k_ring_analysis(int64_t nside, int64_t L,
-                                                       const Tin *__restrict__ maps,
-                                                       const double *__restrict__ mask,
-                                                       const void *__restrict__ twall,
-                                                       int64_t twcnt,
-                                                       const uint8_t *__restrict__ shifted,
-                                                       typename vec2<T>::type *__restrict__ out,
-                                                       int mcap, int hcap, int bsmin)
+__global__ void __launch_bounds__(512) k_ring_forward(int64_t nside, int64_t L, int64_t ncomp, int cpc,
+                                                      const Tin *__restrict__ maps,
+                                                      const double *__restrict__ mask, bool vec,
+                                                      const void *__restrict__ twall, int64_t twcnt,
+                                                      const uint8_t *__restrict__ shifted,
+                                                      typename vec2<T>::type *__restrict__ out, int64_t i0,
+                                                      int64_t cnt, int mcap, int hcap, int bsmin, int buf)
 {
     using T2 = typename vec2<T>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int64_t r = blockIdx.y, c = blockIdx.x;
-    const int64_t nring = 4 * nside - 1, npix = 12 * nside * nside;
+    const int64_t r = launch_ring(nside, i0, cnt, blockIdx.y), nring = 4 * nside - 1, npix = 12 * nside * nside;
     const int n = (int)ring_nphi(nside, r), h = n / 2;
-    if (mcap > 0 && use_bluestein(h, mcap)) return;
-    if (ring_big(h, hcap, (int)nside, bsmin)) return;   // left to k_ring_analysis_big
+    const bool bs = mcap > 0 && use_bluestein(h, mcap);
+    if (hcap > 0 && ring_big(h, hcap, (int)nside, bsmin)) return;   // left to k_ring_analysis_big
     const int64_t off = ring_offset(nside, r);
-    T2 *A = reinterpret_cast<T2 *>(smem_raw);
-    T2 *B = A + hcap;
-    const T2 *tw = TwTable<T2>::get(twall, twcnt) + twiddle_offset(n);
-    load_ring<T>(maps + c * npix + off, mask ? mask + off : nullptr, h, A,
-                 [](int, T2 z) { return z; });
-    __syncthreads();
-    T2 *Z = fft_shared(A, B, h, tw, -1);
-    ring_outputs<T>(Z, n, L, tw, shifted[r] != 0, (T)(4.0 * M_PI / (double)npix),
-                    out + (c * nring + r) * L);
-}
-
-// Bluestein path, single precision: one CTA per (block of `cpc` components, ring), the
-// component block the fast grid index.
-//   X_k = sum_j z_j omega_h^{jk} = c_k sum_j (z_j c_j) conj(c_{k-j}),  c_j = e^{-i pi j^2 / h}
-// evaluated as a circular convolution of length M: the transform of the wrapped conjugate
-// chirp once per CTA, then per component one forward and one inverse FFT.  The chirp is
-// read exactly from the ring's table: c_j = omega_{2h}^{j^2 mod 2h}.
-template <typename Tin>
-__global__ void __launch_bounds__(512) k_ring_analysis_bluestein(int64_t nside, int64_t L,
-                                                                 int64_t ncomp, int cpc, int mcap,
-                                                                 int hcap, int bsmin,
-                                                                 const Tin *__restrict__ maps,
-                                                                 const double *__restrict__ mask,
-                                                                 const void *__restrict__ twall,
-                                                                 int64_t twcnt,
-                                                                 const uint8_t *__restrict__ shifted,
-                                                                 float2 *__restrict__ out)
-{
-    using T2 = float2;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int64_t r = blockIdx.y;
-    const int n = (int)ring_nphi(nside, r), h = n / 2;
-    if (!use_bluestein(h, mcap) || ring_big(h, hcap, (int)nside, bsmin)) return;
-    const int M = next_pow2(2 * h - 1);
-    const int64_t nring = 4 * nside - 1, npix = 12 * nside * nside;
-    const int64_t off = ring_offset(nside, r);
-    T2 *buf0 = reinterpret_cast<T2 *>(smem_raw);
-    T2 *buf1 = buf0 + mcap, *buf2 = buf1 + mcap;
-    const T2 *tw32 = TwTable<T2>::get(twall, twcnt);
-    const T2 *tw = tw32 + twiddle_offset(n);     // omega_n^k, k < h
-    const T2 *twM = tw32 + twiddle_offset(M);    // omega_M^k, k < M / 2 (M = 4i, i <= nside)
-    auto chirp = [&](int j) {
-        const unsigned q = ((unsigned)j * (unsigned)j) % (unsigned)n;
-        return twiddle_n(tw, h, (int)q, -1);
-    };
-    for (int m = threadIdx.x; m < M; m += blockDim.x) {
-        T2 v = make_float2(0.f, 0.f);
-        if (m < h) v = chirp(m);
-        else if (m > M - h) v = chirp(M - m);
-        v.y = -v.y;
-        buf0[m] = v;
-    }
-    __syncthreads();
-    const T2 *FB = fft_shared<1>(buf0, buf1, M, twM, -1);
-    T2 *X = (FB == buf0) ? buf1 : buf0;
-    T2 *Y = buf2;
-    const float invM = 1.0f / (float)M;
     const bool sh = shifted[r] != 0;
-    const float w = (float)(4.0 * M_PI / (double)npix);
-    const int64_t c1 = (int64_t)(blockIdx.x + 1) * cpc < ncomp ? (int64_t)(blockIdx.x + 1) * cpc : ncomp;
-    for (int64_t c = (int64_t)blockIdx.x * cpc; c < c1; ++c) {
-        for (int j = h + threadIdx.x; j < M; j += blockDim.x) X[j] = make_float2(0.f, 0.f);
-        load_ring<float>(maps + c * npix + off, mask ? mask + off : nullptr, h, X,
-                         [&](int t, T2 z) { return cmul(z, chirp(t)); });
-        __syncthreads();
-        T2 *FA = fft_shared<1>(X, Y, M, twM, -1);
-        T2 *G = (FA == X) ? Y : X;
-        for (int m = threadIdx.x; m < M; m += blockDim.x) {
-            T2 v = cmul(FA[m], FB[m]);
-            v.x *= invM;
-            v.y *= invM;
-            FA[m] = v;
+    T2 *b0 = reinterpret_cast<T2 *>(smem_raw), *b1 = b0 + buf, *b2 = b1 + buf;
+    const T2 *twT = TwTable<T2>::get(twall, twcnt);
+    const T2 *tw = twT + twiddle_offset(n);
+    const int M = bs ? next_pow2(2 * h - 1) : 0;
+    const T2 *twM = bs ? twT + twiddle_offset(M) : nullptr;
+    T2 *FB = nullptr, *X = b0, *Y = b1;
+    if (bs) {
+        FB = bs_filter(h, n, M, tw, twM, -1, b0, b1);
+        X = FB == b0 ? b1 : b0;
+        Y = b2;
+    }
+    const T w = (T)(4.0 * M_PI / (double)npix);
+    const int64_t cend = (int64_t)(blockIdx.x + 1) * cpc < ncomp ? (int64_t)(blockIdx.x + 1) * cpc : ncomp;
+    for (int64_t c = (int64_t)blockIdx.x * cpc; c < cend; ++c) {
+        const double *mk = mask ? mask + off : nullptr;
+        const T2 *Z;
+        if (bs) {
+            load_ring<T>(maps + c * npix + off, mk, vec, h, X,
+                         [&](int t, T2 z) { return cmul(z, bs_chirp(tw, h, n, t, -1)); });
+            __syncthreads();
+            Z = bs_apply(X, Y, FB, h, n, M, tw, twM, -1);
+        } else {
+            load_ring<T>(maps + c * npix + off, mk, vec, h, X, [](int, T2 z) { return z; });
+            __syncthreads();
+            Z = fft_shared(X, Y, h, tw, -1);
         }
-        __syncthreads();
-        T2 *R = fft_shared<1>(FA, G, M, twM, +1);
-        T2 *Z = (R == FA) ? G : FA;
-        for (int k = threadIdx.x; k < h; k += blockDim.x) Z[k] = cmul(R[k], chirp(k));
-        __syncthreads();
-        ring_outputs<float>(Z, n, L, tw, sh, w, out + (c * nring + r) * L);
+        ring_outputs<T>(Z, n, L, tw, sh, w, out + (c * nring + r) * L);
         __syncthreads();
     }
 }
@@ -768,10 +744,7 @@ __global__ void __launch_bounds__(512) k_ring_synthesis(int64_t nside, int64_t L
 
 
 // Inverse ring transform from the folded spectra of k_fold_lanes: one CTA per (ring, block of
-// cpc components).  i0 > 0: the cap rings of length 4 i, i0 <= i < i0 + cnt, of both
-// hemispheres; i0 = 0: the belt.  Rings whose half-length has a prime factor above 64 go through
-// Bluestein's method (M <= mcap: three buffers of M), the others through the mixed-radix FFT.
-// A launch covers rings of one shared-memory size, so that short rings run many CTAs per SM.
+// cpc components), with the rings and buffers of k_ring_forward.
 // With the fold before it: 2235 -> 790 us for a (Q, U) pair at Nside 1024 (a ring per CTA reading
 // its coefficients 128 lanes apart and taking prime factors up to 1021 as one radix), 163 -> 61
 // us for one FP64 map at Nside 256.
@@ -785,8 +758,8 @@ __global__ void __launch_bounds__(512) k_ring_inverse(int64_t nside, int64_t nco
 {
     using T2 = typename vec2<T>::type;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int64_t b = blockIdx.y, nring = 4 * nside - 1, npix = 12 * nside * nside;
-    const int64_t r = i0 == 0 ? nside - 1 + b : (b < cnt ? i0 - 1 + b : 4 * nside - 1 - (i0 + b - cnt));
+    const int64_t nring = 4 * nside - 1, npix = 12 * nside * nside;
+    const int64_t r = launch_ring(nside, i0, cnt, blockIdx.y);
     const int n = (int)ring_nphi(nside, r), h = n / 2;
     const bool bs = mcap > 0 && use_bluestein(h, mcap);
     if (hcap > 0 && ring_big(h, hcap, (int)nside, bsmin)) return;   // left to k_ring_synthesis_big
@@ -887,12 +860,12 @@ __global__ void __launch_bounds__(512) k_ring_analysis_big(int64_t nside, int64_
             for (int64_t c = 0; c < ncomp; ++c) {
                 float2 *Z;
                 if (bs) {
-                    load_ring<float>(maps + c * npix + off, mask ? mask + off : nullptr, h, X,
+                    load_ring<float>(maps + c * npix + off, mask ? mask + off : nullptr, false, h, X,
                                      [&](int t, float2 z) { return cmul(z, bs_chirp(tw, h, n, t, -1)); });
                     __syncthreads();
                     Z = bs_apply(X, Y, FB, h, n, M, tw, twM, -1);
                 } else {
-                    load_ring<float>(maps + c * npix + off, mask ? mask + off : nullptr, h, X,
+                    load_ring<float>(maps + c * npix + off, mask ? mask + off : nullptr, false, h, X,
                                      [](int, float2 z) { return z; });
                     __syncthreads();
                     Z = fft_shared(X, Y, h, tw, -1);
@@ -902,7 +875,7 @@ __global__ void __launch_bounds__(512) k_ring_analysis_big(int64_t nside, int64_
             }
         } else {
             for (int64_t c = 0; c < ncomp; ++c) {
-                load_ring<T>(maps + c * npix + off, mask ? mask + off : nullptr, h, b0,
+                load_ring<T>(maps + c * npix + off, mask ? mask + off : nullptr, false, h, b0,
                              [](int, T2 z) { return z; });
                 __syncthreads();
                 T2 *Z = fft_shared(b0, b1, h, tw, -1);
@@ -1052,84 +1025,98 @@ extern "C" int64_t gm_ring_big_scratch_bytes(int64_t nside, int64_t nslots)
     return nside < 1 || nslots < 1 ? 0 : nslots * 3 * 4 * nside * (int64_t)sizeof(float2);
 }
 
+// Whether some ring goes to the *_big kernels (ring_big of the longest ring).
+static bool any_ring_big(int64_t nside, int hcap, int bsmin)
+{
+    return 2 * nside > hcap || (bsmin > 0 && next_pow2((int)(4 * nside - 1)) > bsmin);
+}
+
+// The launches of the ring kernels: the belt (length 4 nside), then the caps by powers of two of
+// their length.  run(i0, cnt, buf, buffers, threads, mcap, rows): buf complex values in each of 2
+// buffers (3 with Bluestein rings, whose M fits buf).  Threads: an eighth of the points where the
+// rings of all components fill the chip many times over (64 maps at Nside 512: 5.5 -> 4.0 ms),
+// else two to four times as many, for the latency of a ring (one FP64 map at Nside 256: 66 us
+// with an eighth, 53 us).
+template <typename T, typename Run>
+static int for_ring_classes(int64_t nside, int64_t ncomp, int hcap, bool big, Run run)
+{
+    int mcap = bluestein_mcap(nside);
+    if (sizeof(T) == 8 && mcap > 4096) mcap = 4096;   // three buffers of M in 227 KB
+    auto one = [&](int64_t i0, int64_t cnt, int hmax, int M) {
+        if (big && hmax > hcap) hmax = hcap;          // longer rings go to the *_big kernels
+        const int buf = M > hmax ? M : hmax;
+        const int64_t rows = i0 ? 2 * cnt : 2 * nside + 1;
+        int threads = rows * ncomp >= 148 * 64 ? buf / 8 : (M ? buf / 4 : buf / 2);
+        threads = threads >= 512 ? 512 : (threads >= 256 ? 256 : (threads >= 128 ? 128 : 64));
+        return run(i0, cnt, buf, M ? 3 : 2, threads, M ? mcap : 0, rows);
+    };
+    const int hb = (int)(2 * nside);
+    int st = one(0, 0, hb, use_bluestein(hb, mcap) ? next_pow2(2 * hb - 1) : 0);
+    for (int64_t lo = 1, hi = 128; st == GM_OK && lo < nside; lo = hi + 1, hi *= 2) {
+        const int64_t top = hi < nside - 1 ? hi : nside - 1;
+        const int hm = (int)(2 * top), M = next_pow2(2 * hm - 1);
+        // above the first class every ring has the same M: beyond mcap none takes Bluestein
+        st = one(lo, top - lo + 1, hm, M <= mcap ? M : (lo == 1 ? mcap : 0));
+    }
+    return st;
+}
+
+template <typename T, typename Tin>
+static int ring_analysis(int64_t nside, int64_t L, int64_t ncomp, const void *maps, const double *mask, const void *tw,
+                         const uint8_t *shifted, void *ringspec, int hcap, int bsmin, bool big, void *scratch,
+                         int64_t slot, int64_t nslots, cudaStream_t s)
+{
+    using T2 = typename vec2<T>::type;
+    const int64_t twcnt = gm_ring_twiddle_count(nside), nring = 4 * nside - 1;
+    const bool vec = reinterpret_cast<uintptr_t>(maps) % (2 * sizeof(Tin)) == 0 && reinterpret_cast<uintptr_t>(mask) % 16 == 0;
+    int st = for_ring_classes<T>(nside, ncomp, hcap, big, [&](int64_t i0, int64_t cnt, int buf, int nbuf, int threads, int mcap, int64_t rows) {
+        const size_t bytes = (size_t)nbuf * buf * sizeof(T2);
+        const int e = set_smem(k_ring_forward<T, Tin>, bytes);
+        if (e) return e;
+        const int cpc = nbuf == 3 ? 8 : 1;   // components that share the transform of the chirp
+        dim3 grid((unsigned)((ncomp + cpc - 1) / cpc), (unsigned)rows);
+        k_ring_forward<T, Tin><<<grid, threads, bytes, s>>>(nside, L, ncomp, cpc, (const Tin *)maps, mask, vec, tw, twcnt,
+                                                            shifted, (T2 *)ringspec, i0, cnt, mcap, big ? hcap : 0, bsmin,
+                                                            buf);
+        return check_launch("gm_ring_analysis");
+    });
+    if (st || !big) return st;
+    const unsigned gbig = (unsigned)(nslots < nring ? nslots : nring);
+    k_ring_analysis_big<T, Tin><<<gbig, 512, 0, s>>>(nside, L, ncomp, (const Tin *)maps, mask, tw, twcnt, shifted,
+                                                     (T2 *)ringspec, hcap, bsmin, scratch, slot);
+    return check_launch("gm_ring_analysis");
+}
+
 extern "C" int gm_ring_analysis_ws(int precision, int64_t nside, int64_t L, int64_t ncomp,
                                    const void *maps, int map_dtype_bytes, const double *mask,
                                    const void *tw, const uint8_t *shifted, void *ringspec,
                                    void *scratch, int64_t scratch_bytes, int64_t hcap_max,
                                    int64_t bs_min, void *stream)
 {
-    const bool big = scratch != nullptr;
+    const bool ws = scratch != nullptr;
     if (nside < 1 || nside > 8192 || L < 1 || ncomp < 1 || ncomp > 65535) return GM_ERR_BAD_SHAPE;
-    if (!big && !ring_shape_ok(precision, nside, L, ncomp)) return GM_ERR_BAD_SHAPE;
+    if (!ws && !ring_shape_ok(precision, nside, L, ncomp)) return GM_ERR_BAD_SHAPE;
     if (!maps || !tw || !shifted || !ringspec) return GM_ERR_BAD_PTR;
     if (map_dtype_bytes != 8 && map_dtype_bytes != 4) return GM_ERR_UNSUPPORTED;
-    const int64_t nslots = big ? scratch_bytes / gm_ring_big_scratch_bytes(nside, 1) : 0;
-    if (big && nslots < 1) return GM_ERR_BAD_SHAPE;
-    const int64_t nring = 4 * nside - 1, cnt = gm_ring_twiddle_count(nside);
-    int hcap = ring_hcap(precision, nside, big);
-    if (big && hcap_max > 0 && hcap_max < hcap) hcap = (int)hcap_max;
-    // single precision only: FP64 has no Bluestein path
-    const int bsmin = big && precision == GM_MIXED ? (bs_min > 0 ? (int)bs_min : 8192) : 0;
-    const size_t smem = 2 * (size_t)hcap * (precision == GM_FP64 ? sizeof(double2) : sizeof(float2));
-    const int64_t slot = gm_ring_big_scratch_bytes(nside, 1);
-    int threads = nside >= 256 ? 512 : 128;
-    dim3 grid((unsigned)ncomp, (unsigned)nring);
+    if (precision != GM_FP64 && precision != GM_MIXED) return GM_ERR_UNSUPPORTED;
+    const int64_t slot = gm_ring_big_scratch_bytes(nside, 1), nslots = ws ? scratch_bytes / slot : 0;
+    if (ws && nslots < 1) return GM_ERR_BAD_SHAPE;
+    int hcap = ring_hcap(precision, nside, ws);
+    if (ws && hcap_max > 0 && hcap_max < hcap) hcap = (int)hcap_max;
+    // single precision only: FP64 has no Bluestein path in global memory
+    const int bsmin = ws && precision == GM_MIXED ? (bs_min > 0 ? (int)bs_min : 8192) : 0;
+    const bool big = ws && any_ring_big(nside, hcap, bsmin);
     cudaStream_t s = as_stream(stream);
-    int st;
+#define GM_RING(T, TIN)                                                                                           \
+    return ring_analysis<T, TIN>(nside, L, ncomp, maps, mask, tw, shifted, ringspec, hcap, bsmin, big, scratch,   \
+                                 slot, nslots, s)
     if (precision == GM_FP64) {
-        const unsigned gbig = (unsigned)(nslots < nring ? nslots : nring);
-        if (map_dtype_bytes == 8) {
-            if ((st = set_smem(k_ring_analysis<double, double>, smem))) return st;
-            k_ring_analysis<double, double><<<grid, threads, smem, s>>>(
-                nside, L, (const double *)maps, mask, tw, cnt, shifted, (double2 *)ringspec, 0, hcap, 0);
-            if (big)
-                k_ring_analysis_big<double, double><<<gbig, 512, 0, s>>>(
-                    nside, L, ncomp, (const double *)maps, mask, tw, cnt, shifted, (double2 *)ringspec,
-                    hcap, 0, scratch, slot);
-        } else {
-            if ((st = set_smem(k_ring_analysis<double, float>, smem))) return st;
-            k_ring_analysis<double, float><<<grid, threads, smem, s>>>(
-                nside, L, (const float *)maps, mask, tw, cnt, shifted, (double2 *)ringspec, 0, hcap, 0);
-            if (big)
-                k_ring_analysis_big<double, float><<<gbig, 512, 0, s>>>(
-                    nside, L, ncomp, (const float *)maps, mask, tw, cnt, shifted, (double2 *)ringspec,
-                    hcap, 0, scratch, slot);
-        }
-    } else if (precision == GM_MIXED) {
-        const int mcap = bluestein_mcap(nside);
-        const size_t bs_smem = 3 * (size_t)mcap * sizeof(float2);
-        const int cpc = 8;
-        dim3 bs_grid((unsigned)((ncomp + cpc - 1) / cpc), (unsigned)nring);
-        const unsigned gbig = (unsigned)(nslots < nring ? nslots : nring);
-        if (map_dtype_bytes == 8) {
-            if ((st = set_smem(k_ring_analysis<float, double>, smem))) return st;
-            k_ring_analysis<float, double><<<grid, threads, smem, s>>>(
-                nside, L, (const double *)maps, mask, tw, cnt, shifted, (float2 *)ringspec, mcap, hcap, bsmin);
-            if ((st = set_smem(k_ring_analysis_bluestein<double>, bs_smem))) return st;
-            k_ring_analysis_bluestein<double><<<bs_grid, 512, bs_smem, s>>>(
-                nside, L, ncomp, cpc, mcap, hcap, bsmin, (const double *)maps, mask, tw, cnt, shifted,
-                (float2 *)ringspec);
-            if (big)
-                k_ring_analysis_big<float, double><<<gbig, 512, 0, s>>>(
-                    nside, L, ncomp, (const double *)maps, mask, tw, cnt, shifted, (float2 *)ringspec,
-                    hcap, bsmin, scratch, slot);
-        } else {
-            if ((st = set_smem(k_ring_analysis<float, float>, smem))) return st;
-            k_ring_analysis<float, float><<<grid, threads, smem, s>>>(
-                nside, L, (const float *)maps, mask, tw, cnt, shifted, (float2 *)ringspec, mcap, hcap, bsmin);
-            if ((st = set_smem(k_ring_analysis_bluestein<float>, bs_smem))) return st;
-            k_ring_analysis_bluestein<float><<<bs_grid, 512, bs_smem, s>>>(
-                nside, L, ncomp, cpc, mcap, hcap, bsmin, (const float *)maps, mask, tw, cnt, shifted,
-                (float2 *)ringspec);
-            if (big)
-                k_ring_analysis_big<float, float><<<gbig, 512, 0, s>>>(
-                    nside, L, ncomp, (const float *)maps, mask, tw, cnt, shifted, (float2 *)ringspec,
-                    hcap, bsmin, scratch, slot);
-        }
-    } else {
-        return GM_ERR_UNSUPPORTED;
+        if (map_dtype_bytes == 8) GM_RING(double, double);
+        GM_RING(double, float);
     }
-    return check_launch("gm_ring_analysis");
+    if (map_dtype_bytes == 8) GM_RING(float, double);
+    GM_RING(float, float);
+#undef GM_RING
 }
 
 extern "C" int gm_ring_analysis(int precision, int64_t nside, int64_t L, int64_t ncomp,
@@ -1245,12 +1232,6 @@ extern "C" int gm_ring_synthesis(int precision, int64_t nside, int64_t L, int64_
                                 stream);
 }
 
-// Whether some ring goes to the *_big kernels (ring_big of the longest ring).
-static bool any_ring_big(int64_t nside, int hcap, int bsmin)
-{
-    return 2 * nside > hcap || (bsmin > 0 && next_pow2((int)(4 * nside - 1)) > bsmin);
-}
-
 extern "C" int64_t gm_ring_fold_bytes(int precision, int64_t nside)
 {
     if (nside < 1) return 0;
@@ -1264,37 +1245,22 @@ static int ring_synthesis_fold(int64_t nside, int64_t L, int64_t ncomp, const vo
 {
     using T2 = typename vec2<T>::type;
     const int64_t cnt = gm_ring_twiddle_count(nside), sstride = 2 * nside + 1;
-    const int hc = big ? hcap : 0;
-    int mcap = bluestein_mcap(nside);
-    if (sizeof(T) == 8 && mcap > 4096) mcap = 4096;   // three buffers of M in 227 KB
     for (int64_t c0 = 0; c0 < ncomp; c0 += chunk) {
         const int64_t cw = ncomp - c0 < chunk ? ncomp - c0 : chunk;
         fold_lanes<T, false>(nside, L, ncomp, c0, cw, syn, nullptr, shifted, nullptr, work, sstride, s);
         int st = check_launch("gm_ring_synthesis_fold");
         if (st) return st;
-        // rings up to half-length hmax, with buffers for Bluestein rings of length M (0: none)
-        auto run = [&](int64_t i0, int64_t n, int hmax, int M) {
-            const int cpc = 8, buf = M > hmax ? M : hmax;
-            const size_t bytes = (size_t)(M ? 3 : 2) * buf * sizeof(T2);
-            int e = set_smem(k_ring_inverse<T>, bytes);
+        st = for_ring_classes<T>(nside, cw, hcap, big, [&](int64_t i0, int64_t n, int buf, int nbuf, int threads, int mcap, int64_t rows) {
+            const size_t bytes = (size_t)nbuf * buf * sizeof(T2);
+            const int e = set_smem(k_ring_inverse<T>, bytes);
             if (e) return e;
-            const int threads = hmax <= 256 ? 128 : (hmax <= 512 ? 256 : 512);
-            dim3 grid((unsigned)((cw + cpc - 1) / cpc), (unsigned)(i0 ? 2 * n : 2 * nside + 1));
-            k_ring_inverse<T><<<grid, threads, bytes, s>>>(nside, cw, cpc, sstride, (const T2 *)work, tw, cnt, shifted,
-                                                           maps, c0, i0, n, M ? mcap : 0, hc, bsmin, buf);
+            const int cpc = nbuf == 3 ? 8 : 1;
+            dim3 grid((unsigned)((cw + cpc - 1) / cpc), (unsigned)rows);
+            k_ring_inverse<T><<<grid, threads, bytes, s>>>(nside, cw, cpc, sstride, (const T2 *)work, tw, cnt, shifted, maps,
+                                                           c0, i0, n, mcap, big ? hcap : 0, bsmin, buf);
             return check_launch("gm_ring_synthesis_fold");
-        };
-        // the belt (length 4 nside), then the caps by powers of two of their length
-        const int hb = (int)(2 * nside);
-        const int hfit = big && hb > hcap ? hcap : hb;
-        if ((st = run(0, 0, hfit, use_bluestein(hb, mcap) ? next_pow2(2 * hb - 1) : 0))) return st;
-        for (int64_t lo = 1, hi = 128; lo < nside; lo = hi + 1, hi *= 2) {
-            const int64_t top = hi < nside - 1 ? hi : nside - 1;
-            const int hm = (int)(2 * top), M = next_pow2(2 * hm - 1);
-            // above the first class every ring has the same M: beyond mcap none takes Bluestein
-            const int Mc = M <= mcap ? M : (lo == 1 ? mcap : 0);
-            if ((st = run(lo, top - lo + 1, big && hm > hcap ? hcap : hm, Mc))) return st;
-        }
+        });
+        if (st) return st;
     }
     return GM_OK;
 }
