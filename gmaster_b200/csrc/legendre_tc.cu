@@ -737,34 +737,35 @@ __global__ void k_prep_syn(int64_t lmax, int spin, int sp, int H, int NR,
 // and n - k read each other's orders, so they are summed together and every synthesis
 // value is read once.  The image of order m = k + t n is then
 //   (-1)^t w n P_k - rhs(m), scaled by `scale`, as f16 hi/lo.
-// Reads the synthesis and rhs_map once, writes each image row once (coalesced across the
-// row threads); rows beyond 2H and the absent south ring of the equator lane keep the
-// zeros the pack wrote.
-// Occupancy bound per spin (measured at Nside 2048: spin 0 without spills at 16 CTAs per SM,
-// 15.0 -> 11.6 ms; spin 2 at 10, 23.9 -> 21.7 ms, where 16 would spill).
+// A thread takes the two rows (re, im) of one item and hemisphere: 8-byte loads of the synthesis,
+// one right-hand side for both rows, 4-byte stores of the images, and the conjugation is a sign
+// of the second row.  The residue pairs of a lane are spread over grid.y CTAs, and rings of few
+// residues sum their aliases with several loads in flight.  Rows beyond 2H and the absent south
+// ring of the equator lane keep the zeros the pack wrote.
+// Bound by memory: reads the synthesis and rhs_map once, writes each image row once.  One CTA per
+// lane with a thread per row and 2-byte stores took 2.03 ms for 32 (Q, U) fields at Nside 512 (2.4
+// TB/s) and 0.92 ms for 16 at Nside 256, where 512 CTAs leave the chip half idle; 0.94 and 0.24
+// ms here.
 template <int SPIN>
-__global__ void __launch_bounds__(128, SPIN == 0 ? 16 : 10) k_fold_tc(int64_t nside, int64_t L, int ncomp,
-                                                 const float *__restrict__ synd_a,
-                                                 const float *__restrict__ synd_b, int R2,
-                                                 const float4 *__restrict__ rhs_map,
-                                                 const uint8_t *__restrict__ shifted,
-                                                 uint8_t *__restrict__ img_a,
-                                                 uint8_t *__restrict__ img_b, float scale)
+__global__ void __launch_bounds__(64, SPIN == 0 ? 24 : 16) k_fold_tc(int64_t nside, int64_t L, int ncomp,
+                                                const float *__restrict__ synd_a,
+                                                const float *__restrict__ synd_b, int R2,
+                                                const float4 *__restrict__ rhs_map,
+                                                const uint8_t *__restrict__ shifted,
+                                                uint8_t *__restrict__ img_a,
+                                                uint8_t *__restrict__ img_b, float scale)
 {
     const int64_t j = blockIdx.x;
-    const int r = threadIdx.x;
     const int64_t nlanes = 2 * nside, npix = 12 * nside * nside, NG = (nlanes + kKC - 1) / kKC;
     const int n = (int)ring_nphi(nside, north_ring(j));
     const bool sh = shifted[north_ring(j)] != 0;
     const int H = SPIN == 0 ? 2 * ncomp : ncomp;
+    const int r = 2 * (int)threadIdx.x;                 // rows r (re) and r + 1 (im) of an item
     const bool south = r >= H;
     if (r >= 2 * H || (south && j == nlanes - 1)) return;
     const float wn = (float)(4.0 * M_PI / (double)npix * (double)n);
-    const int rr = south ? r - H : r;
-    const int item = rr >> 1;
-    const bool im = rr & 1;
-    const float cs = im ? -1.0f : 1.0f;                 // conjugation of this row
-    const int64_t stride = nlanes * R2;
+    const int item = (south ? r - H : r) >> 1;
+    const int64_t stride = nlanes * R2;                 // floats between orders
     const float *pa = synd_a + j * R2 + r;
     const float *pb = (SPIN ? synd_b : synd_a) + j * R2 + r;
     const uint32_t roff = tc::sw128_mn_offset(128, (uint32_t)r, (uint32_t)(j % kKC));
@@ -773,111 +774,104 @@ __global__ void __launch_bounds__(128, SPIN == 0 ? 16 : 10) k_fold_tc(int64_t ns
     uint8_t *ib = SPIN ? img_b + (j / kKC) * 2 * (int64_t)kAImg + roff : nullptr;
     const float4 *rb = rhs_map + j * ncomp;
 
-    // rhs of this row at order m for variant v (0: image a, 1: image b)
-    auto rhs = [&](int64_t m, int v) -> float {
+    auto ld = [&](const float *p, int64_t m) { return *reinterpret_cast<const float2 *>(p + m * stride); };
+    auto put = [&](uint8_t *img, int64_t m, float x, float y) {
+        const __half2 hi = __floats2half2_rn(x, y);
+        const float2 h = __half22float2(hi);
+        *reinterpret_cast<__half2 *>(img + m * istride) = hi;
+        *reinterpret_cast<__half2 *>(img + m * istride + kAImg) = __floats2half2_rn(x - h.x, y - h.y);
+    };
+    // images of order m: f times the folded sums less the right-hand side
+    auto out = [&](int64_t m, float f, float2 sa, float2 sb) {
         const float4 *b = rb + m * nlanes * ncomp;
         if (SPIN == 0) {
             const float4 q = b[item];
-            return south ? (im ? q.w : q.z) : (im ? q.y : q.x);
+            put(ia, m, (f * sa.x - (south ? q.z : q.x)) * scale, (f * sa.y - (south ? q.w : q.y)) * scale);
+            return;
         }
         const float4 q = b[2 * item], u = b[2 * item + 1];
         const float qr = south ? q.z : q.x, qi = south ? q.w : q.y;
         const float ur = south ? u.z : u.x, ui = south ? u.w : u.y;
         // image a rows [P_N | M_S], image b rows [M_N | P_S]; P = Q + iU, M = Q - iU
-        const bool plus = (v == 0) ? !south : south;
-        return plus ? (im ? qi + ur : qr - ui) : (im ? qi - ur : qr + ui);
+        const float2 P = make_float2(qr - ui, qi + ur), M = make_float2(qr + ui, qi - ur);
+        const float2 ra = south ? M : P, rv = south ? P : M;
+        put(ia, m, (f * sa.x - ra.x) * scale, (f * sa.y - ra.y) * scale);
+        put(ib, m, (f * sb.x - rv.x) * scale, (f * sb.y - rv.y) * scale);
     };
-    auto put = [&](uint8_t *img, int64_t m, float val) {
-        const float x = val * scale;
-        const __half hi = __float2half_rn(x);
-        const __half lo = __float2half_rn(x - __half2float(hi));
-        *reinterpret_cast<__half *>(img + m * istride) = hi;
-        *reinterpret_cast<__half *>(img + m * istride + kAImg) = lo;
-    };
-    // write the images of residue k from its sums (pa_k: variant a, pb_k: variant b)
-    auto emit = [&](int k, float sa, float sb) {
+    auto emit = [&](int k, float2 sa, float2 sb) {
         int t = 0;
+#pragma unroll 2
+        for (int64_t m = k; m < L; m += n, ++t) out(m, (sh && (t & 1)) ? -wn : wn, sa, sb);
+    };
+    // sums over the orders k + t n with the sign (-1)^t of a shifted ring
+    auto sums = [&](int k, float2 &A, float2 &B) {
+        A = B = make_float2(0.f, 0.f);
+        int t = 0;
+#pragma unroll 4
         for (int64_t m = k; m < L; m += n, ++t) {
-            const float f = (sh && (t & 1)) ? -wn : wn;
-            put(ia, m, f * sa - rhs(m, 0));
-            if (SPIN) put(ib, m, f * sb - rhs(m, 1));
+            const float sg = (sh && (t & 1)) ? -1.f : 1.f;
+            const float2 a = ld(pa, m);
+            A.x += sg * a.x;
+            A.y += sg * a.y;
+            if (SPIN) {
+                const float2 b = ld(pb, m);
+                B.x += sg * b.x;
+                B.y += sg * b.y;
+            }
         }
+        if (!SPIN) B = A;
     };
     const float neg = sh ? -1.0f : 1.0f;   // sign of an order read as a negative alias, relative
                                            // to its sign as a positive alias
+    // P + neg conj(Q)
+    auto with_conj = [&](float2 P, float2 Q) { return make_float2(P.x + neg * Q.x, P.y - neg * Q.y); };
 
+    // this CTA's residue pairs (k, n - k), k <= n / 2
+    const int np = n / 2 + 1, per = (np + (int)gridDim.y - 1) / (int)gridDim.y;
+    int k = (int)blockIdx.y * per;
+    const int kend = k + per < np ? k + per : np;
+    if (k == 0 && kend > 0) {
+        // residue 0: orders t n, and their conjugates as negative aliases for t >= 1
+        float2 A, B;
+        sums(0, A, B);
+        const float2 a0 = ld(pa, 0), b0 = SPIN ? ld(pb, 0) : a0;
+        const float2 A1 = make_float2(A.x - a0.x, A.y - a0.y), B1 = make_float2(B.x - b0.x, B.y - b0.y);
+        emit(0, make_float2(A.x + B1.x, A.y - B1.y), make_float2(B.x + A1.x, B.y - A1.y));
+        ++k;
+    }
     if (n >= L) {
         // rings at least as long as lmax + 1 (the belt): order k is its residue's only
         // positive alias and n - k (when below L) its only negative one, so the residue
-        // pairs are independent and the loop keeps several loads in flight.  The same
-        // sums as the general loop below, in the same order of operations.
-        emit(0, pa[0], pb[0]);
+        // pairs are independent and the loop keeps several loads in flight
 #pragma unroll 4
-        for (int k = 1; k <= n / 2 && k < L; ++k) {
+        for (; k < kend; ++k) {
+            if (k >= L) break;
             const int k2 = n - k;
-            const float ak = pa[(int64_t)k * stride], bk = SPIN ? pb[(int64_t)k * stride] : ak;
+            const float2 ak = ld(pa, k), bk = SPIN ? ld(pb, k) : ak;
             if (k2 == k) {
-                put(ia, k, wn * (ak + neg * cs * bk) - rhs(k, 0));
-                if (SPIN) put(ib, k, wn * (bk + neg * cs * ak) - rhs(k, 1));
+                out(k, wn, with_conj(ak, bk), with_conj(bk, ak));
             } else if (k2 < L) {
-                const float a2 = pa[(int64_t)k2 * stride], b2 = SPIN ? pb[(int64_t)k2 * stride] : a2;
-                put(ia, k, wn * (ak + neg * cs * b2) - rhs(k, 0));
-                if (SPIN) put(ib, k, wn * (bk + neg * cs * a2) - rhs(k, 1));
-                put(ia, k2, wn * (neg * cs * bk + a2) - rhs(k2, 0));
-                if (SPIN) put(ib, k2, wn * (neg * cs * ak + b2) - rhs(k2, 1));
+                const float2 a2 = ld(pa, k2), b2 = SPIN ? ld(pb, k2) : a2;
+                out(k, wn, with_conj(ak, b2), with_conj(bk, a2));
+                out(k2, wn, with_conj(a2, bk), with_conj(b2, ak));
             } else {
-                put(ia, k, wn * ak - rhs(k, 0));
-                if (SPIN) put(ib, k, wn * bk - rhs(k, 1));
+                out(k, wn, ak, bk);
             }
         }
         return;
     }
-
-    // residue 0: orders t n (t >= 0), and t n (t >= 1) as negative aliases
-    {
-        float s0a = 0.f, s0b = 0.f;
-        int t = 0;
-        for (int64_t mm = 0; mm < L; mm += n, ++t) {
-            const float sg = (sh && (t & 1)) ? -1.f : 1.f;
-            const float a = pa[mm * stride], b = SPIN ? pb[mm * stride] : a;
-            s0a += sg * a;
-            if (SPIN) s0b += sg * b;
-            if (mm > 0) {
-                s0a += sg * cs * b;                 // conj of the partner row
-                if (SPIN) s0b += sg * cs * a;
-            }
-        }
-        emit(0, s0a, s0b);
-    }
-    // residue pairs (k, n - k), 0 < k < n / 2, and the self-paired residue n / 2
-    for (int k = 1; 2 * k <= n && k < L; ++k) {
+    for (; k < kend; ++k) {
+        if (k >= L) break;
         const int k2 = n - k;
-        float pka = 0.f, pkb = 0.f, p2a = 0.f, p2b = 0.f;
-        int t = 0;
-        for (int64_t mm = k; mm < L; mm += n, ++t) {
-            const float sg = (sh && (t & 1)) ? -1.f : 1.f;
-            const float a = pa[mm * stride], b = SPIN ? pb[mm * stride] : a;
-            pka += sg * a;
-            if (SPIN) pkb += sg * b;
-            p2a += neg * sg * cs * b;
-            if (SPIN) p2b += neg * sg * cs * a;
+        float2 A, B, A2, B2;
+        sums(k, A, B);
+        if (k2 == k) {
+            emit(k, with_conj(A, B), with_conj(B, A));
+            continue;
         }
-        if (k2 != k) {
-            t = 0;
-            for (int64_t mm = k2; mm < L; mm += n, ++t) {
-                const float sg = (sh && (t & 1)) ? -1.f : 1.f;
-                const float a = pa[mm * stride], b = SPIN ? pb[mm * stride] : a;
-                p2a += sg * a;
-                if (SPIN) p2b += sg * b;
-                pka += neg * sg * cs * b;
-                if (SPIN) pkb += neg * sg * cs * a;
-            }
-            emit(k, pka, pkb);
-            if (k2 < L) emit(k2, p2a, p2b);
-        } else {
-            // k = n / 2: the set is its own partner; p2 holds the conjugate part
-            emit(k, pka + p2a, pkb + p2b);
-        }
+        sums(k2, A2, B2);
+        emit(k, with_conj(A, B2), with_conj(B, A2));
+        if (k2 < L) emit(k2, with_conj(A2, B), with_conj(B2, A));
     }
 }
 
@@ -1192,7 +1186,10 @@ extern "C" int gm_tc_fold(int64_t nside, int64_t lmax, int spin, int64_t ncomp, 
         return GM_ERR_BAD_PTR;
     const int H = spin == 0 ? (int)(2 * ncomp) : (int)ncomp;
     auto kern = spin == 0 ? k_fold_tc<0> : k_fold_tc<2>;
-    kern<<<(unsigned)(2 * nside), 128, 0, as_stream(stream)>>>(
+    // residue pairs over enough CTAs for two rounds of a full chip (24 of 64 threads per SM)
+    const int64_t want = 2 * 148 * 24, split = (want + 2 * nside - 1) / (2 * nside);
+    const dim3 grid((unsigned)(2 * nside), (unsigned)(split < 16 ? split : 16));
+    kern<<<grid, (H + 31) / 32 * 32, 0, as_stream(stream)>>>(
         nside, lmax + 1, (int)ncomp, synd_a, synd_b, 2 * H, (const float4 *)rhs_map, shifted,
         (uint8_t *)img_a, (uint8_t *)img_b, (float)img_scale);
     return check_launch("gm_tc_fold");
