@@ -10,83 +10,89 @@
 // within its ring): prev[p] = the masked pixel at or before p, next[p] = at or after p
 // (ring-local indices, -1 for a ring without masked pixels).  k_mask_apodize then visits
 // rings outwards from the query's own ring, alternating north and south, two candidates
-// per ring, and stops in each direction once the ring's latitude alone puts it beyond the
-// best chord found (or the apodisation radius).  The result is the exact minimum over all
-// masked pixels, like the k-d tree's.
+// per ring, passing over rings without a masked pixel within the radius of the query's warp
+// and those whose latitude alone puts them beyond the best chord found, until the latitude
+// alone exceeds the radius.  The result is the exact minimum over all masked pixels, like the
+// k-d tree's.
 //
 // Chords are evaluated as |v_q - v_c|^2 = dz^2 + ds^2 + 4 s_q s_c sin^2(dphi / 2) with
 // z = cos(theta), s = sin(theta): the same Euclidean distance between unit vectors, free of
 // the cancellation of 2 - 2 v_q.v_c at small separations.
-
-#include <climits>
 
 #include "gm_common.cuh"
 
 namespace gm {
 namespace {
 
-constexpr int kRunThreads = 1024;
+constexpr int kRunThreads = 512;
 constexpr int kApoThreads = 256;
 constexpr double kTwoPi = 6.283185307179586;   // 2 pi rounded to double, as numpy's 2*np.pi
 constexpr double kInvTwoPi = 0.15915494309189535;
 
-// One CTA per ring (grid-stride over rings).  Thread t scans a contiguous chunk of the ring;
-// two block-wide scans give the last masked pixel before each chunk and the first after.
+// One CTA per ring (grid-stride over rings).  The ring's masked pixels become one bit each (a
+// ballot per 32 pixels, read coalesced and once); one warp then finds for every word the last
+// non-empty word before it and the first after it, and every pixel takes its neighbours from
+// its own word or from those two.  Bound by memory (8 bytes read, 8 written a pixel): 105 -> 53 us
+// at Nside 1024 against block scans of per-thread chunks.
 __global__ void __launch_bounds__(kRunThreads) k_ring_runs(int64_t nside,
                                                            const double *__restrict__ mask,
                                                            int32_t *__restrict__ prev,
                                                            int32_t *__restrict__ next)
 {
-    __shared__ int sp[kRunThreads], sn[kRunThreads];
-    const int t = threadIdx.x;
+    extern __shared__ unsigned bits[];   // words of the ring, then the two neighbour lists
+    const int t = threadIdx.x, lane = t & 31;
     const int64_t nring = 4 * nside - 1;
+    const int wmax = (int)((4 * nside + 31) / 32);
+    int *before = reinterpret_cast<int *>(bits + wmax), *after = before + wmax;
     for (int64_t r = blockIdx.x; r < nring; r += gridDim.x) {
-        const int n = (int)ring_nphi(nside, r);
+        const int n = (int)ring_nphi(nside, r), nwords = (n + 31) / 32;
         const int64_t off = ring_offset(nside, r);
-        const int chunk = (n + kRunThreads - 1) / kRunThreads;
-        const int b = min(n, t * chunk), e = min(n, b + chunk);
-        int last = -1, first = INT_MAX;
-        for (int i = b; i < e; ++i) {
-            if (mask[off + i] <= 0.0) {
-                if (first == INT_MAX) first = i;
-                last = i;
-            }
+        for (int i = t; i < nwords * 32; i += kRunThreads) {
+            const unsigned w = __ballot_sync(0xffffffffu, i < n && mask[off + i] <= 0.0);
+            if (lane == 0) bits[i >> 5] = w;
         }
-        sp[t] = last;
-        sn[t] = first;
         __syncthreads();
-        // inclusive prefix max of sp (left to right) and suffix min of sn (right to left)
-        for (int d = 1; d < kRunThreads; d <<= 1) {
-            const int a = t >= d ? sp[t - d] : -1;
-            const int c = t + d < kRunThreads ? sn[t + d] : INT_MAX;
-            __syncthreads();
-            sp[t] = max(sp[t], a);
-            sn[t] = min(sn[t], c);
-            __syncthreads();
-        }
-        const int ring_last = sp[kRunThreads - 1], ring_first = sn[0];
-        int carry_p = t > 0 ? sp[t - 1] : -1;
-        int carry_n = t + 1 < kRunThreads ? sn[t + 1] : INT_MAX;
-        __syncthreads();   // every thread has read sp / sn before the next ring rewrites them
-        if (ring_last < 0) {
-            for (int i = b; i < e; ++i) {
-                prev[off + i] = -1;
-                next[off + i] = -1;
+        if (t < 64) {
+            // warp 0: last non-empty word at or before each word, warp 1: first at or after
+            const bool fwd = t < 32;
+            int carry = -1;
+            for (int base = 0; base < nwords; base += 32) {
+                const int k = base + lane, w = fwd ? k : nwords - 1 - k;
+                int v = k < nwords && bits[w] ? w : -1;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int u = __shfl_up_sync(0xffffffffu, v, o);
+                    if (lane >= o && v < 0) v = u;
+                }
+                if (v < 0) v = carry;
+                if (k < nwords) (fwd ? before : after)[w] = v;
+                carry = __shfl_sync(0xffffffffu, v, 31);
             }
-            continue;
         }
-        if (carry_p < 0) carry_p = ring_last;        // wrap: the ring's last masked pixel
-        if (carry_n == INT_MAX) carry_n = ring_first;  // wrap: the ring's first masked pixel
-        int run = carry_p;
-        for (int i = b; i < e; ++i) {
-            if (mask[off + i] <= 0.0) run = i;
-            prev[off + i] = run;
+        __syncthreads();
+        const int lastw = before[nwords - 1], firstw = after[0];
+        const int ring_last = lastw < 0 ? -1 : 32 * lastw + 31 - __clz(bits[lastw]);
+        const int ring_first = firstw < 0 ? -1 : 32 * firstw + __ffs(bits[firstw]) - 1;
+        for (int i = t; i < n; i += kRunThreads) {
+            const int w = i >> 5;
+            const unsigned own = bits[w];
+            const unsigned lo = own & (0xffffffffu >> (31 - (i & 31))), hi = own & (0xffffffffu << (i & 31));
+            int p, q;
+            if (lo) {
+                p = 32 * w + 31 - __clz(lo);
+            } else {
+                const int u = w > 0 ? before[w - 1] : -1;
+                p = u < 0 ? ring_last : 32 * u + 31 - __clz(bits[u]);   // wrap: the ring's last masked pixel
+            }
+            if (hi) {
+                q = 32 * w + __ffs(hi) - 1;
+            } else {
+                const int u = w + 1 < nwords ? after[w + 1] : -1;
+                q = u < 0 ? ring_first : 32 * u + __ffs(bits[u]) - 1;   // wrap: the ring's first masked pixel
+            }
+            prev[off + i] = p;
+            next[off + i] = q;
         }
-        run = carry_n;
-        for (int i = e - 1; i >= b; --i) {
-            if (mask[off + i] <= 0.0) run = i;
-            next[off + i] = run;
-        }
+        __syncthreads();   // every thread has read the words before the next ring rewrites them
     }
 }
 
@@ -141,9 +147,41 @@ __device__ __forceinline__ bool probe(int64_t nside, int64_t jj, const Rings &rg
     return true;
 }
 
+// Whether ring jj has a masked pixel that some pixel of ring j between longitudes phi_a and phi_b
+// could find within the radius: the longitudes within reach widen [phi_a, phi_b] by
+// 2 asin x <= 2 (x + (pi / 2 - 1) x^3) on [0, 1], x^2 = (chord2_max - lb) / w, taken with a margin for its
+// single-precision evaluation and one pixel each side.
+__device__ __forceinline__ bool ring_in_reach(int64_t nside, int64_t jj, double lb, double w, const Rings &rg,
+                                              const int32_t *__restrict__ prev, double phi_a, double phi_b,
+                                              double chord2_max)
+{
+    const int nn = (int)ring_nphi(nside, jj);
+    const int32_t *run = prev + ring_offset(nside, jj);
+    const float x2 = (float)((chord2_max - lb) / fmax(w, 1e-300)) * 1.0001f;
+    if (!(x2 < 1.0f)) return run[0] >= 0;   // the whole ring
+    const float x = sqrtf(x2);
+    const double reach = 2.0 * 1.0001 * (double)(x + 0.570797f * x * x2);
+    const double inv = rg.inv[jj], phi0 = rg.phi0[jj];
+    const double a = floor((phi_a - reach - phi0) * inv) - 1.0, b = ceil((phi_b + reach - phi0) * inv) + 1.0;
+    if (b - a + 1.0 >= (double)nn) return run[0] >= 0;
+    // a >= -2 nn and b <= 3 nn: both lie within a few turns
+    int k = (int)b % nn;
+    if (k < 0) k += nn;
+    const int c = run[k];   // the last masked pixel at or before the right end, cyclically
+    if (c < 0) return false;
+    const int back = c <= k ? k - c : k - c + nn;
+    return back <= (int)(b - a);
+}
+
 // mode 0: C1 taper, 1: C2 taper (out = mask * f(x) for unmasked pixels closer than the
 // radius, x = sqrt(0.5 d^2 / threshold)); mode 2: zeroing step (out = 0 for masked pixels
 // and for pixels closer than the radius to a masked one, else the mask value).
+//
+// Bound by the instructions of the probes.  A warp is 32 neighbouring pixels of one ring: its
+// lanes first test 32 rings at a time, outwards from the warp's own, for masked pixels within
+// reach of the whole warp, and only the rings found are probed per pixel, in the same order.
+// Most pixels have none: at Nside 1024 with a radius of one degree (36 rings) every pixel probed
+// them all, 2.29 ms; 0.39 ms here.
 __global__ void __launch_bounds__(kApoThreads) k_mask_apodize(
     int64_t nside, Rings rg, const double *__restrict__ mask,
     const int32_t *__restrict__ prev, const int32_t *__restrict__ next, double chord2_max,
@@ -153,24 +191,42 @@ __global__ void __launch_bounds__(kApoThreads) k_mask_apodize(
     const int64_t j = blockIdx.y;
     const int64_t n = ring_nphi(nside, j);
     const int64_t i = (int64_t)blockIdx.x * kApoThreads + threadIdx.x;
-    if (i >= n) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t iw = i - lane;   // the warp's first pixel
+    if (iw >= n) return;
     const int64_t p = ring_offset(nside, j) + i;
-    const double m = mask[p];
-    if (mode == 2 ? (m <= 0.0) : !(m > 0.0)) {
-        out[p] = mode == 2 ? 0.0 : m;
-        return;
-    }
+    const double m = i < n ? mask[p] : 0.0;
+    const bool search = i < n && (mode == 2 ? !(m <= 0.0) : m > 0.0);
+    if (i < n && !search) out[p] = mode == 2 ? 0.0 : m;
+    if (!__any_sync(0xffffffffu, search)) return;
     Query q;
     q.z = rg.z[j];
     q.s = rg.s[j];
     q.phi = fma((double)i, rg.step[j], rg.phi0[j]);
     q.best = chord2_max;
     q.found = false;
-    bool up = true, dn = true;
-    for (int64_t d = 0; up || dn; ++d) {
-        if (up) up = j + d < nring && probe(nside, j + d, rg, prev, next, q);
-        if (dn) dn = j - 1 - d >= 0 && probe(nside, j - 1 - d, rg, prev, next, q);
+    const double phi_a = fma((double)iw, rg.step[j], rg.phi0[j]);
+    const double phi_b = fma((double)(iw + 31 < n ? iw + 31 : n - 1), rg.step[j], rg.phi0[j]);
+    // slot 2 d: ring j + d, slot 2 d + 1: ring j - 1 - d
+    auto ring_of = [&](int64_t slot) { return (slot & 1) ? j - 1 - (slot >> 1) : j + (slot >> 1); };
+    for (int64_t base = 0;; base += 32) {
+        const int64_t jj = ring_of(base + lane);
+        bool near = false, hit = false;
+        if (jj >= 0 && jj < nring) {
+            const double dz = q.z - rg.z[jj], ds = q.s - rg.s[jj], lb = dz * dz + ds * ds;
+            near = lb < chord2_max;
+            if (near) hit = ring_in_reach(nside, jj, lb, 4.0 * q.s * rg.s[jj], rg, prev, phi_a, phi_b, chord2_max);
+        }
+        unsigned todo = __ballot_sync(0xffffffffu, hit);
+        while (todo) {
+            const int64_t ring = ring_of(base + __ffs(todo) - 1);
+            todo &= todo - 1;
+            if (search) probe(nside, ring, rg, prev, next, q);
+        }
+        // latitudes alone put every later ring out of reach (lb grows outwards)
+        if (!__any_sync(0xffffffffu, near)) break;
     }
+    if (!search) return;
     if (!q.found) {
         out[p] = m;
         return;
@@ -195,8 +251,9 @@ extern "C" int gm_mask_ring_runs(int64_t nside, const double *mask, int32_t *pre
     if (nside < 1 || nside > 16384) return GM_ERR_BAD_SHAPE;
     if (!mask || !prev || !next) return GM_ERR_BAD_PTR;
     const int64_t nring = 4 * nside - 1;
-    const int grid = (int)(nring < 296 ? nring : 296);
-    k_ring_runs<<<grid, kRunThreads, 0, as_stream(stream)>>>(nside, mask, prev, next);
+    const int grid = (int)(nring < 592 ? nring : 592);
+    const size_t smem = 3 * (size_t)((4 * nside + 31) / 32) * sizeof(int);   // 24 KB at Nside 16384
+    k_ring_runs<<<grid, kRunThreads, smem, as_stream(stream)>>>(nside, mask, prev, next);
     return check_launch("gm_mask_ring_runs");
 }
 

@@ -233,7 +233,8 @@ def mask_apodization(mask_in, aposize, apotype="C1"):
     scale = 2.5 if apotype == "Smooth" else 1.2
     if int(4 * npix * (1 - np.cos(scale * radius))) < 2:
         raise ValueError("Your apodization scale is too small for this pixel size")
-    if not bool((mask <= 0).any()):
+    # without a masked pixel nothing is smoothed (the C1 / C2 kernels then leave the mask as it is)
+    if apotype == "Smooth" and not bool((mask <= 0).any()):
         return result(mask.clone())
     dev = mask.device
     prev = torch.empty(npix, dtype=torch.int32, device=dev)
