@@ -24,6 +24,8 @@ that loop for a whole batch at once:
   maps overlaps the T transforms.
 """
 
+import copy
+
 import numpy as np
 import torch
 
@@ -93,8 +95,7 @@ def fields_from_maps(mask, maps, *, spin=None, n_iter=None, beam=None, lmax=None
     alms = alms[0] if len(alms) == 1 else torch.cat(alms)
     fields = []
     for i in range(nsims):
-        f = NmtField(mask_t, None, spin=spin, n_iter=n_iter, beam=beam, lmax=lmax, lite=True,
-                     precision=precision)
+        f = copy.copy(proto)   # the geometry, mask and beam of the batch
         f.alm = alms[i]
         fields.append(f)
     return fields

@@ -182,6 +182,7 @@ class Plan:
         # healpy packing helpers (host)
         m = np.arange(self.L)
         self.mstart = m * (2 * self.lmax + 1 - m) // 2
+        self._passes = {}   # (spin, ncomp, precision, kind, settings) -> tile and checkpoint arguments
 
 
 def get_plan(nside, lmax, device=None):
@@ -265,6 +266,25 @@ def pack_rhs(plan, spec, prec):
     return rhs
 
 
+def _pass_setup(plan, spin, ncomp, prec, kind):
+    """(tile, ck_args) of a Legendre pass, looked up once per plan, pass and settings; the tables
+    that ck_args points into are kept with it."""
+    from . import sht_tc
+
+    key = (spin, ncomp, prec, kind, autotune.autotune_enabled(), sht_tc.USE_CHECKPOINTS, sht_tc.USE_TILE_SKIP,
+           sht_tc.CK_MEMORY_SHARE)
+    have = plan._passes.get(key)
+    if have is None:
+        tile = autotune.tile_for(plan, spin, ncomp, prec, kind)
+        ck = ck_args(plan, spin, prec)
+        keep = None
+        if ck is not None:
+            tp = sht_tc.get_tc_plan(plan.nside, plan.lmax, plan.device)
+            keep = (tp.ck_segoff[spin], tp.ck[spin], tp.ck_masks.get(spin))
+        have = plan._passes[key] = (tile, ck, keep)
+    return have[0], have[1]
+
+
 def ck_args(plan, spin, prec):
     """Checkpoint-table arguments (segoff, state and shift of the s' = -s and +s variants,
     their lane-group masks or None)
@@ -313,8 +333,7 @@ def run_legendre(plan, spin, ncomp, prec, kind, tile, src, dst, scale=1.0, ck=No
 
 def legendre_analysis(plan, spin, rhs, alm, scale, prec):
     ncomp = rhs.shape[2]
-    tile = autotune.tile_for(plan, spin, ncomp, prec, "ana")
-    ck = ck_args(plan, spin, prec)
+    tile, ck = _pass_setup(plan, spin, ncomp, prec, "ana")
     _timed(f"legendre_analysis_s{spin}", plan, spin, ncomp,
            lambda: run_legendre(plan, spin, ncomp, prec, "ana", tile, rhs, alm, scale, ck))
 
@@ -322,8 +341,7 @@ def legendre_analysis(plan, spin, rhs, alm, scale, prec):
 def legendre_synthesis(plan, spin, alm, ncomp, prec, out=None):
     syn = out if out is not None else torch.empty(
         (plan.L, plan.nlanes, ncomp, 4), dtype=_real_dtype(prec), device=plan.device)
-    tile = autotune.tile_for(plan, spin, ncomp, prec, "syn")
-    ck = ck_args(plan, spin, prec)
+    tile, ck = _pass_setup(plan, spin, ncomp, prec, "syn")
     _timed(f"legendre_synthesis_s{spin}", plan, spin, ncomp,
            lambda: run_legendre(plan, spin, ncomp, prec, "syn", tile, alm, syn, ck=ck))
     return syn

@@ -162,8 +162,8 @@ _TARGET_LOG2 = 13
 
 def pow2_scale(t):
     """Power of two that brings max |t| to about 2^13 (1.0 for an all-zero tensor)."""
-    lo, hi = torch.aminmax(t)
-    amax = max(abs(float(lo)), abs(float(hi)))
+    lo, hi = torch.stack(torch.aminmax(t)).tolist()
+    amax = max(abs(lo), abs(hi))
     if not amax > 0.0 or not np.isfinite(amax):
         return 1.0
     return float(2.0 ** (_TARGET_LOG2 - int(np.ceil(np.log2(amax)))))
@@ -309,6 +309,18 @@ def _full_path_bytes(tp, spin, ncomp, n_iter):
     return max(spec + base, later)
 
 
+def _fits(need, share, device):
+    """Whether `need` bytes stay within `share` of the free device memory.  The driver's answer can
+    take tens of milliseconds on a shared machine, so it is asked only for buffers above an
+    eighth of the card; smaller ones are taken to fit, and a transform that runs out of memory
+    all the same starts again over windows of orders."""
+    if need <= torch.cuda.get_device_properties(device).total_memory // 8:
+        return True
+    free, _ = torch.cuda.mem_get_info(device)
+    free += torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
+    return need <= share * free
+
+
 def map2alm_tc(maps, spin, nside, lmax, n_iter, mask=None, window=None, ring_spectra=None):
     """Batched analysis: maps (ncomp, npix) float64/float32 CUDA -> (ncomp, nelem) complex128
     (spin 2: rows E, B per field), with n_iter Jacobi iterations.  `mask` (npix,), if
@@ -326,15 +338,25 @@ def map2alm_tc(maps, spin, nside, lmax, n_iter, mask=None, window=None, ring_spe
     _check_batch(spin, ncomp)
     tp = get_tc_plan(nside, lmax, maps.device)
     p = tp.plan
-    if window is None:
-        free, _ = torch.cuda.mem_get_info(p.device)
-        free += torch.cuda.memory_reserved(p.device) - torch.cuda.memory_allocated(p.device)
-        if _full_path_bytes(tp, spin, ncomp, n_iter) > 0.95 * free:
-            window = window_orders(tp, spin, ncomp)
+    if window is None and not _fits(_full_path_bytes(tp, spin, ncomp, n_iter), 0.95, p.device):
+        window = window_orders(tp, spin, ncomp)
     if window is not None:
         return map2alm_tc_windowed(maps, spin, nside, lmax, n_iter, mask=mask, window=window)
     if ring_spectra is not None and ring_spectra.shape != (ncomp, p.nring, p.L):
         raise ValueError("ring_spectra must be (ncomp, nring, L)")
+    try:
+        return _map2alm_full(tp, maps, spin, n_iter, mask, [ring_spectra])
+    except torch.cuda.OutOfMemoryError:
+        window = window_orders(tp, spin, ncomp)
+    return map2alm_tc_windowed(maps, spin, nside, lmax, n_iter, mask=mask, window=window)
+
+
+def _map2alm_full(tp, maps, spin, n_iter, mask, spectra):
+    """map2alm_tc with all orders at once; `spectra` is a one-element list (the ring spectra or
+    None) that is emptied, so that they are released after packing unless the caller holds them."""
+    p = tp.plan
+    ncomp = maps.shape[0]
+    ring_spectra = spectra.pop()
     spec = ring_spectra if ring_spectra is not None else sht.ring_analysis(p, maps, _lib.MIXED, mask=mask)
     ring_spectra = None   # the spectra are released after packing unless the caller holds them
     b = _Batch(tp, spin, ncomp)
@@ -466,21 +488,27 @@ def alm2map_tc(alm, spin, nside, lmax, window=None):
     b.from_api(alm.to(torch.complex128))
     H, _ = _rows(spin, ncomp)
     if window is None:
-        free, _ = torch.cuda.mem_get_info(p.device)
-        free += torch.cuda.memory_reserved(p.device) - torch.cuda.memory_allocated(p.device)
         full = (len(_variants(spin)) * p.L * p.nlanes * 2 * H * 4
                 + tp.nchunks[spin] * _lib.load().gm_tc_syn_image_bytes(1) + p.L * p.nlanes * ncomp * 16)
-        if full > 0.9 * free:
+        try:
+            if _fits(full, 0.9, p.device):
+                syn = _synthesis_full(b)
+            else:
+                window = window_orders(tp, spin, ncomp)
+        except torch.cuda.OutOfMemoryError:
             window = window_orders(tp, spin, ncomp)
     if window is not None:
         syn = _synthesis_windowed(b, int(max(1, min(p.L, window))))
-        maps = sht.ring_synthesis(p, syn, _lib.MIXED)
-        _check(tp)
-        return maps
-    synd = b.synthesis()
-    syn = torch.empty((p.L, p.nlanes, ncomp, 4), dtype=torch.float32, device=p.device)
-    _lib.call("gm_tc_synd_to_syn", p.nside, p.lmax, spin, ncomp, _lib.ptr(synd[0]),
-              _lib.ptr(synd[1]) if spin else None, _lib.ptr(syn), _lib.stream_handle(p.device))
     maps = sht.ring_synthesis(p, syn, _lib.MIXED)
     _check(tp)
     return maps
+
+
+def _synthesis_full(b):
+    """Ring coefficients syn (L, nlanes, ncomp, 4) float32 of the alm accumulator, all orders at once."""
+    p = b.tp.plan
+    synd = b.synthesis()
+    syn = torch.empty((p.L, p.nlanes, b.ncomp, 4), dtype=torch.float32, device=p.device)
+    _lib.call("gm_tc_synd_to_syn", p.nside, p.lmax, b.spin, b.ncomp, _lib.ptr(synd[0]),
+              _lib.ptr(synd[1]) if b.spin else None, _lib.ptr(syn), _lib.stream_handle(p.device))
+    return syn

@@ -52,9 +52,14 @@ class NmtMapInfo:
         self.nside = nside
         self.npix = 12 * nside ** 2
         self.nx = self.ny = -1
-        theta, phi0, nphi, offsets = sht.ring_geometry(nside)
-        self.theta, self.phi0, self.nphi, self.offsets = theta, phi0, nphi, offsets
         self.weight = 4 * np.pi / self.npix
+
+    def __getattr__(self, name):
+        # the ring geometry on first use: a field needs none of it on the host
+        if name in ("theta", "phi0", "nphi", "offsets"):
+            self.theta, self.phi0, self.nphi, self.offsets = sht.ring_geometry(self.nside)
+            return self.__dict__[name]
+        raise AttributeError(name)
 
     def __eq__(self, other):
         return isinstance(other, NmtMapInfo) and self.nside == other.nside
