@@ -13,6 +13,7 @@ variant of the reference are outside this build.
 """
 
 import ctypes
+import functools
 import itertools
 
 import numpy as np
@@ -124,6 +125,36 @@ def _kernels(cell, spins, lmax, l_toeplitz, l_exact, dl_band):
     return {k: (None if v is None else v.contiguous()) for k, v in out.items()}
 
 
+@functools.lru_cache(maxsize=64)
+def _term_table(nmaps, have):
+    """Term table of the components `nmaps` of the four fields and the kernels present per
+    contraction: ((wick, name) of every kernel used, (kernel, row of A, row of B) and sign of
+    every term, term range of every output block)."""
+    na, nb, nc, nd = nmaps
+    off = (0, na * nc, na * nc + na * nd, na * nc + na * nd + nb * nc)
+    kindex, rows, signs, bptr = {}, [], [], [0]
+    outputs = itertools.product(range(na), range(nb), range(nc), range(nd))
+    for ia, ib, ic, id_ in outputs:
+        inputs = itertools.product(range(na), range(nb), range(nc), range(nd), range(2))
+        for iap, ibp, icp, idp, wick in inputs:
+            if wick == 0:   # <a1 b1><a2 b2>
+                fa = _family(na, nc, ia, ic, iap, icp)
+                fb = _family(nb, nd, ib, id_, ibp, idp)
+                ra, rb = off[0] + icp + nc * iap, off[3] + idp + nd * ibp
+            else:           # <a1 b2><a2 b1>
+                fa = _family(na, nd, ia, id_, iap, idp)
+                fb = _family(nb, nc, ib, ic, ibp, icp)
+                ra, rb = off[1] + idp + nd * iap, off[2] + icp + nc * ibp
+            sign, name = _paired(fa, fb)
+            if name is None or name not in have[wick]:
+                continue
+            kindex.setdefault((wick, name), len(kindex))
+            rows.append((kindex[wick, name], ra, rb))
+            signs.append(sign)
+        bptr.append(len(rows))
+    return tuple(kindex), tuple(rows), tuple(signs), tuple(bptr)
+
+
 class NmtCovarianceWorkspace:
     """Coupling kernels for the Gaussian covariance of the spectra of (fla1, fla2) and
     (flb1, flb2) (covariance.py:197-660): same interface as the reference's."""
@@ -193,33 +224,9 @@ class NmtCovarianceWorkspace:
         """Flattened term table: per output block X = (ia nb + ib) nclsb + (ic nd + id) the
         (kernel, row of A, row of B, sign) of every non-zero term (covariance.py:407-429),
         with rows into the concatenated spectra [c11; c12; c21; c22]."""
-        na, nb, nc, nd = self.nmaps
-        off = (0, na * nc, na * nc + na * nd, na * nc + na * nd + nb * nc)
-        kernels, kindex = [], {}
-        rows, signs, bptr = [], [], [0]
-        outputs = itertools.product(range(na), range(nb), range(nc), range(nd))
-        for ia, ib, ic, id_ in outputs:
-            inputs = itertools.product(range(na), range(nb), range(nc), range(nd), range(2))
-            for iap, ibp, icp, idp, wick in inputs:
-                if wick == 0:   # <a1 b1><a2 b2>
-                    fa = _family(na, nc, ia, ic, iap, icp)
-                    fb = _family(nb, nd, ib, id_, ibp, idp)
-                    ra, rb = off[0] + icp + nc * iap, off[3] + idp + nd * ibp
-                else:           # <a1 b2><a2 b1>
-                    fa = _family(na, nd, ia, id_, iap, idp)
-                    fb = _family(nb, nc, ib, ic, ibp, icp)
-                    ra, rb = off[1] + idp + nd * iap, off[2] + icp + nc * ibp
-                sign, name = _paired(fa, fb)
-                xi = None if name is None else self.xiSS[wick][name]
-                if xi is None:
-                    continue
-                if (wick, name) not in kindex:
-                    kindex[wick, name] = len(kernels)
-                    kernels.append(xi)
-                rows.append((kindex[wick, name], ra, rb))
-                signs.append(sign)
-            bptr.append(len(rows))
-        return kernels, rows, signs, bptr
+        have = tuple(tuple(n for n in KERNEL_NAMES if xi[n] is not None) for xi in self.xiSS)
+        used, rows, signs, bptr = _term_table(self.nmaps, have)
+        return [self.xiSS[wick][name] for wick, name in used], list(rows), list(signs), list(bptr)
 
     def gaussian_covariance(self, cla1b1, cla1b2, cla2b1, cla2b2, wa, wb=None, coupled=False):
         """Covariance of the two power spectra: (nbands_a ncls_a, nbands_b ncls_b) for the
