@@ -356,28 +356,33 @@ __global__ void k_toeplitz_fill(int64_t lmax, int64_t lt, int64_t le, int64_t dl
 
 // ---------------------------------------------------------------- binning
 
-// Binned block: out[b][b'] = sum_{l in b} wfl[l] sum_{l' in b'} M[l][l'] beam[l'] inv_fl[l'].
-__global__ void k_bin_block(int64_t lmax, int64_t nb, const double *__restrict__ M,
-                            const int32_t *__restrict__ band_ptr, const int32_t *__restrict__ band_ells,
-                            const double *__restrict__ wfl, const double *__restrict__ inv_fl,
-                            const double *__restrict__ beam, double *__restrict__ out)
+// Binned block: out[b][b'] = sum_{l in b} wfl[l] sum_{l' in b'} M[l][l'] beam[l'] inv_fl[l'].  One warp
+// per pair of bands: lanes along l', the rows of b in turn (several loads in flight), then a sum
+// over the lanes.  A CTA of 256 threads per pair, with a division per element and a tree in
+// shared memory, took 38 us a block at lmax 1535 with bands of ten; 16 us here.
+constexpr int kBinWarps = 8;
+__global__ void __launch_bounds__(32 * kBinWarps) k_bin_block(
+    int64_t lmax, int64_t nb, const double *__restrict__ M, const int32_t *__restrict__ band_ptr,
+    const int32_t *__restrict__ band_ells, const double *__restrict__ wfl, const double *__restrict__ inv_fl,
+    const double *__restrict__ beam, double *__restrict__ out)
 {
-    const int64_t b = blockIdx.y, bp = blockIdx.x, n = lmax + 1;
+    const int64_t b = blockIdx.y, bp = (int64_t)blockIdx.x * kBinWarps + (threadIdx.x >> 5), n = lmax + 1;
+    if (bp >= nb) return;
+    const int lane = threadIdx.x & 31;
     const int i0 = band_ptr[b], i1 = band_ptr[b + 1], k0 = band_ptr[bp], k1 = band_ptr[bp + 1];
-    const int nk = k1 - k0, cnt = (i1 - i0) * nk;
     double s = 0.0;
-    for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
-        const int l = band_ells[i0 + t / nk], lp = band_ells[k0 + t % nk];
-        s += wfl[l] * M[(int64_t)l * n + lp] * beam[lp] * inv_fl[lp];
+    for (int k = k0 + lane; k < k1; k += 32) {
+        const int lp = band_ells[k];
+        double t = 0.0;
+#pragma unroll 4
+        for (int i = i0; i < i1; ++i) {
+            const int l = band_ells[i];
+            t = fma(wfl[l], M[(int64_t)l * n + lp], t);
+        }
+        s += t * beam[lp] * inv_fl[lp];
     }
-    __shared__ double red[256];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-        if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[b * nb + bp] = red[0];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) out[b * nb + bp] = s;
 }
 
 // Place binned blocks into the (ncls nb)^2 matrix, band-major channel-minor.
@@ -926,6 +931,30 @@ __global__ void __launch_bounds__(64) k_lu_prepare(int n, const double *__restri
 // steps (two barriers, a row read and two reductions each); with the interchanges applied one by
 // one and 32-step substitutions inside a block a solve of n = 92 took 42 us, of 612 438
 // us; here 6.8 and 77 us.
+// Sums of CB values over the lanes: lane c < CB returns value c's (CB = 4: the lanes exchange halves
+// of the values over their two low bits first, six shuffles instead of twenty).  The additions
+// pair the lanes in the same order for every CB.
+template <int CB>
+__device__ __forceinline__ double lane_sums(const double (&v)[CB], int lane)
+{
+    static_assert(CB == 1 || CB == 4, "columns per CTA");
+    double s;
+    if constexpr (CB == 1) {
+        s = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 2);
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+    } else {
+        const bool b1 = lane & 2, b0 = lane & 1;
+        const double k0 = b1 ? v[2] : v[0], k1 = b1 ? v[3] : v[1];   // kept, and given to the partner
+        const double g0 = b1 ? v[0] : v[2], g1 = b1 ? v[1] : v[3];
+        const double h0 = k0 + __shfl_xor_sync(0xffffffffu, g0, 2), h1 = k1 + __shfl_xor_sync(0xffffffffu, g1, 2);
+        s = (b0 ? h1 : h0) + __shfl_xor_sync(0xffffffffu, b0 ? h0 : h1, 1);
+    }
+    s += __shfl_xor_sync(0xffffffffu, s, 4);
+    s += __shfl_xor_sync(0xffffffffu, s, 8);
+    s += __shfl_xor_sync(0xffffffffu, s, 16);
+    return s;
+}
+
 // load(row, column): entry of b.
 template <int CB, class Load>
 __device__ __forceinline__ void lu_solve_columns(int n, const double *__restrict__ lu,
@@ -958,21 +987,13 @@ __device__ __forceinline__ void lu_solve_columns(int n, const double *__restrict
                 for (int c = 0; c < CB; ++c) acc[c] = fma(l, xs[j * CB + c], acc[c]);
             }
         }
-#pragma unroll
-        for (int c = 0; c < CB; ++c)
-            for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
-        if (lane == 0)
-#pragma unroll
-            for (int c = 0; c < CB; ++c) part[r][c] = xs[row * CB + c] - acc[c];
+        const double sum = lane_sums<CB>(acc, lane);
+        if (lane < CB) part[r][lane] = xs[row * CB + lane] - sum;
         __syncthreads();
 #pragma unroll
-        for (int c = 0; c < CB; ++c) {
-            acc[c] = di * part[lane][c];
-            for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
-        }
-        if (lane == 0)
-#pragma unroll
-            for (int c = 0; c < CB; ++c) xs[row * CB + c] = acc[c];
+        for (int c = 0; c < CB; ++c) acc[c] = di * part[lane][c];
+        const double v = lane_sums<CB>(acc, lane);
+        if (lane < CB) xs[row * CB + lane] = v;
         __syncthreads();
     };
     for (int blk = 0; blk < nblk; ++blk) step(blk, 0, blk * kLuSB, 0);
@@ -1148,18 +1169,18 @@ extern "C" int gm_bin_coupling_csr(int64_t lmax, int64_t nbands, int ncls, const
         return GM_ERR_BAD_PTR;
     cudaStream_t s = as_stream(stream);
     const int64_t n = lmax + 1, nn = n * n, nb2 = nbands * nbands;
-    dim3 grid((unsigned)nbands, (unsigned)nbands);
+    dim3 grid((unsigned)((nbands + kBinWarps - 1) / kBinWarps), (unsigned)nbands);
     // block slots: tt 0, te 1, pp 2, mm 3
     if (ncls == 1) {
-        k_bin_block<<<grid, 256, 0, s>>>(lmax, nbands, blocks, band_ptr, band_ells, wfl, inv_fl,
+        k_bin_block<<<grid, 32 * kBinWarps, 0, s>>>(lmax, nbands, blocks, band_ptr, band_ells, wfl, inv_fl,
                                          beam, scratch);
     } else if (ncls == 2) {
-        k_bin_block<<<grid, 256, 0, s>>>(lmax, nbands, blocks + nn, band_ptr, band_ells, wfl,
+        k_bin_block<<<grid, 32 * kBinWarps, 0, s>>>(lmax, nbands, blocks + nn, band_ptr, band_ells, wfl,
                                          inv_fl, beam, scratch);
     } else {
-        k_bin_block<<<grid, 256, 0, s>>>(lmax, nbands, blocks + 2 * nn, band_ptr, band_ells, wfl,
+        k_bin_block<<<grid, 32 * kBinWarps, 0, s>>>(lmax, nbands, blocks + 2 * nn, band_ptr, band_ells, wfl,
                                          inv_fl, beam, scratch);
-        k_bin_block<<<grid, 256, 0, s>>>(lmax, nbands, blocks + 3 * nn, band_ptr, band_ells, wfl,
+        k_bin_block<<<grid, 32 * kBinWarps, 0, s>>>(lmax, nbands, blocks + 3 * nn, band_ptr, band_ells, wfl,
                                          inv_fl, beam, scratch + nb2);
     }
     const int64_t N = ncls * nbands;
