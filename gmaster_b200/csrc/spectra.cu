@@ -426,6 +426,25 @@ __global__ void k_bin_cells(int64_t lmax, int64_t nb, int64_t ncls, const double
 
 // ---------------------------------------------------------------- LU
 
+// Order of pivot candidates: NaN, then by magnitude (zero is 1).
+__device__ __forceinline__ unsigned long long pivot_key(double v)
+{
+    const double f = fabs(v);
+    return f >= 0.0 ? (unsigned long long)__double_as_longlong(f) + 1ull : 0ull;
+}
+
+// The warp's largest key and its lowest row: the key's halves and the row one after the other
+// through the integer reductions (a shuffle tree of (key, row) takes 15 steps).
+__device__ __forceinline__ void best_pivot(unsigned long long &q, int &r)
+{
+    const unsigned hi = (unsigned)(q >> 32), lo = (unsigned)q;
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    const bool mine = hi == mh && lo == ml;
+    r = __reduce_min_sync(0xffffffffu, mine ? r : 0x7fffffff);
+    q = ((unsigned long long)mh << 32) | ml;
+}
+
 // Blocked LU, panel step in shared memory: columns [k0, k0 + kb) of rows k0..n-1 of the
 // row-major (n, n) matrix, one CTA, partial pivoting (largest magnitude, lowest row on ties; a
 // NaN is never chosen over a number).  Row interchanges are confined to the panel here; k_lu_rest
@@ -434,8 +453,7 @@ __global__ void k_bin_cells(int64_t lmax, int64_t nb, int64_t ncls, const double
 //
 // Bound by latency: two barriers, a warp reduction of the pivot candidates and kb - k
 // multiply-adds a row per column.  The panel is read and written once; held in global memory it
-// took 7 us a column, here 1.6 (a 612 x 612 matrix: panels 4.3 -> 1.0 ms, with the other
-// columns' kernels 5.4 -> 1.4 ms).
+// took 7 us a column, here 1.6 at 612 rows (bound by the shared-memory traffic of the update).
 __global__ void __launch_bounds__(1024) k_lu_panel_smem(int n, int k0, int kb, double *__restrict__ a,
                                                         int32_t *__restrict__ piv, int32_t *__restrict__ status)
 {
@@ -450,33 +468,18 @@ __global__ void __launch_bounds__(1024) k_lu_panel_smem(int n, int k0, int kb, d
         pan[(int64_t)c * ld + i] = a[(int64_t)(k0 + i) * n + k0 + c];
     }
     __syncthreads();
-    // order of candidates: NaN, then by magnitude
-    auto key_of = [](double v) -> unsigned long long {
-        const double f = fabs(v);
-        return f >= 0.0 ? (unsigned long long)__double_as_longlong(f) + 1ull : 0ull;
-    };
     for (int k = 0; k < kb; ++k) {
         double *col = pan + (int64_t)k * ld;
         unsigned long long key = 0;
         int row = k;
         for (int i = k + tid; i < rows; i += blockDim.x) {
-            const unsigned long long q = key_of(col[i]);
+            const unsigned long long q = pivot_key(col[i]);
             if (q > key) {
                 key = q;
                 row = i;
             }
         }
-        // the warp's largest key and its lowest row: the key's halves and the row one after the
-        // other through the integer reductions (a shuffle tree of (key, row) takes 15 steps)
-        auto best = [](unsigned long long &q, int &r) {
-            const unsigned hi = (unsigned)(q >> 32), lo = (unsigned)q;
-            const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-            const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
-            const bool mine = hi == mh && lo == ml;
-            r = __reduce_min_sync(0xffffffffu, mine ? r : 0x7fffffff);
-            q = ((unsigned long long)mh << 32) | ml;
-        };
-        best(key, row);
+        best_pivot(key, row);
         if (lane == 0) {
             skey[k & 1][warp] = key;
             srow[k & 1][warp] = row;
@@ -484,7 +487,7 @@ __global__ void __launch_bounds__(1024) k_lu_panel_smem(int n, int k0, int kb, d
         __syncthreads();
         key = lane < nw ? skey[k & 1][lane] : 0ull;
         row = lane < nw ? srow[k & 1][lane] : 0x7fffffff;
-        best(key, row);
+        best_pivot(key, row);
         if (key == 0ull) row = k;   // no number in the column
         if (tid == 0) {
             piv[k0 + k] = k0 + row;
@@ -513,6 +516,71 @@ __global__ void __launch_bounds__(1024) k_lu_panel_smem(int n, int k0, int kb, d
         const int i = (int)(e / kb), c = (int)(e % kb);
         a[(int64_t)(k0 + i) * n + k0 + c] = pan[(int64_t)c * ld + i];
     }
+}
+
+// The panel step with every row in the registers of a thread (rows <= NT, kb <= KB): the update of
+// a column then reads only the pivot row from shared memory, where the form above moves two
+// entries a row and column through it: panels of a 612 x 612 matrix 1.0 -> 0.66 ms.
+template <int KB, int NT>
+__global__ void __launch_bounds__(NT) k_lu_panel_reg(int n, int k0, int kb, double *__restrict__ a,
+                                                     int32_t *__restrict__ piv, int32_t *__restrict__ status)
+{
+    __shared__ __align__(16) double prow[KB], krow[KB];
+    __shared__ unsigned long long skey[32];
+    __shared__ int srow[32];
+    const int rows = n - k0, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    const bool mine = tid < rows;
+    if (k0 == 0 && tid == 0) *status = 0;
+    double x[KB];
+    double *src = a + (int64_t)(k0 + tid) * n + k0;
+#pragma unroll
+    for (int c = 0; c < KB; ++c) x[c] = mine && c < kb ? src[c] : 0.0;
+#pragma unroll
+    for (int k = 0; k < KB; ++k) {
+        if (k >= kb) break;
+        unsigned long long key = mine && tid >= k ? pivot_key(x[k]) : 0ull;
+        int row = mine && tid >= k ? tid : 0x7fffffff;
+        best_pivot(key, row);
+        if (lane == 0) {
+            skey[warp] = key;
+            srow[warp] = row;
+        }
+        __syncthreads();
+        key = lane < nw ? skey[lane] : 0ull;
+        row = lane < nw ? srow[lane] : 0x7fffffff;
+        best_pivot(key, row);
+        if (key == 0ull) row = k;   // no number in the column
+        if (tid == 0) {
+            piv[k0 + k] = k0 + row;
+            if (key == 1ull && *status == 0) *status = k0 + k + 1;
+        }
+        if (tid == row)
+#pragma unroll
+            for (int c = 0; c < KB; ++c) prow[c] = x[c];
+        if (tid == k && row != k)
+#pragma unroll
+            for (int c = 0; c < KB; ++c) krow[c] = x[c];
+        __syncthreads();
+        if (row != k) {
+            if (tid == row)
+#pragma unroll
+                for (int c = 0; c < KB; ++c) x[c] = krow[c];
+            if (tid == k)
+#pragma unroll
+                for (int c = 0; c < KB; ++c) x[c] = prow[c];
+        }
+        if (tid > k) {
+            const double d = prow[k], inv = d != 0.0 ? 1.0 / d : 0.0;
+            const double l = x[k] * inv;
+            x[k] = l;
+#pragma unroll
+            for (int c = k + 1; c < KB; ++c) x[c] = fma(-l, prow[c], x[c]);
+        }
+    }
+    if (mine)
+#pragma unroll
+        for (int c = 0; c < KB; ++c)
+            if (c < kb) src[c] = x[c];
 }
 
 // Blocked LU, the columns outside the panel [k0, k0 + kb), kb <= 32: the panel's row
@@ -1238,16 +1306,26 @@ extern "C" int gm_lu_factor(int64_t n, double *a, int32_t *piv, int32_t *status,
         set_error("gm_lu_factor attr", e);
         return GM_ERR_LAUNCH;
     }
-    for (int64_t k0 = 0; k0 < n; k0 += w) {
-        const int kb = (int)(n - k0 < w ? n - k0 : w);
-        const int64_t rows = n - k0, k1 = k0 + kb;
+    for (int64_t k0 = 0; k0 < n;) {
+        const int64_t rows = n - k0;
+        // rows in registers: 32 columns of up to 640 rows, 16 of up to 1024; else the widest panel
+        // that fits shared memory (one for all of n <= 160)
+        const int width = n <= 160 ? w : (rows <= 640 ? 32 : (rows <= 1024 ? 16 : w));
+        const int kb = (int)(rows < width ? rows : width);
+        const int64_t k1 = k0 + kb;
         const int threads = rows >= 1024 ? 1024 : (int)((rows + 31) / 32 * 32);
-        k_lu_panel_smem<<<1, threads, smem, s>>>((int)n, (int)k0, kb, a, piv, status);
+        if (n > 160 && rows <= 640)
+            k_lu_panel_reg<32, 640><<<1, threads, 0, s>>>((int)n, (int)k0, kb, a, piv, status);
+        else if (n > 160 && rows <= 1024)
+            k_lu_panel_reg<16, 1024><<<1, threads, 0, s>>>((int)n, (int)k0, kb, a, piv, status);
+        else
+            k_lu_panel_smem<<<1, threads, smem, s>>>((int)n, (int)k0, kb, a, piv, status);
         if (n > kb) k_lu_rest<<<(unsigned)((n - kb + 127) / 128), 128, 0, s>>>((int)n, (int)k0, kb, a, piv);
         if (k1 < n) {
             const int st = gm_lu_update(n, a, k0, k1, stream);
             if (st != GM_OK) return st;
         }
+        k0 = k1;
     }
     return check_launch("gm_lu_factor");
 }
