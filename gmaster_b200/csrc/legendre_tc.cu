@@ -677,7 +677,8 @@ __global__ void __launch_bounds__(128) k_pack_tc(int64_t nside, int64_t L, int n
 // Rows: spin 0 [a | s a] (src row r mod H); spin 2 variant -2 (lambda+): [2a | s -2a]
 // (src row r); variant +2 (lambda-): [-2a | s 2a] (src r < H ? H + r : r - H); s = (-1)^(l+m).
 // With `rel` set the chunks start at the order's first row instead: chunk cc covers
-// l0 + 64 cc + [0, 64) (the layout of the checkpointed synthesis, legendre_ck.cu).
+// l0 + 64 cc + [0, 64) (the layout of the checkpointed synthesis, legendre_ck.cu).  Every byte of
+// every chunk is written (zeros for rows past 2H and degrees out of range).
 __global__ void k_prep_syn(int64_t lmax, int spin, int sp, int H, int NR,
                            const double *__restrict__ alm_i, const int64_t *__restrict__ choff,
                            uint8_t *__restrict__ simg, double scale, int64_t mbeg, int rel)
@@ -1102,11 +1103,6 @@ extern "C" int gm_tc_prep_syn_window(int64_t lmax, int spin, int sp, int64_t nco
     const int H = spin == 0 ? (int)(2 * ncomp) : (int)ncomp;
     const int NR = spin == 0 ? H : 2 * H;
     cudaStream_t s = as_stream(stream);
-    cudaError_t e = cudaMemsetAsync(simg, 0, (size_t)simg_bytes, s);
-    if (e != cudaSuccess) {
-        set_error("gm_tc_prep_syn memset", e);
-        return GM_ERR_LAUNCH;
-    }
     k_prep_syn<<<dim3(16, (unsigned)(mend - mbeg)), 256, 0, s>>>(lmax, spin, sp, H, NR, alm_i, choff,
                                                                 (uint8_t *)simg, alm_scale, mbeg, 0);
     return check_launch("gm_tc_prep_syn");
@@ -1122,11 +1118,6 @@ extern "C" int gm_ck_prep_syn(int64_t lmax, int spin, int sp, int64_t ncomp, con
     const int H = spin == 0 ? (int)(2 * ncomp) : (int)ncomp;
     const int NR = spin == 0 ? H : 2 * H;
     cudaStream_t s = as_stream(stream);
-    cudaError_t e = cudaMemsetAsync(simg, 0, (size_t)simg_bytes, s);
-    if (e != cudaSuccess) {
-        set_error("gm_ck_prep_syn memset", e);
-        return GM_ERR_LAUNCH;
-    }
     k_prep_syn<<<dim3(16, (unsigned)(lmax + 1)), 256, 0, s>>>(lmax, spin, sp, H, NR, alm_i, choff,
                                                               (uint8_t *)simg, alm_scale, 0, 1);
     return check_launch("gm_ck_prep_syn");
