@@ -116,6 +116,8 @@ SIGNATURES = {
                                  _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_int, _c_vp], _c_int),
     "gm_legendre_synthesis_ck": ([_c_int, _c_i64, _c_i64, _c_i64, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp,
                                   _c_vp, _c_vp, _c_vp, _c_vp, _c_int, _c_vp], _c_int),
+    "gm_refine": ([_c_int, _c_int, _c_i64, _c_i64, _c_i64, _c_i64] + [_c_vp] * 7 + [_c_int, _c_int] + [_c_vp] * 8,
+                  _c_int),
     "gm_ck_offsets": ([_c_i64, _c_int, _c_vp, _c_vp], _c_int),
     "gm_ck_table_entries": ([_c_i64, _c_i64, _c_int], _c_i64),
     "gm_ck_build": ([_c_i64, _c_i64, _c_int, _c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp],

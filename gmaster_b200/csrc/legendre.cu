@@ -732,3 +732,29 @@ extern "C" int gm_legendre_synthesis(int precision, int spin, int64_t nside, int
         return dispatch_syn<float>(spin, nside, lmax, ncomp, lane_geom, seeds, alm, syn, s);
     return GM_ERR_UNSUPPORTED;
 }
+
+// The Jacobi refinement of one field's analysis, n_iter times synthesis, ring-fold residual and
+// analysis, issued by one call.  segoff: checkpointed rows (legendre_rows.cu); NULL: the FP64
+// recurrence.
+extern "C" int gm_refine(int precision, int spin, int64_t nside, int64_t lmax, int64_t ncomp, int64_t n_iter,
+                         const double *lane_geom, const double *seeds, const void *rhs_map, const uint8_t *shifted,
+                         void *syn, void *res, double *alm, int tile_syn, int tile_ana, const int64_t *segoff,
+                         const void *ck_a, const uint8_t *cn_a, const void *ck_b, const uint8_t *cn_b,
+                         const uint64_t *mask_a, const uint64_t *mask_b, void *stream)
+{
+    if (segoff && precision != GM_MIXED) return GM_ERR_UNSUPPORTED;
+    for (int64_t it = 0; it < n_iter; ++it) {
+        int st = segoff ? gm_legendre_synthesis_ck(spin, nside, lmax, ncomp, lane_geom, alm, syn, segoff, ck_a, cn_a,
+                                                   ck_b, cn_b, mask_a, mask_b, tile_syn, stream)
+                        : gm_legendre_synthesis_tile(precision, spin, nside, lmax, ncomp, lane_geom, seeds, alm, syn,
+                                                     tile_syn, stream);
+        if (st == GM_OK) st = gm_fold_residual(precision, nside, lmax + 1, ncomp, syn, rhs_map, shifted, res, stream);
+        if (st == GM_OK)
+            st = segoff ? gm_legendre_analysis_ck(spin, nside, lmax, ncomp, lane_geom, res, alm, -1.0, segoff, ck_a, cn_a,
+                                                  ck_b, cn_b, mask_a, mask_b, tile_ana, stream)
+                        : gm_legendre_analysis_tile(precision, spin, nside, lmax, ncomp, lane_geom, seeds, res, alm, -1.0,
+                                                    tile_ana, stream);
+        if (st != GM_OK) return st;
+    }
+    return GM_OK;
+}

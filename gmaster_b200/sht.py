@@ -374,6 +374,17 @@ def ring_synthesis(plan, syn, prec):
 
 # ----------------------------------------------------------------------------- transforms
 
+def _refine(plan, spin, alm, rhs_map, syn, res, n_iter, prec):
+    """The Jacobi iterations of map2alm_device, all launches issued by one call."""
+    ncomp = rhs_map.shape[2]
+    tile_ana, ck = _pass_setup(plan, spin, ncomp, prec, "ana")
+    tile_syn, _ = _pass_setup(plan, spin, ncomp, prec, "syn")
+    _lib.call("gm_refine", prec, spin, plan.nside, plan.lmax, ncomp, n_iter, _lib.ptr(plan.geom), _lib.ptr(plan.seeds),
+              _lib.ptr(rhs_map), _lib.ptr(plan.shifted), _lib.ptr(syn), _lib.ptr(res), _lib.ptr(alm), tile_syn, tile_ana,
+              *(ck if ck is not None else (None,) * 7), _lib.stream_handle(plan.device))
+    _lib.CALLS["gm_refine"] += 3 * n_iter - 1   # launches of the call
+
+
 def map2alm_device(maps, spin, nside, lmax, n_iter, precision="mixed"):
     """Analysis of ``maps`` (ncomp, npix) on the GPU with ``n_iter`` Jacobi iterations.
 
@@ -395,6 +406,9 @@ def map2alm_device(maps, spin, nside, lmax, n_iter, precision="mixed"):
     if n_iter > 0:
         syn = torch.empty_like(rhs_map)
         res = torch.empty_like(rhs_map)
+        if TIMER is None:
+            _refine(plan, spin, alm, rhs_map, syn, res, int(n_iter), prec)
+            return alm
         for _ in range(int(n_iter)):
             legendre_synthesis(plan, spin, alm, ncomp, prec, out=syn)
             fold_residual(plan, syn, rhs_map, prec, out=res)

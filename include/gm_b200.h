@@ -369,6 +369,14 @@ int gm_legendre_synthesis_ck(int spin, int64_t nside, int64_t lmax, int64_t ncom
                              const int64_t *segoff, const void *ck_a, const uint8_t *cn_a,
                              const void *ck_b, const uint8_t *cn_b, const uint64_t *mask_a,
                              const uint64_t *mask_b, int tile, void *stream);
+/* n_iter Jacobi steps alm <- alm - A(S(alm) - map) of one field by one call (healpix.py:1059-1068):
+ * the tiled or (segoff not NULL, mixed precision) checkpointed synthesis into syn,
+ * gm_fold_residual into res, the analysis with scale -1. */
+int gm_refine(int precision, int spin, int64_t nside, int64_t lmax, int64_t ncomp, int64_t n_iter,
+              const double *lane_geom, const double *seeds, const void *rhs_map,
+              const uint8_t *shifted, void *syn, void *res, double *alm, int tile_syn, int tile_ana,
+              const int64_t *segoff, const void *ck_a, const uint8_t *cn_a, const void *ck_b,
+              const uint8_t *cn_b, const uint64_t *mask_a, const uint64_t *mask_b, void *stream);
 
 /* ---- checkpointed batched Legendre contraction (replaces march_v2.cu:155-407 for batched
  * maps; the reference's window tables march_v2.py:388-450 are its per-geometry constants).
