@@ -1,11 +1,14 @@
 // Checkpointed Legendre / Wigner-d contraction on the tcgen05 tensor cores (sm_100a).
 //
 // The rows lambda^{s'}_lm(theta) are generated in single precision by the three-term
-// recurrence in its difference form
-//     C_l = c1_l (x - 1) + E_l,   D_l = b_l D_{l-1} + C_l v_{l-1},   v_l = v_{l-1} + D_l
-// (c1 = alpha, b = beta, E = alpha - beta - 1 - alpha s'c0/|s'|; algebraically the same as
-// v_l = alpha (x - c) v_{l-1} - beta v_{l-2}), restarted every kSeg = 128 rows from a
-// state computed once per geometry by the FP64 recurrence (the checkpoint table).  The
+// recurrence in its difference form, the difference D_l = v_l - v_{l-1} = alpha_l d_l carried
+// scaled (beta_l = alpha_l / alpha_{l-1} exactly):
+//     d_l = d_{l-1} + ((x - 1) + e_l) v_{l-1},   v_l = v_{l-1} + alpha_l d_l,
+// e = 1 - (beta + 1) / alpha - s'c0/|s'| (algebraically the same as
+// v_l = alpha (x - c) v_{l-1} - beta v_{l-2}): three operations and two coefficients a row.
+// They restart every kSeg = 128 rows from a state computed once per geometry by the FP64
+// recurrence (the checkpoint table), and what the rounding of x - 1 leaves off is added to d
+// every eighth row (it is one direction for all rows of a lane).  The
 // difference form keeps each rounding unamplified near the poles and turning points, where
 // the plain form multiplies it by 1/sin(phi) (phi the local oscillation phase); over 128 rows
 // from an exact start the FP32 rows stay within ~2e-6 of the row scale sqrt((2l+1)/4pi).
@@ -18,8 +21,8 @@
 //     order at the same time share that order's right-hand-side images through L2 and each
 //     alm element receives exactly one addition per launch, from one unit;
 //   * the synthesis runs two sets of 8 generator warps on alternate segments.
-// A checkpoint stores the pre-state (v_{l_s - 1}, D_{l_s}) of the segment's first row l_s,
-// so that row is the uniform step with coefficients (c1, E, b) = (0, 0, 1).  The state is
+// A checkpoint stores the pre-state (v_{l_s - 1}, D_{l_s}) of the segment's first row l_s:
+// v = v_{l_s - 1} + D and d = D / alpha_{l_s} start the segment.  The state is
 // kept in FP32 with a shift n in {0..5}: actual = stored * 2^(-64 n).  Lanes whose rows are
 // still far below 2^-16 (the seed region of high orders, where a segment can grow by 2^230)
 // carry n > 0, emit v * 2^(-64 n) and renormalise every 8 rows; a warp in which every lane
@@ -68,7 +71,7 @@ constexpr uint32_t kAImgG = 2u * 128u * kKG * 2u;   // a group's hi and lo image
 constexpr uint32_t kTileA = 2u * kSB * kKG * 2u;    // tile: 256 rows x 32 lanes, hi + lo (32 KB)
 constexpr int kStageLd = kSB + 1;                   // epilogue staging row stride (floats)
 // the epilogue stages 128 rows x kStageLd floats in the tiles and coefficient rows
-static_assert(128 * kStageLd * 4 <= kSetsA * kTileA + kSB * 16, "epilogue staging does not fit");
+static_assert(128 * kStageLd * 4 <= kSetsA * kTileA + kSB * 8, "epilogue staging does not fit");
 // synthesis
 constexpr int kLT = 256;                            // lanes per CTA (MMA N)
 constexpr int kKL = 64;                             // rows per chunk (MMA K)
@@ -159,15 +162,21 @@ __host__ __device__ __forceinline__ int64_t first_row(int64_t m, int sp)
     return m > a ? m : a;
 }
 
-// Difference-form coefficients of the step to row l of order m (coefficient base mb).
-__device__ __forceinline__ float4 diff_coef(const double *__restrict__ coef, int64_t mb, int64_t l,
-                                            int64_t L, double sgn_c, bool restart)
+// Coefficients (e, alpha) of the step from row l - 1 to row l of order m (coefficient base mb);
+// past the last row the step is v = v (those rows meet no image row or are not written).
+__device__ __forceinline__ float2 step_coef(const double *__restrict__ coef, int64_t mb, int64_t l,
+                                            int64_t L, double sgn_c)
 {
-    if (restart) return make_float4(0.f, 0.f, 1.f, 0.f);   // D = D, v = v + D
-    if (l >= L) return make_float4(0.f, -1.f, 0.f, 0.f);   // v = 0 from here on
+    if (l >= L) return make_float2(0.f, 0.f);
     const Coef c = load_coef(coef, mb + l);
-    return make_float4((float)c.alpha, (float)(c.alpha - c.beta - 1.0 - sgn_c * c.alpha * c.c0),
-                       (float)c.beta, 0.f);
+    return make_float2((float)(1.0 - (c.beta + 1.0) / c.alpha - sgn_c * c.c0), (float)c.alpha);
+}
+
+// 1 / alpha_l at a segment's first row l, zero at the order's first row l0 (where d = 0).
+__device__ __forceinline__ float inv_alpha(const double *__restrict__ coef, int64_t mb, int64_t l, int64_t l0,
+                                           int64_t L)
+{
+    return l > l0 && l < L ? (float)(1.0 / load_coef(coef, mb + l).alpha) : 0.f;
 }
 
 // A warp-uniform bounded wait: every lane waits, and the warp goes on only if all did.
@@ -177,62 +186,83 @@ __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volati
     return __all_sync(0xffffffffu, ok);
 }
 
-// One step of the FP32 difference form with coefficients q = (c1, E, b):
-//   C = c1 (x - 1) + E,  D <- C v + b D,  v <- v + D.
-// b D is formed off the dependent chain, so a row costs two dependent operations.
-__device__ __forceinline__ void diff_step(const float4 &q, float y, float &v, float &D)
-{
-    const float C = fmaf(q.x, y, q.y);
-    const float bD = q.z * D;
-    D = fmaf(C, v, bD);
-    v = v + D;
-}
+// State of a lane: y = x - 1 and dy = 8 (x - 1 - y) in single precision, the row v, its scaled
+// difference d and the shift n.
+struct Row {
+    float y, dy, v, d;
+    int n;
+
+    __device__ __forceinline__ void start(const float2 &st, int shift, double xm1, float r)
+    {
+        y = (float)xm1;
+        dy = (float)(8.0 * (xm1 - (double)y));
+        v = st.x + st.y;
+        d = st.y * r;
+        n = shift;
+    }
+    __device__ __forceinline__ void step(float e, float al)
+    {
+        d = fmaf(y + e, v, d);
+        v = fmaf(al, d, v);
+    }
+};
 
 // Sixty-four rows of one lane (eight chunks of eight), split into f16 hi/lo and stored as
 // 16-byte chunks: chunk cc at base + ((cc ^ sw) << 4), its lo plane lo_delta bytes further.
+// A chunk's coefficients (two rows per 16-byte load) are loaded before the previous chunk is
+// stored, so that the loads' latency is behind its rows and conversions: with eight warps an SM
+// (the shared memory holds no more tiles) the generators are bound by latency and issue slots.
+// Against the four-operation rows (c1, E, b), 32 QU fields at Nside 512: synthesis 1.25 -> 1.19
+// ms a launch, analysis 1.38 ms either way (its rows are not what bounds it), error of the alms
+// against exact sums 3.6e-6 -> 3.4e-6.
 // SCALED: some lane of the warp still carries a shift n > 0 (decided once per 64 rows; a
 // lane's shift only decreases): such lanes emit v * 2^(-64 n) and renormalise every 8 rows.
 template <bool SCALED>
-__device__ __forceinline__ void gen64(const float4 *__restrict__ cw, float y, float &v, float &D, int &n,
-                                      uint32_t base, uint32_t lo_delta, uint32_t sw)
+__device__ __forceinline__ void gen64(const float2 *__restrict__ cw, Row &w, uint32_t base, uint32_t lo_delta,
+                                      uint32_t sw)
 {
-#pragma unroll 2
+    const float4 *__restrict__ c4 = reinterpret_cast<const float4 *>(cw);
+    float4 q[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) q[e] = c4[e];
+#pragma unroll 4
     for (int cc = 0; cc < 8; ++cc) {
         float vals[8];
-        if (SCALED) {
-            const float sc = n == 0 ? 1.0f : (n == 1 ? 0x1p-64f : 0.0f);
+        float4 nq[4];
+        const int nc = cc < 7 ? cc + 1 : 7;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                diff_step(cw[8 * cc + e], y, v, D);
-                vals[e] = v * sc;
-            }
-            // 8 rows grow a value by at most 2^63 (alpha <= sqrt(2m) + 1 at Nside <= 8192),
-            // so a renormalisation at 2^48 keeps every shifted value below 2^111
-            if (n != 0 && fabsf(v) > 0x1p48f) {
-                v *= 0x1p-64f;
-                D *= 0x1p-64f;
-                --n;
-            }
-        } else {
+        for (int e = 0; e < 4; ++e) nq[e] = c4[4 * nc + e];
+        const float sc = !SCALED || w.n == 0 ? 1.0f : (w.n == 1 ? 0x1p-64f : 0.0f);
+        w.d = fmaf(w.dy, w.v, w.d);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                diff_step(cw[8 * cc + e], y, v, D);
-                vals[e] = v;
-            }
+        for (int e = 0; e < 4; ++e) {
+            vals[2 * e] = SCALED ? w.v * sc : w.v;
+            w.step(q[e].x, q[e].y);
+            vals[2 * e + 1] = SCALED ? w.v * sc : w.v;
+            w.step(q[e].z, q[e].w);
+        }
+        // 8 rows grow a value by at most 2^63 (alpha <= sqrt(2m) + 1 at Nside <= 8192), so a
+        // renormalisation at 2^48 keeps every shifted value below 2^111
+        if (SCALED && w.n != 0 && fabsf(w.v) > 0x1p48f) {
+            w.v *= 0x1p-64f;
+            w.d *= 0x1p-64f;
+            --w.n;
         }
         uint4 hi, lo;
         pack8(vals, hi, lo);
         const uint32_t off = ((uint32_t)cc ^ sw) << 4;
         sts128(base + off, hi);
         sts128(base + lo_delta + off, lo);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) q[e] = nq[e];
     }
 }
 
-__device__ __forceinline__ void gen_rows64(const float4 *__restrict__ cw, float y, float &v, float &D,
-                                           int &n, uint32_t base, uint32_t lo_delta, uint32_t sw)
+__device__ __forceinline__ void gen_rows64(const float2 *__restrict__ cw, Row &w, uint32_t base,
+                                           uint32_t lo_delta, uint32_t sw)
 {
-    if (__any_sync(0xffffffffu, n != 0)) gen64<true>(cw, y, v, D, n, base, lo_delta, sw);
-    else gen64<false>(cw, y, v, D, n, base, lo_delta, sw);
+    if (__any_sync(0xffffffffu, w.n != 0)) gen64<true>(cw, w, base, lo_delta, sw);
+    else gen64<false>(cw, w, base, lo_delta, sw);
 }
 
 // ----------------------------------------------------------------------- checkpoint table
@@ -378,7 +408,8 @@ __global__ void __launch_bounds__(kThrA, 1) k_ana_ck(CkParams p, const uint8_t *
     uint8_t *smem = smem_raw + (base - tc::smem_u32(smem_raw));
     uint8_t *sA = smem;                                              // kImgBufA image buffers
     uint8_t *sB = smem + kImgBufA * kAImgG;                          // kSetsA tiles
-    float4 *sCf = reinterpret_cast<float4 *>(sB + kSetsA * kTileA); // kSB coefficient rows
+    float2 *sCf = reinterpret_cast<float2 *>(sB + kSetsA * kTileA); // kSB coefficient rows
+    float *sR = reinterpret_cast<float *>(sCf + kSB);                // 1 / alpha of the segments' first rows
     const int64_t L = p.lmax + 1, NG = (p.nlanes + kKC - 1) / kKC, NGK = (p.nlanes + kKG - 1) / kKG;
     const int64_t U = p.uoff[L];
     const int64_t G = gridDim.x, c = blockIdx.x;
@@ -492,13 +523,16 @@ __global__ void __launch_bounds__(kThrA, 1) k_ana_ck(CkParams p, const uint8_t *
                                  (uint32_t)(2 * sseg) * 1024 + (t & 7) * 128;
         uint32_t js = 0;   // groups generated into this set's tile
         bool dead = false;
-        // this thread's coefficient row of a unit, loaded one unit ahead
+        // this thread's coefficient row of a unit, loaded one unit ahead (z: 1 / alpha at a
+        // segment's first row)
         auto unit_coef = [&](int64_t uu) {
             const int64_t mm = unit_order(p.uoff, L, uu);
-            const int64_t lbb = first_row(mm, p.sp) + (uu - p.uoff[mm]) * kSB;
-            return diff_coef(p.coef, alm_idx(p.lmax, 0, mm), lbb + tid, L, sgn_c, (tid & (kSeg - 1)) == 0);
+            const int64_t l0 = first_row(mm, p.sp), l = l0 + (uu - p.uoff[mm]) * kSB + tid;
+            const int64_t mbb = alm_idx(p.lmax, 0, mm);
+            const float2 q = step_coef(p.coef, mbb, l + 1, L, sgn_c);
+            return make_float3(q.x, q.y, (tid & (kSeg - 1)) == 0 ? inv_alpha(p.coef, mbb, l, l0, L) : 0.f);
         };
-        float4 ncoef = c < U ? unit_coef(c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float3 ncoef = c < U ? unit_coef(c) : make_float3(0.f, 0.f, 0.f);
         for (int64_t u = c; u < U; u += G) {
             const int64_t m = unit_order(p.uoff, L, u);
             const int64_t s = u - p.uoff[m];
@@ -507,7 +541,10 @@ __global__ void __launch_bounds__(kThrA, 1) k_ana_ck(CkParams p, const uint8_t *
             // coefficient rows of the unit (the previous unit's rows are no longer read: every
             // generator has passed its epilogue)
             gen_barrier_a();
-            if (!dead) sCf[tid] = ncoef;
+            if (!dead) {
+                sCf[tid] = make_float2(ncoef.x, ncoef.y);
+                if ((tid & (kSeg - 1)) == 0) sR[tid / kSeg] = ncoef.z;
+            }
             gen_barrier_a();
             if (!dead && u + G < U) ncoef = unit_coef(u + G);
             // this thread's segment; the second half of an order's last superblock may lie
@@ -543,9 +580,8 @@ __global__ void __launch_bounds__(kThrA, 1) k_ana_ck(CkParams p, const uint8_t *
                     g = gnext;
                     continue;
                 }
-                float v = nst.x, D = nst.y;
-                const float y = (float)(nx - 1.0);
-                int n = nn;
+                Row w;
+                w.start(nst, nn, nx - 1.0, sR[sseg]);
                 if (gnext >= 0) fetch(gnext);
                 g = gnext;
                 if (!warp_wait(&sh.b_free[S], (js & 1) ^ 1, abort, err)) {
@@ -554,8 +590,8 @@ __global__ void __launch_bounds__(kThrA, 1) k_ana_ck(CkParams p, const uint8_t *
                 }
                 // 128 rows of the lane: MN blocks 2 sseg (rows 0-63) and 2 sseg + 1; a thread
                 // stores 8 consecutive rows as 16 bytes, the lo plane kTileA / 2 bytes further
-                gen_rows64(sCf + kSeg * sseg, y, v, D, n, rowbase, kTileA / 2, (uint32_t)(t & 7));
-                gen_rows64(sCf + kSeg * sseg + kHalf, y, v, D, n, rowbase + 1024, kTileA / 2, (uint32_t)(t & 7));
+                gen_rows64(sCf + kSeg * sseg, w, rowbase, kTileA / 2, (uint32_t)(t & 7));
+                gen_rows64(sCf + kSeg * sseg + kHalf, w, rowbase + 1024, kTileA / 2, (uint32_t)(t & 7));
                 tc::fence_async_smem();
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(&sh.b_full[S]);
@@ -684,7 +720,8 @@ __global__ void __launch_bounds__(kThrS, 1) k_syn_ck(CkParams p, const uint8_t *
     uint8_t *smem = smem_raw + (base - tc::smem_u32(smem_raw));
     uint8_t *sA = smem;                                              // 2 x (hi, lo) alm images
     uint8_t *sB = smem + 4 * kSImg;                                  // 2 sets x (hi, lo) tiles
-    float4 *sCf = reinterpret_cast<float4 *>(sB + 4 * kBTileS);     // 2 sets x kSeg rows
+    float2 *sCf = reinterpret_cast<float2 *>(sB + 4 * kBTileS);     // 2 sets x kSeg rows
+    float *sR = reinterpret_cast<float *>(sCf + 2 * kSeg);           // 1 / alpha of their first rows
     const int64_t L = p.lmax + 1;
     const int64_t m = blockIdx.y, tile = blockIdx.x;
     const int64_t l0 = first_row(m, p.sp);
@@ -801,8 +838,8 @@ __global__ void __launch_bounds__(kThrS, 1) k_syn_ck(CkParams p, const uint8_t *
         const bool valid = jl < p.nlanes;
         const double sgn_c = sgn_of(p.sp);
         const int64_t mb = alm_idx(p.lmax, 0, m);
-        const float y = valid ? (float)(p.geom[jl] - 1.0) : 0.f;
-        float4 *cwin = sCf + kSeg * S;
+        const double xm1 = valid ? p.geom[jl] - 1.0 : 0.0;
+        float2 *cwin = sCf + kSeg * S;
         const uint32_t b0 = tc::smem_u32(sB + S * 2 * kBTileS);
         const uint32_t rowoff = (uint32_t)((t >> 3) * 1024 + (t & 7) * 128);
         uint32_t js = 0;   // chunks generated by this set
@@ -810,7 +847,8 @@ __global__ void __launch_bounds__(kThrS, 1) k_syn_ck(CkParams p, const uint8_t *
         // state and coefficient row of the set's next segment, loaded one segment ahead
         float2 nst = make_float2(0.f, 0.f);
         int nn = 0;
-        float4 ncoef = make_float4(0.f, 0.f, 0.f, 0.f);
+        float2 ncoef = make_float2(0.f, 0.f);
+        float nr = 0.f;
         auto fetch = [&](int i) {
             nst = make_float2(0.f, 0.f);
             nn = 0;
@@ -821,16 +859,18 @@ __global__ void __launch_bounds__(kThrS, 1) k_syn_ck(CkParams p, const uint8_t *
                 nst = __ldg(p.ck + idx);
                 nn = __ldg(p.cn + idx);
             }
-            if (t < kSeg) ncoef = diff_coef(p.coef, mb, l0 + kSeg * k + t, L, sgn_c, t == 0);
+            if (t < kSeg) ncoef = step_coef(p.coef, mb, l0 + kSeg * k + t + 1, L, sgn_c);
+            if (t == 0) nr = inv_alpha(p.coef, mb, l0 + kSeg * k, l0, L);
         };
         fetch(S);
         for (int i = S; i < nact; i += 2) {
             set_barrier_s(S);   // the set's previous segment is generated: its rows are free
             if (!dead && t < kSeg) cwin[t] = ncoef;
+            if (!dead && t == 0) sR[S] = nr;
             set_barrier_s(S);
             if (dead) continue;
-            float v = nst.x, D = nst.y;
-            int n = nn;
+            Row w;
+            w.start(nst, nn, xm1, sR[S]);
             fetch(i + 2);
             const int nh = chunks_in(i);
             for (int half = 0; half < nh; ++half, ++js) {
@@ -839,7 +879,7 @@ __global__ void __launch_bounds__(kThrS, 1) k_syn_ck(CkParams p, const uint8_t *
                     break;
                 }
                 // tile: K-major SW128, 256 N rows (lanes) of 64 K values (rows l)
-                gen_rows64(cwin + kKL * half, y, v, D, n, b0 + rowoff, kBTileS, (uint32_t)(t & 7));
+                gen_rows64(cwin + kKL * half, w, b0 + rowoff, kBTileS, (uint32_t)(t & 7));
                 tc::fence_async_smem();
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(&sh.b_full[S]);
@@ -980,7 +1020,7 @@ static int ck_analysis(int64_t nside, int64_t lmax, int spin, int sp, int64_t nc
         return GM_ERR_BAD_SHAPE;
     if (!geom || !coef || !segoff || !uoff || !ck_state || !ck_shift || !img || !alm_i || !err)
         return GM_ERR_BAD_PTR;
-    const size_t smem = kImgBufA * kAImgG + kSetsA * kTileA + kSB * sizeof(float4) + 1024;
+    const size_t smem = kImgBufA * kAImgG + kSetsA * kTileA + kSB * sizeof(float2) + 2 * sizeof(float) + 1024;
     auto kern = spin == 0 ? k_ana_ck<0> : k_ana_ck<2>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) {
@@ -1065,7 +1105,7 @@ static int ck_synthesis(int64_t nside, int64_t lmax, int spin, int sp, int64_t n
         return GM_ERR_BAD_SHAPE;
     if (!geom || !coef || !segoff || !ck_state || !ck_shift || !simg || !choff || !synd || !err)
         return GM_ERR_BAD_PTR;
-    const size_t smem = 4 * kSImg + 4 * kBTileS + 2 * kSeg * sizeof(float4) + 1024;
+    const size_t smem = 4 * kSImg + 4 * kBTileS + 2 * kSeg * sizeof(float2) + 2 * sizeof(float) + 1024;
     auto kern = spin == 0 ? k_syn_ck<0> : k_syn_ck<2>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) {
