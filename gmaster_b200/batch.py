@@ -296,7 +296,7 @@ def _upload(x, dev):
 def _stream_ring_spectra(t_maps, mask_t, dev, parts=4):
     """Copy host T maps (nsims, npix) to the device in `parts` pieces on the side stream and
     compute each piece's masked single-precision ring spectra on the current stream once
-    it has arrived.  Returns (device maps, [spectra])."""
+    it has arrived.  Returns (device maps, [spectra], event of the last copy)."""
     h = t_maps if isinstance(t_maps, torch.Tensor) else torch.from_numpy(np.ascontiguousarray(t_maps))
     if h.dtype != torch.float64:
         h = h.to(torch.float64)
@@ -320,7 +320,7 @@ def _stream_ring_spectra(t_maps, mask_t, dev, parts=4):
     for (a, b), ev in zip(zip(bounds[:-1], bounds[1:]), events):
         main.wait_event(ev)
         sht.ring_analysis(plan, d[a:b], _lib.MIXED, mask=mask_t, out=spec[a:b])
-    return d, [spec]
+    return d, [spec], events[-1]
 
 
 def mc_bandpowers(mask, t_maps, qu_maps, w00, w02, w22, *, n_iter=None, precision=None):
@@ -330,7 +330,8 @@ def mc_bandpowers(mask, t_maps, qu_maps, w00, w02, w22, *, n_iter=None, precisio
     host memory (pinned host memory lets the copies run asynchronously: the (Q, U) maps
     are copied while the T fields are transformed).  Returns three lists over the
     simulations: TT (1, nb); TE, TB (2, nb); EE, EB, BE, BB (4, nb) -- the per-simulation
-    result of ``w.decouple_cell(compute_coupled_cell(f1, f2))``.
+    result of ``w.decouple_cell(compute_coupled_cell(f1, f2))``.  The maps have been read when
+    the call returns (the bandpowers may still be on their way): their buffers can be refilled.
     """
     dev = torch.device("cuda", torch.cuda.current_device())
     mask_t = as_device(mask, torch.float64)
@@ -342,20 +343,27 @@ def mc_bandpowers(mask, t_maps, qu_maps, w00, w02, w22, *, n_iter=None, precisio
     if streamed:
         # T maps in parts: the ring transform of each part runs as soon as it has arrived,
         # behind the copies of the next parts and of the (Q, U) maps
-        t_dev, spec_box = _stream_ring_spectra(t_maps, mask_t, dev)
+        t_dev, spec_box, ev_t = _stream_ring_spectra(t_maps, mask_t, dev)
         qu_dev, ev_qu = _upload(qu_maps, dev)
     else:
         t_dev, ev_t = _upload(t_maps, dev)
         qu_dev, ev_qu = _upload(qu_maps, dev)
         if ev_t is not None:
             main.wait_event(ev_t)
-    ft = fields_from_maps(mask_t, t_dev, spin=0, n_iter=n_iter, precision=precision,
-                          ring_spectra=spec_box)
-    del t_dev, spec_box
-    if ev_qu is not None:
-        main.wait_event(ev_qu)
-    fp = fields_from_maps(mask_t, qu_dev, spin=2, n_iter=n_iter, precision=precision)
-    del qu_dev
-    return (decouple_cells(w00, compute_coupled_cells(ft, ft)),
-            decouple_cells(w02, compute_coupled_cells(ft, fp)),
-            decouple_cells(w22, compute_coupled_cells(fp, fp)))
+    try:
+        ft = fields_from_maps(mask_t, t_dev, spin=0, n_iter=n_iter, precision=precision,
+                              ring_spectra=spec_box)
+        del t_dev, spec_box
+        if ev_qu is not None:
+            main.wait_event(ev_qu)
+        fp = fields_from_maps(mask_t, qu_dev, spin=2, n_iter=n_iter, precision=precision)
+        del qu_dev
+        return (decouple_cells(w00, compute_coupled_cells(ft, ft)),
+                decouple_cells(w02, compute_coupled_cells(ft, fp)),
+                decouple_cells(w22, compute_coupled_cells(fp, fp)))
+    finally:
+        # the caller may refill pinned map buffers as soon as the call returns; nothing in the
+        # double-precision transforms waits for the copies on the host
+        for ev in (ev_t, ev_qu):
+            if ev is not None:
+                ev.synchronize()

@@ -136,6 +136,40 @@ def test_mc_bandpowers_equals_step_by_step_api(cuda):
 
 
 @pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_mc_bandpowers_has_read_pinned_maps_on_return(cuda, precision):
+    """Pinned map buffers refilled right after the call do not change its bandpowers, also where
+    the copies start late (behind 0.3 s of other work of the copy stream) and the workspaces'
+    factors have been checked before."""
+    from gmaster_b200 import batch
+
+    nside, nsims = 16, 3
+    rng = np.random.default_rng(22)
+    t = torch.from_numpy(rng.normal(size=(nsims, 12 * nside ** 2))).pin_memory()
+    qu = torch.from_numpy(rng.normal(size=(nsims, 2, 12 * nside ** 2))).pin_memory()
+    mask = _mask(nside, seed=5)
+    b = nmt.NmtBin.from_nside_linear(nside, 4)
+    f0 = nmt.NmtField(mask, None, spin=0, precision=precision)
+    f2 = nmt.NmtField(mask, None, spin=2, precision=precision)
+    ws = [nmt.NmtWorkspace.from_fields(x, y, b) for x, y in ((f0, f0), (f0, f2), (f2, f2))]
+    want = nmt.mc_bandpowers(mask, t, qu, *ws, n_iter=1, precision=precision)
+    torch.cuda.synchronize()
+    keep = t.clone(), qu.clone()
+    for _ in range(2):
+        with torch.cuda.stream(batch._copy_stream(torch.device("cuda", torch.cuda.current_device()))):
+            torch.cuda._sleep(600_000_000)
+        got = nmt.mc_bandpowers(mask, t, qu, *ws, n_iter=1, precision=precision)
+        t.zero_()
+        qu.zero_()
+        torch.cuda.synchronize()
+        t.copy_(keep[0])
+        qu.copy_(keep[1])
+        for g, w in zip(got, want):
+            for gi, wi in zip(g, w):
+                np.testing.assert_allclose(gi.cpu().numpy(), wi.cpu().numpy(), rtol=1e-12,
+                                           atol=1e-12 * float(wi.abs().max()))
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
 def test_simulation_graph_matches_eager_pipeline(cuda, precision):
     """The graph-captured per-simulation estimator gives each simulation's
     decouple_cell(compute_coupled_cell(...)) bandpowers (pseudo-C_ell sums order chunks
