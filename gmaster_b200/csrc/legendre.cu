@@ -21,9 +21,10 @@
 //
 // A CTA is up to four warps of one order; the rows go in segments of up to 128 whose
 // coefficients its threads compute once, then in blocks of eight without barriers: a warp whose
-// lanes are all below 2^-300 only steps.  Spin s sums 2a and -2a directly (four values a row
-// instead of eight).  Small sizes are bound by the chain of rows (m = 0) and the reduction
-// trees, large ones by the FP64 pipe: (3 + 2 NC) operations per row and lane (spin 0), 14 (spin
+// lanes are all below 2^-300 only steps.  Spin s takes the sum F and the difference G of the
+// two variants' rows, formed in double precision, against Q and U (four values a row, E and B:
+// at m = 0, where G = 0, E takes Q alone and B takes U alone).  Small sizes are bound by the chain of rows (m = 0) and the reduction
+// trees, large ones by the FP64 pipe: (3 + 2 NC) operations per row and lane (spin 0), 16 (spin
 // s).  Against windows of 32 rows with coefficients by square roots and divisions in each, and
 // eight sums a row: FP64 analysis / synthesis at Nside 128 56 / 44 -> 35 / 21 us, at Nside 1024
 // 10.0 / 8.1 -> 5.1 / 3.9 ms (spin 0) and 26.8 / 21.5 -> 13.0 / 9.9 ms (spin 2); mixed spin 1 at
@@ -192,7 +193,7 @@ template <int SPIN, int NC> struct Shape {
 };
 
 // Eight rows of one warp into red[8 NV].  rh: spin 0, per map Sum re, im, Diff re, im; spin s,
-// P_N, P_S, M_N, M_S (re, im).
+// Q Sum, Q Diff, U Sum, U Diff (re, im).
 template <typename T, int SPIN, int NC, int R, bool PART>
 __device__ __forceinline__ void ana8(RowState<Shape<SPIN, NC>::NVAR, R> &w, const T (&rh)[R][4 * NC],
                                      const Coef *__restrict__ cf, double *__restrict__ red, int lane)
@@ -212,25 +213,29 @@ __device__ __forceinline__ void ana8(RowState<Shape<SPIN, NC>::NVAR, R> &w, cons
             const Coef c = cf[i + s];
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                T val[NVAR];
+                double lam[NVAR];
 #pragma unroll
-                for (int q = 0; q < NVAR; ++q) val[q] = !PART || w.k[q][r] == 0 ? (T)w.v[q][r] : (T)0;
+                for (int q = 0; q < NVAR; ++q) lam[q] = !PART || w.k[q][r] == 0 ? w.v[q][r] : 0.0;
                 if (SPIN == 0) {
+                    const T val = (T)lam[0];
 #pragma unroll
                     for (int e = 0; e < NC; ++e) {
-                        acc[s * NV + 2 * e] += val[0] * rh[r][4 * e + 2 * (s & 1)];
-                        acc[s * NV + 2 * e + 1] += val[0] * rh[r][4 * e + 2 * (s & 1) + 1];
+                        acc[s * NV + 2 * e] += val * rh[r][4 * e + 2 * (s & 1)];
+                        acc[s * NV + 2 * e + 1] += val * rh[r][4 * e + 2 * (s & 1) + 1];
                     }
                 } else {
-                    const T vp = (s & 1) ? -val[NVAR - 1] : val[NVAR - 1], vm = (s & 1) ? -val[0] : val[0];
+                    // E += F Q_p + i G U_d, B += F U_p - i G Q_d
+                    const T f = (T)(lam[0] + lam[NVAR - 1]), g = (T)(lam[0] - lam[NVAR - 1]);
+                    const T *qp = rh[r] + 2 * (s & 1), *qd = rh[r] + 2 - 2 * (s & 1), *up = qp + 4, *ud = qd + 4;
                     T *a = acc + s * NV;
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        a[e] += val[0] * rh[r][e];
-                        a[e] += vp * rh[r][2 + e];
-                        a[2 + e] += val[NVAR - 1] * rh[r][4 + e];
-                        a[2 + e] += vm * rh[r][6 + e];
-                    }
+                    a[0] += f * qp[0];
+                    a[0] -= g * ud[1];
+                    a[1] += f * qp[1];
+                    a[1] += g * ud[0];
+                    a[2] += f * up[0];
+                    a[2] += g * qd[1];
+                    a[3] += f * up[1];
+                    a[3] -= g * qd[0];
                 }
                 w.step(c, r);
             }
@@ -277,21 +282,11 @@ __global__ void __launch_bounds__(kThreads) k_legendre_ana(
 #pragma unroll
             for (int q = 0; q < 4 * NC; ++q) rh[r][q] = g[q / 4][q % 4];
         } else {
-            // north = (Sum + Diff) / 2, south = (Sum - Diff) / 2; P = Q + iU, M = Q - iU.  The
-            // southern rows are the northern ones of the other variant times (-1)^(l + m + s):
-            // the sign of a segment's even rows goes into the southern right-hand sides
-            const T h = (T)0.5, hs = (l0 + m + sv) & 1 ? (T)-0.5 : (T)0.5;
-            const T *q = g[0], *u = g[NC - 1];
-            const T qnr = h * (q[0] + q[2]), qni = h * (q[1] + q[3]), qsr = hs * (q[0] - q[2]), qsi = hs * (q[1] - q[3]);
-            const T unr = h * (u[0] + u[2]), uni = h * (u[1] + u[3]), usr = hs * (u[0] - u[2]), usi = hs * (u[1] - u[3]);
-            rh[r][0] = qnr - uni;
-            rh[r][1] = qni + unr;
-            rh[r][2] = qsr - usi;
-            rh[r][3] = qsi + usr;
-            rh[r][4] = qnr + uni;
-            rh[r][5] = qni - unr;
-            rh[r][6] = qsr + usi;
-            rh[r][7] = qsi - usr;
+            // the southern rows are the northern ones of the other variant times (-1)^(l + m + s):
+            // where a segment's even rows have it odd, Sum and Diff change places
+            const int p = (l0 + m + sv) & 1;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) rh[r][q] = p ? g[q / 4][(q + 2) % 4] : g[q / 4][q % 4];
         }
     }
 
@@ -340,13 +335,12 @@ __global__ void __launch_bounds__(kThreads) k_legendre_ana(
                     }
                 }
             } else {
-                // E = -(+sa + -sa) / 2, B = i (+sa - -sa) / 2
                 double *e = alm + 2 * (c0 * nelem + idx), *b = e + 2 * nelem;
-                const double hs = 0.5 * scale;
-                atomicAdd(e, -hs * (sum[0] + sum[2]));
-                atomicAdd(e + 1, -hs * (sum[1] + sum[3]));
-                atomicAdd(b, -hs * (sum[1] - sum[3]));
-                atomicAdd(b + 1, hs * (sum[0] - sum[2]));
+                const double hs = -0.5 * scale;
+                atomicAdd(e, hs * sum[0]);
+                atomicAdd(e + 1, hs * sum[1]);
+                atomicAdd(b, hs * sum[2]);
+                atomicAdd(b + 1, hs * sum[3]);
             }
         }
     }
@@ -355,8 +349,8 @@ __global__ void __launch_bounds__(kThreads) k_legendre_ana(
 // ---------------------------------------------------------------- synthesis
 
 // Eight rows of one warp added to the accumulators.  aw[row][.]: spin 0, (re, im) per map; spin s,
-// +sa and -sa (re, im).  acc: spin 0, per map the even and odd rows (re, im); spin s, U_N, V_N
-// (of +sa, -sa), U_S, V_S.
+// E and B (re, im).  acc: spin 0, per map the even and odd rows (re, im); spin s, Q Sum, Q Diff,
+// U Sum, U Diff (re, im): F of an even row and G of an odd one go to the hemispheres' sum.
 template <typename T, int SPIN, int NC, int R, bool PART>
 __device__ __forceinline__ void syn8(RowState<Shape<SPIN, NC>::NVAR, R> &w, T (&acc)[R][4 * NC],
                                      const Coef *__restrict__ cf, const T *__restrict__ aw)
@@ -370,25 +364,29 @@ __device__ __forceinline__ void syn8(RowState<Shape<SPIN, NC>::NVAR, R> &w, T (&
         for (int q = 0; q < 2 * NA; ++q) a[q] = aw[s * 2 * NA + q];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            T val[NVAR];
+            double lam[NVAR];
 #pragma unroll
-            for (int q = 0; q < NVAR; ++q) val[q] = !PART || w.k[q][r] == 0 ? (T)w.v[q][r] : (T)0;
+            for (int q = 0; q < NVAR; ++q) lam[q] = !PART || w.k[q][r] == 0 ? w.v[q][r] : 0.0;
             T *o = acc[r];
             if (SPIN == 0) {
+                const T val = (T)lam[0];
 #pragma unroll
                 for (int e = 0; e < NC; ++e) {
-                    o[4 * e + 2 * (s & 1)] += val[0] * a[2 * e];
-                    o[4 * e + 2 * (s & 1) + 1] += val[0] * a[2 * e + 1];
+                    o[4 * e + 2 * (s & 1)] += val * a[2 * e];
+                    o[4 * e + 2 * (s & 1) + 1] += val * a[2 * e + 1];
                 }
             } else {
-                const T vp = (s & 1) ? -val[NVAR - 1] : val[NVAR - 1], vm = (s & 1) ? -val[0] : val[0];
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    o[e] += val[0] * a[e];
-                    o[2 + e] += val[NVAR - 1] * a[2 + e];
-                    o[4 + e] += vp * a[e];
-                    o[6 + e] += vm * a[2 + e];
-                }
+                // -2 Q = F E + i G B, -2 U = F B - i G E
+                const T f = (T)(lam[0] + lam[NVAR - 1]), g = (T)(lam[0] - lam[NVAR - 1]);
+                T *qp = o + 2 * (s & 1), *qd = o + 2 - 2 * (s & 1), *up = qp + 4, *ud = qd + 4;
+                qp[0] += f * a[0];
+                qp[1] += f * a[1];
+                up[0] += f * a[2];
+                up[1] += f * a[3];
+                qd[0] -= g * a[3];
+                qd[1] += g * a[2];
+                ud[0] += g * a[1];
+                ud[1] -= g * a[0];
             }
             w.step(c, r);
         }
@@ -404,7 +402,7 @@ __global__ void __launch_bounds__(kThreads) k_legendre_syn(
 {
     using S = Shape<SPIN, NC>;
     constexpr int NVAR = S::NVAR, kRows = 128;
-    constexpr int NA = SPIN == 0 ? NC : 2;  // complex alm rows per degree (maps, or +sa and -sa)
+    constexpr int NA = SPIN == 0 ? NC : 2;  // complex alm rows per degree (maps, or E and B)
     __shared__ Coef cf[kRows];
     __shared__ T aw[kRows * 2 * NA];
     const int64_t L = lmax + 1, nlanes = 2 * nside, nelem = L * (L + 1) / 2;
@@ -445,11 +443,10 @@ __global__ void __launch_bounds__(kThreads) k_legendre_syn(
                     e = src[0];
                     b = src[nelem];
                 }
-                // +sa = -(E + iB), -sa = -(E - iB)
-                o[0] = (T)(b.y - e.x);
-                o[1] = (T)(-e.y - b.x);
-                o[2] = (T)(-e.x - b.y);
-                o[3] = (T)(b.x - e.y);
+                o[0] = (T)e.x;
+                o[1] = (T)e.y;
+                o[2] = (T)b.x;
+                o[3] = (T)b.y;
             }
         }
         __syncthreads();
@@ -472,7 +469,8 @@ __global__ void __launch_bounds__(kThreads) k_legendre_syn(
         }
     }
 
-    const T hs = (l0 + m + sv) & 1 ? (T)-0.5 : (T)0.5;   // (-1)^(l + m + s) of the even rows
+    // Sum and Diff change places where even rows have odd l + m + s
+    const T h = (T)-0.5, hs = (l0 + m + sv) & 1 ? (T)0.5 : (T)-0.5;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int64_t j = jw + r * 32 + lane;
@@ -489,17 +487,15 @@ __global__ void __launch_bounds__(kThreads) k_legendre_syn(
                 o[3] = a[4 * c + 1] - a[4 * c + 3];
             }
         } else {
-            // Q = (U + V) / 2, U map = (U - V) / 2i, both hemispheres
-            T *oq = syn + (((int64_t)m * nlanes + j) * ncomp + c0) * 4, *ou = oq + 4;
-            const T h = (T)0.5;
-            oq[0] = h * (a[0] + a[2]);
-            oq[1] = h * (a[1] + a[3]);
-            oq[2] = hs * (a[4] + a[6]);
-            oq[3] = hs * (a[5] + a[7]);
-            ou[0] = h * (a[1] - a[3]);
-            ou[1] = -h * (a[0] - a[2]);
-            ou[2] = hs * (a[5] - a[7]);
-            ou[3] = -hs * (a[4] - a[6]);
+            T *o = syn + (((int64_t)m * nlanes + j) * ncomp + c0) * 4;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const T *q = a + 4 * c;   // north = Sum + Diff, south = Sum - Diff
+                o[4 * c] = h * (q[0] + q[2]);
+                o[4 * c + 1] = h * (q[1] + q[3]);
+                o[4 * c + 2] = hs * (q[0] - q[2]);
+                o[4 * c + 3] = hs * (q[1] - q[3]);
+            }
         }
     }
 }

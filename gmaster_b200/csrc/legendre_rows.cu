@@ -14,13 +14,20 @@
 // Packing.  All arithmetic is on pairs of floats (fma.rn.f32x2: two FMAs per issue slot; the
 // FMA rate is that of scalar code, 128 a clock and SM, but at half the issue slots, which the
 // reduction's selects, adds and loads take).  A pair is two lanes of one warp for spin 0, and
-// the two row variants s' = -2, +2 of one lane for spin 2: the contraction
-//     2a_l  = sum  v^- P_N + s v^+ P_S,    -2a_l = sum  v^+ M_N + s v^- M_S,
-// s = (-1)^(l+m), P = Q + iU, M = Q - iU, is then four packed FMAs a row and lane whose two
-// halves are added with the sign s, fixed by the row's index, once per block of rows.
+// the two row variants s' = -2, +2 of one lane for spin 2.  There the contraction takes their
+// sum F = v^- + v^+ and difference G = v^- - v^+ (two scalar additions a row and lane):
+//     -2 E_l = sum  F Q_p + i G U_d,    -2 B_l = sum  F U_p - i G Q_d,
+// p the hemispheres' sum and d their difference where l + m is even, the other way round where
+// it is odd: four packed FMAs of (F, G), for odd rows of (G, F), whose two halves are added
+// once per block of rows.  E and B are never formed from each other's rounded values: at m = 0
+// (G = 0) E takes Q alone and B takes U alone, and elsewhere a B far below E carries the
+// rounding of the products G Q only.  Summing 2a and -2a instead (P = Q + iU, M = Q - iU, no
+// F and G) takes 4 % less time (field, spin 2, Nside 512: 6.8 against 7.1 ms) and leaves the
+// rounding of E in B: with U = 1e-3 Q the error of B at m = 0, Nside 512, is 7e-5 of B there, 3e-7
+// here.
 //
 // Bound and split.  The FMA pipe: (3 + 2 NC) packed FMAs per row and two lanes for spin 0, 7
-// per row and lane for spin 2, plus one shuffle per row, value and thread in the analysis
+// and two additions per row and lane for spin 2, plus one shuffle per row, value and thread in the analysis
 // (the shuffle unit takes one instruction a clock and SM, a quarter of the FMA issue rate, so
 // a thread sums its 2R or R lanes first).  At Nside 512 the pipe is 60-64 % busy (a packed FMA
 // of three different operands issues at 1.37 a clock and SM instead of 2: the register file's
@@ -239,6 +246,15 @@ template <int SPIN, int R> struct Rows {
         return __any_sync(0xffffffffu, any != 0);
     }
 
+    // Spin 2: sum and difference of the two variants' values, in this order (even rows) or the
+    // other (odd rows).
+    static __device__ __forceinline__ u64 variant_sums(u64 val, bool odd)
+    {
+        float a, b;
+        unpack(val, a, b);
+        return odd ? pack(a - b, a + b) : pack(a + b, a - b);
+    }
+
     __device__ __forceinline__ void step(int u, u64 e, u64 al)
     {
         const u64 C = add2(y[u], e);
@@ -278,11 +294,13 @@ __device__ __forceinline__ float reduce_scatter(float (&v)[V], int lane)
 
 // Eight rows of one warp: the row values times the right-hand sides, summed over the warp's
 // lanes into red[8 NV] (value v of row s at s NV + v).  rh[u][.]: spin 0, per map Sum re, im
-// and Diff re, im (each two lanes); spin 2, (P_N, P_S) re, im and (M_S, M_N) re, im.
+// and Diff re, im (each two lanes); spin 2, the factors of (F, G) that give E re, E im, B re,
+// B im on even rows, and of (G, F) for -(B im), B re, E im, -(E re) on odd rows.
 template <int SPIN, int NC, int R, bool SCALED>
 __device__ __forceinline__ void ana8(Rows<SPIN, R> &w, const u64 (&rh)[R][4 * NC], const float4 *__restrict__ cf,
                                      float *__restrict__ red, int lane)
 {
+    using W = Rows<SPIN, R>;
     constexpr int NV = SPIN == 0 ? 2 * NC : 4;
     constexpr int V = NV == 16 ? 32 : 16;
     constexpr int RB = V / NV;
@@ -312,7 +330,10 @@ __device__ __forceinline__ void ana8(Rows<SPIN, R> &w, const u64 (&rh)[R][4 * NC
                     }
                 } else {
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) acc[s * 4 + q] = fma2(val, rh[u][q], acc[s * 4 + q]);
+                    for (int q = 0; q < 4; ++q) {
+                        u64 &a = acc[s * 4 + ((s & 1) ? 3 - q : q)];
+                        a = fma2(W::variant_sums(val, s & 1), rh[u][q], a);
+                    }
                 }
                 w.step(u, e, al);
             }
@@ -322,10 +343,8 @@ __device__ __forceinline__ void ana8(Rows<SPIN, R> &w, const u64 (&rh)[R][4 * NC
         for (int q = 0; q < V; ++q) {
             float a, b;
             unpack(acc[q], a, b);
-            // spin 2: the south half carries (-1)^(row); P_S is the second half, M_S the first
             const int s = q / NV, k = q % NV;
-            if (SPIN == 0 || (s & 1) == 0) out[q] = a + b;
-            else out[q] = k < 2 ? a - b : b - a;
+            out[q] = SPIN == 2 && (s & 1) && (k == 0 || k == 3) ? -a - b : a + b;
         }
         const float tot = reduce_scatter<V>(out, lane);
         if (lane < V) red[i * NV + lane] = tot;
@@ -384,21 +403,14 @@ __global__ void __launch_bounds__(32 * max_warps(SPIN, R), ana_ctas(SPIN, NC, R)
                 q = src[0];
                 p = src[1];
             }
-            // north = (Sum + Diff) / 2, south = (Sum - Diff) / 2; P = Q + iU, M = Q - iU
-            const float qnr = 0.5f * (q.x + q.z), qni = 0.5f * (q.y + q.w);
-            float qsr = 0.5f * (q.x - q.z), qsi = 0.5f * (q.y - q.w);
-            const float unr = 0.5f * (p.x + p.z), uni = 0.5f * (p.y + p.w);
-            float usr = 0.5f * (p.x - p.z), usi = 0.5f * (p.y - p.w);
-            if ((l0 + m) & 1) {   // (-1)^(l+m) of the segments' even rows
-                qsr = -qsr;
-                qsi = -qsi;
-                usr = -usr;
-                usi = -usi;
+            if ((l0 + m) & 1) {   // the segments' even rows have odd l + m: Sum and Diff change places
+                q = make_float4(q.z, q.w, q.x, q.y);
+                p = make_float4(p.z, p.w, p.x, p.y);
             }
-            rh[u][0] = pack(qnr - uni, qsr - usi);
-            rh[u][1] = pack(qni + unr, qsi + usr);
-            rh[u][2] = pack(qsr + usi, qnr + uni);
-            rh[u][3] = pack(qsi - usr, qni - unr);
+            rh[u][0] = pack(q.x, -p.w);
+            rh[u][1] = pack(q.y, p.z);
+            rh[u][2] = pack(p.x, q.w);
+            rh[u][3] = pack(p.y, -q.z);
         }
     }
 
@@ -452,13 +464,12 @@ __global__ void __launch_bounds__(32 * max_warps(SPIN, R), ana_ctas(SPIN, NC, R)
                     }
                 }
             } else {
-                // E = -(2a + -2a) / 2, B = i (2a - -2a) / 2
                 double *e = alm + 2 * (c0 * nelem + idx), *b = e + 2 * nelem;
-                const double hs = 0.5 * scale;
-                atomicAdd(e, -hs * (sv[0] + sv[2]));
-                atomicAdd(e + 1, -hs * (sv[1] + sv[3]));
-                atomicAdd(b, -hs * (sv[1] - sv[3]));
-                atomicAdd(b + 1, hs * (sv[0] - sv[2]));
+                const double hs = -0.5 * scale;
+                atomicAdd(e, hs * sv[0]);
+                atomicAdd(e + 1, hs * sv[1]);
+                atomicAdd(b, hs * sv[2]);
+                atomicAdd(b + 1, hs * sv[3]);
             }
         }
     }
@@ -467,11 +478,14 @@ __global__ void __launch_bounds__(32 * max_warps(SPIN, R), ana_ctas(SPIN, NC, R)
 // ---------------------------------------------------------------- synthesis
 
 // Eight rows of one warp added to the accumulators.  aw[row][.]: spin 0, per map (re, re, im,
-// im); spin 2, (2a re, s 2a re, 2a im, s 2a im) and (s -2a re, -2a re, s -2a im, -2a im).
+// im); spin 2, the factors of (F, G) in Q re, Q im and U re, U im (even rows; odd rows of (G, F)).
+// acc of spin 2: (Sum, Diff) of Q re, Q im, U re, U im: F of an even row and G of an odd one go
+// to the hemispheres' sum, the others to their difference.
 template <int SPIN, int NC, int R, bool SCALED>
 __device__ __forceinline__ void syn8(Rows<SPIN, R> &w, u64 (&acc)[R][4 * NC], const float4 *__restrict__ cf,
                                      const float4 *__restrict__ aw)
 {
+    using W = Rows<SPIN, R>;
     constexpr int NA = SPIN == 0 ? NC : 2;
     u64 sc[R];
     if (SCALED) {
@@ -497,7 +511,7 @@ __device__ __forceinline__ void syn8(Rows<SPIN, R> &w, u64 (&acc)[R][4 * NC], co
                 }
             } else {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) acc[u][q] = fma2(val, a[q], acc[u][q]);
+                for (int q = 0; q < 4; ++q) acc[u][q] = fma2(W::variant_sums(val, s & 1), a[q], acc[u][q]);
             }
             w.step(u, e, al);
         }
@@ -560,12 +574,10 @@ __global__ void __launch_bounds__(32 * max_warps(SPIN, R)) k_rows_syn(int64_t ns
                     e = src[0];
                     b = src[nelem];
                 }
-                // 2a = -(E + iB), -2a = -(E - iB)
-                const float pr = (float)(b.y - e.x), pi = (float)(-e.y - b.x);
-                const float mr = (float)(-e.x - b.y), mi = (float)(b.x - e.y);
-                const float s = ((lb + i + m) & 1) ? -1.f : 1.f;
-                aw[i * 2] = make_float4(pr, s * pr, pi, s * pi);
-                aw[i * 2 + 1] = make_float4(s * mr, mr, s * mi, mi);
+                // 2 Q = -F E - i G B, 2 U = -F B + i G E
+                const float er = (float)e.x, ei = (float)e.y, br = (float)b.x, bi = (float)b.y;
+                aw[i * 2] = (i & 1) ? make_float4(bi, -er, -br, -ei) : make_float4(-er, bi, -ei, -br);
+                aw[i * 2 + 1] = (i & 1) ? make_float4(-ei, -br, er, -bi) : make_float4(-br, -ei, -bi, er);
             }
         }
         const bool on = (act & mine) != 0ull;
@@ -608,15 +620,15 @@ __global__ void __launch_bounds__(32 * max_warps(SPIN, R)) k_rows_syn(int64_t ns
         } else {
             const int64_t j = W::lane_of(jw, u, 0, lane);
             if (j >= nlanes) continue;
-            // halves: (U_N, U_S) of 2a and (V_S, V_N) of -2a; Q = (U + V) / 2, U map = (U - V) / 2i
-            float unr, usr, uni, usi, vnr, vsr, vni, vsi;
-            unpack(acc[u][0], unr, usr);
-            unpack(acc[u][1], uni, usi);
-            unpack(acc[u][2], vsr, vnr);
-            unpack(acc[u][3], vsi, vni);
-            out[j * ncomp] = make_float4(0.5f * (unr + vnr), 0.5f * (uni + vni), 0.5f * (usr + vsr), 0.5f * (usi + vsi));
-            out[j * ncomp + 1] = make_float4(0.5f * (uni - vni), -0.5f * (unr - vnr), 0.5f * (usi - vsi),
-                                             -0.5f * (usr - vsr));
+            // north = Sum + Diff, south = Sum - Diff, the other way round where even rows have odd l + m
+            const float hs = (l0 + m) & 1 ? -0.5f : 0.5f;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                float sr, dr, si, di;
+                unpack(acc[u][2 * c], sr, dr);
+                unpack(acc[u][2 * c + 1], si, di);
+                out[j * ncomp + c] = make_float4(0.5f * (sr + dr), 0.5f * (si + di), hs * (sr - dr), hs * (si - di));
+            }
         }
     }
 }
