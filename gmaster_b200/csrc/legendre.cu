@@ -107,23 +107,37 @@ __device__ __forceinline__ Coef step_coef(int l, int m, int s)
     return Coef{e + c, e - c, 1.0 / r1};
 }
 
-template <typename T, int V>
-__device__ __forceinline__ T warp_reduce_scatter(T (&v)[V], int lane)
+// Sum of each of the V values of all 32 threads: thread t returns value t % V.  The last LD of the
+// five levels add in double precision.
+template <int LD, typename T, int V>
+__device__ __forceinline__ double warp_reduce_scatter(T (&v)[V], int lane)
 {
+    double w[V];
 #pragma unroll
-    for (int h = V / 2; h >= 1; h >>= 1) {
+    for (int h = V / 2, level = 5; h >= 1; h >>= 1, --level) {
         const bool upper = (lane & h) != 0;
 #pragma unroll
         for (int i = 0; i < h; ++i) {
-            T send = upper ? v[i] : v[i + h];
-            T keep = upper ? v[i + h] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+            if (level > LD) {
+                const T send = upper ? v[i] : v[i + h], keep = upper ? v[i + h] : v[i];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+                w[i] = (double)v[i];
+            } else {
+                const double send = upper ? w[i] : w[i + h], keep = upper ? w[i + h] : w[i];
+                w[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+            }
         }
     }
-    T r = v[0];
 #pragma unroll
-    for (int h = V; h < 32; h <<= 1) r += __shfl_xor_sync(0xffffffffu, r, h);
-    return r;
+    for (int h = V, level = V == 16 ? 1 : 0; h < 32; h <<= 1, --level) {
+        if (level > LD) {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], h);
+            w[0] = (double)v[0];
+        } else {
+            w[0] += __shfl_xor_sync(0xffffffffu, w[0], h);
+        }
+    }
+    return w[0];
 }
 
 __device__ __forceinline__ int64_t alm_index(int64_t lmax, int64_t l, int64_t m)
@@ -226,6 +240,12 @@ __device__ __forceinline__ void ana8(RowState<Shape<SPIN, NC>::NVAR, R> &w, cons
     // values per reduction tree: 32 where the registers allow (half the trees, of one more level)
     constexpr int V = (NV * 8 >= 32 && R <= 2) || NV == 16 ? 32 : 16;
     constexpr int RB = V / NV;
+    // Spin s adds the F and the G terms in one chain of 2 R products; the last levels of the tree in
+    // double precision take off as much rounding as that adds over two chains and trees of R
+    // products each (in units of a product's: 3, 10, 36, 136 and 5 x 2 R less 2 R a level against 2,
+    // 6, 20, 72 and 5 x 2 R).
+    constexpr int LD = SPIN == 0 || sizeof(T) == 8 ? 0 : (R <= 2 ? 1 : (R == 4 ? 2 : 4));
+    static_assert(V == 16 || V == 32, "levels of the tree");
     static_assert(RB % 2 == 0 && 8 % RB == 0, "row parity is fixed by the row index");
 #pragma unroll 1
     for (int i = 0; i < 8; i += RB) {
@@ -264,8 +284,8 @@ __device__ __forceinline__ void ana8(RowState<Shape<SPIN, NC>::NVAR, R> &w, cons
                 w.step(c, r);
             }
         }
-        const T tot = warp_reduce_scatter<T, V>(acc, lane);
-        if (lane < V) red[i * NV + lane] = (double)tot;
+        const double tot = warp_reduce_scatter<LD>(acc, lane);
+        if (lane < V) red[i * NV + lane] = tot;
     }
     w.rescale();
 }
@@ -427,8 +447,14 @@ __global__ void __launch_bounds__(kThreads) k_legendre_syn(
     using S = Shape<SPIN, NC>;
     constexpr int NVAR = S::NVAR, kRows = 128;
     constexpr int NA = SPIN == 0 ? NC : 2;  // complex alm rows per degree (maps, or E and B)
+    // Spin s in single precision: the sums of the rows done, kept apart from the running one of 32
+    // rows (even rows' F and odd rows' G terms share an accumulator: one over all rows would add
+    // twice as many terms as sums of F and G apart).  Spin 1, Nside 512: relative error of a pass
+    // 1.5e-7; one accumulator over all rows 5.7e-7, F and G apart 4.1e-7.
+    constexpr bool kTwoLevel = SPIN != 0 && sizeof(T) == 4;
     __shared__ Coef cf[kRows];
     __shared__ T aw[kRows * 2 * NA];
+    __shared__ T done[kTwoLevel ? R * 4 * NC : 1][kTwoLevel ? kThreads : 1];
     const int64_t L = lmax + 1, nlanes = 2 * nside, nelem = L * (L + 1) / 2;
     const int m = blockIdx.y;
     const int64_t c0 = (int64_t)blockIdx.z * NC;
@@ -443,7 +469,10 @@ __global__ void __launch_bounds__(kThreads) k_legendre_syn(
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
-        for (int q = 0; q < 4 * NC; ++q) acc[r][q] = (T)0;
+        for (int q = 0; q < 4 * NC; ++q) {
+            acc[r][q] = (T)0;
+            if (kTwoLevel) done[r * 4 * NC + q][threadIdx.x] = (T)0;
+        }
 
     for (int64_t lb = l0; lb < L; lb += kRows) {
         const int nrow = (int)(L - lb < kRows ? L - lb : kRows);
@@ -490,7 +519,19 @@ __global__ void __launch_bounds__(kThreads) k_legendre_syn(
                 }
                 w.rescale();
             }
+            if (kTwoLevel && ((i & 24) == 24 || i + 8 >= nrow)) {
+#pragma unroll
+                for (int q = 0; q < R * 4 * NC; ++q) {
+                    T &d = done[q][threadIdx.x];
+                    d += acc[q / (4 * NC)][q % (4 * NC)];
+                    acc[q / (4 * NC)][q % (4 * NC)] = (T)0;
+                }
+            }
         }
+    }
+    if (kTwoLevel) {
+#pragma unroll
+        for (int q = 0; q < R * 4 * NC; ++q) acc[q / (4 * NC)][q % (4 * NC)] = done[q][threadIdx.x];
     }
 
     // Sum and Diff change places where even rows have odd l + m + s

@@ -59,3 +59,30 @@ def test_synthesis_of_order_zero_keeps_e_and_b_apart(cuda, nside, lmax, spin, pr
     want = sht.legendre_synthesis(plan, spin, alm, 2, _lib.FP64)
     err = (got - want)[0, :, 1].norm() / want[0, :, 1].norm()
     assert float(err) < 4e-6
+
+
+@pytest.mark.parametrize("nside,lmax,spin,tiles", [(256, 767, 1, {0: 0, 1: 1, 2: 2, 3: 9}),
+                                                   (256, 767, 4, {0: 0, 2: 2}), (64, 191, 1, {0: 0})])
+def test_single_precision_sums_of_spin_s_err_no_more_than_those_of_spin_zero(cuda, nside, lmax, spin, tiles):
+    """Mixed passes from double-precision rows: the error is that of the single-precision sums,
+    R lanes a thread and 32 threads a tree (analysis) or the rows of an order (synthesis), for E and B
+    as for one spin-0 map with the same R (tiles: spin s -> spin 0); 3 % for the draw."""
+    plan, prec, real, gen = _setup(nside, lmax, "mixed")
+    rhs = torch.randn((plan.L, plan.nlanes, 2, 4), generator=gen, device="cuda", dtype=real)
+    alm = torch.randn((2, plan.nelem), generator=gen, device="cuda", dtype=torch.complex128)
+
+    def errors(s, tile):
+        nc = 1 if s == 0 else 2
+        out = []
+        for kind, src in (("ana", rhs[:, :, :nc].contiguous()), ("syn", alm[:nc].contiguous())):
+            shape, kinds = ((nc, plan.nelem), (torch.complex128,) * 2) if kind == "ana" else (
+                (plan.L, plan.nlanes, nc, 4), (torch.float32, torch.float64))
+            got, want = (torch.zeros(shape, dtype=k, device="cuda") for k in kinds)
+            sht.run_legendre(plan, s, nc, prec, kind, tile, src, got)
+            sht.run_legendre(plan, s, nc, _lib.FP64, kind, -1, src.double() if kind == "ana" else src, want)
+            out.append(float((got - want).norm() / want.norm()))
+        return out
+
+    for tile, same in tiles.items():
+        for got, ref in zip(errors(spin, tile), errors(0, same)):
+            assert got < 1.03 * ref
