@@ -480,26 +480,18 @@ __global__ void __launch_bounds__(kThreads) k_legendre_syn(
         for (int i = threadIdx.x; i < kRows; i += blockDim.x) {
             const bool in = i < nrow;
             cf[i] = in ? step_coef((int)lb + i, m, sv) : Coef{0.0, 0.0, 0.0};
-            const double2 *src = reinterpret_cast<const double2 *>(alm) + c0 * nelem + (in ? alm_index(lmax, lb + i, m) : 0);
+            const double *src = alm + 2 * (c0 * nelem + (in ? alm_index(lmax, lb + i, m) : 0));   // 8-byte aligned
             T *o = aw + i * 2 * NA;
             if (SPIN == 0) {
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
-                    double2 a = make_double2(0.0, 0.0);
-                    if (in && c0 + c < ncomp) a = src[c * nelem];
-                    o[2 * c] = (T)a.x;
-                    o[2 * c + 1] = (T)a.y;
+                    const bool have = in && c0 + c < ncomp;
+                    o[2 * c] = have ? (T)src[2 * c * nelem] : (T)0;
+                    o[2 * c + 1] = have ? (T)src[2 * c * nelem + 1] : (T)0;
                 }
             } else {
-                double2 e = make_double2(0.0, 0.0), b = e;
-                if (in) {
-                    e = src[0];
-                    b = src[nelem];
-                }
-                o[0] = (T)e.x;
-                o[1] = (T)e.y;
-                o[2] = (T)b.x;
-                o[3] = (T)b.y;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) o[q] = in ? (T)src[2 * (q / 2) * nelem + q % 2] : (T)0;
             }
         }
         __syncthreads();

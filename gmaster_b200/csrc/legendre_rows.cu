@@ -134,6 +134,23 @@ __device__ __forceinline__ float4 step_coef(int l, int m, int s)
     return make_float4((float)(e + c), (float)(e - c), a, a);
 }
 
+// Four floats of an array aligned to 16 bytes (wide) or to its elements.
+__device__ __forceinline__ float4 load4(const float *p, bool wide)
+{
+    return wide ? *reinterpret_cast<const float4 *>(p) : make_float4(p[0], p[1], p[2], p[3]);
+}
+__device__ __forceinline__ void store4(float *p, float4 v, bool wide)
+{
+    if (wide) {
+        *reinterpret_cast<float4 *>(p) = v;
+    } else {
+        p[0] = v.x;
+        p[1] = v.y;
+        p[2] = v.z;
+        p[3] = v.w;
+    }
+}
+
 __device__ __forceinline__ int64_t alm_index(int64_t lmax, int64_t l, int64_t m)
 {
     return m * (2 * lmax + 1 - m) / 2 + l;
@@ -359,7 +376,7 @@ __host__ __device__ constexpr int ana_ctas(int spin, int nc, int r) { return spi
 template <int SPIN, int NC, int R>
 __global__ void __launch_bounds__(32 * max_warps(SPIN, R), ana_ctas(SPIN, NC, R)) k_rows_ana(int64_t nside, int64_t lmax, int64_t ncomp,
                                                           const double *__restrict__ geom,
-                                                          const float *__restrict__ rhs,
+                                                          const float *__restrict__ rhs, bool wide,
                                                           double *__restrict__ alm, double scale, Tab tab)
 {
     constexpr int NV = SPIN == 0 ? 2 * NC : 4;
@@ -386,9 +403,9 @@ __global__ void __launch_bounds__(32 * max_warps(SPIN, R), ana_ctas(SPIN, NC, R)
             for (int c = 0; c < NC; ++c) {
                 float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
                 if (c0 + c < ncomp) {
-                    const float4 *src = reinterpret_cast<const float4 *>(rhs) + (int64_t)m * nlanes * ncomp + c0 + c;
-                    if (j0 < nlanes) a = src[j0 * ncomp];
-                    if (j1 < nlanes) b = src[j1 * ncomp];
+                    const float *src = rhs + 4 * ((int64_t)m * nlanes * ncomp + c0 + c);
+                    if (j0 < nlanes) a = load4(src + 4 * j0 * ncomp, wide);
+                    if (j1 < nlanes) b = load4(src + 4 * j1 * ncomp, wide);
                 }
                 rh[u][4 * c] = pack(a.x, b.x);
                 rh[u][4 * c + 1] = pack(a.y, b.y);
@@ -399,9 +416,9 @@ __global__ void __launch_bounds__(32 * max_warps(SPIN, R), ana_ctas(SPIN, NC, R)
             const int64_t j = W::lane_of(jw, u, 0, lane);
             float4 q = make_float4(0.f, 0.f, 0.f, 0.f), p = q;
             if (j < nlanes) {
-                const float4 *src = reinterpret_cast<const float4 *>(rhs) + ((int64_t)m * nlanes + j) * ncomp + c0;
-                q = src[0];
-                p = src[1];
+                const float *src = rhs + 4 * (((int64_t)m * nlanes + j) * ncomp + c0);
+                q = load4(src, wide);
+                p = load4(src + 4, wide);
             }
             if ((l0 + m) & 1) {   // the segments' even rows have odd l + m: Sum and Diff change places
                 q = make_float4(q.z, q.w, q.x, q.y);
@@ -523,7 +540,7 @@ template <int SPIN, int NC, int R>
 __global__ void __launch_bounds__(32 * max_warps(SPIN, R)) k_rows_syn(int64_t nside, int64_t lmax, int64_t ncomp,
                                                           const double *__restrict__ geom,
                                                           const double *__restrict__ alm,
-                                                          float *__restrict__ syn, Tab tab)
+                                                          float *__restrict__ syn, bool wide, Tab tab)
 {
     constexpr int NVAR = SPIN == 0 ? 1 : 2;
     constexpr int NA = SPIN == 0 ? NC : 2;
@@ -567,22 +584,18 @@ __global__ void __launch_bounds__(32 * max_warps(SPIN, R)) k_rows_syn(int64_t ns
             const bool in = i < nrow;
             cf[i] = in ? step_coef(lb + i, m, SPIN) : make_float4(0.f, 0.f, 0.f, 0.f);
             const int64_t idx = in ? alm_index(lmax, lb + i, m) : 0;
-            const double2 *src = reinterpret_cast<const double2 *>(alm) + c0 * nelem + idx;
+            const double *src = alm + 2 * (c0 * nelem + idx);   // 8-byte aligned
             if (SPIN == 0) {
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
-                    double2 a = make_double2(0.0, 0.0);
-                    if (in && c0 + c < ncomp) a = src[c * nelem];
-                    aw[i * NC + c] = make_float4((float)a.x, (float)a.x, (float)a.y, (float)a.y);
+                    const bool have = in && c0 + c < ncomp;
+                    const float re = have ? (float)src[2 * c * nelem] : 0.f, im = have ? (float)src[2 * c * nelem + 1] : 0.f;
+                    aw[i * NC + c] = make_float4(re, re, im, im);
                 }
             } else {
-                double2 e = make_double2(0.0, 0.0), b = e;
-                if (in) {
-                    e = src[0];
-                    b = src[nelem];
-                }
                 // 2 Q = -F E - i G B, 2 U = -F B + i G E
-                const float er = (float)e.x, ei = (float)e.y, br = (float)b.x, bi = (float)b.y;
+                const float er = in ? (float)src[0] : 0.f, ei = in ? (float)src[1] : 0.f;
+                const float br = in ? (float)src[2 * nelem] : 0.f, bi = in ? (float)src[2 * nelem + 1] : 0.f;
                 aw[i * 2] = (i & 1) ? make_float4(bi, -er, -br, -ei) : make_float4(-er, bi, -ei, -br);
                 aw[i * 2 + 1] = (i & 1) ? make_float4(-ei, -br, er, -bi) : make_float4(-br, -ei, -bi, er);
             }
@@ -616,7 +629,7 @@ __global__ void __launch_bounds__(32 * max_warps(SPIN, R)) k_rows_syn(int64_t ns
         for (int q = 0; q < R * 4; ++q) acc[q / 4][q % 4] = done[q][threadIdx.x];
     }
 
-    float4 *out = reinterpret_cast<float4 *>(syn) + (int64_t)m * nlanes * ncomp + c0;
+    float *out = syn + 4 * ((int64_t)m * nlanes * ncomp + c0);
 #pragma unroll
     for (int u = 0; u < R; ++u) {
         if (SPIN == 0) {
@@ -631,8 +644,8 @@ __global__ void __launch_bounds__(32 * max_warps(SPIN, R)) k_rows_syn(int64_t ns
                 for (int h = 0; h < 2; ++h) {
                     const int64_t j = W::lane_of(jw, u, h, lane);
                     if (j < nlanes)
-                        out[j * ncomp + c] = make_float4(e[h][0] + e[h][2], e[h][1] + e[h][3], e[h][0] - e[h][2],
-                                                         e[h][1] - e[h][3]);
+                        store4(out + 4 * (j * ncomp + c),
+                               make_float4(e[h][0] + e[h][2], e[h][1] + e[h][3], e[h][0] - e[h][2], e[h][1] - e[h][3]), wide);
                 }
             }
         } else {
@@ -645,7 +658,8 @@ __global__ void __launch_bounds__(32 * max_warps(SPIN, R)) k_rows_syn(int64_t ns
                 float sr, dr, si, di;
                 unpack(acc[u][2 * c], sr, dr);
                 unpack(acc[u][2 * c + 1], si, di);
-                out[j * ncomp + c] = make_float4(0.5f * (sr + dr), 0.5f * (si + di), hs * (sr - dr), hs * (si - di));
+                store4(out + 4 * (j * ncomp + c),
+                       make_float4(0.5f * (sr + dr), 0.5f * (si + di), hs * (sr - dr), hs * (si - di)), wide);
             }
         }
     }
@@ -671,7 +685,8 @@ static int launch_rows_ana(int64_t nside, int64_t lmax, int64_t ncomp, const dou
     const int64_t nlanes = 2 * nside;
     const int nw = rows_warps<SPIN, R>(nlanes), per = nw * Rows<SPIN, R>::kLanes, nc = SPIN == 0 ? NC : 2;
     dim3 grid((unsigned)((nlanes + per - 1) / per), (unsigned)(lmax + 1), (unsigned)((ncomp + nc - 1) / nc));
-    k_rows_ana<SPIN, NC, R><<<grid, 32 * nw, 0, s>>>(nside, lmax, ncomp, geom, (const float *)rhs, alm, scale, tab);
+    k_rows_ana<SPIN, NC, R><<<grid, 32 * nw, 0, s>>>(nside, lmax, ncomp, geom, (const float *)rhs,
+                                                        reinterpret_cast<uintptr_t>(rhs) % 16 == 0, alm, scale, tab);
     return check_launch("gm_legendre_analysis_ck");
 }
 
@@ -682,7 +697,8 @@ static int launch_rows_syn(int64_t nside, int64_t lmax, int64_t ncomp, const dou
     const int64_t nlanes = 2 * nside;
     const int nw = rows_warps<SPIN, R>(nlanes), per = nw * Rows<SPIN, R>::kLanes, nc = SPIN == 0 ? NC : 2;
     dim3 grid((unsigned)((nlanes + per - 1) / per), (unsigned)(lmax + 1), (unsigned)((ncomp + nc - 1) / nc));
-    k_rows_syn<SPIN, NC, R><<<grid, 32 * nw, 0, s>>>(nside, lmax, ncomp, geom, alm, (float *)syn, tab);
+    k_rows_syn<SPIN, NC, R><<<grid, 32 * nw, 0, s>>>(nside, lmax, ncomp, geom, alm, (float *)syn,
+                                                        reinterpret_cast<uintptr_t>(syn) % 16 == 0, tab);
     return check_launch("gm_legendre_synthesis_ck");
 }
 

@@ -735,7 +735,8 @@ __global__ void k_prep_syn(int64_t lmax, int spin, int sp, int H, int NR,
 // and n - k read each other's orders, so they are summed together and every synthesis
 // value is read once.  The image of order m = k + t n is then
 //   (-1)^t w n P_k - rhs(m), scaled by `scale`, as f16 hi/lo.
-// A thread takes the two rows (re, im) of one item and hemisphere: 8-byte loads of the synthesis,
+// A thread takes the two rows (re, im) of one item and hemisphere: 8-byte loads of the synthesis
+// (WIDE; two loads where its arrays are aligned to 4 bytes only),
 // one right-hand side for both rows, 4-byte stores of the images, and the conjugation is a sign
 // of the second row.  The residue pairs of a lane are spread over grid.y CTAs, and rings of few
 // residues sum their aliases with several loads in flight.  Rows beyond 2H and the absent south
@@ -744,7 +745,7 @@ __global__ void k_prep_syn(int64_t lmax, int spin, int sp, int H, int NR,
 // lane with a thread per row and 2-byte stores took 2.03 ms for 32 (Q, U) fields at Nside 512 (2.4
 // TB/s) and 0.92 ms for 16 at Nside 256, where 512 CTAs leave the chip half idle; 0.94 and 0.24
 // ms here.
-template <int SPIN>
+template <int SPIN, bool WIDE>
 __global__ void __launch_bounds__(64, SPIN == 0 ? 24 : 16) k_fold_tc(int64_t nside, int64_t L, int ncomp,
                                                 const float *__restrict__ synd_a,
                                                 const float *__restrict__ synd_b, int R2,
@@ -772,7 +773,10 @@ __global__ void __launch_bounds__(64, SPIN == 0 ? 24 : 16) k_fold_tc(int64_t nsi
     uint8_t *ib = SPIN ? img_b + (j / kKC) * 2 * (int64_t)kAImg + roff : nullptr;
     const float4 *rb = rhs_map + j * ncomp;
 
-    auto ld = [&](const float *p, int64_t m) { return *reinterpret_cast<const float2 *>(p + m * stride); };
+    auto ld = [&](const float *p, int64_t m) {
+        const float *q = p + m * stride;
+        return WIDE ? *reinterpret_cast<const float2 *>(q) : make_float2(q[0], q[1]);
+    };
     auto put = [&](uint8_t *img, int64_t m, float x, float y) {
         const __half2 hi = __floats2half2_rn(x, y);
         const float2 h = __half22float2(hi);
@@ -997,6 +1001,9 @@ static bool window_ok(int64_t lmax, int64_t mbeg, int64_t mend)
     return mbeg >= 0 && mbeg < mend && mend <= lmax + 1;
 }
 
+// Analysis images are read by bulk copies (16-byte boundaries) and written two rows at a time.
+static bool image_aligned(const void *img) { return reinterpret_cast<uintptr_t>(img) % 16 == 0; }
+
 extern "C" int gm_tc_pack_window(int64_t nside, int64_t lmax, int spin, int64_t ncomp,
                                  const void *ringspec, void *rhs_map, void *img_a, void *img_b,
                                  double img_scale, int64_t mbeg, int64_t mend, void *stream)
@@ -1004,7 +1011,7 @@ extern "C" int gm_tc_pack_window(int64_t nside, int64_t lmax, int spin, int64_t 
     if (nside < 1 || lmax < 0 || !tc_shape_ok(spin, ncomp) || !(img_scale > 0.0) ||
         !window_ok(lmax, mbeg, mend))
         return GM_ERR_BAD_SHAPE;
-    if (!ringspec || !img_a || (spin && !img_b)) return GM_ERR_BAD_PTR;
+    if (!ringspec || !img_a || (spin && !img_b) || !image_aligned(img_a) || !image_aligned(img_b)) return GM_ERR_BAD_PTR;
     const int64_t NG = gm_tc_lane_groups(nside);
     cudaStream_t s = as_stream(stream);
     // the kernel writes every row of every lane; only the padding lanes of a last, partial
@@ -1170,10 +1177,13 @@ extern "C" int gm_tc_fold(int64_t nside, int64_t lmax, int spin, int64_t ncomp, 
                           void *img_a, void *img_b, double img_scale, void *stream)
 {
     if (nside < 1 || lmax < 2 || !tc_shape_ok(spin, ncomp) || !(img_scale > 0.0)) return GM_ERR_BAD_SHAPE;
-    if (!synd_a || (spin && !synd_b) || !rhs_map || !shifted || !img_a || (spin && !img_b))
+    if (!synd_a || (spin && !synd_b) || !rhs_map || !shifted || !img_a || (spin && !img_b) || !image_aligned(img_a) ||
+        !image_aligned(img_b))
         return GM_ERR_BAD_PTR;
     const int H = spin == 0 ? (int)(2 * ncomp) : (int)ncomp;
-    auto kern = spin == 0 ? k_fold_tc<0> : k_fold_tc<2>;
+    const bool wide = ((reinterpret_cast<uintptr_t>(synd_a) | reinterpret_cast<uintptr_t>(spin ? synd_b : synd_a)) & 7) == 0;
+    auto kern = wide ? (spin == 0 ? k_fold_tc<0, true> : k_fold_tc<2, true>)
+                     : (spin == 0 ? k_fold_tc<0, false> : k_fold_tc<2, false>);
     // residue pairs over enough CTAs for two rounds of a full chip (24 of 64 threads per SM)
     const int64_t want = 2 * 148 * 24, split = (want + 2 * nside - 1) / (2 * nside);
     const dim3 grid((unsigned)(2 * nside), (unsigned)(split < 16 ? split : 16));

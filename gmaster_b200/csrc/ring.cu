@@ -554,8 +554,9 @@ __device__ __forceinline__ void residue_sums(const T *__restrict__ syn, int64_t 
     ps[1] = si;
 }
 
-// Both hemispheres' coefficients of one order: (north re, im, south re, im).
-template <typename T> struct alignas(16) Quad {
+// Both hemispheres' coefficients of one order: (north re, im, south re, im), of 16-byte aligned
+// arrays or (not WIDE) of arrays aligned to their elements only.
+template <typename T, bool WIDE> struct alignas(WIDE ? 16 : sizeof(T)) Quad {
     T x, y, z, w;
 };
 
@@ -575,16 +576,17 @@ template <typename T> struct alignas(16) Quad {
 // one map (1.2 GB: 2.7 TB/s), 370 -> 78 us at Nside 512 with a (Q, U) pair.
 __host__ __device__ constexpr int fold_threads(int J) { return J == 8 ? 512 : 256; }
 
-template <typename T, int J, bool RESIDUAL>
+template <typename T, int J, bool RESIDUAL, bool WIDE>
 __global__ void __launch_bounds__(fold_threads(J)) k_fold_lanes(int64_t nside, int64_t L, int64_t ncomp, int64_t cbeg, int64_t cw,
-                                                    const Quad<T> *__restrict__ syn,
-                                                    const Quad<T> *__restrict__ rhs_map,
-                                                    const uint8_t *__restrict__ shifted, Quad<T> *__restrict__ out,
+                                                    const Quad<T, WIDE> *__restrict__ syn,
+                                                    const Quad<T, WIDE> *__restrict__ rhs_map,
+                                                    const uint8_t *__restrict__ shifted, Quad<T, WIDE> *__restrict__ out,
                                                     typename vec2<T>::type *__restrict__ spec, int64_t sstride)
 {
     using T2 = typename vec2<T>::type;
+    using Q4 = Quad<T, WIDE>;
     constexpr int NT = fold_threads(J), Q = NT / J;
-    __shared__ Quad<T> pa[NT], pb[NT];
+    __shared__ Q4 pa[NT], pb[NT];
     const int64_t nlanes = 2 * nside, stride = nlanes * ncomp;
     const int q = threadIdx.x / J;
     const int64_t item = (int64_t)blockIdx.x * J + threadIdx.x % J;
@@ -595,19 +597,19 @@ __global__ void __launch_bounds__(fold_threads(J)) k_fold_lanes(int64_t nside, i
     const bool sh = shifted[north_ring(j)] != 0, two = j != nlanes - 1;
     const T sigma = sh ? (T)-1 : (T)1;
     const T wn = (T)(4.0 * M_PI / (double)(12 * nside * nside) * (double)n);
-    const Quad<T> *src = syn + col;
+    const Q4 *src = syn + col;
     int s = 1;
     while (2 * s * np <= Q) s *= 2;
     const int part = q & (s - 1);
 
     // aliases k + t n, t = t0, t0 + s, ...
     auto sum = [&](int k, int t0) {
-        Quad<T> a{0, 0, 0, 0};
+        Q4 a{0, 0, 0, 0};
         const int64_t dm = (int64_t)s * n;
         int t = t0;
 #pragma unroll 4
         for (int64_t m = k + (int64_t)t0 * n; m < L; m += dm, t += s) {
-            const Quad<T> v = src[m * stride];
+            const Q4 v = src[m * stride];
             const T sg = (sh && (t & 1)) ? (T)-1 : (T)1;
             a.x += sg * v.x;
             a.y += sg * v.y;
@@ -616,12 +618,12 @@ __global__ void __launch_bounds__(fold_threads(J)) k_fold_lanes(int64_t nside, i
         }
         return a;
     };
-    auto pair_sums = [&](int p, Quad<T> &A, Quad<T> &B) {
+    auto pair_sums = [&](int p, Q4 &A, Q4 &B) {
         // residue 0 leaves order 0 to the caller
         A = sum(p, p == 0 && part == 0 ? s : part);
-        B = (p > 0 && 2 * p < n) ? sum(n - p, part) : Quad<T>{0, 0, 0, 0};
+        B = (p > 0 && 2 * p < n) ? sum(n - p, part) : Q4{0, 0, 0, 0};
     };
-    auto emit = [&](int k, const Quad<T> &P) {
+    auto emit = [&](int k, const Q4 &P) {
         if (RESIDUAL) {
             const int64_t dm = (int64_t)s * n;
             int t = part;
@@ -630,8 +632,8 @@ __global__ void __launch_bounds__(fold_threads(J)) k_fold_lanes(int64_t nside, i
                 const T f = (sh && (t & 1)) ? -wn : wn;
                 const T nr = f * P.x, ni = f * P.y, sr = two ? f * P.z : (T)0, si = two ? f * P.w : (T)0;
                 const int64_t idx = m * stride + col;
-                const Quad<T> b = rhs_map[idx];
-                out[idx] = Quad<T>{nr + sr - b.x, ni + si - b.y, nr - sr - b.z, ni - si - b.w};
+                const Q4 b = rhs_map[idx];
+                out[idx] = Q4{nr + sr - b.x, ni + si - b.y, nr - sr - b.z, ni - si - b.w};
             }
         } else if (part == 0 && 2 * k <= n) {
             const int64_t base = (c - cbeg) * (4 * nside - 1);
@@ -639,22 +641,22 @@ __global__ void __launch_bounds__(fold_threads(J)) k_fold_lanes(int64_t nside, i
             if (two) spec[(base + south_ring(nside, j)) * sstride + k] = make2<T2, T>(P.z, P.w);
         }
     };
-    auto finish = [&](int p, const Quad<T> &A, const Quad<T> &B) {
+    auto finish = [&](int p, const Q4 &A, const Q4 &B) {
         if (p == 0) {
-            const Quad<T> z = src[0];
-            emit(0, Quad<T>{z.x + 2 * A.x, z.y, z.z + 2 * A.z, z.w});
+            const Q4 z = src[0];
+            emit(0, Q4{z.x + 2 * A.x, z.y, z.z + 2 * A.z, z.w});
         } else if (2 * p == n) {
-            emit(p, Quad<T>{A.x + sigma * A.x, A.y - sigma * A.y, A.z + sigma * A.z, A.w - sigma * A.w});
+            emit(p, Q4{A.x + sigma * A.x, A.y - sigma * A.y, A.z + sigma * A.z, A.w - sigma * A.w});
         } else {
-            emit(p, Quad<T>{A.x + sigma * B.x, A.y - sigma * B.y, A.z + sigma * B.z, A.w - sigma * B.w});
+            emit(p, Q4{A.x + sigma * B.x, A.y - sigma * B.y, A.z + sigma * B.z, A.w - sigma * B.w});
             if (RESIDUAL)
-                emit(n - p, Quad<T>{B.x + sigma * A.x, B.y - sigma * A.y, B.z + sigma * A.z, B.w - sigma * A.w});
+                emit(n - p, Q4{B.x + sigma * A.x, B.y - sigma * A.y, B.z + sigma * A.z, B.w - sigma * A.w});
         }
     };
 
     const int p0 = q / s;
     if (s > 1 && ok && p0 < np) {
-        Quad<T> A, B;
+        Q4 A, B;
         pair_sums(p0, A, B);
         pa[threadIdx.x] = A;
         pb[threadIdx.x] = B;
@@ -663,17 +665,17 @@ __global__ void __launch_bounds__(fold_threads(J)) k_fold_lanes(int64_t nside, i
     if (!ok) return;
     if (s > 1) {
         if (p0 >= np) return;
-        Quad<T> A{0, 0, 0, 0}, B{0, 0, 0, 0};
+        Q4 A{0, 0, 0, 0}, B{0, 0, 0, 0};
         for (int u = 0; u < s; ++u) {
             const int e = (p0 * s + u) * J + (int)(threadIdx.x % J);
-            const Quad<T> a = pa[e], b = pb[e];
+            const Q4 a = pa[e], b = pb[e];
             A.x += a.x; A.y += a.y; A.z += a.z; A.w += a.w;
             B.x += b.x; B.y += b.y; B.z += b.z; B.w += b.w;
         }
         finish(p0, A, B);
     } else {
         for (int p = p0; p < np; p += Q) {
-            Quad<T> A, B;
+            Q4 A, B;
             pair_sums(p, A, B);
             finish(p, A, B);
         }
@@ -1150,7 +1152,7 @@ extern "C" int gm_pack_rhs(int precision, int64_t nside, int64_t L, int64_t ncom
 
 // Columns per CTA: eight (a full 128-byte line a row in single precision) where that leaves two
 // CTAs per SM, else two.
-template <typename T, bool RESIDUAL>
+template <typename T, bool RESIDUAL, bool WIDE = true>
 static void fold_lanes(int64_t nside, int64_t L, int64_t ncomp, int64_t cbeg, int64_t cw, const void *syn,
                        const void *rhs_map, const uint8_t *shifted, void *out, void *spec, int64_t sstride,
                        cudaStream_t s)
@@ -1158,12 +1160,12 @@ static void fold_lanes(int64_t nside, int64_t L, int64_t ncomp, int64_t cbeg, in
     using T2 = typename vec2<T>::type;
     const int64_t items = 2 * nside * cw;
     auto run = [&](auto kernel, int J) {
-        kernel<<<(unsigned)((items + J - 1) / J), fold_threads(J), 0, s>>>(nside, L, ncomp, cbeg, cw, (const Quad<T> *)syn,
-                                                               (const Quad<T> *)rhs_map, shifted, (Quad<T> *)out,
-                                                               (T2 *)spec, sstride);
+        kernel<<<(unsigned)((items + J - 1) / J), fold_threads(J), 0, s>>>(
+            nside, L, ncomp, cbeg, cw, (const Quad<T, WIDE> *)syn, (const Quad<T, WIDE> *)rhs_map, shifted,
+            (Quad<T, WIDE> *)out, (T2 *)spec, sstride);
     };
-    if (items >= 8 * 296) run(k_fold_lanes<T, 8, RESIDUAL>, 8);
-    else run(k_fold_lanes<T, 2, RESIDUAL>, 2);
+    if (items >= 8 * 296) run(k_fold_lanes<T, 8, RESIDUAL, WIDE>, 8);
+    else run(k_fold_lanes<T, 2, RESIDUAL, WIDE>, 2);
 }
 
 extern "C" int gm_fold_residual(int precision, int64_t nside, int64_t L, int64_t ncomp,
@@ -1173,12 +1175,12 @@ extern "C" int gm_fold_residual(int precision, int64_t nside, int64_t L, int64_t
     if (nside < 1 || L < 1 || ncomp < 1 || ncomp > 65535) return GM_ERR_BAD_SHAPE;
     if (!syn || !rhs_map || !shifted || !rhs_out) return GM_ERR_BAD_PTR;
     cudaStream_t s = as_stream(stream);
-    if (precision == GM_FP64)
-        fold_lanes<double, true>(nside, L, ncomp, 0, ncomp, syn, rhs_map, shifted, rhs_out, nullptr, 0, s);
-    else if (precision == GM_MIXED)
-        fold_lanes<float, true>(nside, L, ncomp, 0, ncomp, syn, rhs_map, shifted, rhs_out, nullptr, 0, s);
-    else
-        return GM_ERR_UNSUPPORTED;
+    const bool wide = ((reinterpret_cast<uintptr_t>(syn) | reinterpret_cast<uintptr_t>(rhs_map) |
+                        reinterpret_cast<uintptr_t>(rhs_out)) & 15) == 0;
+    auto run = [&](auto fold) { fold(nside, L, ncomp, 0, ncomp, syn, rhs_map, shifted, rhs_out, nullptr, 0, s); };
+    if (precision == GM_FP64) run(wide ? fold_lanes<double, true, true> : fold_lanes<double, true, false>);
+    else if (precision == GM_MIXED) run(wide ? fold_lanes<float, true, true> : fold_lanes<float, true, false>);
+    else return GM_ERR_UNSUPPORTED;
     return check_launch("gm_fold_residual");
 }
 

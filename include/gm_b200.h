@@ -303,7 +303,7 @@ int64_t gm_tc_syn_image_bytes(int64_t nchunks);
 int gm_tc_coef_table(int64_t lmax, int spin, double *tab, void *stream);
 /* Ring spectra (ncomp, nring, L) complex64 -> rhs_map (L, nlanes, ncomp) float4
  * [G_N re, im, G_S re, im] and the analysis images scaled by img_scale (img_b only for
- * spin 2). */
+ * spin 2).  Images are 16-byte aligned, here and in gm_tc_fold (GM_ERR_BAD_PTR otherwise). */
 int gm_tc_pack(int64_t nside, int64_t lmax, int spin, int64_t ncomp, const void *ringspec,
                void *rhs_map, void *img_a, void *img_b, double img_scale, void *stream);
 /* alm_i += scale * analysis of the rows of `img` for row variant sp (0, -2, +2).
