@@ -22,6 +22,20 @@ inline int check_launch(const char *where)
     return GM_OK;
 }
 
+// Lets launches of `kernel` ask for up to `limit` bytes of dynamic shared memory.  The limit
+// belongs to the kernel, not to a launch: `limit` is the most that any launch takes, the same in
+// every call, so that a host thread never lowers it between another's call and its launch.
+template <typename K>
+inline int allow_smem(K kernel, int limit, const char *where)
+{
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+    if (err != cudaSuccess) {
+        set_error(where, err);
+        return GM_ERR_LAUNCH;
+    }
+    return GM_OK;
+}
+
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 
 template <typename T> struct vec2;

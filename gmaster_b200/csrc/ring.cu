@@ -1000,17 +1000,8 @@ static int ring_shape_ok(int precision, int64_t nside, int64_t L, int64_t ncomp)
     return 1;
 }
 
-template <typename K>
-static int set_smem(K kernel, size_t bytes)
-{
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)bytes);
-    if (e != cudaSuccess) {
-        set_error("cudaFuncSetAttribute", e);
-        return GM_ERR_LAUNCH;
-    }
-    return GM_OK;
-}
+// Most dynamic shared memory of the ring kernels: 227 KB less their static arrays.
+constexpr int kRingSmem = 227 * 1024 - 336;
 
 // Shared memory of the ring kernels: ping-pong buffers of hcap complex values.
 static int ring_hcap(int precision, int64_t nside, bool big)
@@ -1073,7 +1064,7 @@ static int ring_analysis(int64_t nside, int64_t L, int64_t ncomp, const void *ma
     const bool vec = reinterpret_cast<uintptr_t>(maps) % (2 * sizeof(Tin)) == 0 && reinterpret_cast<uintptr_t>(mask) % 16 == 0;
     int st = for_ring_classes<T>(nside, ncomp, hcap, big, [&](int64_t i0, int64_t cnt, int buf, int nbuf, int threads, int mcap, int64_t rows) {
         const size_t bytes = (size_t)nbuf * buf * sizeof(T2);
-        const int e = set_smem(k_ring_forward<T, Tin>, bytes);
+        const int e = allow_smem(k_ring_forward<T, Tin>, kRingSmem, "gm_ring_analysis attr");
         if (e) return e;
         const int cpc = nbuf == 3 ? 8 : 1;   // components that share the transform of the chirp
         dim3 grid((unsigned)((ncomp + cpc - 1) / cpc), (unsigned)rows);
@@ -1207,14 +1198,14 @@ extern "C" int gm_ring_synthesis_ws(int precision, int64_t nside, int64_t L, int
     cudaStream_t s = as_stream(stream);
     int st;
     if (precision == GM_FP64) {
-        if ((st = set_smem(k_ring_synthesis<double>, smem))) return st;
+        if ((st = allow_smem(k_ring_synthesis<double>, kRingSmem, "gm_ring_synthesis attr"))) return st;
         k_ring_synthesis<double><<<grid, threads, smem, s>>>(nside, L, ncomp, (const double *)syn,
                                                              tw, cnt, shifted, maps, hcap, 0);
         if (big)
             k_ring_synthesis_big<double><<<gbig, 512, 0, s>>>(nside, L, ncomp, (const double *)syn, tw, cnt,
                                                               shifted, maps, hcap, 0, scratch, slot);
     } else if (precision == GM_MIXED) {
-        if ((st = set_smem(k_ring_synthesis<float>, smem))) return st;
+        if ((st = allow_smem(k_ring_synthesis<float>, kRingSmem, "gm_ring_synthesis attr"))) return st;
         k_ring_synthesis<float><<<grid, threads, smem, s>>>(nside, L, ncomp, (const float *)syn,
                                                             tw, cnt, shifted, maps, hcap, bsmin);
         if (big)
@@ -1254,7 +1245,7 @@ static int ring_synthesis_fold(int64_t nside, int64_t L, int64_t ncomp, const vo
         if (st) return st;
         st = for_ring_classes<T>(nside, cw, hcap, big, [&](int64_t i0, int64_t n, int buf, int nbuf, int threads, int mcap, int64_t rows) {
             const size_t bytes = (size_t)nbuf * buf * sizeof(T2);
-            const int e = set_smem(k_ring_inverse<T>, bytes);
+            const int e = allow_smem(k_ring_inverse<T>, kRingSmem, "gm_ring_synthesis_fold attr");
             if (e) return e;
             const int cpc = nbuf == 3 ? 8 : 1;
             dim3 grid((unsigned)((cw + cpc - 1) / cpc), (unsigned)rows);

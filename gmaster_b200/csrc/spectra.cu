@@ -1273,11 +1273,14 @@ extern "C" int gm_bin_cells_csr(int64_t lmax, int64_t nbands, int64_t ncls, cons
     return check_launch("gm_bin_cells");
 }
 
+// Shared memory of a panel or of the right-hand sides of a CTA.
+constexpr int kLuSmem = 200 * 1024;
+
 // Panel width of the shared-memory panels: the widest of 32, 16, 8, 4 columns that fit (the
 // whole matrix up to n = 160), 0 when none does.
 static int lu_panel_width(int64_t n)
 {
-    const int64_t fit = 200 * 1024 / (8 * (n | 1));
+    const int64_t fit = kLuSmem / (8 * (n | 1));
     if (fit >= n) return (int)n;
     for (int kb = kLuPan; kb >= 4; kb /= 2)
         if (fit >= kb) return kb;
@@ -1306,11 +1309,8 @@ extern "C" int gm_lu_factor(int64_t n, double *a, int32_t *piv, int32_t *status,
         return GM_OK;
     }
     const size_t smem = (size_t)w * (n | 1) * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(k_lu_panel_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) {
-        set_error("gm_lu_factor attr", e);
-        return GM_ERR_LAUNCH;
-    }
+    const int sa = allow_smem(k_lu_panel_smem, kLuSmem, "gm_lu_factor attr");
+    if (sa != GM_OK) return sa;
     for (int64_t k0 = 0; k0 < n;) {
         const int64_t rows = n - k0;
         // rows in registers: 32 columns of up to 640 rows, 16 of up to 1024; else the widest panel
@@ -1369,14 +1369,10 @@ extern "C" int gm_lu_solve(int64_t n, const double *lu, const int32_t *piv, int6
     if (n < 1 || nrhs < 1) return GM_ERR_BAD_SHAPE;
     if (!lu || !piv || !b) return GM_ERR_BAD_PTR;
     const size_t smem = (size_t)n * kLuCB * sizeof(double);
-    if (smem <= 200 * 1024) {
+    if (smem <= kLuSmem) {
         // the columns of b fit in shared memory: the blocked solve
-        cudaError_t e = cudaFuncSetAttribute(k_lu_solve_blk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) {
-            set_error("gm_lu_solve attr", e);
-            return GM_ERR_LAUNCH;
-        }
+        const int sa = allow_smem(k_lu_solve_blk, kLuSmem, "gm_lu_solve attr");
+        if (sa != GM_OK) return sa;
         k_lu_solve_blk<<<(unsigned)((nrhs + kLuCB - 1) / kLuCB), 256, smem, as_stream(stream)>>>(n, lu, piv,
                                                                                                 nrhs, b);
         return check_launch("gm_lu_solve");
@@ -1395,7 +1391,7 @@ extern "C" int64_t gm_lu_prepared_bytes(int64_t n)
 }
 
 // The columns of b in shared memory: 4 per CTA up to this many rows.
-constexpr int64_t kLuPreparedMax = 200 * 1024 / (4 * 8);
+constexpr int64_t kLuPreparedMax = kLuSmem / (4 * 8);
 
 extern "C" int gm_lu_prepare(int64_t n, const double *lu, const int32_t *piv, void *work, void *stream)
 {
@@ -1405,11 +1401,8 @@ extern "C" int gm_lu_prepare(int64_t n, const double *lu, const int32_t *piv, vo
     double *inv = (double *)work;
     int32_t *perm = (int32_t *)(inv + nblk * 2 * kLuSB * kLuSB);
     const size_t smem = 2 * (size_t)n * sizeof(int32_t);
-    cudaError_t e = cudaFuncSetAttribute(k_lu_prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) {
-        set_error("gm_lu_prepare attr", e);
-        return GM_ERR_LAUNCH;
-    }
+    const int sa = allow_smem(k_lu_prepare, 2 * (int)kLuPreparedMax * (int)sizeof(int32_t), "gm_lu_prepare attr");
+    if (sa != GM_OK) return sa;
     k_lu_prepare<<<(unsigned)(1 + nblk), 64, smem, as_stream(stream)>>>((int)n, lu, piv, perm, inv);
     return check_launch("gm_lu_prepare");
 }
@@ -1427,11 +1420,8 @@ extern "C" int gm_lu_solve_prepared(int64_t n, const double *lu, const void *wor
     auto kern = wide ? k_lu_solve_prepared<4> : k_lu_solve_prepared<1>;
     const int cb = wide ? 4 : 1;
     const size_t smem = (size_t)nblk * kLuSB * cb * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) {
-        set_error("gm_lu_solve_prepared attr", e);
-        return GM_ERR_LAUNCH;
-    }
+    const int sa = allow_smem(kern, kLuSmem, "gm_lu_solve_prepared attr");
+    if (sa != GM_OK) return sa;
     kern<<<(unsigned)((nrhs + cb - 1) / cb), 1024, smem, as_stream(stream)>>>((int)n, lu, perm, inv, nrhs, b, x);
     return check_launch("gm_lu_solve_prepared");
 }
@@ -1456,11 +1446,8 @@ extern "C" int gm_decouple_cells(int64_t nbands, int64_t ncls, int64_t ncells, c
     auto kern = wide ? k_decouple<4> : k_decouple<1>;
     const int cb = wide ? 4 : 1;
     const size_t smem = (size_t)nblk * kLuSB * cb * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) {
-        set_error("gm_decouple_cells attr", e);
-        return GM_ERR_LAUNCH;
-    }
+    const int sa = allow_smem(kern, kLuSmem, "gm_decouple_cells attr");
+    if (sa != GM_OK) return sa;
     kern<<<(unsigned)((ncells + cb - 1) / cb), 1024, smem, as_stream(stream)>>>(
         (int)n, (int)ncls, ld, c, band_ptr, band_ells, wfl, lu, perm, inv, ncells, x);
     return check_launch("gm_decouple_cells");
