@@ -83,12 +83,9 @@ def fields_from_maps(mask, maps, *, spin=None, n_iter=None, beam=None, lmax=None
                                               n_iter, "fp64") for i in range(chunk.shape[0])])
         else:
             # the ring stage multiplies by the mask as it reads the maps: no masked copy
-            spec = None
-            if ring_spectra and s0 == 0 and nsims <= per_launch:
-                spec = ring_spectra.pop()
             a = sht_tc.map2alm_tc(flat, spin, nside, lm, n_iter,
-                                  mask=None if masked_on_input else mask_t, ring_spectra=spec)
-            del spec
+                                  mask=None if masked_on_input else mask_t,
+                                  ring_spectra=ring_spectra if ring_spectra and nsims <= per_launch else None)
         del flat, chunk
         alms.append(a.reshape(-1, nmaps, a.shape[1]))
     # one launch's alms are used as they are (a concatenation would hold a second copy)

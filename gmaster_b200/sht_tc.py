@@ -294,10 +294,10 @@ def window_orders(tp, spin, ncomp, budget=None):
     return int(max(1, min(tp.plan.L, budget // per)))
 
 
-def _full_path_bytes(tp, spin, ncomp, n_iter):
+def _full_path_bytes(tp, spin, ncomp, n_iter, held=False):
     """Peak device bytes of the single-window map2alm: the ring spectra, right-hand sides
-    and images while packing; then (spectra released) the right-hand sides, images, alm
-    accumulator and synthesis buffers."""
+    and images while packing; then (spectra released, unless `held` by the caller) the
+    right-hand sides, images, alm accumulator and synthesis buffers."""
     p = tp.plan
     H, NR = _rows(spin, ncomp)
     nv = len(_variants(spin))
@@ -306,7 +306,7 @@ def _full_path_bytes(tp, spin, ncomp, n_iter):
     later = base + p.nelem * NR * 8
     if n_iter > 0:
         later += nv * p.L * p.nlanes * 2 * H * 4 + tp.nchunks[spin] * _lib.load().gm_tc_syn_image_bytes(1)
-    return max(spec + base, later)
+    return max(spec + base, later + (spec if held else 0))
 
 
 def _fits(need, share, device):
@@ -333,19 +333,24 @@ def map2alm_tc(maps, spin, nside, lmax, n_iter, mask=None, window=None, ring_spe
     the free device memory (or `window`, a number of orders, is given) the transform runs
     over windows of orders instead (`map2alm_tc_windowed`).  `ring_spectra`, if given, are
     the single-precision ring spectra of the (masked) maps, already computed (a caller
-    that streams the maps in can transform each part as it arrives)."""
+    that streams the maps in can transform each part as it arrives): a tensor, which the
+    caller keeps, or a one-element list that holds it and is emptied, so that the spectra are
+    released once they are packed."""
     ncomp = maps.shape[0]
     _check_batch(spin, ncomp)
     tp = get_tc_plan(nside, lmax, maps.device)
     p = tp.plan
-    if window is None and not _fits(_full_path_bytes(tp, spin, ncomp, n_iter), 0.95, p.device):
+    box = (ring_spectra or [None]) if isinstance(ring_spectra, list) else [ring_spectra]
+    held = isinstance(ring_spectra, torch.Tensor)
+    if window is None and not _fits(_full_path_bytes(tp, spin, ncomp, n_iter, held), 0.95, p.device):
         window = window_orders(tp, spin, ncomp)
     if window is not None:
+        box.clear()
         return map2alm_tc_windowed(maps, spin, nside, lmax, n_iter, mask=mask, window=window)
-    if ring_spectra is not None and ring_spectra.shape != (ncomp, p.nring, p.L):
+    if box[0] is not None and box[0].shape != (ncomp, p.nring, p.L):
         raise ValueError("ring_spectra must be (ncomp, nring, L)")
     try:
-        return _map2alm_full(tp, maps, spin, n_iter, mask, [ring_spectra])
+        return _map2alm_full(tp, maps, spin, n_iter, mask, box)
     except torch.cuda.OutOfMemoryError:
         window = window_orders(tp, spin, ncomp)
     return map2alm_tc_windowed(maps, spin, nside, lmax, n_iter, mask=mask, window=window)
@@ -353,12 +358,12 @@ def map2alm_tc(maps, spin, nside, lmax, n_iter, mask=None, window=None, ring_spe
 
 def _map2alm_full(tp, maps, spin, n_iter, mask, spectra):
     """map2alm_tc with all orders at once; `spectra` is a one-element list (the ring spectra or
-    None) that is emptied, so that they are released after packing unless the caller holds them."""
+    None) that is emptied, so that they are released after packing unless a caller holds them."""
     p = tp.plan
     ncomp = maps.shape[0]
-    ring_spectra = spectra.pop()
-    spec = ring_spectra if ring_spectra is not None else sht.ring_analysis(p, maps, _lib.MIXED, mask=mask)
-    ring_spectra = None   # the spectra are released after packing unless the caller holds them
+    spec = spectra.pop()
+    if spec is None:
+        spec = sht.ring_analysis(p, maps, _lib.MIXED, mask=mask)
     b = _Batch(tp, spin, ncomp)
     # the spin-2 rows G_Q -+ i G_U are at most twice the largest ring value
     b.img_scale = pow2_scale(spec.view(torch.float32)) / (2.0 if spin else 1.0)
