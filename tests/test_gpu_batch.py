@@ -105,6 +105,27 @@ def test_batch_shape_errors(cuda):
         nmt.fields_from_maps(mask, np.zeros((2, 2, 12 * 64)), spin=0)
 
 
+def test_fields_of_a_batch_share_only_the_mask(cuda):
+    """Changing the beam, the alms or the geometry of one field in place leaves the others."""
+    nside = 16
+    maps = np.random.default_rng(3).normal(size=(3, 12 * nside ** 2))
+    beam = np.linspace(1.0, 0.5, 3 * nside)
+    mask = torch.from_numpy(_mask(nside)).cuda()
+    fields = nmt.fields_from_maps(mask, maps, n_iter=0, beam=beam, precision="mixed")
+    keep = fields[1].alm.clone()
+    fields[0].beam.zero_()
+    fields[0].alm.zero_()
+    fields[0].ainfo.lmax = 3
+    fields[0].ainfo_mask.mstart[:] = 0
+    fields[0].minfo.nside = 1
+    for f in fields[1:]:
+        np.testing.assert_array_equal(f.beam.cpu().numpy(), beam)
+        assert f.ainfo.lmax == 3 * nside - 1 and f.minfo.nside == nside
+        assert f.ainfo_mask.mstart[-1] > 0
+        assert f.mask is fields[0].mask
+    assert torch.equal(fields[1].alm, keep)
+
+
 def test_mc_bandpowers_equals_step_by_step_api(cuda):
     """mc_bandpowers on device maps and on pinned host maps (copied on a side stream)
     gives the results of fields_from_maps / compute_coupled_cells / decouple_cells (to the
