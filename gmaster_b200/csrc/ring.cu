@@ -249,9 +249,12 @@ __host__ __device__ __forceinline__ int next_pow2(int x)
     return m;
 }
 
+// Largest prime factor transformed by a direct stage.
+constexpr int kDirectPrime = 64;
+
 __host__ __device__ __forceinline__ bool use_bluestein(int h, int mcap)
 {
-    return largest_prime_factor(h) > 64 && next_pow2(2 * h - 1) <= mcap;
+    return largest_prime_factor(h) > kDirectPrime && next_pow2(2 * h - 1) <= mcap;
 }
 
 // Largest power-of-two FFT length of the Bluestein path: its table must exist (a ring
@@ -413,12 +416,13 @@ __device__ __forceinline__ void ring_outputs(const T2 *__restrict__ Z, int n, in
     }
 }
 
-// Rings of a launch (forward and inverse): i0 > 0, the cap rings of length 4 i, i0 <= i < i0 + cnt, of
-// both hemispheres; i0 = 0, the belt.  A launch covers rings of one shared-memory size, so
-// that short rings run many CTAs per SM.
+// Ring of row b of a launch (forward and inverse): the cap rings of length 4 i, i0 <= i < i0 + cnt,
+// longest first (the north and the south one), then the belt.
 __device__ __forceinline__ int64_t launch_ring(int64_t nside, int64_t i0, int64_t cnt, int64_t b)
 {
-    return i0 == 0 ? nside - 1 + b : (b < cnt ? i0 - 1 + b : 4 * nside - 1 - (i0 + b - cnt));
+    if (b >= 2 * cnt) return nside - 1 + b - 2 * cnt;
+    const int64_t i = i0 + cnt - 1 - (b >> 1);
+    return b & 1 ? 4 * nside - 1 - i : i - 1;
 }
 
 // Forward ring transform: one CTA per (ring, block of cpc components), the component block the
@@ -427,7 +431,7 @@ __device__ __forceinline__ int64_t launch_ring(int64_t nside, int64_t i0, int64_
 // three buffers of M; the transform of the chirp once per CTA), the others through the
 // mixed-radix FFT.  Bound by the passes over shared memory (one per radix) and their barriers:
 // an eighth of the points as threads, two radix-4 butterflies each, fills an SM with CTAs.
-template <typename T, typename Tin>
+template <typename T, typename Tin, bool BS>
 __global__ void __launch_bounds__(512) k_ring_forward(int64_t nside, int64_t L, int64_t ncomp, int cpc,
                                                       const Tin *__restrict__ maps,
                                                       const double *__restrict__ mask, bool vec,
@@ -440,7 +444,7 @@ __global__ void __launch_bounds__(512) k_ring_forward(int64_t nside, int64_t L, 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int64_t r = launch_ring(nside, i0, cnt, blockIdx.y), nring = 4 * nside - 1, npix = 12 * nside * nside;
     const int n = (int)ring_nphi(nside, r), h = n / 2;
-    const bool bs = mcap > 0 && use_bluestein(h, mcap);
+    const bool bs = BS && use_bluestein(h, mcap);
     if (hcap > 0 && ring_big(h, hcap, (int)nside, bsmin)) return;   // left to k_ring_analysis_big
     const int64_t off = ring_offset(nside, r);
     const bool sh = shifted[r] != 0;
@@ -750,7 +754,7 @@ __global__ void __launch_bounds__(512) k_ring_synthesis(int64_t nside, int64_t L
 // With the fold before it: 2235 -> 790 us for a (Q, U) pair at Nside 1024 (a ring per CTA reading
 // its coefficients 128 lanes apart and taking prime factors up to 1021 as one radix), 163 -> 61
 // us for one FP64 map at Nside 256.
-template <typename T>
+template <typename T, bool BS>
 __global__ void __launch_bounds__(512) k_ring_inverse(int64_t nside, int64_t ncomp, int cpc, int64_t sstride,
                                                       const typename vec2<T>::type *__restrict__ spec,
                                                       const void *__restrict__ twall, int64_t twcnt,
@@ -763,7 +767,7 @@ __global__ void __launch_bounds__(512) k_ring_inverse(int64_t nside, int64_t nco
     const int64_t nring = 4 * nside - 1, npix = 12 * nside * nside;
     const int64_t r = launch_ring(nside, i0, cnt, blockIdx.y);
     const int n = (int)ring_nphi(nside, r), h = n / 2;
-    const bool bs = mcap > 0 && use_bluestein(h, mcap);
+    const bool bs = BS && use_bluestein(h, mcap);
     if (hcap > 0 && ring_big(h, hcap, (int)nside, bsmin)) return;   // left to k_ring_synthesis_big
     const int64_t off = ring_offset(nside, r);
     const bool sh = shifted[r] != 0;
@@ -1024,32 +1028,58 @@ static bool any_ring_big(int64_t nside, int hcap, int bsmin)
     return 2 * nside > hcap || (bsmin > 0 && next_pow2((int)(4 * nside - 1)) > bsmin);
 }
 
-// The launches of the ring kernels: the belt (length 4 nside), then the caps by powers of two of
-// their length.  run(i0, cnt, buf, buffers, threads, mcap, rows): buf complex values in each of 2
-// buffers (3 with Bluestein rings, whose M fits buf).  Threads: an eighth of the points where the
-// rings of all components fill the chip many times over (64 maps at Nside 512: 5.5 -> 4.0 ms),
-// else two to four times as many, for the latency of a ring (one FP64 map at Nside 256: 66 us
-// with an eighth, 53 us).
+// The launches of the ring kernels: the belt (length 4 nside) and the caps by powers of two of their
+// length; all rings up to Nside 128 in one.  run(i0, cnt, rows, buf, buffers, threads, cpc, mcap):
+// cap rings i0 .. i0 + cnt - 1 of both hemispheres, then the belt where rows says so; buf complex
+// values in each of 2 buffers (3 with Bluestein rings, whose M fits buf).  The longest caps, where
+// none takes Bluestein, share the belt's launch: longest first, the belt fills up behind their
+// direct sums over primes (one FP64 map at Nside 2048: 8.6 -> 6.8 ms).  Threads: an eighth of the
+// points where the rings of all components fill the chip many times over (64 maps at Nside 512:
+// 5.5 -> 4.0 ms), else two to four times as many, for the latency of a ring (one FP64 map at Nside
+// 256: 66 us with an eighth, 53 us).  cpc components of a CTA share the transform of the chirp
+// where that leaves two rounds of CTAs (eight everywhere: 16 maps at Nside 64 78 us, 21 here).
 template <typename T, typename Run>
 static int for_ring_classes(int64_t nside, int64_t ncomp, int hcap, bool big, Run run)
 {
     int mcap = bluestein_mcap(nside);
     if (sizeof(T) == 8 && mcap > 4096) mcap = 4096;   // three buffers of M in 227 KB
-    auto one = [&](int64_t i0, int64_t cnt, int hmax, int M) {
+    auto one = [&](int64_t i0, int64_t cnt, bool belt, int hmax, int M) {
         if (big && hmax > hcap) hmax = hcap;          // longer rings go to the *_big kernels
         const int buf = M > hmax ? M : hmax;
-        const int64_t rows = i0 ? 2 * cnt : 2 * nside + 1;
+        const int64_t rows = 2 * cnt + (belt ? 2 * nside + 1 : 0);
         int threads = rows * ncomp >= 148 * 64 ? buf / 8 : (M ? buf / 4 : buf / 2);
         threads = threads >= 512 ? 512 : (threads >= 256 ? 256 : (threads >= 128 ? 128 : 64));
-        return run(i0, cnt, buf, M ? 3 : 2, threads, M ? mcap : 0, rows);
+        int cpc = 1;
+        if (M) {
+            const int64_t room = kRingSmem / (3 * (int64_t)buf * 2 * sizeof(T)), cap = 2048 / threads;
+            const int64_t fill = rows * ncomp / (2 * 148 * (room < cap ? room : cap));
+            cpc = fill < 1 ? 1 : (fill < 8 ? (int)fill : 8);
+        }
+        return run(i0, cnt, rows, buf, M ? 3 : 2, threads, cpc, M ? mcap : 0);
     };
-    const int hb = (int)(2 * nside);
-    int st = one(0, 0, hb, use_bluestein(hb, mcap) ? next_pow2(2 * hb - 1) : 0);
-    for (int64_t lo = 1, hi = 128; st == GM_OK && lo < nside; lo = hi + 1, hi *= 2) {
-        const int64_t top = hi < nside - 1 ? hi : nside - 1;
-        const int hm = (int)(2 * top), M = next_pow2(2 * hm - 1);
-        // above the first class every ring has the same M: beyond mcap none takes Bluestein
-        st = one(lo, top - lo + 1, hm, M <= mcap ? M : (lo == 1 ? mcap : 0));
+    // M of the caps lo .. top (one power of two above the first class), 0 without Bluestein rings
+    auto caps_M = [&](int64_t lo, int64_t top) {
+        // rings of up to 512 pixels on a full chip: direct FP64 sums over primes up to 127 cost less
+        // than three transforms of 512 points (64 maps at Nside 128: 380 -> 279 us)
+        if (sizeof(T) == 8 && top <= 128 && (4 * nside - 1) * ncomp >= 148 * 64) return 0;
+        const int64_t first = lo > kDirectPrime ? lo : kDirectPrime + 1;
+        if (first > top || next_pow2((int)(4 * first - 1)) > mcap) return 0;
+        const int M = next_pow2((int)(4 * top - 1));
+        return M < mcap ? M : mcap;
+    };
+    const int hb = (int)(2 * nside), Mb = use_bluestein(hb, mcap) ? next_pow2(2 * hb - 1) : 0;
+    if (nside <= 128) {
+        const int M = caps_M(1, nside - 1);
+        return one(1, nside - 1, true, hb, M > Mb ? M : Mb);
+    }
+    int64_t hi = 128;
+    while (2 * hi < nside - 1) hi *= 2;
+    const bool joint = Mb == 0 && caps_M(hi + 1, nside - 1) == 0;   // the last class and the belt
+    int st = joint ? GM_OK : one(1, 0, true, hb, Mb);
+    for (int64_t lo = 1, h = 128; st == GM_OK && lo < nside; lo = h + 1, h *= 2) {
+        const int64_t top = h < nside - 1 ? h : nside - 1;
+        const bool last = joint && top == nside - 1;
+        st = one(lo, top - lo + 1, last, last ? hb : (int)(2 * top), caps_M(lo, top));
     }
     return st;
 }
@@ -1062,13 +1092,14 @@ static int ring_analysis(int64_t nside, int64_t L, int64_t ncomp, const void *ma
     using T2 = typename vec2<T>::type;
     const int64_t twcnt = gm_ring_twiddle_count(nside), nring = 4 * nside - 1;
     const bool vec = reinterpret_cast<uintptr_t>(maps) % (2 * sizeof(Tin)) == 0 && reinterpret_cast<uintptr_t>(mask) % 16 == 0;
-    int st = for_ring_classes<T>(nside, ncomp, hcap, big, [&](int64_t i0, int64_t cnt, int buf, int nbuf, int threads, int mcap, int64_t rows) {
+    int st = for_ring_classes<T>(nside, ncomp, hcap, big, [&](int64_t i0, int64_t cnt, int64_t rows, int buf, int nbuf,
+                                                              int threads, int cpc, int mcap) {
         const size_t bytes = (size_t)nbuf * buf * sizeof(T2);
-        const int e = allow_smem(k_ring_forward<T, Tin>, kRingSmem, "gm_ring_analysis attr");
+        auto kernel = nbuf == 3 ? k_ring_forward<T, Tin, true> : k_ring_forward<T, Tin, false>;
+        const int e = allow_smem(kernel, kRingSmem, "gm_ring_analysis attr");
         if (e) return e;
-        const int cpc = nbuf == 3 ? 8 : 1;   // components that share the transform of the chirp
         dim3 grid((unsigned)((ncomp + cpc - 1) / cpc), (unsigned)rows);
-        k_ring_forward<T, Tin><<<grid, threads, bytes, s>>>(nside, L, ncomp, cpc, (const Tin *)maps, mask, vec, tw, twcnt,
+        kernel<<<grid, threads, bytes, s>>>(nside, L, ncomp, cpc, (const Tin *)maps, mask, vec, tw, twcnt,
                                                             shifted, (T2 *)ringspec, i0, cnt, mcap, big ? hcap : 0, bsmin,
                                                             buf);
         return check_launch("gm_ring_analysis");
@@ -1243,13 +1274,14 @@ static int ring_synthesis_fold(int64_t nside, int64_t L, int64_t ncomp, const vo
         fold_lanes<T, false>(nside, L, ncomp, c0, cw, syn, nullptr, shifted, nullptr, work, sstride, s);
         int st = check_launch("gm_ring_synthesis_fold");
         if (st) return st;
-        st = for_ring_classes<T>(nside, cw, hcap, big, [&](int64_t i0, int64_t n, int buf, int nbuf, int threads, int mcap, int64_t rows) {
+        st = for_ring_classes<T>(nside, cw, hcap, big, [&](int64_t i0, int64_t n, int64_t rows, int buf, int nbuf,
+                                                           int threads, int cpc, int mcap) {
             const size_t bytes = (size_t)nbuf * buf * sizeof(T2);
-            const int e = allow_smem(k_ring_inverse<T>, kRingSmem, "gm_ring_synthesis_fold attr");
+            auto kernel = nbuf == 3 ? k_ring_inverse<T, true> : k_ring_inverse<T, false>;
+            const int e = allow_smem(kernel, kRingSmem, "gm_ring_synthesis_fold attr");
             if (e) return e;
-            const int cpc = nbuf == 3 ? 8 : 1;
             dim3 grid((unsigned)((cw + cpc - 1) / cpc), (unsigned)rows);
-            k_ring_inverse<T><<<grid, threads, bytes, s>>>(nside, cw, cpc, sstride, (const T2 *)work, tw, cnt, shifted, maps,
+            kernel<<<grid, threads, bytes, s>>>(nside, cw, cpc, sstride, (const T2 *)work, tw, cnt, shifted, maps,
                                                            c0, i0, n, mcap, big ? hcap : 0, bsmin, buf);
             return check_launch("gm_ring_synthesis_fold");
         });
