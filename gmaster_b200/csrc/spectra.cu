@@ -20,8 +20,7 @@ __device__ __forceinline__ int64_t alm_idx(int64_t lmax, int64_t l, int64_t m)
 
 // ---------------------------------------------------------------- pseudo-C_ell
 
-constexpr int kPclLanes = 32;    // degrees per CTA (one per lane: coalesced over l)
-constexpr int kPclWarps = 32;    // orders interleaved over the warps of a CTA
+constexpr int kPclThreads = 1024;
 constexpr int kPclPairs = 64;    // field pairs of one launch
 
 // Field pairs of a launch: pair p has the alms a (N1 rows of nelem) and b (N2 rows), spectra out
@@ -31,19 +30,24 @@ struct PclPairs {
     double *out[kPclPairs];
 };
 
-// grid (l-blocks of 32, pairs), 1024 threads: lane = degree l, warp w sums the orders m = w,
-// w + 32, ... <= l of every component product (each alm read once); the partial sums are then
-// added in a fixed order, so the result does not depend on scheduling (equal inputs give
-// bit-equal spectra).  Bound by the latency of the order loop at small lmax and by memory at
-// large: 32 warps keep it at lmax / 32 steps, and a batch of pairs is one launch.  32 pairs of
-// (E, B) at lmax 767: 74 us (4.1 TB/s); 911 us in 32 launches of eight warps and one product a CTA.
-template <int N1, int N2>
-__global__ void __launch_bounds__(kPclLanes * kPclWarps) k_pseudo_cl(int64_t lmax, const __grid_constant__ PclPairs p)
+// grid (blocks of LANES degrees, the longest sums first; pairs), 1024 threads: a thread takes degree
+// l and sums the orders m = w, w + 1024 / LANES, ... <= l of every component product (each alm read
+// once); the partial sums are then added in a fixed order, so the result does not depend on
+// scheduling (equal inputs give bit-equal spectra).  Bound by the latency of the order loop at small
+// lmax and by memory at large: 32 warps keep it at lmax / 32 steps, and a batch of pairs is one
+// launch.  32 pairs of (E, B) at lmax 767: 74 us (4.1 TB/s); 911 us in 32 launches of eight warps and
+// one product a CTA.  LANES = 32 up to 512 degrees, 16 up to 1024, 8 above: one pair has few blocks of
+// 32 (two (E, B) fields at lmax 767 / 3071 / 6143: 19 / 148 / 381 -> 13 / 74 / 251 us), where 32
+// pairs at lmax 767 lose 5 % with 16 and 25 % with 8.
+template <int N1, int N2, int LANES>
+__global__ void __launch_bounds__(kPclThreads) k_pseudo_cl(int64_t lmax, const __grid_constant__ PclPairs p)
 {
-    __shared__ double part[N1 * N2][kPclWarps][kPclLanes];
+    constexpr int kGroups = kPclThreads / LANES, kOut = N1 * N2 * LANES;
+    constexpr int kPer = kPclThreads / kOut < 32 ? kPclThreads / kOut : 32;   // threads per result
+    __shared__ double part[N1 * N2][kGroups][LANES + 1];
     const int64_t L = lmax + 1, nelem = L * (L + 1) / 2;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t l = (int64_t)blockIdx.x * kPclLanes + lane;
+    const int lane = threadIdx.x % LANES, w = threadIdx.x / LANES;
+    const int64_t l = (int64_t)(gridDim.x - 1 - blockIdx.x) * LANES + lane;
     const double2 *a = p.a[blockIdx.y], *b = p.b[blockIdx.y];
     const bool same = N1 == N2 && a == b;
     double s[N1 * N2];
@@ -51,7 +55,7 @@ __global__ void __launch_bounds__(kPclLanes * kPclWarps) k_pseudo_cl(int64_t lma
     for (int q = 0; q < N1 * N2; ++q) s[q] = 0.0;
     if (l < L) {
 #pragma unroll 4
-        for (int64_t m = w; m <= l; m += kPclWarps) {
+        for (int64_t m = w; m <= l; m += kGroups) {
             const int64_t k = alm_idx(lmax, l, m);
             double2 x[N1], y[N2];
 #pragma unroll
@@ -70,12 +74,17 @@ __global__ void __launch_bounds__(kPclLanes * kPclWarps) k_pseudo_cl(int64_t lma
 #pragma unroll
     for (int q = 0; q < N1 * N2; ++q) part[q][w][lane] = s[q];
     __syncthreads();
-    if (w < N1 * N2 && l < L) {
-        double t = 0.0;
+    // kPer neighbouring threads add a result's partial sums, always in the same order
+    const int o = threadIdx.x / kPer, i = threadIdx.x % kPer, d = o % LANES;
+    double t = 0.0;
+    if (o < kOut) {
 #pragma unroll
-        for (int q = 0; q < kPclWarps; ++q) t += part[w][q][lane];
-        p.out[blockIdx.y][w * L + l] = t / (2.0 * (double)l + 1.0);
+        for (int g = i; g < kGroups; g += kPer) t += part[o / LANES][g][d];
     }
+#pragma unroll
+    for (int h = kPer / 2; h >= 1; h >>= 1) t += __shfl_xor_sync(0xffffffffu, t, h);
+    const int64_t lo = (int64_t)(gridDim.x - 1 - blockIdx.x) * LANES + d;
+    if (o < kOut && i == 0 && lo < L) p.out[blockIdx.y][(o / LANES) * L + lo] = t / (2.0 * (double)lo + 1.0);
 }
 
 // ---------------------------------------------------------------- Wigner-3j coupling
@@ -1143,12 +1152,15 @@ extern "C" int gm_pseudo_cl_pairs(int64_t lmax, int64_t npairs, int64_t n1, cons
             p.b[i] = (const double2 *)alm2[f] + (whole ? 0 : q % n2) * nelem;
             p.out[i] = cls[f] + q * L;
         }
-        const dim3 grid((unsigned)((L + kPclLanes - 1) / kPclLanes), (unsigned)cnt);
-        const int threads = kPclLanes * kPclWarps;
-        if (!whole || (n1 == 1 && n2 == 1)) k_pseudo_cl<1, 1><<<grid, threads, 0, s>>>(lmax, p);
-        else if (n1 == 1) k_pseudo_cl<1, 2><<<grid, threads, 0, s>>>(lmax, p);
-        else if (n2 == 1) k_pseudo_cl<2, 1><<<grid, threads, 0, s>>>(lmax, p);
-        else k_pseudo_cl<2, 2><<<grid, threads, 0, s>>>(lmax, p);
+        const int lanes = L <= 512 ? 32 : (L <= 1024 ? 16 : 8);   // by lmax alone: a pair's sums do not depend on the batch
+        const dim3 grid((unsigned)((L + lanes - 1) / lanes), (unsigned)cnt);
+        auto run = [&](auto k32, auto k16, auto k8) {
+            (lanes == 32 ? k32 : (lanes == 16 ? k16 : k8))<<<grid, kPclThreads, 0, s>>>(lmax, p);
+        };
+        if (!whole || (n1 == 1 && n2 == 1)) run(k_pseudo_cl<1, 1, 32>, k_pseudo_cl<1, 1, 16>, k_pseudo_cl<1, 1, 8>);
+        else if (n1 == 1) run(k_pseudo_cl<1, 2, 32>, k_pseudo_cl<1, 2, 16>, k_pseudo_cl<1, 2, 8>);
+        else if (n2 == 1) run(k_pseudo_cl<2, 1, 32>, k_pseudo_cl<2, 1, 16>, k_pseudo_cl<2, 1, 8>);
+        else run(k_pseudo_cl<2, 2, 32>, k_pseudo_cl<2, 2, 16>, k_pseudo_cl<2, 2, 8>);
         const int st = check_launch("gm_pseudo_cl");
         if (st != GM_OK) return st;
     }
