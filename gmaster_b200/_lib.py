@@ -101,6 +101,9 @@ SIGNATURES = {
     "gm_tc_selftest": ([_c_i64, _c_i64, _c_int, _c_int, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp], _c_int),
     "gm_tc_selftest_timeout": ([_c_i64, _c_i64, _c_vp, _c_vp, _c_vp, _c_vp, _c_i64, _c_vp], _c_int),
     "gm_mask_ring_runs": ([_c_i64, _c_vp, _c_vp, _c_vp, _c_vp], _c_int),
+    "gm_mask_ring_gaps": ([_c_i64, _c_vp, _c_vp, _c_vp], _c_int),
+    "gm_mask_apodize_gaps": ([_c_i64, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_dbl, _c_dbl, _c_int, _c_vp, _c_vp],
+                             _c_int),
     "gm_cov_binned": ([_c_i64, _c_i64, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_i64, _c_vp, _c_vp, _c_vp,
                        _c_i64, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp], _c_int),
     "gm_cov_bands": ([_c_i64, _c_i64, _c_i64, _c_vp, _c_i64, _c_vp, _c_vp, _c_vp, _c_vp, _c_i64, _c_vp, _c_vp,

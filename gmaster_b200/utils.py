@@ -200,7 +200,7 @@ def mask_apodization(mask_in, aposize, apotype="C1"):
     x = sqrt((1 - cos theta) / (1 - cos theta_*)), unmasked pixels closer than theta_* are
     multiplied by x - sin(2 pi x) / (2 pi) ("C1") or (1 - cos(pi x)) / 2 ("C2").  The
     distance is exact over all masked pixels (the reference queries a k-d tree of their unit
-    vectors; here the CUDA kernel walks the HEALPix rings, gm_mask_apodize).
+    vectors; here the CUDA kernel walks the HEALPix rings, gm_mask_apodize_gaps).
 
     "Smooth": pixels within 2.5 theta_* of a masked pixel are zeroed, the result is
     smoothed with a Gaussian beam of standard deviation theta_* (map2alm with n_iter = 3,
@@ -238,24 +238,25 @@ def mask_apodization(mask_in, aposize, apotype="C1"):
     scale = 2.5 if apotype == "Smooth" else 1.2
     if int(4 * npix * (1 - np.cos(scale * radius))) < 2:
         raise ValueError("Your apodization scale is too small for this pixel size")
-    # without a masked pixel nothing is smoothed (the C1 / C2 kernels then leave the mask as it is)
+    # without a masked pixel nothing is smoothed (the C1 / C2 kernel then copies the mask)
     if apotype == "Smooth" and not bool((mask <= 0).any()):
         return result(mask.clone())
     dev = mask.device
-    prev = torch.empty(npix, dtype=torch.int32, device=dev)
-    nxt = torch.empty(npix, dtype=torch.int32, device=dev)
+    nring = 4 * nside - 1
+    prev, nxt, gaps = torch.empty(2 * npix + nring, dtype=torch.int32, device=dev).split([npix, npix, nring])
     out = torch.empty_like(mask)
     stream = _lib.stream_handle(dev)
     _lib.call("gm_mask_ring_runs", nside, _lib.ptr(mask), _lib.ptr(prev), _lib.ptr(nxt), stream)
+    _lib.call("gm_mask_ring_gaps", nside, _lib.ptr(prev), _lib.ptr(gaps), stream)
     table = _apo_ring_table(nside, dev)
     if apotype == "Smooth":
         reach = min(2.5 * radius + max_pixel_radius(nside), np.pi)
         chord2 = 4.0 * np.sin(0.5 * reach) ** 2
         if reach >= np.pi:
             chord2 = 5.0   # every pixel is within reach
-        _lib.call("gm_mask_apodize", nside, _lib.ptr(table), _lib.ptr(mask), _lib.ptr(prev),
-                  _lib.ptr(nxt), float(chord2), 0.0, 2, _lib.ptr(out), stream)
-        del prev, nxt
+        _lib.call("gm_mask_apodize_gaps", nside, _lib.ptr(table), _lib.ptr(mask), _lib.ptr(prev),
+                  _lib.ptr(nxt), _lib.ptr(gaps), float(chord2), 0.0, 2, _lib.ptr(out), stream)
+        del prev, nxt, gaps
         lmax = 3 * nside - 1
         prec = get_precision()
         alm = sht.map2alm_device(out[None], 0, nside, lmax, 3, prec)
@@ -264,8 +265,8 @@ def mask_apodization(mask_in, aposize, apotype="C1"):
         smoothed = sht.alm2map_device(alm * beam[None], 0, nside, lmax, prec)[0]
         return smoothed * mask
     threshold = 1 - np.cos(radius)
-    _lib.call("gm_mask_apodize", nside, _lib.ptr(table), _lib.ptr(mask), _lib.ptr(prev),
-              _lib.ptr(nxt), float(2 * threshold), float(threshold),
+    _lib.call("gm_mask_apodize_gaps", nside, _lib.ptr(table), _lib.ptr(mask), _lib.ptr(prev),
+              _lib.ptr(nxt), _lib.ptr(gaps), float(2 * threshold), float(threshold),
               0 if apotype == "C1" else 1, _lib.ptr(out), stream)
     return result(out)
 

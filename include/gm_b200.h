@@ -488,12 +488,19 @@ int gm_tc_alm_layout(int64_t lmax, int spin, int64_t nfield, double *alm_i, doub
  * mask * f(x), x = sqrt(d^2 / 2 / threshold), for pixels with mask > 0 and d^2 <
  * chord2_max, else out = mask; f = x - sin(2 pi x)/(2 pi) (C1) or (1 - cos(pi x))/2 (C2).
  * mode 2 (zeroing step of "Smooth"): out = 0 for masked pixels and for pixels with d^2 <
- * chord2_max, else mask.  out may not alias mask. */
+ * chord2_max, else mask.  out may not alias mask.
+ * gm_mask_ring_gaps: gaps[j] = rings from ring j to the nearest one with a masked pixel (0: itself,
+ * INT32_MAX: none), from `prev` of gm_mask_ring_runs; gaps is a caller-owned int32 (4 nside - 1)
+ * buffer.  gm_mask_apodize_gaps: gm_mask_apodize that starts its search there (NULL: the same). */
 int gm_mask_ring_runs(int64_t nside, const double *mask, int32_t *prev, int32_t *next,
                       void *stream);
 int gm_mask_apodize(int64_t nside, const double *ring_table, const double *mask,
                     const int32_t *prev, const int32_t *next, double chord2_max,
                     double threshold, int mode, double *out, void *stream);
+int gm_mask_ring_gaps(int64_t nside, const int32_t *prev, int32_t *gaps, void *stream);
+int gm_mask_apodize_gaps(int64_t nside, const double *ring_table, const double *mask,
+                         const int32_t *prev, const int32_t *next, const int32_t *gaps,
+                         double chord2_max, double threshold, int mode, double *out, void *stream);
 
 /* ---------------------------------------------------------- Gaussian covariance */
 
