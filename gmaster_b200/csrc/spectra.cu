@@ -370,33 +370,50 @@ __global__ void k_toeplitz_fill(int64_t lmax, int64_t lt, int64_t le, int64_t dl
 
 // ---------------------------------------------------------------- binning
 
-// Binned block: out[b][b'] = sum_{l in b} wfl[l] sum_{l' in b'} M[l][l'] beam[l'] inv_fl[l'].  One warp
-// per pair of bands: lanes along l', the rows of b in turn (several loads in flight), then a sum
-// over the lanes.  A CTA of 256 threads per pair, with a division per element and a tree in
-// shared memory, took 38 us a block at lmax 1535 with bands of ten; 16 us here.
+// Binned block: out[b][b'] = sum_{l in b} wfl[l] sum_{l' in b'} M[l][l'] beam[l'] inv_fl[l'].  ROWS warps
+// per pair of bands: lanes along l', every ROWS-th row of b in turn (several loads in flight),
+// then a sum over the lanes and the warps.  Bound by the latency of the rows.  A CTA of 256 threads
+// per pair, with a division per element and a tree in shared memory, took 38 us a block at lmax 1535
+// with bands of ten; 16 us here with one warp.  Few or wide bands take eight: three bands of 50
+// degrees at Nside 64 78 us a binned workspace with one warp, 56 with eight; one of 766, 2.2 and 0.39 ms.
 constexpr int kBinWarps = 8;
+template <int ROWS>
 __global__ void __launch_bounds__(32 * kBinWarps) k_bin_block(
     int64_t lmax, int64_t nb, const double *__restrict__ M, const int32_t *__restrict__ band_ptr,
     const int32_t *__restrict__ band_ells, const double *__restrict__ wfl, const double *__restrict__ inv_fl,
     const double *__restrict__ beam, double *__restrict__ out)
 {
-    const int64_t b = blockIdx.y, bp = (int64_t)blockIdx.x * kBinWarps + (threadIdx.x >> 5), n = lmax + 1;
-    if (bp >= nb) return;
-    const int lane = threadIdx.x & 31;
-    const int i0 = band_ptr[b], i1 = band_ptr[b + 1], k0 = band_ptr[bp], k1 = band_ptr[bp + 1];
+    constexpr int kPairs = kBinWarps / ROWS;
+    __shared__ double part[kBinWarps];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t b = blockIdx.y, bp = (int64_t)blockIdx.x * kPairs + w / ROWS, n = lmax + 1;
     double s = 0.0;
-    for (int k = k0 + lane; k < k1; k += 32) {
-        const int lp = band_ells[k];
-        double t = 0.0;
+    if (bp < nb) {
+        const int i0 = band_ptr[b] + w % ROWS, i1 = band_ptr[b + 1], k0 = band_ptr[bp], k1 = band_ptr[bp + 1];
+        for (int k = k0 + lane; k < k1; k += 32) {
+            const int lp = band_ells[k];
+            double t = 0.0;
 #pragma unroll 4
-        for (int i = i0; i < i1; ++i) {
-            const int l = band_ells[i];
-            t = fma(wfl[l], M[(int64_t)l * n + lp], t);
+            for (int i = i0; i < i1; i += ROWS) {
+                const int l = band_ells[i];
+                t = fma(wfl[l], M[(int64_t)l * n + lp], t);
+            }
+            s += t * beam[lp] * inv_fl[lp];
         }
-        s += t * beam[lp] * inv_fl[lp];
     }
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) out[b * nb + bp] = s;
+    if (ROWS == 1) {
+        if (lane == 0 && bp < nb) out[b * nb + bp] = s;
+        return;
+    }
+    if (lane == 0) part[w] = s;
+    __syncthreads();
+    if (threadIdx.x < kPairs) {
+        const int64_t q = (int64_t)blockIdx.x * kPairs + threadIdx.x;
+        double t = 0.0;
+        for (int r = 0; r < ROWS; ++r) t += part[threadIdx.x * ROWS + r];
+        if (q < nb) out[b * nb + q] = t;
+    }
 }
 
 // Place binned blocks into the (ncls nb)^2 matrix, band-major channel-minor.
@@ -1254,19 +1271,22 @@ extern "C" int gm_bin_coupling_csr(int64_t lmax, int64_t nbands, int ncls, const
         return GM_ERR_BAD_PTR;
     cudaStream_t s = as_stream(stream);
     const int64_t n = lmax + 1, nn = n * n, nb2 = nbands * nbands;
-    dim3 grid((unsigned)((nbands + kBinWarps - 1) / kBinWarps), (unsigned)nbands);
+    // eight warps a pair where one would leave the chip idle (nbands <= 48) or walk 64 rows and more
+    const bool split = n >= 8 * nbands && (nbands <= 48 || n >= 64 * nbands);
+    const int64_t pairs = split ? 1 : kBinWarps;
+    const dim3 grid((unsigned)((nbands + pairs - 1) / pairs), (unsigned)nbands);
+    auto bin = [&](const double *M, double *to) {
+        (split ? k_bin_block<kBinWarps> : k_bin_block<1>)<<<grid, 32 * kBinWarps, 0, s>>>(
+            lmax, nbands, M, band_ptr, band_ells, wfl, inv_fl, beam, to);
+    };
     // block slots: tt 0, te 1, pp 2, mm 3
     if (ncls == 1) {
-        k_bin_block<<<grid, 32 * kBinWarps, 0, s>>>(lmax, nbands, blocks, band_ptr, band_ells, wfl, inv_fl,
-                                         beam, scratch);
+        bin(blocks, scratch);
     } else if (ncls == 2) {
-        k_bin_block<<<grid, 32 * kBinWarps, 0, s>>>(lmax, nbands, blocks + nn, band_ptr, band_ells, wfl,
-                                         inv_fl, beam, scratch);
+        bin(blocks + nn, scratch);
     } else {
-        k_bin_block<<<grid, 32 * kBinWarps, 0, s>>>(lmax, nbands, blocks + 2 * nn, band_ptr, band_ells, wfl,
-                                         inv_fl, beam, scratch);
-        k_bin_block<<<grid, 32 * kBinWarps, 0, s>>>(lmax, nbands, blocks + 3 * nn, band_ptr, band_ells, wfl,
-                                         inv_fl, beam, scratch + nb2);
+        bin(blocks + 2 * nn, scratch);
+        bin(blocks + 3 * nn, scratch + nb2);
     }
     const int64_t N = ncls * nbands;
     k_place_binned<<<(unsigned)((N * N + 255) / 256), 256, 0, s>>>(nbands, ncls, scratch, out);
