@@ -1309,7 +1309,7 @@ extern "C" int gm_bin_cells_csr(int64_t lmax, int64_t nbands, int64_t ncls, cons
 constexpr int kLuSmem = 200 * 1024;
 
 // Panel width of the shared-memory panels: the widest of 32, 16, 8, 4 columns that fit (the
-// whole matrix up to n = 160), 0 when none does.
+// whole matrix up to n = 159), 0 when none does.
 static int lu_panel_width(int64_t n)
 {
     const int64_t fit = kLuSmem / (8 * (n | 1));
@@ -1345,15 +1345,16 @@ extern "C" int gm_lu_factor(int64_t n, double *a, int32_t *piv, int32_t *status,
     if (sa != GM_OK) return sa;
     for (int64_t k0 = 0; k0 < n;) {
         const int64_t rows = n - k0;
-        // rows in registers: 32 columns of up to 640 rows, 16 of up to 1024; else the widest panel
-        // that fits shared memory (one for all of n <= 160)
-        const int width = n <= 160 ? w : (rows <= 640 ? 32 : (rows <= 1024 ? 16 : w));
+        // one panel in shared memory where the whole matrix fits; else rows in registers, 32 columns
+        // of up to 640 rows, 16 of up to 1024, or the widest panel that fits shared memory
+        const bool whole = w == n;
+        const int width = whole ? w : (rows <= 640 ? 32 : (rows <= 1024 ? 16 : w));
         const int kb = (int)(rows < width ? rows : width);
         const int64_t k1 = k0 + kb;
         const int threads = rows >= 1024 ? 1024 : (int)((rows + 31) / 32 * 32);
-        if (n > 160 && rows <= 640)
+        if (!whole && rows <= 640)
             k_lu_panel_reg<32, 640><<<1, threads, 0, s>>>((int)n, (int)k0, kb, a, piv, status);
-        else if (n > 160 && rows <= 1024)
+        else if (!whole && rows <= 1024)
             k_lu_panel_reg<16, 1024><<<1, threads, 0, s>>>((int)n, (int)k0, kb, a, piv, status);
         else
             k_lu_panel_smem<<<1, threads, smem, s>>>((int)n, (int)k0, kb, a, piv, status);

@@ -1,4 +1,4 @@
-"""Shared-memory LU panels and prepared solves at the edges of their ranges: one panel (n <= 160),
+"""Shared-memory LU panels and prepared solves at the edges of their ranges: one panel (n <= 159),
 every panel width, last panels and 32-row blocks in part, right-hand sides that fill a CTA in
 part; pivots equal to numpy's choice rule.  Bound: solves of well-conditioned matrices to 1e-11
 (n eps times a modest growth), residuals |PA - LU| to 1e-13 of |A|."""
@@ -12,7 +12,7 @@ from gmaster_b200.workspaces import LUFactor
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 160, 161, 256, 781, 1600, 3300])
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 158, 159, 160, 161, 256, 781, 1600, 3300])
 def test_factors_and_solves(cuda, n):
     rng = np.random.default_rng(n)
     a = rng.normal(size=(n, n))
