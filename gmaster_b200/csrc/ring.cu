@@ -1298,7 +1298,8 @@ extern "C" int gm_ring_synthesis_fold(int precision, int64_t nside, int64_t L, i
     if (nside < 1 || nside > 8192 || L < 1 || ncomp < 1 || ncomp > 65535) return GM_ERR_BAD_SHAPE;
     if (precision != GM_FP64 && precision != GM_MIXED) return GM_ERR_UNSUPPORTED;
     if (!syn || !tw || !shifted || !maps || !work || !scratch) return GM_ERR_BAD_PTR;
-    if ((reinterpret_cast<uintptr_t>(maps) | reinterpret_cast<uintptr_t>(syn)) & 15) return GM_ERR_BAD_PTR;
+    if ((reinterpret_cast<uintptr_t>(maps) | reinterpret_cast<uintptr_t>(syn) | reinterpret_cast<uintptr_t>(work)) & 15)
+        return GM_ERR_BAD_PTR;
     const int64_t per = gm_ring_fold_bytes(precision, nside), chunk = work_bytes / per;
     const int64_t slot = gm_ring_big_scratch_bytes(nside, 1), nslots = scratch_bytes / slot;
     if (chunk < 1 || nslots < 1) return GM_ERR_BAD_SHAPE;

@@ -120,7 +120,7 @@ int gm_ring_synthesis_ws(int precision, int64_t nside, int64_t L, int64_t ncomp,
  * prime factor above 64 by Bluestein's method in both precisions (the entries above take the
  * mixed-radix FFT).  work holds the folded spectra of as many components at a time as
  * work_bytes allow, gm_ring_fold_bytes each; scratch as in gm_ring_synthesis_ws (required).
- * syn and maps must be 16-byte aligned. */
+ * syn, maps and work must be 16-byte aligned (GM_ERR_BAD_PTR otherwise). */
 int64_t gm_ring_fold_bytes(int precision, int64_t nside);
 int gm_ring_synthesis_fold(int precision, int64_t nside, int64_t L, int64_t ncomp, const void *syn,
                            const void *tw, const uint8_t *shifted, double *maps, void *work,

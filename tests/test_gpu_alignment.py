@@ -18,7 +18,7 @@ def _gen(seed):
 def _offset(t, by=1):
     """A copy of t that starts `by` real elements after a 16-byte boundary."""
     flat = torch.view_as_real(t).reshape(-1) if t.is_complex() else t.reshape(-1)
-    buf = torch.empty(flat.numel() + 4, dtype=flat.dtype, device=t.device)
+    buf = torch.empty(flat.numel() + max(4, by), dtype=flat.dtype, device=t.device)
     out = buf[by:by + flat.numel()]
     out.copy_(flat)
     assert out.data_ptr() % 16 != 0
@@ -100,3 +100,20 @@ def test_batched_fold(cuda, spin, ncomp):
         _lib.call("gm_tc_fold", nside, lmax, spin, ncomp, _lib.ptr(synd[0]), _lib.ptr(synd[-1]) if spin else None,
                   _lib.ptr(rhs), _lib.ptr(p.shifted), _lib.ptr(off), _lib.ptr(img[-1]) if spin else None, 64.0,
                   _lib.stream_handle(p.device))
+
+
+def test_ring_synthesis_fold_refuses_what_it_cannot_read(cuda):
+    plan = sht.get_plan(8, 23)
+    syn = torch.randn((plan.L, plan.nlanes, 1, 4), generator=_gen(6), device="cuda")
+    maps = torch.empty(plan.npix, dtype=torch.float64, device="cuda")
+    work = torch.empty(int(_lib.load().gm_ring_fold_bytes(_lib.MIXED, 8)), dtype=torch.uint8, device="cuda")
+    scratch, nbytes = sht._ring_scratch(plan, _lib.MIXED)
+
+    def call(s, m, w):
+        _lib.call("gm_ring_synthesis_fold", _lib.MIXED, 8, plan.L, 1, _lib.ptr(s), _lib.ptr(plan.tw), _lib.ptr(plan.shifted),
+                  _lib.ptr(m), _lib.ptr(w), work.numel(), _lib.ptr(scratch), nbytes, 0, 0, _lib.stream_handle(plan.device))
+
+    call(syn, maps, work)
+    for args in ((_offset(syn), maps, work), (syn, _offset(maps), work), (syn, maps, _offset(work, 8))):
+        with pytest.raises(_lib.GMError):
+            call(*args)
