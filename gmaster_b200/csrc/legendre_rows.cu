@@ -370,8 +370,12 @@ __device__ __forceinline__ void ana8(Rows<SPIN, R> &w, const u64 (&rh)[R][4 * NC
 }
 
 // Resident CTAs asked for: four of one spin-0 map at R = 4 (128 registers; 139 and three CTAs
-// measured 18.0 instead of 16.9 ms at Nside 2048).
-__host__ __device__ constexpr int ana_ctas(int spin, int nc, int r) { return spin == 0 && nc == 1 && r == 4 ? 4 : 1; }
+// measured 18.0 instead of 16.9 ms at Nside 2048), two of eight warps of spin 2 at R = 4 (122
+// registers; 172 and one CTA took 7.9 instead of 6.9 ms at Nside 1024, 1.31 instead of 1.04 at 512).
+__host__ __device__ constexpr int ana_ctas(int spin, int nc, int r)
+{
+    return spin == 0 && nc == 1 && r == 4 ? 4 : (spin == 2 && r == 4 ? 2 : 1);
+}
 
 template <int SPIN, int NC, int R>
 __global__ void __launch_bounds__(32 * max_warps(SPIN, R), ana_ctas(SPIN, NC, R)) k_rows_ana(int64_t nside, int64_t lmax, int64_t ncomp,
