@@ -21,14 +21,14 @@
 //
 // A CTA is up to four warps of one order; the rows go in segments of up to 128 whose
 // coefficients its threads compute once, then in blocks of eight without barriers: a warp whose
-// lanes are all below 2^-300 only steps.  Spin s takes the sum F and the difference G of the
-// two variants' rows, formed in double precision, against Q and U (four values a row, E and B:
-// at m = 0, where G = 0, E takes Q alone and B takes U alone).  Small sizes are bound by the chain of rows (m = 0) and the reduction
-// trees, large ones by the FP64 pipe: (3 + 2 NC) operations per row and lane (spin 0), 16 (spin
-// s).  Against windows of 32 rows with coefficients by square roots and divisions in each, and
-// eight sums a row: FP64 analysis / synthesis at Nside 128 56 / 44 -> 35 / 21 us, at Nside 1024
-// 10.0 / 8.1 -> 5.1 / 3.9 ms (spin 0) and 26.8 / 21.5 -> 13.0 / 9.9 ms (spin 2); mixed spin 1 at
-// Nside 1024 20.1 / 18.4 -> 9.6 / 8.7 ms.
+// lanes are all below 2^-300 only steps.  Spin s takes the sum F and the difference G of the two
+// variants' rows, formed in double precision, against Q and U (four values a row, E and B: at m = 0,
+// where G = 0, E takes Q alone and B takes U alone).  Small sizes are bound by the chain of rows
+// (m = 0) and the reduction trees, large ones by the FP64 pipe: (3 + 2 NC) operations per row and
+// lane (spin 0), 16 (spin s).  Against windows of 32 rows with coefficients by square roots and
+// divisions in each, and eight sums a row: FP64 analysis / synthesis at Nside 128 58 / 44 -> 33 / 23
+// us, at Nside 1024 10.0 / 8.1 -> 5.2 / 4.0 ms (spin 0) and 26.8 / 21.5 -> 13.3 / 10.9 ms (spin 2);
+// mixed spin 1 at Nside 1024 20.1 / 18.3 -> 10.9 / 9.7 ms.
 //
 // Replaces gmaster/_native/cuda/march_v2.cu:155-407 (march_analysis /
 // march_synthesis: float32 difference-form recurrence, SIMT FMA contraction).

@@ -22,18 +22,18 @@
 // once per block of rows.  E and B are never formed from each other's rounded values: at m = 0
 // (G = 0) E takes Q alone and B takes U alone, and elsewhere a B far below E carries the
 // rounding of the products G Q only.  Summing 2a and -2a instead (P = Q + iU, M = Q - iU, no
-// F and G) takes 4 % less time (field, spin 2, Nside 512: 6.8 against 7.1 ms) and leaves the
+// F and G) takes 3 % less time (field, spin 2, Nside 512: 6.8 against 7.0 ms) and leaves the
 // rounding of E in B: with U = 1e-3 Q the error of B at m = 0, Nside 512, is 7e-5 of B there, 3e-7
 // here.
 //
-// Bound and split.  The FMA pipe: (3 + 2 NC) packed FMAs per row and two lanes for spin 0, 7
-// and two additions per row and lane for spin 2, plus one shuffle per row, value and thread in the analysis
-// (the shuffle unit takes one instruction a clock and SM, a quarter of the FMA issue rate, so
-// a thread sums its 2R or R lanes first).  At Nside 512 the pipe is 60-64 % busy (a packed FMA
-// of three different operands issues at 1.37 a clock and SM instead of 2: the register file's
-// bandwidth), IPC 1.7-2.1.  Against the four-operation scalar rows with a warp tree per 32
-// values: analysis / synthesis at Nside 2048 40.6 / 25.2 -> 17.4 / 14.0 ms (spin 0), at Nside
-// 512 2.37 / 1.32 -> 0.99 / 0.72 ms (spin 2).  A CTA is up to eight warps of one order m; a warp's
+// Bound and split.  The FMA pipe: (3 + 2 NC) packed FMAs per row and two lanes for spin 0, 7 and
+// two additions per row and lane for spin 2, plus one shuffle per row, value and thread in the
+// analysis (the shuffle unit takes one instruction a clock and SM, a quarter of the FMA issue
+// rate, so a thread sums its 2R or R lanes first).  At Nside 512 the pipe is 56-62 % busy (a packed
+// FMA of three different operands issues at 1.37 a clock and SM instead of 2: the register file's
+// bandwidth), IPC 1.8-2.2.  Against the four-operation scalar rows with a warp tree per 32
+// values: analysis / synthesis at Nside 2048 40.6 / 25.2 -> 17.0 / 14.0 ms (spin 0), at Nside
+// 512 2.37 / 1.32 -> 1.04 / 0.77 ms (spin 2).  A CTA is up to eight warps of one order m; a warp's
 // lanes are contiguous and it skips the segments whose checkpoint states are zero on all of
 // them.
 //

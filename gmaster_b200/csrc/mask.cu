@@ -9,10 +9,10 @@
 // up from the pixel just above it.  k_ring_runs stores both for every pixel (cyclically
 // within its ring): prev[p] = the masked pixel at or before p, next[p] = at or after p
 // (ring-local indices, -1 for a ring without masked pixels).  k_mask_apodize then visits
-// rings outwards from the query's own ring, alternating north and south, two candidates
-// per ring, passing over rings without a masked pixel within the radius of the query's warp
-// and those whose latitude alone puts them beyond the best chord found, until the latitude
-// alone exceeds the radius.  The result is the exact minimum over all masked pixels, like the
+// rings outwards from the query's own ring or the nearest one with a masked pixel (k_ring_gaps),
+// alternating north and south, two candidates per ring, passing over rings without a masked pixel
+// that could improve a pixel of the query's warp, until the latitude alone puts every later ring
+// beyond the worst chord that the warp still has.  The result is the exact minimum over all masked pixels, like the
 // k-d tree's.
 //
 // Chords are evaluated as |v_q - v_c|^2 = dz^2 + ds^2 + 4 s_q s_c sin^2(dphi / 2) with

@@ -229,8 +229,8 @@ __device__ T2 *fft_shared(T2 *a, T2 *b, int h, const T2 *__restrict__ tw, int si
 // ---------------------------------------------------------------- analysis
 
 // Rings whose half-length h has a prime factor above 64 are transformed by Bluestein's
-// chirp-z method in single precision (three power-of-two FFTs of length
-// M = nextpow2(2h - 1) <= mcap), instead of a generic radix-p stage costing h p.
+// chirp-z method (three power-of-two FFTs of length M = nextpow2(2h - 1) <= mcap), instead of a
+// generic radix-p stage costing h p.
 __host__ __device__ __forceinline__ int largest_prime_factor(int h)
 {
     int p = 1;
@@ -751,8 +751,8 @@ __global__ void __launch_bounds__(512) k_ring_synthesis(int64_t nside, int64_t L
 
 // Inverse ring transform from the folded spectra of k_fold_lanes: one CTA per (ring, block of
 // cpc components), with the rings and buffers of k_ring_forward.
-// With the fold before it: 2235 -> 790 us for a (Q, U) pair at Nside 1024 (a ring per CTA reading
-// its coefficients 128 lanes apart and taking prime factors up to 1021 as one radix), 163 -> 61
+// With the fold before it: 2.22 -> 0.75 ms for a (Q, U) pair at Nside 1024 (a ring per CTA reading
+// its coefficients 128 lanes apart and taking prime factors up to 1021 as one radix), 180 -> 65
 // us for one FP64 map at Nside 256.
 template <typename T, bool BS>
 __global__ void __launch_bounds__(512) k_ring_inverse(int64_t nside, int64_t ncomp, int cpc, int64_t sstride,
@@ -825,9 +825,9 @@ __global__ void __launch_bounds__(512) k_ring_inverse(int64_t nside, int64_t nco
 // power-of-two length M.  __syncthreads orders the CTA's global-memory accesses.
 
 // T = float: three buffers of Mmax complex floats per slot (Bluestein rings included).
-// T = double: no Bluestein path (the mixed-radix FFT takes every ring, as in the FP64
-// shared-memory kernel); two buffers of 2 nside complex doubles per slot, which fit the
-// same slot bytes (64 nside <= 96 nside).
+// T = double: no Bluestein path here (the FP64 shared-memory kernels have one up to M = 4096; the
+// mixed-radix FFT takes every ring that is too long for them); two buffers of 2 nside complex
+// doubles per slot, which fit the same slot bytes (64 nside <= 96 nside).
 template <typename T, typename Tin>
 __global__ void __launch_bounds__(512) k_ring_analysis_big(int64_t nside, int64_t L, int64_t ncomp,
                                                            const Tin *__restrict__ maps,
@@ -1035,7 +1035,7 @@ static bool any_ring_big(int64_t nside, int hcap, int bsmin)
 // none takes Bluestein, share the belt's launch: longest first, the belt fills up behind their
 // direct sums over primes (one FP64 map at Nside 2048: 8.6 -> 6.8 ms).  Threads: an eighth of the
 // points where the rings of all components fill the chip many times over (64 maps at Nside 512:
-// 5.5 -> 4.0 ms), else two to four times as many, for the latency of a ring (one FP64 map at Nside
+// 5.5 -> 3.6 ms), else two to four times as many, for the latency of a ring (one FP64 map at Nside
 // 256: 66 us with an eighth, 53 us).  cpc components of a CTA share the transform of the chirp
 // where that leaves two rounds of CTAs (eight everywhere: 16 maps at Nside 64 78 us, 21 here).
 template <typename T, typename Run>

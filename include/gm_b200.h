@@ -140,7 +140,8 @@ int64_t gm_seed_table_len(int64_t L);
  * spin 0: ncomp maps -> nalm = ncomp rows; spin s in 1..8: ncomp = 2 nfields ->
  * nalm = 2 nfields rows (E, B per field, healpix.py:800-814); other spins return
  * GM_ERR_UNSUPPORTED.
- * lane_geom: (3, nlanes) float64 [cos theta, log2 sin(theta/2), log2 cos(theta/2)].
+ * lane_geom: (3, nlanes) float64 [cos theta, log2 sin(theta/2), log2 cos(theta/2)] of the northern
+ * HEALPix rings (cos theta - 1 in double precision is taken from nside itself, rounded once).
  * seeds: gm_seed_table_len(L) doubles (see gmaster_b200/sht.py).
  * alm is accumulated with double-precision atomics: zero it first for a fresh analysis. */
 int gm_legendre_analysis(int precision, int spin, int64_t nside, int64_t lmax,
