@@ -364,11 +364,17 @@ def ring_synthesis(plan, syn, prec):
     ncomp = syn.shape[2]
     maps = torch.empty((ncomp, plan.npix), dtype=torch.float64, device=plan.device)
     per = int(_lib.load().gm_ring_fold_bytes(prec, plan.nside))
-    work = torch.empty(per * max(1, min(ncomp, RING_FOLD_BYTES // per)), dtype=torch.uint8, device=plan.device)
     scratch, sbytes = _ring_scratch(plan, prec)
-    _lib.call("gm_ring_synthesis_fold", prec, plan.nside, plan.L, ncomp, _lib.ptr(syn), _lib.ptr(plan.tw),
-              _lib.ptr(plan.shifted), _lib.ptr(maps), _lib.ptr(work), work.numel(), _lib.ptr(scratch), sbytes,
-              RING_TUNING["hcap_max"], RING_TUNING["bs_min"], _lib.stream_handle(plan.device))
+    head = (prec, plan.nside, plan.L, ncomp, _lib.ptr(syn), _lib.ptr(plan.tw), _lib.ptr(plan.shifted), _lib.ptr(maps))
+    tail = (_lib.ptr(scratch), sbytes, RING_TUNING["hcap_max"], RING_TUNING["bs_min"], _lib.stream_handle(plan.device))
+    try:
+        work = torch.empty(per * max(1, min(ncomp, RING_FOLD_BYTES // per)), dtype=torch.uint8, device=plan.device)
+    except torch.cuda.OutOfMemoryError:
+        work = None   # the kernel without folded spectra, two to seven times slower
+    if work is None:
+        _lib.call("gm_ring_synthesis_ws", *head, *tail)
+    else:
+        _lib.call("gm_ring_synthesis_fold", *head, _lib.ptr(work), work.numel(), *tail)
     return maps
 
 

@@ -334,7 +334,8 @@ int gm_tc_analysis_noalloc(int64_t nside, int64_t lmax, int spin, int sp, int64_
                            const void *img, double *alm_i, double scale, int64_t nctas,
                            int32_t *err, void *stream);
 
-/* Synthesis operand images from alm_scale * alm_i for row variant sp (device choff). */
+/* Synthesis operand images from alm_scale * alm_i for row variant sp (device choff).  Every byte of
+ * the chunks is written, here and in gm_ck_prep_syn; simg_bytes is not read. */
 int gm_tc_prep_syn(int64_t lmax, int spin, int sp, int64_t ncomp, const double *alm_i,
                    const int64_t *choff, void *simg, int64_t simg_bytes, double alm_scale,
                    void *stream);
