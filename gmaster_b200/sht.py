@@ -272,7 +272,7 @@ def _pass_setup(plan, spin, ncomp, prec, kind):
     from . import sht_tc
 
     key = (spin, ncomp, prec, kind, autotune.autotune_enabled(), sht_tc.USE_CHECKPOINTS, sht_tc.USE_TILE_SKIP,
-           sht_tc.CK_MEMORY_SHARE)
+           sht_tc.CK_MEMORY_SHARE, sht_tc.CK_MAX_LANES)
     have = plan._passes.get(key)
     if have is None:
         tile = autotune.tile_for(plan, spin, ncomp, prec, kind)

@@ -40,3 +40,26 @@ def test_rows_match_fp64(cuda, spin, ncomp, nside, lmax):
         for g, w in zip(both(_lib.MIXED, tile, ck), want):
             err = float(torch.linalg.vector_norm(g - w) / torch.linalg.vector_norm(w))
             assert err < 3e-6, (tile, err)
+
+
+def test_a_pass_follows_the_settings_of_the_tables(cuda, monkeypatch):
+    """Each setting that decides whether a pass takes the tables is looked at again when it changes."""
+    from gmaster_b200 import sht_tc
+
+    plan = sht.get_plan(16, 47)
+    rhs = torch.randn((plan.L, plan.nlanes, 1, 4), device="cuda")
+    alm = torch.zeros((1, plan.nelem), dtype=torch.complex128, device="cuda")
+
+    def entry():
+        before = dict(_lib.CALLS)
+        sht.legendre_analysis(plan, 0, rhs, alm, 1.0, _lib.MIXED)
+        return {k for k, v in _lib.CALLS.items() if v != before.get(k, 0) and k.startswith("gm_legendre_analysis")}
+
+    entry()
+    assert entry() == {"gm_legendre_analysis_ck"}
+    for name, value in (("CK_MAX_LANES", 0), ("CK_MEMORY_SHARE", 0.0), ("USE_CHECKPOINTS", False)):
+        with monkeypatch.context() as m:
+            m.setattr(sht_tc, name, value)
+            entry()
+            assert entry() == {"gm_legendre_analysis_tile"}, name
+        assert entry() == {"gm_legendre_analysis_ck"}
