@@ -949,8 +949,8 @@ def kdtree_apodization_sample(mask_np, nside, apo_deg, nquery=2_000_000, seed=0)
 def run_apodize(args):
     """C1 apodisation of binary masks of the configuration recipes (|b| > 20 deg about a
     tilted pole plus holes) on the GPU: Nside 2048 (2000 holes of 5', 1 deg) and Nside
-    8192 (10000 holes of 2', 0.5 deg).  One step = gm_mask_ring_runs, gm_mask_ring_gaps and
-    gm_mask_apodize_gaps through `mask_apodization` on a device-resident mask; e2e adds the host->device copy of
+    8192 (10000 holes of 2', 0.5 deg).  One step = gm_mask_ring_runs + gm_mask_apodize_gaps
+    through `mask_apodization` on a device-resident mask; e2e adds the host->device copy of
     the mask from pinned memory and the copy of the result back."""
     import torch
 

@@ -150,7 +150,7 @@ _lib = None
 # Kernel launches made by each entry point (for launch accounting); default 1.
 LAUNCHES = {"gm_last_error": 0, "gm_version": 0, "gm_ring_twiddle_count": 0,
             "gm_seed_table_len": 0, "gm_bin_coupling_csr": 3, "gm_tc_lane_groups": 0,
-            "gm_tc_ana_image_bytes": 0, "gm_tc_ana_scratch_bytes": 0,
+            "gm_mask_apodize_gaps": 2, "gm_tc_ana_image_bytes": 0, "gm_tc_ana_scratch_bytes": 0,
             "gm_tc_syn_chunk_offsets": 0, "gm_tc_syn_image_bytes": 0, "gm_legendre_tiles": 0,
             "gm_coupling_units": 0, "gm_ring_big_scratch_bytes": 0, "gm_ring_fold_bytes": 0, "gm_lu_prepared_bytes": 0, "gm_ring_synthesis_fold": 3, "gm_ck_offsets": 0,
             "gm_ck_table_entries": 0, "gm_ck_syn_chunk_offsets": 0, "gm_ck_segments": 0,

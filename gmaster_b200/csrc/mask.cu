@@ -26,7 +26,6 @@ namespace {
 
 constexpr int kRunThreads = 512;
 constexpr int kApoThreads = 256;
-constexpr int kApoGroups = 2;   // pixels of a thread, kApoThreads apart
 constexpr int kGapThreads = 1024;
 constexpr double kTwoPi = 6.283185307179586;   // 2 pi rounded to double, as numpy's 2*np.pi
 constexpr double kInvTwoPi = 0.15915494309189535;
@@ -220,9 +219,9 @@ __device__ __forceinline__ bool ring_in_reach(int64_t nside, int64_t jj, double 
 // 1024 with a radius of one degree (36 rings) every pixel probed them all, 2.29 ms; 0.38 ms here.
 // After every four probes the rings that can no longer improve the worst of the warp's distances are
 // dropped: a search on to the radius took 16.9 instead of 0.73 ms with every second pixel masked at
-// random at 20 degrees, and one through the empty rings 2.9 instead of 0.12 ms without masked pixels.  Two
-// groups of pixels a thread: half the CTAs, 7 % (four: a quarter, 50 % slower, the rings' probes of a
-// CTA one after the other).
+// random at 20 degrees, and one through the empty rings 2.9 instead of 0.12 ms without masked pixels.
+// GROUPS pixels a thread: two from Nside 512 on, half the CTAs, 7 % (four: a quarter, 50 % slower, the
+// rings' probes of a CTA one after the other).
 // The warp's 32 pixels iw ... of ring j (n pixels, gap rings from the nearest one with a masked
 // pixel); m: the mask of the thread's pixel i, p its place.
 __device__ __forceinline__ void apodize_warp(int64_t nside, const Rings &rg, const int32_t *__restrict__ prev,
@@ -284,19 +283,20 @@ __device__ __forceinline__ void apodize_warp(int64_t nside, const Rings &rg, con
     out[p] = m * f;
 }
 
+template <int GROUPS>
 __global__ void __launch_bounds__(kApoThreads) k_mask_apodize(
     int64_t nside, Rings rg, const double *__restrict__ mask,
     const int32_t *__restrict__ prev, const int32_t *__restrict__ next, const int32_t *__restrict__ gaps,
     double chord2_max, double threshold, int mode, double *__restrict__ out)
 {
     const int64_t j = blockIdx.y, n = ring_nphi(nside, j), off = ring_offset(nside, j);
-    const int64_t i0 = (int64_t)blockIdx.x * kApoGroups * kApoThreads + threadIdx.x;
-    double m[kApoGroups];
+    const int64_t i0 = (int64_t)blockIdx.x * GROUPS * kApoThreads + threadIdx.x;
+    double m[GROUPS];
 #pragma unroll
-    for (int e = 0; e < kApoGroups; ++e) m[e] = i0 + e * kApoThreads < n ? mask[off + i0 + e * kApoThreads] : 0.0;
+    for (int e = 0; e < GROUPS; ++e) m[e] = i0 + e * kApoThreads < n ? mask[off + i0 + e * kApoThreads] : 0.0;
     const int gap = gaps ? gaps[j] : 0;
 #pragma unroll
-    for (int e = 0; e < kApoGroups; ++e) {
+    for (int e = 0; e < GROUPS; ++e) {
         const int64_t i = i0 + e * kApoThreads, iw = i - (threadIdx.x & 31);
         if (iw >= n) return;
         if (gap != INT32_MAX) apodize_warp(nside, rg, prev, next, chord2_max, threshold, mode, out, j, n, iw, gap, m[e], off + i);
@@ -338,7 +338,7 @@ extern "C" int gm_mask_apodize(int64_t nside, const double *ring_table, const do
 }
 
 extern "C" int gm_mask_apodize_gaps(int64_t nside, const double *ring_table, const double *mask,
-                                    const int32_t *prev, const int32_t *next, const int32_t *gaps,
+                                    const int32_t *prev, const int32_t *next, int32_t *gaps,
                                     double chord2_max, double threshold, int mode, double *out, void *stream)
 {
     if (nside < 1 || nside > 16384) return GM_ERR_BAD_SHAPE;
@@ -346,11 +346,19 @@ extern "C" int gm_mask_apodize_gaps(int64_t nside, const double *ring_table, con
     if (mode < 0 || mode > 2) return GM_ERR_UNSUPPORTED;
     if (!(chord2_max > 0.0) || (mode != 2 && !(threshold > 0.0))) return GM_ERR_BAD_SHAPE;
     const int64_t nring = 4 * nside - 1;
-    const int64_t per = kApoGroups * kApoThreads;
+    // below Nside 512 the table of the nearest rings (5 us) takes longer than the few rings that it
+    // passes over, and half the CTAs would not fill the chip several times
+    const bool large = nside >= 512;
+    if (!large) gaps = nullptr;
+    if (gaps) {
+        const int st = gm_mask_ring_gaps(nside, prev, gaps, stream);
+        if (st != GM_OK) return st;
+    }
+    const int64_t per = (large ? 2 : 1) * kApoThreads;
     const dim3 grid((unsigned)((4 * nside + per - 1) / per), (unsigned)nring);
     const Rings rg{ring_table, ring_table + nring, ring_table + 2 * nring, ring_table + 3 * nring,
                    ring_table + 4 * nring};
-    k_mask_apodize<<<grid, kApoThreads, 0, as_stream(stream)>>>(nside, rg, mask, prev, next, gaps,
+    (large ? k_mask_apodize<2> : k_mask_apodize<1>)<<<grid, kApoThreads, 0, as_stream(stream)>>>(nside, rg, mask, prev, next, gaps,
                                                                  chord2_max, threshold, mode, out);
     return check_launch("gm_mask_apodize");
 }

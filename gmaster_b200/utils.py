@@ -242,12 +242,12 @@ def mask_apodization(mask_in, aposize, apotype="C1"):
     if apotype == "Smooth" and not bool((mask <= 0).any()):
         return result(mask.clone())
     dev = mask.device
-    nring = 4 * nside - 1
-    prev, nxt, gaps = torch.empty(2 * npix + nring, dtype=torch.int32, device=dev).split([npix, npix, nring])
+    prev = torch.empty(npix + 4 * nside - 1, dtype=torch.int32, device=dev)
+    nxt = torch.empty(npix, dtype=torch.int32, device=dev)
+    gaps = _lib.ptr(prev) + 4 * npix   # one entry per ring behind those of the pixels
     out = torch.empty_like(mask)
     stream = _lib.stream_handle(dev)
     _lib.call("gm_mask_ring_runs", nside, _lib.ptr(mask), _lib.ptr(prev), _lib.ptr(nxt), stream)
-    _lib.call("gm_mask_ring_gaps", nside, _lib.ptr(prev), _lib.ptr(gaps), stream)
     table = _apo_ring_table(nside, dev)
     if apotype == "Smooth":
         reach = min(2.5 * radius + max_pixel_radius(nside), np.pi)
@@ -255,8 +255,8 @@ def mask_apodization(mask_in, aposize, apotype="C1"):
         if reach >= np.pi:
             chord2 = 5.0   # every pixel is within reach
         _lib.call("gm_mask_apodize_gaps", nside, _lib.ptr(table), _lib.ptr(mask), _lib.ptr(prev),
-                  _lib.ptr(nxt), _lib.ptr(gaps), float(chord2), 0.0, 2, _lib.ptr(out), stream)
-        del prev, nxt, gaps
+                  _lib.ptr(nxt), gaps, float(chord2), 0.0, 2, _lib.ptr(out), stream)
+        del prev, nxt
         lmax = 3 * nside - 1
         prec = get_precision()
         alm = sht.map2alm_device(out[None], 0, nside, lmax, 3, prec)
@@ -266,7 +266,7 @@ def mask_apodization(mask_in, aposize, apotype="C1"):
         return smoothed * mask
     threshold = 1 - np.cos(radius)
     _lib.call("gm_mask_apodize_gaps", nside, _lib.ptr(table), _lib.ptr(mask), _lib.ptr(prev),
-              _lib.ptr(nxt), _lib.ptr(gaps), float(2 * threshold), float(threshold),
+              _lib.ptr(nxt), gaps, float(2 * threshold), float(threshold),
               0 if apotype == "C1" else 1, _lib.ptr(out), stream)
     return result(out)
 

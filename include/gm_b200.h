@@ -493,7 +493,8 @@ int gm_tc_alm_layout(int64_t lmax, int spin, int64_t nfield, double *alm_i, doub
  * chord2_max, else mask.  out may not alias mask.
  * gm_mask_ring_gaps: gaps[j] = rings from ring j to the nearest one with a masked pixel (0: itself,
  * INT32_MAX: none), from `prev` of gm_mask_ring_runs; gaps is a caller-owned int32 (4 nside - 1)
- * buffer.  gm_mask_apodize_gaps: gm_mask_apodize that starts its search there (NULL: the same). */
+ * buffer.  gm_mask_apodize_gaps: gm_mask_apodize with such a buffer as scratch: from nside 512 on
+ * it fills it and starts its search there (NULL: gm_mask_apodize). */
 int gm_mask_ring_runs(int64_t nside, const double *mask, int32_t *prev, int32_t *next,
                       void *stream);
 int gm_mask_apodize(int64_t nside, const double *ring_table, const double *mask,
@@ -501,7 +502,7 @@ int gm_mask_apodize(int64_t nside, const double *ring_table, const double *mask,
                     double threshold, int mode, double *out, void *stream);
 int gm_mask_ring_gaps(int64_t nside, const int32_t *prev, int32_t *gaps, void *stream);
 int gm_mask_apodize_gaps(int64_t nside, const double *ring_table, const double *mask,
-                         const int32_t *prev, const int32_t *next, const int32_t *gaps,
+                         const int32_t *prev, const int32_t *next, int32_t *gaps,
                          double chord2_max, double threshold, int mode, double *out, void *stream);
 
 /* ---------------------------------------------------------- Gaussian covariance */
